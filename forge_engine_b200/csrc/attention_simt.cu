@@ -1,147 +1,503 @@
-// Causal grouped-query attention over cache pages, one query token per block.
+// Causal grouped-query attention over cache pages in plain 32-bit arithmetic.
 //
 // The plain form upstream uses for prefill is softmax(q k^T * scale + mask) v with the
 // softmax in 32-bit (src/forge_engine/qwen3.py:187-206); its decode kernel walks the
 // pages position by position with an online softmax in 32-bit
-// (src/forge_engine/kernels/cuda_paged.py:276-347).  This kernel is the general form
+// (src/forge_engine/kernels/cuda_paged.py:276-347).  These kernels are the general form
 // of both: any number of new tokens per request, keys read from pages (the new
-// tokens' keys have been written before it runs), optional window.  It is the true
+// tokens' keys have been written before they run), optional window.  They are the true
 // 32-bit attention and the fallback for shapes the tensor-core kernels refuse.
 //
-// Work split: block = (token, q head), 4 warps.  Keys [lo, pos] are cut into chunks
-// of 32 starting at lo; warp w takes chunks w, w+4, ...; inside a chunk a lane owns
-// one key for the score and D/32 output elements for the value sum.  The four
-// partial (max, sum, acc) are merged in a fixed order.  Nothing depends on what else
-// is in the batch.
+// attention_simt_span: single tokens (decoding, or a caller that names no entries).  A block takes
+//   the query heads of one kv head (up to 16) over one span of 128 key positions, whose keys and
+//   values pass through a ring in shared memory; attention_simt_merge adds a token's spans up in
+//   order.  Bound by the bytes of keys and values; the spans are what keeps the chip busy at few
+//   requests.
+// attention_simt_tile: entries of several tokens.  A block takes 32 rows (token, query head) of one
+//   kv head over all their keys in tiles of 64, as two small FFMA products from shared memory.
+//
+// Spans and tiles are counted from position 0, every sum runs over positions (or elements of a
+// head: even and odd ones apart) in ascending order, and which kernel a token takes depends on how
+// many its entry brings: nothing depends on what else is in the batch.
 #include "attention_common.cuh"
 
-#define ATT_WARPS 4
-#define ATT_MAX_D 256
+namespace {
 
-template <typename T>
-__global__ void __launch_bounds__(ATT_WARPS * 32)
-attention_simt_kernel(const T* __restrict__ q, int q_stride, PagedKV cache,
-                      const int* __restrict__ positions, const int* __restrict__ token_entry,
-                      int window, float scale, T* __restrict__ out, int num_q_heads, int* status) {
-  extern __shared__ float smem[];
-  const int D = cache.head_dim;
-  float* qs = smem;                        // [D]
-  float* part_acc = smem + D;              // [ATT_WARPS][D]
-  float* part_m = part_acc + ATT_WARPS * D;  // [ATT_WARPS]
-  float* part_l = part_m + ATT_WARPS;      // [ATT_WARPS]
+constexpr int SPAN = 128;          // key positions of a block of the span kernel
+constexpr int SPAN_KEYS = 32;      // of one stage of its ring
+constexpr int SPAN_STAGES = 3;
+constexpr int SPAN_THREADS = 128;
+constexpr int TILE_ROWS = 32, TILE_KEYS = 64, TILE_THREADS = 128;
+constexpr int P_PITCH = TILE_KEYS + 4;
 
-  const int token = blockIdx.x, head = blockIdx.y;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kvh = head / (num_q_heads / cache.num_kv_heads);
-  const int pos = positions[token];
-  const int entry = token_entry[token];
-  const int lo = window > 0 ? max(0, pos - window + 1) : 0;
-  const T* kbase = (const T*)cache.k;
-  const T* vbase = (const T*)cache.v;
-  const int* table = cache.block_table + (size_t)entry * cache.max_pages;
+struct Simt {
+  const void* q;
+  int q_stride;
+  PagedKV cache;
+  const int* positions;
+  const int* token_entry;
+  const int* cu_tokens;     // null: every token is a unit of its own
+  int units, window;
+  float scale;
+  void* out;
+  int num_q_heads, groups, spans, row_tiles;
+  float* partial;           // [unit][kv head][row tile][span][row][D + 2]
+  int* status;
+};
 
-  const T* qrow = q + (size_t)token * q_stride + (size_t)head * D;
-  for (int i = threadIdx.x; i < D; i += blockDim.x) qs[i] = to_float(qrow[i]);
-  __syncthreads();
+__device__ __forceinline__ void copy16(void* dst, const void* src, bool valid) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
+               ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(valid ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int PENDING>
+__device__ __forceinline__ void wait() { asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory"); }
 
-  const int nd = (D + 31) >> 5;
-  float acc[ATT_MAX_D / 32];
-#pragma unroll
-  for (int i = 0; i < ATT_MAX_D / 32; ++i) acc[i] = 0.f;
-  float m = -INFINITY, l = 0.f;
+__device__ __forceinline__ void fma2(uint64_t& acc, uint64_t a, uint64_t b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ float sum2(uint64_t acc) {
+  return __uint_as_float((unsigned)acc) + __uint_as_float((unsigned)(acc >> 32));
+}
+__device__ __forceinline__ void pairs4(const float* p, uint64_t (&out)[2]) {
+  const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p);
+  out[0] = v.x;
+  out[1] = v.y;
+}
+__device__ __forceinline__ void pairs4(const bf16* p, uint64_t (&out)[2]) {
+  const uint2 raw = *reinterpret_cast<const uint2*>(p);
+  out[0] = (uint64_t)(raw.x << 16) | ((uint64_t)(raw.x & 0xffff0000u) << 32);
+  out[1] = (uint64_t)(raw.y << 16) | ((uint64_t)(raw.y & 0xffff0000u) << 32);
+}
 
-  const int n_keys = pos - lo + 1;
-  const int n_chunks = (n_keys + 31) >> 5;
-  for (int c = warp; c < n_chunks; c += ATT_WARPS) {
-    const int key = lo + (c << 5) + lane;
-    bool valid = key <= pos;
-    long long off = -1;
-    if (valid) {
-      const int logical = key / cache.page_size;
-      int page = -1;
-      if (logical < cache.max_pages) page = table[logical];
-      if (page < 0 || page >= cache.num_pages) {
-        atomicOr(status, FE_STATUS_BAD_PAGE);
-        valid = false;
-      } else {
-        off = (long long)kv_offset(cache, page, kvh, key - logical * cache.page_size);
-      }
-    }
-    float s = -INFINITY;
-    if (valid) {
-      const T* kp = kbase + off;
-      float dot = 0.f;
-      for (int d = 0; d < D; d += 8) {
-        float kk[8];
-        load8(kp + d, kk);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) dot += qs[d + e] * kk[e];
-      }
-      s = dot * scale;
-    }
-    const float m_new = fmaxf(m, warp_max(s));
-    const float p = valid ? expf(s - m_new) : 0.f;
-    const float corr = (m == -INFINITY) ? 0.f : expf(m - m_new);
-    l = l * corr + warp_sum(p);
-    m = m_new;
-#pragma unroll
-    for (int i = 0; i < ATT_MAX_D / 32; ++i) acc[i] *= corr;
-    const int in_chunk = min(32, n_keys - (c << 5));
-    for (int j = 0; j < in_chunk; ++j) {
-      const float pj = __shfl_sync(0xffffffffu, p, j);
-      const long long oj = __shfl_sync(0xffffffffu, off, j);
-      if (oj < 0) continue;
-      const T* vp = vbase + oj;
-#pragma unroll
-      for (int i = 0; i < ATT_MAX_D / 32; ++i) {
-        const int d = lane + (i << 5);
-        if (i < nd && d < D) acc[i] += pj * to_float(vp[d]);
-      }
-    }
+// Where key position `key` of an entry lies, in elements of the cache; -1 (and a status bit) without a page.
+__device__ __forceinline__ long long key_offset(const PagedKV& c, const int* table, int kvh, int key, int* status) {
+  const int logical = key / c.page_size;
+  const int page = logical < c.max_pages ? table[logical] : -1;
+  if (page < 0 || page >= c.num_pages) {
+    atomicOr(status, FE_STATUS_BAD_PAGE);
+    return -1;
   }
+  return (long long)kv_offset(c, page, kvh, key - logical * c.page_size);
+}
 
-  if (lane == 0) { part_m[warp] = m; part_l[warp] = l; }
-#pragma unroll
-  for (int i = 0; i < ATT_MAX_D / 32; ++i) {
-    const int d = lane + (i << 5);
-    if (i < nd && d < D) part_acc[warp * D + d] = acc[i];
-  }
-  __syncthreads();
-  float big = -INFINITY;
-#pragma unroll
-  for (int w = 0; w < ATT_WARPS; ++w) big = fmaxf(big, part_m[w]);
-  T* orow = out + (size_t)token * num_q_heads * D + (size_t)head * D;
-  for (int d = threadIdx.x; d < D; d += blockDim.x) {
-    float num = 0.f, den = 0.f;
-#pragma unroll
-    for (int w = 0; w < ATT_WARPS; ++w) {
-      const float f = (part_m[w] == -INFINITY) ? 0.f : expf(part_m[w] - big);
-      num += part_acc[w * D + d] * f;
-      den += part_l[w] * f;
-    }
-    orow[d] = from_float<T>(den > 0.f ? num / den : 0.f);
+// KEYS keys from `first` on (those in [lo, hi] are needed), as they lie in memory: k rows with 16
+// bytes of padding, v rows without.  ok[i]: whether key i counts.
+template <typename T, int KEYS, int THREADS>
+__device__ __forceinline__ void stage_keys(const Simt& p, const int* table, int kvh, int first, int lo, int hi, T* ks, T* vs, int* ok) {
+  constexpr int CH = 16 / (int)sizeof(T), TPK = THREADS / KEYS;     // threads of a key
+  const int D = p.cache.head_dim, i = threadIdx.x / TPK, part = threadIdx.x % TPK;
+  const int key = first + i;
+  const long long off = key >= lo && key <= hi ? key_offset(p.cache, table, kvh, key, p.status) : -1;
+  if (part == 0) ok[i] = off >= 0;
+  const T* k = (const T*)p.cache.k + (off < 0 ? 0 : off);
+  const T* v = (const T*)p.cache.v + (off < 0 ? 0 : off);
+  for (int d = part * CH; d < D; d += TPK * CH) {
+    copy16(ks + i * (D + CH) + d, k + d, off >= 0);
+    copy16(vs + i * D + d, v + d, off >= 0);
   }
 }
 
+template <typename T, int R, int DMAX>
+__global__ void __launch_bounds__(SPAN_THREADS) attention_simt_span_kernel(const Simt p) {
+  constexpr int CH = 16 / (int)sizeof(T), PER = (DMAX + SPAN_THREADS - 1) / SPAN_THREADS;
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ __align__(16) float ps[R][SPAN_KEYS];
+  __shared__ float corr[R];
+  __shared__ int ok[SPAN_STAGES][SPAN_KEYS];
+  pdl_trigger();
+  pdl_wait();
+  const int D = p.cache.head_dim, unit = blockIdx.x, span = blockIdx.z, kvh = blockIdx.y / p.row_tiles, tile = blockIdx.y % p.row_tiles;
+  int token = unit, entry;
+  if (p.cu_tokens != nullptr) {
+    token = p.cu_tokens[unit];
+    if (p.cu_tokens[unit + 1] - token != 1) return;
+    entry = unit;
+  } else {
+    entry = p.token_entry[unit];
+  }
+  const int pos = p.positions[token];
+  const int lo = p.window > 0 ? max(0, pos - p.window + 1) : 0;
+  const int begin = span * SPAN, end = min(begin + SPAN, pos + 1);
+  if (span == 0 && pos >= p.spans * SPAN && threadIdx.x == 0) atomicOr(p.status, FE_STATUS_BAD_PAGE);   // past the block table
+  if (end <= max(begin, lo)) return;
+  const int rows = min(R, p.groups - tile * R);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float* qs = (float*)smem;                                     // [R][D]
+  T* ks = (T*)(qs + R * D);                                     // [stage][key][D + CH]
+  T* vs = ks + SPAN_STAGES * SPAN_KEYS * (D + CH);              // [stage][key][D]
+  const int* table = p.cache.block_table + (size_t)entry * p.cache.max_pages;
+  const int first = max(begin, lo) / SPAN_KEYS * SPAN_KEYS, steps = (end - first + SPAN_KEYS - 1) / SPAN_KEYS;
+#pragma unroll
+  for (int s = 0; s < SPAN_STAGES - 1; ++s) {
+    if (s < steps)
+      stage_keys<T, SPAN_KEYS, SPAN_THREADS>(p, table, kvh, first + s * SPAN_KEYS, lo, end - 1, ks + s * SPAN_KEYS * (D + CH),
+                                             vs + s * SPAN_KEYS * D, ok[s]);
+    commit();
+  }
+  const int head0 = kvh * p.groups + tile * R;
+  const T* q = (const T*)p.q + (size_t)token * p.q_stride + (size_t)head0 * D;
+  for (int i = threadIdx.x; i < R * D; i += SPAN_THREADS) qs[i] = i < rows * D ? to_float(q[i]) : 0.f;
+
+  float m[(R + 3) / 4], l[(R + 3) / 4], acc[R][PER];
+#pragma unroll
+  for (int i = 0; i < (R + 3) / 4; ++i) m[i] = -INFINITY, l[i] = 0.f;
+#pragma unroll
+  for (int i = 0; i < R; ++i)
+#pragma unroll
+    for (int j = 0; j < PER; ++j) acc[i][j] = 0.f;
+
+  for (int step = 0; step < steps; ++step) {
+    const int s = step % SPAN_STAGES;
+    wait<SPAN_STAGES - 2>();
+    __syncthreads();               // this stage has landed; everyone is done with the one before it
+    const int next = step + SPAN_STAGES - 1, to = next % SPAN_STAGES;
+    if (next < steps)
+      stage_keys<T, SPAN_KEYS, SPAN_THREADS>(p, table, kvh, first + next * SPAN_KEYS, lo, end - 1, ks + to * SPAN_KEYS * (D + CH),
+                                             vs + to * SPAN_KEYS * D, ok[to]);
+    commit();
+    const T* krow = ks + (s * SPAN_KEYS + lane) * (D + CH);
+#pragma unroll
+    for (int i = 0; i < (R + 3) / 4; ++i) {
+      const int r = warp + 4 * i;
+      if (r < rows) {
+        uint64_t dot = 0;
+        const float* qrow = qs + r * D;
+#pragma unroll 4
+        for (int d = 0; d < D; d += 4) {
+          uint64_t a[2], b[2];
+          pairs4(qrow + d, a);
+          pairs4(krow + d, b);
+          fma2(dot, a[0], b[0]);
+          fma2(dot, a[1], b[1]);
+        }
+        const float score = ok[s][lane] ? sum2(dot) * p.scale : -INFINITY;
+        const float top = fmaxf(m[i], warp_max(score));
+        const float e = score == -INFINITY ? 0.f : expf(score - top);
+        const float c = m[i] == -INFINITY ? 0.f : expf(m[i] - top);
+        l[i] = l[i] * c + warp_sum(e);
+        m[i] = top;
+        ps[r][lane] = e;
+        if (lane == 0) corr[r] = c;
+      }
+    }
+    __syncthreads();
+    const T* vt = vs + s * SPAN_KEYS * D;
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+      const int d = threadIdx.x + j * SPAN_THREADS;
+      if (d < D) {
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+          if (r < rows) acc[r][j] *= corr[r];
+#pragma unroll 2
+        for (int key = 0; key < SPAN_KEYS; key += 4) {
+          float v[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) v[e] = to_float(vt[(key + e) * D + d]);
+#pragma unroll
+          for (int r = 0; r < R; ++r) {
+            if (r < rows) {
+              const float4 e = *reinterpret_cast<const float4*>(&ps[r][key]);
+              acc[r][j] = fmaf(e.x, v[0], acc[r][j]);
+              acc[r][j] = fmaf(e.y, v[1], acc[r][j]);
+              acc[r][j] = fmaf(e.z, v[2], acc[r][j]);
+              acc[r][j] = fmaf(e.w, v[3], acc[r][j]);
+            }
+          }
+        }
+      }
+    }
+  }
+  float* part = p.partial + ((((size_t)unit * gridDim.y + blockIdx.y) * p.spans + span) * R) * (D + 2);
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    if (r < rows) {
+#pragma unroll
+      for (int j = 0; j < PER; ++j) {
+        const int d = threadIdx.x + j * SPAN_THREADS;
+        if (d < D) part[r * (D + 2) + d] = acc[r][j];
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < (R + 3) / 4; ++i) {
+    const int r = warp + 4 * i;
+    if (r < rows && lane == 0) {
+      part[r * (D + 2) + D] = m[i];
+      part[r * (D + 2) + D + 1] = l[i];
+    }
+  }
+}
+
+// One block per (query head, unit): its spans in ascending order.
+template <typename T>
+__global__ void __launch_bounds__(128) attention_simt_merge_kernel(const Simt p, int R) {
+  __shared__ float best;
+  pdl_trigger();
+  pdl_wait();
+  const int D = p.cache.head_dim, unit = blockIdx.x, head = blockIdx.y;
+  int token = unit;
+  if (p.cu_tokens != nullptr) {
+    token = p.cu_tokens[unit];
+    if (p.cu_tokens[unit + 1] - token != 1) return;
+  }
+  const int pos = p.positions[token], lo = p.window > 0 ? max(0, pos - p.window + 1) : 0;
+  // a position past the block table has no spans beyond it
+  const int from = lo / SPAN, to = min(pos / SPAN, p.spans - 1);
+  const int kvh = head / p.groups, within = head - kvh * p.groups;
+  const size_t stride = (size_t)R * (D + 2);
+  const float* part = p.partial + (((size_t)unit * (p.cache.num_kv_heads * p.row_tiles) + kvh * p.row_tiles + within / R) * p.spans) * stride +
+                      (size_t)(within % R) * (D + 2);
+  if (threadIdx.x < 32) {
+    float top = -INFINITY;
+    for (int s = from + (int)threadIdx.x; s <= to; s += 32) top = fmaxf(top, part[s * stride + D]);
+    top = warp_max(top);
+    if (threadIdx.x == 0) best = top;
+  }
+  __syncthreads();
+  const float top = best;
+  T* out = (T*)p.out + ((size_t)token * p.num_q_heads + head) * D;
+  for (int d = threadIdx.x; d < D; d += blockDim.x) {
+    float num = 0.f, den = 0.f;
+#pragma unroll 4
+    for (int s = from; s <= to; ++s) {
+      const float m = part[s * stride + D], f = m == -INFINITY ? 0.f : expf(m - top);
+      num = fmaf(part[s * stride + d], f, num);
+      den = fmaf(part[s * stride + D + 1], f, den);
+    }
+    out[d] = from_float<T>(den > 0.f ? num / den : 0.f);
+  }
+}
+
+template <typename T, int DMAX>
+__global__ void __launch_bounds__(TILE_THREADS) attention_simt_tile_kernel(const Simt p) {
+  constexpr int CH = 16 / (int)sizeof(T), CG = DMAX / 64;      // groups of four output columns of a thread
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ int ok[TILE_KEYS];
+  pdl_trigger();
+  pdl_wait();
+  const int D = p.cache.head_dim, entry = blockIdx.z, kvh = blockIdx.y;
+  const int token0 = p.cu_tokens[entry], count = p.cu_tokens[entry + 1] - token0;
+  if (count <= 1) return;
+  const int total = count * p.groups, tiles = (total + TILE_ROWS - 1) / TILE_ROWS;
+  if ((int)blockIdx.x >= tiles) return;
+  const int row0 = (tiles - 1 - (int)blockIdx.x) * TILE_ROWS;    // the tiles with the most keys first
+  const int qpitch = D + 4;
+  float* qs = (float*)smem;                                     // [row][D + 4]
+  float* ps = qs + TILE_ROWS * qpitch;                          // [row][key]
+  T* ks = (T*)(ps + TILE_ROWS * P_PITCH);                       // [key][D + CH]
+  T* vs = ks + TILE_KEYS * (D + CH);                            // [key][D]
+  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+  for (int i = threadIdx.x; i < TILE_ROWS * D; i += TILE_THREADS) {
+    const int r = i / D, d = i - r * D, row = row0 + r;
+    const int token = token0 + row / p.groups, head = kvh * p.groups + row % p.groups;
+    qs[r * qpitch + d] = row < total ? to_float(((const T*)p.q)[(size_t)token * p.q_stride + (size_t)head * D + d]) : 0.f;
+  }
+  int from[4], upto[4];              // the positions this thread's rows see
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int row = row0 + ty * 4 + i;
+    upto[i] = row < total ? p.positions[token0 + row / p.groups] : -1;
+    from[i] = p.window > 0 ? max(0, upto[i] - p.window + 1) : 0;
+  }
+  const int* table = p.cache.block_table + (size_t)entry * p.cache.max_pages;
+  const int low = p.positions[token0 + row0 / p.groups], high = p.positions[token0 + (min(row0 + TILE_ROWS, total) - 1) / p.groups];
+  const int lo = p.window > 0 ? max(0, low - p.window + 1) : 0;
+  float m[4], l[4], acc[4][CG][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    m[i] = -INFINITY;
+    l[i] = 0.f;
+#pragma unroll
+    for (int g = 0; g < CG; ++g)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[i][g][e] = 0.f;
+  }
+  for (int first = lo / TILE_KEYS * TILE_KEYS; first <= high; first += TILE_KEYS) {
+    __syncthreads();
+    stage_keys<T, TILE_KEYS, TILE_THREADS>(p, table, kvh, first, lo, high, ks, vs, ok);
+    commit();
+    wait<0>();
+    __syncthreads();
+    uint64_t dot[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) dot[i][j] = 0;
+#pragma unroll 4
+    for (int d = 0; d < D; d += 4) {
+      uint64_t a[4][2], b[4][2];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) pairs4(qs + (ty * 4 + i) * qpitch + d, a[i]);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) pairs4(ks + (tx + 16 * j) * (D + CH) + d, b[j]);
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) fma2(dot[i][j], a[i][e], b[j][e]);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float score[4], top = m[i];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int key = first + tx + 16 * j;
+        score[j] = ok[tx + 16 * j] && key >= from[i] && key <= upto[i] ? sum2(dot[i][j]) * p.scale : -INFINITY;
+        top = fmaxf(top, score[j]);
+      }
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+      const float c = m[i] == -INFINITY ? 0.f : expf(m[i] - top);
+      float sum = 0.f;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float e = score[j] == -INFINITY ? 0.f : expf(score[j] - top);
+        ps[(ty * 4 + i) * P_PITCH + tx + 16 * j] = e;
+        sum += e;
+      }
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      l[i] = l[i] * c + sum;
+      m[i] = top;
+#pragma unroll
+      for (int g = 0; g < CG; ++g)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[i][g][e] *= c;
+    }
+    __syncwarp();                    // a row's probabilities are written and read by the same warp
+    // Where some row of the tile does not see some key, that key's value is taken as zero for it: a
+    // zero probability would not keep an infinity out.
+    const bool edge = first < max(0, p.window > 0 ? high - p.window + 1 : 0) || first + TILE_KEYS - 1 > low;
+    for (int key = 0; key < TILE_KEYS; key += 4) {
+      float e[4][4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) load4(ps + (ty * 4 + i) * P_PITCH + key, e[i]);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+#pragma unroll
+        for (int g = 0; g < CG; ++g) {
+          const int d = tx * 4 + 64 * g;
+          if (d < D) {
+            float v[4];
+            load4(vs + (key + u) * D + d, v);
+            if (!edge) {
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) acc[i][g][c] = fmaf(e[i][u], v[c], acc[i][g][c]);
+            } else {
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const bool seen = first + key + u >= from[i] && first + key + u <= upto[i];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) acc[i][g][c] = fmaf(e[i][u], seen ? v[c] : 0.f, acc[i][g][c]);
+              }
+            }
+          }
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int row = row0 + ty * 4 + i;
+    if (row >= total) continue;
+    T* out = (T*)p.out + ((size_t)(token0 + row / p.groups) * p.num_q_heads + kvh * p.groups + row % p.groups) * D;
+#pragma unroll
+    for (int g = 0; g < CG; ++g) {
+      const int d = tx * 4 + 64 * g;
+      if (d < D) {
+        float o[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) o[c] = l[i] > 0.f ? acc[i][g][c] / l[i] : 0.f;
+        store4(out + d, o);
+      }
+    }
+  }
+}
+
+template <typename K, typename... A>
+int launch(K kernel, dim3 grid, int threads, size_t smem, cudaStream_t stream, const A&... args) {
+  if (smem > 48 * 1024) {
+    const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (err != cudaSuccess) return (int)err;
+  }
+  return fe_launch_dependent(kernel, grid, dim3(threads), smem, stream, args...);
+}
+
+int rows_of(int groups) { return groups <= 2 ? 2 : groups <= 4 ? 4 : groups <= 8 ? 8 : 16; }
+
+template <typename T, int DMAX>
+int run_spans(const Simt& p, cudaStream_t stream) {
+  const int R = rows_of(p.groups), D = p.cache.head_dim;
+  const size_t smem = (size_t)R * D * 4 + SPAN_STAGES * SPAN_KEYS * ((size_t)2 * D * sizeof(T) + 16);
+  const dim3 grid(p.units, p.cache.num_kv_heads * p.row_tiles, p.spans);
+  int code;
+  if (R == 2) code = launch(attention_simt_span_kernel<T, 2, DMAX>, grid, SPAN_THREADS, smem, stream, p);
+  else if (R == 4) code = launch(attention_simt_span_kernel<T, 4, DMAX>, grid, SPAN_THREADS, smem, stream, p);
+  else if (R == 8) code = launch(attention_simt_span_kernel<T, 8, DMAX>, grid, SPAN_THREADS, smem, stream, p);
+  else code = launch(attention_simt_span_kernel<T, 16, DMAX>, grid, SPAN_THREADS, smem, stream, p);
+  if (code) return code;
+  return launch(attention_simt_merge_kernel<T>, dim3(p.units, p.num_q_heads), 128, 0, stream, p, R);
+}
+
+template <typename T>
+int run_tiles(const Simt& p, int max_new, cudaStream_t stream) {
+  const int D = p.cache.head_dim;
+  const size_t smem = (size_t)4 * TILE_ROWS * (D + 4 + P_PITCH) + (size_t)TILE_KEYS * (2 * D * sizeof(T) + 16);
+  const dim3 grid((unsigned)(((long long)max_new * p.groups + TILE_ROWS - 1) / TILE_ROWS), p.cache.num_kv_heads, p.units);
+  if (D <= 64) return launch(attention_simt_tile_kernel<T, 64>, grid, TILE_THREADS, smem, stream, p);
+  if (D <= 128) return launch(attention_simt_tile_kernel<T, 128>, grid, TILE_THREADS, smem, stream, p);
+  return launch(attention_simt_tile_kernel<T, 256>, grid, TILE_THREADS, smem, stream, p);
+}
+
+template <typename T>
+int run(const Simt& p, int n_tokens, int max_new, cudaStream_t stream) {
+  // units that bring several tokens, then those that bring one; a step of one prompt has none of these
+  if (p.cu_tokens != nullptr && max_new > 1) {
+    const int code = run_tiles<T>(p, max_new, stream);
+    if (code) return code;
+    if (p.units == 1 && n_tokens > 1) return 0;
+  }
+  return p.cache.head_dim <= 128 ? run_spans<T, 128>(p, stream) : run_spans<T, 256>(p, stream);
+}
+
+}  // namespace
+
+// Floats of workspace for `units` single tokens whose block tables are `max_pages` wide.
+FE_EXPORT long long fe_attention_simt_scratch(int units, int num_q_heads, int num_kv_heads, int head_dim, int max_pages, int page_size) {
+  if (units <= 0 || num_kv_heads <= 0 || num_q_heads % num_kv_heads) return 0;
+  const int groups = num_q_heads / num_kv_heads, R = rows_of(groups);
+  const long long spans = ((long long)max_pages * page_size + SPAN - 1) / SPAN;
+  return (long long)units * num_kv_heads * ((groups + R - 1) / R) * spans * R * (head_dim + 2);
+}
+
+// `cu_tokens` [units + 1] says which tokens each unit (an entry: row u of the block table, positions
+// in order) brings, at most `max_new`; null: every token is a unit and `token_entry` names its row.
 FE_EXPORT int fe_attention_simt(const void* q, int q_stride, int dtype, const void* k_cache,
                                 const void* v_cache, const int* block_table, int max_pages,
                                 int page_size, int num_pages, const int* positions,
-                                const int* token_entry, int window, float scale, void* out,
+                                const int* token_entry, const int* cu_tokens, int units, int max_new,
+                                int window, float scale, void* out,
                                 int num_q_heads, int num_kv_heads, int head_dim, int n_tokens,
-                                int* status, cudaStream_t stream) {
+                                float* workspace, int* status, cudaStream_t stream) {
   if (n_tokens <= 0) return 0;
-  if (head_dim % 8 || head_dim > ATT_MAX_D || head_dim < 8) return FE_ERR_BAD_SHAPE;
-  if (num_q_heads % num_kv_heads || num_q_heads > 65535) return FE_ERR_BAD_SHAPE;
+  if (head_dim % 8 || head_dim > 256 || head_dim < 8) return FE_ERR_BAD_SHAPE;
+  if (num_kv_heads <= 0 || num_q_heads % num_kv_heads || num_q_heads > 65535) return FE_ERR_BAD_SHAPE;
+  if (((uintptr_t)k_cache | (uintptr_t)v_cache) & 15) return FE_ERR_BAD_ALIGN;
+  if (cu_tokens == nullptr) units = n_tokens;
+  if (cu_tokens != nullptr && units > 65535) return FE_ERR_TOO_LARGE;
   PagedKV cache{k_cache, v_cache, block_table, max_pages, page_size, num_pages, num_kv_heads, head_dim};
-  dim3 grid(n_tokens, num_q_heads);
-  const size_t smem = sizeof(float) * (head_dim * (1 + ATT_WARPS) + 2 * ATT_WARPS);
-  if (dtype == FE_DTYPE_F32)
-    attention_simt_kernel<float><<<grid, ATT_WARPS * 32, smem, stream>>>((const float*)q, q_stride,
-        cache, positions, token_entry, window, scale, (float*)out, num_q_heads, status);
-  else if (dtype == FE_DTYPE_BF16)
-    attention_simt_kernel<bf16><<<grid, ATT_WARPS * 32, smem, stream>>>((const bf16*)q, q_stride,
-        cache, positions, token_entry, window, scale, (bf16*)out, num_q_heads, status);
-  else
-    return FE_ERR_BAD_DTYPE;
-  return fe_last_error();
+  const int groups = num_q_heads / num_kv_heads, R = rows_of(groups);
+  const long long spans = ((long long)max_pages * page_size + SPAN - 1) / SPAN;
+  const int row_tiles = (groups + R - 1) / R;
+  if (spans > 65535 || (long long)num_kv_heads * row_tiles > 65535) return FE_ERR_TOO_LARGE;
+  Simt p{q, q_stride, cache, positions, token_entry, cu_tokens, units, window, scale, out, num_q_heads, groups,
+         (int)spans, row_tiles, workspace, status};
+  if (dtype == FE_DTYPE_F32) return run<float>(p, n_tokens, max_new, stream);
+  if (dtype == FE_DTYPE_BF16) return run<bf16>(p, n_tokens, max_new, stream);
+  return FE_ERR_BAD_DTYPE;
 }

@@ -243,6 +243,8 @@ __global__ void __launch_bounds__(32 * (GSK_LOADERS + 8)) gemm_simt_rows_kernel(
       gs_arrive_copied(&full[s]);
       if (++s == stages) s = 0, phase ^= 1u;
     }
+    gs_commit();
+    gs_wait<0>();          // no copy is in flight when the block ends, also after a wait that ran out
   } else {
     const int lc = (warp % (COLS / LC)) * LC + lane % LC, mine = (warp / (COLS / LC)) * ROWS + (lane / LC) * R;
     float acc[R];
@@ -292,10 +294,11 @@ __global__ void __launch_bounds__(32 * (GSK_LOADERS + 8)) gemm_simt_rows_kernel(
       if (lane == 0) gs_arrive(&empty[s]);
       if (++s == stages) s = 0, phase ^= 1u;
     }
-    if (ok && col0 + lc < p.o) {
+    if (col0 + lc < p.o) {
+      // after a wait that ran out the outputs are NaN, which the sampler reports
 #pragma unroll
       for (int i = 0; i < R; ++i)
-        if (mine + i < p.n) gs_store(p, acc[i], mine + i, col0 + lc);
+        if (mine + i < p.n) gs_store(p, ok ? acc[i] : __int_as_float(0x7fffffff), mine + i, col0 + lc);
     }
   }
 }

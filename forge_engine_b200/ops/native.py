@@ -88,7 +88,8 @@ def _declare(handle: ctypes.CDLL) -> None:
         "fe_qk_rope_cache": [p, i, p, p, f, p, p, i, p, p, p, p, p, i, i, i, i, i, i, i, i, p, p],
         "fe_qk_rope_cache_sums": [p, p, p, p, f, p, p, p, p, p, p, p, i, i, i, i, i, i, i, i, p, p],
         "fe_rope_table": [p, p, i, i, f, p, p],
-        "fe_attention_simt": [p, i, i, p, p, p, i, i, i, p, p, i, f, p, i, i, i, i, p, p],
+        "fe_attention_simt": [p, i, i, p, p, p, i, i, i, p, p, p, i, i, i, f, p, i, i, i, i, p, p, p],
+        "fe_attention_simt_scratch": [i, i, i, i, i, i],
         "fe_gemm_simt": [p, i, p, i, p, p, i, i, i, i, i, p],
         "fe_sample": [p, i, i, p, p, p, p, p, p, p, p, p],
         "fe_gemm_tc5": [p, p, p, p, i, i, i, i, i, p, p, p, f, f, p],
@@ -117,7 +118,7 @@ def _declare(handle: ctypes.CDLL) -> None:
         fn.argtypes = argtypes
         fn.restype = c_int
     for name in ("fe_gated_recurrence_scratch", "fe_wkv_scratch", "fe_delta_rule_scratch", "fe_matrix_memory_scratch",
-                 "fe_retention_scratch", "fe_rglru_scratch"):
+                 "fe_retention_scratch", "fe_rglru_scratch", "fe_attention_simt_scratch"):
         getattr(handle, name).restype = ctypes.c_longlong
     handle.fe_uniform_host.argtypes = [c_ulonglong, c_ulonglong]
     handle.fe_uniform_host.restype = c_float
@@ -1419,20 +1420,30 @@ def attention_simt(
     out: torch.Tensor,
     num_q_heads: int,
     status: torch.Tensor,
+    entries: tuple | None = None,
 ) -> None:
-    """General paged causal attention; q row n starts at q + n * q_stride elements."""
+    """General paged causal attention; q row n starts at q + n * q_stride elements.  ``entries`` =
+    (cu_tokens, how many, most tokens of one) says which tokens belong together; without it every
+    token is worked on by itself."""
     num_pages, nkv, page_size, head_dim = k_cache.shape
     n = out.shape[0]
     assert out.shape[1] == num_q_heads * head_dim and out.dtype == q.dtype == k_cache.dtype
+    cu_tokens, units, max_new = (None, n, 1) if entries is None else entries
+    workspace = None
+    if max_new <= 1 or units > 1 or n <= 1:            # some token may come by itself
+        floats = lib().fe_attention_simt_scratch(int(units), num_q_heads, nkv, head_dim, block_table.shape[1], page_size)
+        workspace = _attention_workspace(q.device, max(1, floats))
     check(
         lib().fe_attention_simt(
             ptr(q), int(q_stride), code(q), ptr(k_cache), ptr(v_cache), ptr(block_table),
-            block_table.shape[1], page_size, num_pages, ptr(positions), ptr(token_entry),
-            int(window or 0), float(scale), ptr(out), num_q_heads, nkv, head_dim, n, ptr(status),
+            block_table.shape[1], page_size, num_pages, ptr(positions), ptr(token_entry), ptr(cu_tokens), int(units), int(max_new),
+            int(window or 0), float(scale), ptr(out), num_q_heads, nkv, head_dim, n, ptr(workspace), ptr(status),
             stream(),
         ),
         "attention_simt",
     )
+    global LAUNCHES
+    LAUNCHES += (2 if workspace is not None else 0) + (1 if cu_tokens is not None and max_new > 1 else 0) - 1
 
 
 _balanced_blocks: dict = {}

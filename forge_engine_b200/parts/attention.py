@@ -354,6 +354,7 @@ class GQAttention(Mixer):
                 native.attention_simt(
                     qkv, qkv.shape[1], k_cache, v_cache, table, batch.positions, batch.token_entry,
                     self.spec.window, self.spec.scale, out, self.nq, self.ctx.status,
+                    entries=(batch.cu_tokens, batch.n_entries, batch.max_new),
                 )
         return out
 

@@ -6,6 +6,8 @@ from __future__ import annotations
 import pytest
 import torch
 
+from test_gpu_kernels import dense_attention, paged_layout, status_word
+
 pytestmark = pytest.mark.gpu
 
 DEV = "cuda:0"
@@ -60,3 +62,65 @@ def test_batched_product_with_strided_rows(native, n):
     bound = torch.einsum("nbk,bok->nbo", x.double().abs(), w.double().abs()) * (k + 1) * 2.0**-24
     assert bool(((out[:, :, :o].double() - want).abs() <= bound).all())
     assert float((out[:, :, o:] - 7.0).abs().max()) == 0.0
+
+
+# -- 32-bit attention --------------------------------------------------------------------------------
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("nq, nkv, d, page, window", [
+    (4, 2, 64, 16, None), (16, 8, 128, 16, None), (6, 1, 40, 4, 50), (20, 1, 16, 8, None), (4, 4, 256, 32, 130), (9, 3, 72, 2, 1)])
+def test_attention_of_entries(native, dtype, nq, nkv, d, page, window):
+    """Entries of one token (at both sides of a span of 128 positions) beside entries of several (at both
+    sides of a tile of 32 rows and of 64 keys), each also alone: the same bits, and the dense result."""
+    lengths = [300, 1, 128, 129, 257, 64, 65, 400]
+    counts = [1, 1, 1, 1, 33, 64, 2, 17]
+    k_cache, v_cache, table, keys, values = paged_layout(lengths, page, nkv, d, dtype, seed=d + nq)
+    gen = torch.Generator().manual_seed(5)
+    positions = [p for n, c in zip(lengths, counts) for p in range(n - c, n)]
+    entry = [e for e, c in enumerate(counts) for _ in range(c)]
+    q = torch.randn((len(positions), nq, d), generator=gen).to(dtype)
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)  # noqa: E731
+    cu = [0]
+    for c in counts:
+        cu.append(cu[-1] + c)
+    status = status_word()
+
+    def attend(rows, table, cu_tokens):
+        out = torch.empty((len(rows), nq * d), dtype=dtype, device=DEV)
+        native.attention_simt(q[rows].reshape(len(rows), nq * d).to(DEV), nq * d, k_cache, v_cache, table, ints([positions[r] for r in rows]),
+                              ints([0 if table.shape[0] == 1 else entry[r] for r in rows]), window, d ** -0.5, out, nq, status,
+                              entries=(ints(cu_tokens), len(cu_tokens) - 1, max(b - a for a, b in zip(cu_tokens, cu_tokens[1:]))))
+        return out
+
+    together = attend(list(range(len(positions))), table, cu)
+    assert int(status.item()) == 0
+    for e, count in enumerate(counts):
+        rows = list(range(cu[e], cu[e + 1]))
+        assert torch.equal(attend(rows, table[e : e + 1].contiguous(), [0, count]), together[rows])
+        want = dense_attention(q[rows], keys[e], values[e], torch.tensor([positions[r] for r in rows]), d ** -0.5, window)
+        mine = together[rows].view(count, nq, d).double().cpu()
+        torch.testing.assert_close(mine, want, **(dict(atol=2e-5, rtol=1e-5) if dtype == torch.float32 else dict(atol=2e-2, rtol=2e-2)))
+
+
+def test_attention_marks_missing_pages_and_keeps_later_infinities_out(native):
+    """A position without a page sets the status bit; an infinite value of a later token of the same tile
+    changes no earlier row."""
+    k_cache, v_cache, table, keys, values = paged_layout([40], 8, 1, 16, torch.float32, seed=3)
+    q = torch.randn((40, 2, 16), generator=torch.Generator().manual_seed(1))
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)  # noqa: E731
+
+    def attend(table, positions, cu):
+        out, status = torch.empty((len(positions), 32), device=DEV), status_word()
+        native.attention_simt(q[positions].reshape(len(positions), 32).to(DEV), 32, k_cache, v_cache, table, ints(positions),
+                              ints([0] * len(positions)), None, 0.25, out, 2, status, entries=(ints(cu), 1, len(positions)))
+        return out, int(status.item())
+
+    clean, status = attend(table, list(range(40)), [0, 40])
+    assert status == 0
+    v_cache[int(table[0, 39 // 8]), :, 39 % 8] = float("inf")
+    loud, status = attend(table, list(range(40)), [0, 40])
+    assert status == 0 and torch.equal(loud[:39], clean[:39]) and not bool(torch.isfinite(loud[39]).any())
+    holed = table.clone()
+    holed[0, 1] = -1
+    assert attend(holed, list(range(40)), [0, 40])[1] & 2
+    assert attend(holed, [30], [0, 1])[1] & 2
+    assert attend(table[:, :2].contiguous(), [39], [0, 1])[1] & 2
