@@ -19,19 +19,24 @@
 //   into steps and what else is in the batch change nothing.  With `long_from` > 0 it leaves
 //   entries of that many tokens or more to the three kernels below.
 //
-// Long entries (prompt portions) run chunk by chunk side by side, which is exact for a linear
-// recurrence: with b_t the product of the forget gates from the chunk's first token up to t,
-//     S_t = diag(b_t) S_start + S_local_t,      o_t = (q_t * b_t)^T S_start + o_local_t.
-// gated_recurrence_local  - the kernel above on one chunk of GR_LONG_CHUNK tokens per block,
-//   started from zero: o_local (32-bit, not yet normalised), q_t * b_t, the chunk's last local
-//   state and its b.
-// gated_recurrence_scan   - one thread per state element walks the entry's chunks in order:
-//   S_start of every chunk, and the request's state row after the last.
-// gated_recurrence_finish - per chunk (q * b)^T S_start + o_local as a small 32-bit product from
-//   shared memory, then the head's norm and the store.
-// There is no division by a decay anywhere (a gate may be as small as its lower bound allows),
-// and everything stays 32-bit; against the token-by-token walk only the order of additions
-// differs.
+// Long entries (prompt portions) run in chunks of 64 tokens side by side, which is exact for a linear
+// recurrence: with k_t = 1 - f_t, D(t, s) the product of the forget gates after s up to t, and D(t) that
+// from the chunk's first token up to t,
+//     o_t = (q_t D(t))^T S_start + sum_{s <= t} A_ts v_s,   A_ts = sum_d q_t D(t, s) k_s,
+//     S_end = D(end) S_start + sum_s (D(end, s) k_s) v_s^T.
+// gated_recurrence_chunk  - per head and chunk: q_t D(t), A, the chunk's own end state and D(end).
+//   The chunk is cut into four sub-chunks of 16 tokens.  Inside one, the 16 x 16 products D(t, s) k_s are
+//   built up token by token; between two, D splits into the product from the later one's start up to t,
+//   the whole gates of the sub-chunks in between, and the product after s up to the earlier one's end,
+//   so that A becomes small matrix products.
+// gated_recurrence_scan   - one thread per state element walks the entry's chunks in order: S_start of
+//   every chunk (in the place of its end state), and the request's state row after the last.
+// gated_recurrence_finish - per chunk [q D | A] [S_start; V] as one 32-bit product from shared memory,
+//   then the head's norm and the store.
+// All factors are products of gates: there is no division by a decay anywhere (a gate may be as small
+// as its lower bound allows), and everything stays 32-bit; against the token-by-token walk only the order
+// of additions differs.  What a token costs is 2 dk dv multiply-adds as register tiles of 4 x 4 to 8 x 8
+// (the walk takes five operations per state element and reads two operands of each from shared memory).
 #include "common.cuh"
 
 #define GR_CHUNK 16
@@ -53,10 +58,10 @@ struct GatedRecurrence {
   int heads, dk, dv, ds, kpt;
   int long_from;          // above zero: entries of this many tokens or more belong to the chunk-parallel kernels
   // scratch of the chunk-parallel kernels (32-bit)
-  float* o_local;         // [tokens, heads * dv]
-  float* qb;              // [tokens, heads * dk]
-  float* chunk_state;     // [chunk slots, heads, dk, dv]: the chunk's local end state, then (scan) its start state
-  float* chunk_start;     // [chunk slots, heads, dk, dv]
+  int dkp;                // dk rounded up to fours; the added channels are zero
+  float* qb;              // [tokens, heads, dkp]
+  float* within;          // [chunk slots, heads, 64, 64]: A
+  float* chunk_state;     // [chunk slots, heads, dk, dv]: the chunk's own end state, then (scan) its start state
   float* chunk_decay;     // [chunk slots, heads, dk]
 };
 
@@ -65,6 +70,12 @@ struct GatedRecurrence {
 // tokens apart per chunk, so floor(first / chunk) + e + c never repeats.
 __device__ __forceinline__ int gr_chunk_slot(int first, int entry, int chunk) { return first / GR_LONG_CHUNK + entry + chunk; }
 
+__device__ __forceinline__ void gr_copy16(void* dst, const void* src, bool valid) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
+               ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(valid ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void gr_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void gr_wait_one() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 __device__ __forceinline__ float gr_sigmoid(float x) { return 1.f / (1.f + expf(-x)); }
 
 template <typename TO, int KPT>
@@ -144,13 +155,36 @@ __global__ void __launch_bounds__(1024) gated_recurrence_kernel(GatedRecurrence 
 }
 
 
-// One chunk of a long entry from a zero state (see the head of this file).  A thread keeps the
-// rows s * kpt .. s * kpt + kpt - 1 of its column, so that it reads its gates and queries of a
-// token with 16-byte loads from shared memory; the rows up to KPT are padded with f = 1, q = 0
-// (such a row stays zero), and a pitch of KPT + 4 keeps the eight lanes of a load in different
-// banks.  The running product of the gates and q * b are the work of one thread per channel.
-template <int KPT>
-__global__ void __launch_bounds__(1024) gated_recurrence_local_kernel(GatedRecurrence p) {
+#define GR_SUB 16                                // tokens of a sub-chunk
+#define GR_SUBS (GR_LONG_CHUNK / GR_SUB)
+#define GR_SLICE 128                             // channels (or columns) worked on at a time
+#define GR_AP (GR_LONG_CHUNK + 4)
+
+// Sums of 16 values over the lanes of a warp; lane l gets the sum of value l / 2.
+__device__ __forceinline__ float gr_sum16(float (&x)[16], int lane) {
+#pragma unroll
+  for (int half = 8, bit = 16; half > 0; half >>= 1, bit >>= 1) {
+    const bool upper = (lane & bit) != 0;
+#pragma unroll
+    for (int i = 0; i < half; ++i) {
+      const float send = upper ? x[i] : x[i + half], keep = upper ? x[i + half] : x[i];
+      x[i] = keep + __shfl_xor_sync(0xffffffffu, send, bit);
+    }
+  }
+  return x[0] + __shfl_xor_sync(0xffffffffu, x[0], 1);
+}
+
+__device__ __forceinline__ void gr_outer(float (&acc)[4][4], const float4 a, const float4 b) {
+  const float x[4] = {a.x, a.y, a.z, a.w}, y[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(x[i], y[j], acc[i][j]);
+}
+
+// One chunk of a long entry (see the head of this file).  Tokens past the entry's end have f = 1 and
+// q = k = v = 0.
+__global__ void __launch_bounds__(256, 2) gated_recurrence_chunk_kernel(GatedRecurrence p, int aligned) {
   extern __shared__ __align__(16) float smem[];
   pdl_trigger();
   pdl_wait();
@@ -158,83 +192,278 @@ __global__ void __launch_bounds__(1024) gated_recurrence_local_kernel(GatedRecur
   const int entry_first = p.cu_tokens[entry], entry_count = p.cu_tokens[entry + 1] - entry_first;
   if (entry_count < p.long_from || chunk * GR_LONG_CHUNK >= entry_count) return;
   const int first = entry_first + chunk * GR_LONG_CHUNK, count = min(GR_LONG_CHUNK, entry_count - chunk * GR_LONG_CHUNK);
-  const int dk = p.dk, dv = p.dv, DS = p.ds, kpt = p.kpt;
-  constexpr int KP = KPT >= 8 ? KPT + 4 : KPT;
-  const int pitch = DS * KP;              // floats per token
-  float* fs = smem;                       // [GR_CHUNK][DS][KP]
-  float* qs = fs + GR_CHUNK * pitch;      // [GR_CHUNK][DS][KP]
-  float* vs = qs + GR_CHUNK * pitch;      // [GR_CHUNK][dv]
-  float* bs = vs + GR_CHUNK * dv;         // [dk]: the product of the gates so far
-  const int tid = threadIdx.x;
-  const int v = tid / DS, s = tid - v * DS;
-  const bool live = v < dv;
-  float S[KPT];
-#pragma unroll
-  for (int i = 0; i < KPT; ++i) S[i] = 0.f;
-  for (int idx = tid; idx < GR_CHUNK * pitch; idx += blockDim.x) { fs[idx] = 1.f; qs[idx] = 0.f; }
-  for (int d = tid; d < dk; d += blockDim.x) bs[d] = 1.f;
-  __syncthreads();
-  const float* bias = p.f_bias ? p.f_bias + head * dk : nullptr;
-  const float* low = p.lower + head * dk;
-  for (int c0 = 0; c0 < count; c0 += GR_CHUNK) {
-    const int nt = min(GR_CHUNK, count - c0);
-    for (int idx = tid; idx < nt * dk; idx += blockDim.x) {
-      const int t = idx / dk, d = idx - t * dk;
-      const float* row = p.proj + (size_t)(first + c0 + t) * p.ld;
-      const float zq = row[p.q_off + head * dk + d];
-      const float zf = row[p.f_off + head * dk + d] + (bias ? bias[d] : 0.f);
-      const float l = low[d];
-      const int owner = d / kpt, at = t * pitch + owner * KP + (d - owner * kpt);
-      qs[at] = zq * gr_sigmoid(zq);
-      fs[at] = l + (1.f - l) * gr_sigmoid(zf);
-    }
-    for (int idx = tid; idx < nt * dv; idx += blockDim.x) {
-      const int t = idx / dv, c = idx - t * dv;
-      vs[idx] = p.proj[(size_t)(first + c0 + t) * p.ld + p.v_off + head * dv + c];
-    }
-    __syncthreads();
-    for (int d = tid; d < dk; d += blockDim.x) {
-      const int owner = d / kpt, at = owner * KP + (d - owner * kpt);
-      float b = bs[d];
-      float* dst = p.qb + (size_t)(first + c0) * p.heads * dk + (size_t)head * dk + d;
-      for (int t = 0; t < nt; ++t) {
-        b *= fs[t * pitch + at];
-        dst[(size_t)t * p.heads * dk] = qs[t * pitch + at] * b;
-      }
-      bs[d] = b;
-    }
-    for (int t = 0; t < nt; ++t) {
-      const float vv = live ? vs[t * dv + v] : 0.f;
-      const float4* f4 = reinterpret_cast<const float4*>(fs + t * pitch + s * KP);
-      const float4* q4 = reinterpret_cast<const float4*>(qs + t * pitch + s * KP);
-      float acc = 0.f;
-#pragma unroll
-      for (int i = 0; i < KPT / 4; ++i) {
-        const float4 f = f4[i], q = q4[i];
-        S[4 * i + 0] = fmaf(f.x, S[4 * i + 0], (1.f - f.x) * vv);
-        S[4 * i + 1] = fmaf(f.y, S[4 * i + 1], (1.f - f.y) * vv);
-        S[4 * i + 2] = fmaf(f.z, S[4 * i + 2], (1.f - f.z) * vv);
-        S[4 * i + 3] = fmaf(f.w, S[4 * i + 3], (1.f - f.w) * vv);
-        acc = fmaf(S[4 * i + 0], q.x, acc);
-        acc = fmaf(S[4 * i + 1], q.y, acc);
-        acc = fmaf(S[4 * i + 2], q.z, acc);
-        acc = fmaf(S[4 * i + 3], q.w, acc);
-      }
-      for (int o = DS >> 1; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-      if (live && s == 0) p.o_local[(size_t)(first + c0 + t) * p.heads * dv + (size_t)head * dv + v] = acc;
-    }
-    __syncthreads();
-  }
+  const int dk = p.dk, dv = p.dv;
+  const int dp = min(p.dkp, GR_SLICE) + 4, vp = min(dv, GR_SLICE) + 4;   // pitches: rows of 16 bytes in different banks
+  float* fs = smem;                              // [64][dp]: gates, then what is left of k
+  float* qs = fs + GR_LONG_CHUNK * dp;           // [64][dp]; when q is done, vs [64][vp]
+  float* vs = qs;
+  float* as = qs + GR_LONG_CHUNK * max(dp, vp);  // [64][GR_AP]
+  float* whole = as + GR_LONG_CHUNK * GR_AP;     // [4][dp]: the gates of a whole sub-chunk
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const size_t at = (size_t)gr_chunk_slot(entry_first, entry, chunk) * p.heads + head;
+  for (int i = tid; i < GR_LONG_CHUNK * GR_AP; i += 256) as[i] = 0.f;
+
+  for (int d0 = 0; d0 < dk; d0 += GR_SLICE) {
+    const int nd = min(GR_SLICE, dk - d0), ndp = (nd + 3) & ~3;
+    __syncthreads();
+    if (aligned) {
+      // four channels a thread, all loads of four rows on their way before the first is used
+      const int quads = ndp >> 2, step = 256 / 32;      // a warp takes a row (up to 32 quads)
+      const int d = lane * 4;
+      if (lane < quads) {
+        float low[4], bias[4] = {0.f, 0.f, 0.f, 0.f};
+        load4(p.lower + head * dk + d0 + d, low);
+        if (p.f_bias) load4(p.f_bias + head * dk + d0 + d, bias);
+        const float* base = p.proj + (size_t)head * dk + d0 + d;
 #pragma unroll
-  for (int i = 0; i < KPT; ++i)
-    if (live && i < kpt) p.chunk_state[(at * dk + s * kpt + i) * dv + v] = S[i];
-  for (int d = tid; d < dk; d += blockDim.x) p.chunk_decay[at * dk + d] = bs[d];
+        for (int t0 = 0; t0 < GR_LONG_CHUNK; t0 += 4 * step) {
+          float zf[4][4], zq[4][4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const int t = t0 + u * step + warp;
+            const float* row = base + (size_t)(first + min(t, count - 1)) * p.ld;
+            load4(row + p.f_off, zf[u]);
+            load4(row + p.q_off, zq[u]);
+          }
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const int t = t0 + u * step + warp;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              zq[u][e] = t < count ? zq[u][e] * gr_sigmoid(zq[u][e]) : 0.f;
+              zf[u][e] = t < count ? low[e] + (1.f - low[e]) * gr_sigmoid(zf[u][e] + bias[e]) : 1.f;
+            }
+            store4(qs + t * dp + d, zq[u]);
+            store4(fs + t * dp + d, zf[u]);
+          }
+        }
+      }
+    } else {
+      for (int i = tid; i < GR_LONG_CHUNK * ndp; i += 256) {
+        const int t = i / ndp, d = i - t * ndp;
+        float f = 1.f, q = 0.f;
+        if (t < count && d < nd) {
+          const float* row = p.proj + (size_t)(first + t) * p.ld + (size_t)head * dk + d0 + d;
+          const float zq = row[p.q_off], zf = row[p.f_off] + (p.f_bias ? p.f_bias[head * dk + d0 + d] : 0.f);
+          const float l = p.lower[head * dk + d0 + d];
+          q = zq * gr_sigmoid(zq);
+          f = l + (1.f - l) * gr_sigmoid(zf);
+        }
+        fs[t * dp + d] = f;
+        qs[t * dp + d] = q;
+      }
+    }
+    __syncthreads();
+    {
+      // inside the sub-chunks: two warps each, two tokens s at a time, lanes over the channels
+      constexpr int AT = 2;
+      const int sub = warp >> 1, base = sub * GR_SUB;
+#pragma unroll 1
+      for (int pass = 0; pass < 8 / AT; ++pass) {
+        const int s0 = (warp & 1) * 8 + pass * AT;
+        float w[AT][GR_SLICE / 32], sums[AT][GR_SUB];
+#pragma unroll
+        for (int k = 0; k < AT; ++k)
+#pragma unroll
+          for (int r = 0; r < GR_SLICE / 32; ++r) w[k][r] = 0.f;
+#pragma unroll
+        for (int t = 0; t < GR_SUB; ++t) {
+          float f[GR_SLICE / 32], q[GR_SLICE / 32];
+#pragma unroll
+          for (int r = 0; r < GR_SLICE / 32; ++r) {
+            const bool has = lane + 32 * r < ndp;
+            f[r] = has ? fs[(base + t) * dp + lane + 32 * r] : 1.f;
+            q[r] = has ? qs[(base + t) * dp + lane + 32 * r] : 0.f;
+          }
+#pragma unroll
+          for (int k = 0; k < AT; ++k) {
+            float sum = 0.f;
+#pragma unroll
+            for (int r = 0; r < GR_SLICE / 32; ++r) {
+              w[k][r] = t == s0 + k ? 1.f - f[r] : w[k][r] * f[r];
+              sum = fmaf(q[r], w[k][r], sum);
+            }
+            sums[k][t] = sum;
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < AT; ++k) {
+          const float sum = gr_sum16(sums[k], lane);
+          const int t = lane >> 1;
+          if ((lane & 1) == 0 && t >= s0 + k) as[(base + t) * GR_AP + base + s0 + k] += sum;
+        }
+      }
+    }
+    __syncthreads();
+    // q with the gates from its sub-chunk's start on, k with those up to its sub-chunk's end
+    for (int i = tid; i < ndp * GR_SUBS; i += 256) {
+      const int sub = i / ndp, d = i - sub * ndp;
+      float* f = fs + sub * GR_SUB * dp + d;
+      float* q = qs + sub * GR_SUB * dp + d;
+      float g[GR_SUB], b = 1.f;
+#pragma unroll
+      for (int t = 0; t < GR_SUB; ++t) {
+        g[t] = f[t * dp];
+        b *= g[t];
+        q[t * dp] *= b;
+      }
+      whole[sub * dp + d] = b;
+      b = 1.f;
+#pragma unroll
+      for (int t = GR_SUB - 1; t >= 0; --t) {
+        f[t * dp] = (1.f - g[t]) * b;
+        b *= g[t];
+      }
+    }
+    __syncthreads();
+    // sub-chunks `apart` apart: A's blocks of 16 x 16, 64 threads each; q then takes the gates of the
+    // sub-chunk it has just been multiplied with
+#pragma unroll 1
+    for (int apart = 1; apart < GR_SUBS; ++apart) {
+      const int block = tid >> 6;
+      if (block < GR_SUBS - apart) {
+        const int r = (tid & 63) >> 3, c = tid & 7;
+        const float* q0 = qs + ((apart + block) * GR_SUB + r) * dp;
+        const float* k0 = fs + (block * GR_SUB + c) * dp;
+        float sum[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+#pragma unroll 4
+        for (int d = 0; d < ndp; d += 4) {
+          float a[2][4], b[2][4];
+          load4(q0 + d, a[0]), load4(q0 + 8 * dp + d, a[1]), load4(k0 + d, b[0]), load4(k0 + 8 * dp + d, b[1]);
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+              for (int j = 0; j < 2; ++j) sum[i][j] = fmaf(a[i][e], b[j][e], sum[i][j]);
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+          for (int j = 0; j < 2; ++j) as[((apart + block) * GR_SUB + r + 8 * i) * GR_AP + block * GR_SUB + c + 8 * j] += sum[i][j];
+      }
+      __syncthreads();
+      if (lane * 4 < ndp) {
+        const int d = lane * 4;
+#pragma unroll 4
+        for (int t = warp; t < (GR_SUBS - apart) * GR_SUB; t += 8) {
+          float* q = qs + (apart * GR_SUB + t) * dp + d;
+          float a[4], g[4];
+          load4(q, a), load4(whole + (t / GR_SUB) * dp + d, g);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) a[e] *= g[e];
+          store4(q, a);
+        }
+      }
+      __syncthreads();
+    }
+    if (lane * 4 < ndp) {
+#pragma unroll 4
+      for (int t = warp; t < count; t += 8) {
+        float a[4];
+        load4(qs + t * dp + lane * 4, a);
+        store4(p.qb + ((size_t)(first + t) * p.heads + head) * p.dkp + d0 + lane * 4, a);
+      }
+    }
+    // k with the gates up to the chunk's end
+    for (int d = tid; d < nd; d += 256) {
+      float b = 1.f;
+#pragma unroll
+      for (int sub = GR_SUBS - 1; sub >= 0; --sub) {
+        if (sub < GR_SUBS - 1)
+          for (int t = 0; t < GR_SUB; ++t) fs[(sub * GR_SUB + t) * dp + d] *= b;
+        b *= whole[sub * dp + d];
+      }
+      p.chunk_decay[at * dk + d0 + d] = b;
+    }
+    // the chunk's own end state
+    const int ty = tid >> 4, tx = tid & 15;
+    for (int v0 = 0; v0 < dv; v0 += GR_SLICE) {
+      const int nv = min(GR_SLICE, dv - v0);
+      __syncthreads();
+      if (aligned) {
+        const int c = lane * 4;
+        if (c < nv) {
+          const float* base = p.proj + p.v_off + (size_t)head * dv + v0 + c;
+          float x[8][4];
+#pragma unroll
+          for (int u = 0; u < 8; ++u) load4(base + (size_t)(first + min(u * 8 + warp, count - 1)) * p.ld, x[u]);
+#pragma unroll
+          for (int u = 0; u < 8; ++u) {
+            const int t = u * 8 + warp;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) x[u][e] = t < count ? x[u][e] : 0.f;
+            store4(vs + t * vp + c, x[u]);
+          }
+        }
+      } else {
+        for (int i = tid; i < GR_LONG_CHUNK * nv; i += 256) {
+          const int t = i / nv, c = i - t * nv;
+          vs[t * vp + c] = t < count ? p.proj[(size_t)(first + t) * p.ld + p.v_off + (size_t)head * dv + v0 + c] : 0.f;
+        }
+      }
+      __syncthreads();
+      const bool d_lo = ty * 4 < ndp, d_hi = ty * 4 + 64 < ndp, v_lo = tx * 4 < nv, v_hi = tx * 4 + 64 < nv;
+      float acc[2][2][4][4];
+#pragma unroll
+      for (int a = 0; a < 2; ++a)
+#pragma unroll
+        for (int b = 0; b < 2; ++b)
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[a][b][i][j] = 0.f;
+      const float* kd = fs + ty * 4;
+      const float* vd = vs + tx * 4;
+      const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (ndp > 64 && nv > 64) {
+#pragma unroll 2
+        for (int s = 0; s < GR_LONG_CHUNK; ++s) {
+          const float4 k0 = *reinterpret_cast<const float4*>(kd + s * dp), k1 = d_hi ? *reinterpret_cast<const float4*>(kd + s * dp + 64) : zero;
+          const float4 x0 = *reinterpret_cast<const float4*>(vd + s * vp), x1 = v_hi ? *reinterpret_cast<const float4*>(vd + s * vp + 64) : zero;
+          gr_outer(acc[0][0], k0, x0);
+          gr_outer(acc[0][1], k0, x1);
+          gr_outer(acc[1][0], k1, x0);
+          gr_outer(acc[1][1], k1, x1);
+        }
+      } else if (ndp > 64) {
+#pragma unroll 2
+        for (int s = 0; s < GR_LONG_CHUNK; ++s) {
+          const float4 k0 = *reinterpret_cast<const float4*>(kd + s * dp), k1 = d_hi ? *reinterpret_cast<const float4*>(kd + s * dp + 64) : zero;
+          const float4 x0 = v_lo ? *reinterpret_cast<const float4*>(vd + s * vp) : zero;
+          gr_outer(acc[0][0], k0, x0);
+          gr_outer(acc[1][0], k1, x0);
+        }
+      } else {
+#pragma unroll 2
+        for (int s = 0; s < GR_LONG_CHUNK; ++s) {
+          const float4 k0 = d_lo ? *reinterpret_cast<const float4*>(kd + s * dp) : zero;
+          const float4 x0 = v_lo ? *reinterpret_cast<const float4*>(vd + s * vp) : zero, x1 = v_hi ? *reinterpret_cast<const float4*>(vd + s * vp + 64) : zero;
+          gr_outer(acc[0][0], k0, x0);
+          gr_outer(acc[0][1], k0, x1);
+        }
+      }
+#pragma unroll
+      for (int a = 0; a < 2; ++a)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int d = ty * 4 + 64 * a + i;
+          if (d >= nd) continue;
+          float* dst = p.chunk_state + (at * dk + d0 + d) * dv + v0;
+#pragma unroll
+          for (int b = 0; b < 2; ++b)
+            if (tx * 4 + 64 * b < nv) store4(dst + tx * 4 + 64 * b, acc[a][b][i]);
+        }
+    }
+  }
+  __syncthreads();
+  float* within = p.within + at * GR_LONG_CHUNK * GR_LONG_CHUNK;
+  for (int i = tid; i < GR_LONG_CHUNK * GR_LONG_CHUNK; i += 256) within[i] = as[(i / GR_LONG_CHUNK) * GR_AP + i % GR_LONG_CHUNK];
 }
 
-// One thread per element (d, v) of a head's state: the start state of every chunk of a long
-// entry, in order, and the request's state row after the last chunk.
-__global__ void __launch_bounds__(256) gated_recurrence_scan_kernel(GatedRecurrence p, int* status) {
+// One thread per four neighbouring columns of a state row: the start state of every chunk of a long entry, in
+// order, in the place of the chunk's own end state, and the request's state row after the last chunk.
+__global__ void __launch_bounds__(128) gated_recurrence_scan_kernel(GatedRecurrence p, int* status) {
   pdl_trigger();
   pdl_wait();
   const int head = blockIdx.x, entry = blockIdx.y;
@@ -245,30 +474,50 @@ __global__ void __launch_bounds__(256) gated_recurrence_scan_kernel(GatedRecurre
     if (threadIdx.x == 0 && blockIdx.z == 0) atomicOr(status, FE_STATUS_BAD_PAGE);
     return;
   }
-  const int cell = blockIdx.z * blockDim.x + threadIdx.x;
+  const int cell = (blockIdx.z * blockDim.x + threadIdx.x) * 4;
   if (cell >= p.dk * p.dv) return;
   const int d = cell / p.dv;
   const int chunks = (count + GR_LONG_CHUNK - 1) / GR_LONG_CHUNK;
   float* st = p.state + ((size_t)slot * p.heads + head) * p.dk * p.dv + cell;
-  float state = *st;
+  const bool wide = ((uintptr_t)p.state & 15) == 0;
+  float state[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) state[e] = st[e];
   const size_t stride = (size_t)p.heads * p.dk * p.dv;
-  const float* __restrict__ local = p.chunk_state + ((size_t)gr_chunk_slot(first, entry, 0) * p.heads + head) * p.dk * p.dv + cell;
-  float* __restrict__ start = p.chunk_start + ((size_t)gr_chunk_slot(first, entry, 0) * p.heads + head) * p.dk * p.dv + cell;
+  float* cells = p.chunk_state + ((size_t)gr_chunk_slot(first, entry, 0) * p.heads + head) * p.dk * p.dv + cell;
   const float* __restrict__ decay = p.chunk_decay + ((size_t)gr_chunk_slot(first, entry, 0) * p.heads + head) * p.dk + d;
-#pragma unroll 4
-  for (int c = 0; c < chunks; ++c) {
-    start[c * stride] = state;
-    state = fmaf(decay[(size_t)c * p.heads * p.dk], state, local[c * stride]);
+  for (int c = 0; c < chunks; c += 4) {          // four chunks' loads at a time
+    float own[4][4], keep[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int at = min(c + u, chunks - 1);
+      load4(cells + at * stride, own[u]);
+      keep[u] = decay[(size_t)at * p.heads * p.dk];
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (c + u >= chunks) break;
+      store4(cells + (c + u) * stride, state);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) state[e] = fmaf(keep[u], state[e], own[u][e]);
+    }
   }
-  *st = state;
+  if (wide) {
+    store4(st, state);
+  } else {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) st[e] = state[e];
+  }
 }
 
-// o_t = (q_t * b_t)^T S_start + o_local_t for the tokens of one chunk, then the head's norm.
-// Thread (t, g) of 64 x 4 takes token t and, per round of 32 columns, the columns 4g .. 4g + 3
-// and 16 + 4g .. 16 + 4g + 3 (dv is a multiple of 4); S_start and q * b are read from shared
-// memory 16 bytes at a time.
+// o = [q D | A] [S_start; V] for the 64 tokens of a chunk, then the head's norm.  Both operands pass
+// through shared memory in stretches of 32 rows of the right one; thread (ty, tx) of 8 x 16 keeps tokens
+// ty, ty + 8, .. of the columns 4 tx .. and 64 + 4 tx .. of a pass of 128 columns (dv is a multiple of 4).
+// Where dv takes more than one pass the rows wait in shared memory for the norm.
+#define GR_FK 32
+#define GR_FX (GR_FK + 4)
 template <typename TO>
-__global__ void __launch_bounds__(256) gated_recurrence_finish_kernel(GatedRecurrence p) {
+__global__ void __launch_bounds__(128, 2) gated_recurrence_finish_kernel(GatedRecurrence p, int v_aligned) {
   extern __shared__ __align__(16) float smem[];
   pdl_trigger();
   pdl_wait();
@@ -277,53 +526,131 @@ __global__ void __launch_bounds__(256) gated_recurrence_finish_kernel(GatedRecur
   if (entry_count < p.long_from || chunk * GR_LONG_CHUNK >= entry_count) return;
   const int first = entry_first + chunk * GR_LONG_CHUNK, count = min(GR_LONG_CHUNK, entry_count - chunk * GR_LONG_CHUNK);
   const int dk = p.dk, dv = p.dv;
-  const int dkp = (dk + 3) & ~3;            // rows in fours; the added ones are zero
-  const int qld = dkp + 4;                  // 16-byte rows; a warp's eight tokens read different banks
-  float* ss = smem;                         // [dkp][dv]
-  float* qb = ss + dkp * dv;                // [GR_LONG_CHUNK][qld]
-  float* os = qb + GR_LONG_CHUNK * qld;     // [GR_LONG_CHUNK][dv]
-  const int tid = threadIdx.x;
-  const float* start = p.chunk_start + ((size_t)gr_chunk_slot(entry_first, entry, chunk) * p.heads + head) * dk * dv;
-  for (int i = tid; i < dkp * dv; i += blockDim.x) ss[i] = i < dk * dv ? start[i] : 0.f;
-  for (int i = tid; i < count * qld; i += blockDim.x) {
-    const int t = i / qld, d = i - t * qld;
-    qb[i] = d < dk ? p.qb[(size_t)(first + t) * p.heads * dk + (size_t)head * dk + d] : 0.f;
-  }
-  __syncthreads();
-  const int t = tid >> 2, g = tid & 3;
-  if (t < count) {
-    const float* qt = qb + t * qld;
-    const float* local = p.o_local + (size_t)(first + t) * p.heads * dv + (size_t)head * dv;
-    for (int v0 = 0; v0 < dv; v0 += 32) {
-      const int c0 = v0 + 4 * g, c1 = c0 + 16;
-      const bool has0 = c0 < dv, has1 = c1 < dv;
-      float4 a0 = make_float4(0.f, 0.f, 0.f, 0.f), a1 = a0;
-      for (int d = 0; d < dkp; d += 4) {
-        const float4 q = *reinterpret_cast<const float4*>(qt + d);
-        const float qk[4] = {q.x, q.y, q.z, q.w};
+  const int wide = min(dv, GR_SLICE);
+  const int stage_floats = GR_LONG_CHUNK * GR_FX + GR_FK * wide;
+  float* os = smem + 2 * stage_floats;          // [64][dv], only where dv > 128
+  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+  const size_t at = (size_t)gr_chunk_slot(entry_first, entry, chunk) * p.heads + head;
+  const float* qb = p.qb + ((size_t)first * p.heads + head) * p.dkp;
+  const float* within = p.within + at * GR_LONG_CHUNK * GR_LONG_CHUNK;
+  const float* start = p.chunk_state + at * dk * dv;
+  const float* values = p.proj + (size_t)first * p.ld + p.v_off + (size_t)head * dv;
+  const int q_steps = (p.dkp + GR_FK - 1) / GR_FK, steps = q_steps + (count + GR_FK - 1) / GR_FK;
+
+  auto stage = [&](int step, int v0, int nv) {
+    float* xs = smem + (step & 1) * stage_floats;
+    float* ys = xs + GR_LONG_CHUNK * GR_FX;
+    const bool state = step < q_steps;
+    const int k0 = (state ? step : step - q_steps) * GR_FK;
+    for (int i = tid; i < GR_LONG_CHUNK * (GR_FK / 4); i += 128) {
+      const int t = i / (GR_FK / 4), k = (i % (GR_FK / 4)) * 4;
+      const float* src = state ? qb + (size_t)t * p.heads * p.dkp + k0 + k : within + t * GR_LONG_CHUNK + k0 + k;
+      const bool valid = t < count && (!state || k0 + k < p.dkp);
+      gr_copy16(xs + t * GR_FX + k, valid ? src : within, valid);
+    }
+    for (int i = tid; i < GR_FK * (nv / 4); i += 128) {
+      const int k = i / (nv / 4), c = (i % (nv / 4)) * 4;
+      const bool valid = state ? k0 + k < dk : k0 + k < count;
+      const float* src = !valid ? start : state ? start + (size_t)(k0 + k) * dv + v0 + c : values + (size_t)(k0 + k) * p.ld + v0 + c;
+      if (state || v_aligned) {
+        gr_copy16(ys + k * wide + c, src, valid);
+      } else {
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const float* sr = ss + (d + k) * dv;
-          if (has0) {
-            const float4 x = *reinterpret_cast<const float4*>(sr + c0);
-            a0.x = fmaf(qk[k], x.x, a0.x), a0.y = fmaf(qk[k], x.y, a0.y), a0.z = fmaf(qk[k], x.z, a0.z), a0.w = fmaf(qk[k], x.w, a0.w);
-          }
-          if (has1) {
-            const float4 x = *reinterpret_cast<const float4*>(sr + c1);
-            a1.x = fmaf(qk[k], x.x, a1.x), a1.y = fmaf(qk[k], x.y, a1.y), a1.z = fmaf(qk[k], x.z, a1.z), a1.w = fmaf(qk[k], x.w, a1.w);
+        for (int e = 0; e < 4; ++e) ys[k * wide + c + e] = valid ? src[e] : 0.f;
+      }
+    }
+    gr_commit();
+  };
+
+  for (int v0 = 0; v0 < dv; v0 += GR_SLICE) {
+    const int nv = min(GR_SLICE, dv - v0);
+    const bool has0 = tx * 4 < nv, has1 = tx * 4 + 64 < nv;
+    float acc[2][2][4][4];
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int b = 0; b < 2; ++b)
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) acc[h][b][i][j] = 0.f;
+    __syncthreads();
+    stage(0, v0, nv);
+    for (int step = 0; step < steps; ++step) {
+      if (step + 1 < steps) stage(step + 1, v0, nv);
+      else gr_commit();
+      gr_wait_one();
+      __syncthreads();
+      const float* xs = smem + (step & 1) * stage_floats + ty * GR_FX;
+      const float* ys = smem + (step & 1) * stage_floats + GR_LONG_CHUNK * GR_FX + tx * 4;
+      // the first 32 tokens come before all tokens of the second stretch of V: A is zero there
+      const bool second = step > q_steps;
+#pragma unroll 2
+      for (int k = 0; k < GR_FK; k += 4) {
+        float x[2][4][4];                         // tokens ty + 8 i, and 32 further
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          if (!second) load4(xs + 8 * i * GR_FX + k, x[0][i]);
+          load4(xs + (8 * i + 32) * GR_FX + k, x[1][i]);
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float4 late = make_float4(x[1][0][e], x[1][1][e], x[1][2][e], x[1][3][e]);
+          float4 y0 = make_float4(0.f, 0.f, 0.f, 0.f), y1 = y0;
+          if (has0) y0 = *reinterpret_cast<const float4*>(ys + (k + e) * wide);
+          if (has1) y1 = *reinterpret_cast<const float4*>(ys + (k + e) * wide + 64);
+          gr_outer(acc[1][0], late, y0);
+          if (nv > 64) gr_outer(acc[1][1], late, y1);
+          if (!second) {
+            const float4 early = make_float4(x[0][0][e], x[0][1][e], x[0][2][e], x[0][3][e]);
+            gr_outer(acc[0][0], early, y0);
+            if (nv > 64) gr_outer(acc[0][1], early, y1);
           }
         }
       }
-      if (has0) {
-        const float4 l = *reinterpret_cast<const float4*>(local + c0);
-        *reinterpret_cast<float4*>(os + t * dv + c0) = make_float4(a0.x + l.x, a0.y + l.y, a0.z + l.z, a0.w + l.w);
-      }
-      if (has1) {
-        const float4 l = *reinterpret_cast<const float4*>(local + c1);
-        *reinterpret_cast<float4*>(os + t * dv + c1) = make_float4(a1.x + l.x, a1.y + l.y, a1.z + l.z, a1.w + l.w);
-      }
+      __syncthreads();
+    }
+    if (dv <= GR_SLICE) {
+      float w[2][4];
+#pragma unroll
+      for (int b = 0; b < 2; ++b)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) w[b][j] = tx * 4 + 64 * b < nv ? p.norm_w[tx * 4 + 64 * b + j] : 0.f;
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          float sq = 0.f;
+#pragma unroll
+          for (int b = 0; b < 2; ++b)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) sq = fmaf(acc[h][b][i][j], acc[h][b][i][j], sq);
+#pragma unroll
+          for (int o = 8; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+          const float inv = 1.f / sqrtf(sq / (float)dv + p.eps);
+          const int t = 32 * h + 8 * i + ty;
+          if (t >= count) continue;
+#pragma unroll
+          for (int b = 0; b < 2; ++b) {
+            const int c = tx * 4 + 64 * b;
+            if (c >= nv) continue;
+            float o[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) o[j] = acc[h][b][i][j] * inv * w[b][j];
+            store4((TO*)p.out + ((size_t)(first + t) * p.heads + head) * dv + c, o);
+          }
+        }
+    } else {
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int b = 0; b < 2; ++b)
+          if (tx * 4 + 64 * b < nv)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) store4(os + (32 * h + 8 * i + ty) * dv + v0 + tx * 4 + 64 * b, acc[h][b][i]);
     }
   }
+  if (dv <= GR_SLICE) return;
   __syncthreads();
   const int warp = tid >> 5, lane = tid & 31, warps = blockDim.x >> 5;
   for (int r = warp; r < count; r += warps) {
@@ -350,18 +677,22 @@ static int gr_column_threads(int dk, int dv) {
   return 0;
 }
 
-// Shared memory of gated_recurrence_finish, and whether the chunk-parallel kernels take these sizes.
-static size_t gr_finish_smem(int dk, int dv) {
-  const size_t dkp = (size_t)(dk + 3) / 4 * 4;
-  return sizeof(float) * (dkp * dv + (size_t)GR_LONG_CHUNK * (dkp + 4 + dv));
+// Shared memory of the chunk kernels.
+static size_t gr_chunk_smem(int dk, int dv) {
+  const int dkp = (dk + 3) & ~3, dp = (dkp < GR_SLICE ? dkp : GR_SLICE) + 4, vp = (dv < GR_SLICE ? dv : GR_SLICE) + 4;
+  return sizeof(float) * ((size_t)GR_LONG_CHUNK * (dp + (dp > vp ? dp : vp) + GR_AP) + GR_SUBS * dp);
+}
+static size_t gr_finish_smem(int dv) {
+  const int wide = dv < GR_SLICE ? dv : GR_SLICE;
+  return sizeof(float) * ((size_t)2 * (GR_LONG_CHUNK * GR_FX + GR_FK * wide) + (dv > GR_SLICE ? (size_t)GR_LONG_CHUNK * dv : 0));
 }
 
 // 32-bit floats of scratch the chunk-parallel kernels need for a step of `tokens` tokens in
 // `entries` entries (0: these sizes run token by token whatever the entries' lengths).
 FE_EXPORT long long fe_gated_recurrence_scratch(int tokens, int entries, int heads, int dk, int dv) {
-  if (dv % 4 != 0 || gr_finish_smem(dk, dv) > 200 * 1024 || gr_column_threads(dk, dv) == 0) return 0;
-  const long long slots = tokens / GR_LONG_CHUNK + entries + 1;
-  return (long long)tokens * heads * (dk + dv) + slots * heads * ((long long)2 * dk * dv + dk);
+  if (dv % 4 != 0 || gr_finish_smem(dv) > 220 * 1024 || gr_column_threads(dk, dv) == 0) return 0;
+  const long long slots = tokens / GR_LONG_CHUNK + entries + 1, dkp = (dk + 3) & ~3;
+  return slots * heads * ((long long)dk * dv + GR_LONG_CHUNK * GR_LONG_CHUNK + dkp) + (long long)tokens * heads * dkp;
 }
 
 // Tokens from which on an entry runs chunk by chunk.
@@ -380,17 +711,17 @@ FE_EXPORT int fe_gated_recurrence(const float* proj, long long ld, int q_off, in
   if (ds == 0) return FE_ERR_BAD_SHAPE;
   const int kpt = dk / ds;
   GatedRecurrence p{proj, ld, q_off, f_off, v_off, f_bias, lower, norm_w, eps, state, state_rows, slots, cu_tokens, out,
-                    heads, dk, dv, ds, kpt, 0, nullptr, nullptr, nullptr, nullptr, nullptr};
+                    heads, dk, dv, ds, kpt, 0, (dk + 3) & ~3, nullptr, nullptr, nullptr, nullptr};
   const bool chunked = scratch != nullptr && max_new >= fe_gated_recurrence_long_from() &&
                        fe_gated_recurrence_scratch(tokens, entries, heads, dk, dv) > 0;
   if (chunked) {
     const long long chunk_slots = tokens / GR_LONG_CHUNK + entries + 1;
     p.long_from = fe_gated_recurrence_long_from();
-    p.o_local = scratch;
-    p.qb = p.o_local + (size_t)tokens * heads * dv;
-    p.chunk_state = p.qb + (size_t)tokens * heads * dk;
-    p.chunk_start = p.chunk_state + (size_t)chunk_slots * heads * dk * dv;
-    p.chunk_decay = p.chunk_start + (size_t)chunk_slots * heads * dk * dv;
+    // every part starts on a 16-byte boundary
+    p.chunk_state = scratch;
+    p.within = p.chunk_state + (size_t)chunk_slots * heads * dk * dv;
+    p.qb = p.within + (size_t)chunk_slots * heads * GR_LONG_CHUNK * GR_LONG_CHUNK;
+    p.chunk_decay = p.qb + (size_t)tokens * heads * p.dkp;
   }
   const int threads = (dv * ds + 31) / 32 * 32;
   const size_t smem = sizeof(float) * (size_t)GR_CHUNK * 2 * (dk + dv);
@@ -417,34 +748,27 @@ FE_EXPORT int fe_gated_recurrence(const float* proj, long long ld, int q_off, in
   if (rc || !chunked) return rc ? rc : fe_last_error();
   const int chunks = (max_new + GR_LONG_CHUNK - 1) / GR_LONG_CHUNK;
   if (chunks > 65535) return FE_ERR_TOO_LARGE;
-  const int kpt_built = kpt <= 4 ? 4 : kpt <= 8 ? 8 : kpt <= 16 ? 16 : 32;      // the instantiation's KPT, and its pitch
-  const size_t local_smem = sizeof(float) * ((size_t)GR_CHUNK * (2 * ds * (kpt_built >= 8 ? kpt_built + 4 : kpt_built) + dv) + dk);
-#define GR_LOCAL(KPT)                                                                                                  \
-  do {                                                                                                                 \
-    if (local_smem > 48 * 1024)                                                                                        \
-      cudaFuncSetAttribute(gated_recurrence_local_kernel<KPT>, cudaFuncAttributeMaxDynamicSharedMemorySize,            \
-                           (int)local_smem);                                                                           \
-    rc = fe_launch_dependent(gated_recurrence_local_kernel<KPT>, dim3(heads, entries, chunks), dim3(threads),          \
-                             local_smem, stream, p);                                                                   \
-  } while (0)
-  if (kpt <= 4) GR_LOCAL(4);
-  else if (kpt <= 8) GR_LOCAL(8);
-  else if (kpt <= 16) GR_LOCAL(16);
-  else GR_LOCAL(32);
-#undef GR_LOCAL
+  const size_t chunk_smem = gr_chunk_smem(dk, dv);
+  if (chunk_smem > 48 * 1024)
+    cudaFuncSetAttribute(gated_recurrence_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)chunk_smem);
+  const int v_aligned = ((uintptr_t)proj & 15) == 0 && ld % 4 == 0 && v_off % 4 == 0;
+  const int aligned = v_aligned && q_off % 4 == 0 && f_off % 4 == 0 && dk % 4 == 0 && (((uintptr_t)lower | (uintptr_t)f_bias) & 15) == 0;
+  rc = fe_launch_dependent(gated_recurrence_chunk_kernel, dim3(heads, entries, chunks), dim3(256), chunk_smem, stream, p, aligned);
   if (rc) return rc;
-  rc = fe_launch_dependent(gated_recurrence_scan_kernel, dim3(heads, entries, (dk * dv + 255) / 256), dim3(256), 0, stream,
+  rc = fe_launch_dependent(gated_recurrence_scan_kernel, dim3(heads, entries, (dk * dv + 511) / 512), dim3(128), 0, stream,
                            p, status);
   if (rc) return rc;
-  const size_t finish_smem = gr_finish_smem(dk, dv);
+  const size_t finish_smem = gr_finish_smem(dv);
   if (out_dtype == FE_DTYPE_F32) {
     if (finish_smem > 48 * 1024)
       cudaFuncSetAttribute(gated_recurrence_finish_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)finish_smem);
-    rc = fe_launch_dependent(gated_recurrence_finish_kernel<float>, dim3(heads, entries, chunks), dim3(256), finish_smem, stream, p);
+    rc = fe_launch_dependent(gated_recurrence_finish_kernel<float>, dim3(heads, entries, chunks), dim3(128), finish_smem, stream, p,
+                             v_aligned);
   } else {
     if (finish_smem > 48 * 1024)
       cudaFuncSetAttribute(gated_recurrence_finish_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)finish_smem);
-    rc = fe_launch_dependent(gated_recurrence_finish_kernel<bf16>, dim3(heads, entries, chunks), dim3(256), finish_smem, stream, p);
+    rc = fe_launch_dependent(gated_recurrence_finish_kernel<bf16>, dim3(heads, entries, chunks), dim3(128), finish_smem, stream, p,
+                             v_aligned);
   }
   return rc ? rc : fe_last_error();
 }

@@ -124,3 +124,43 @@ def test_attention_marks_missing_pages_and_keeps_later_infinities_out(native):
     assert attend(holed, list(range(40)), [0, 40])[1] & 2
     assert attend(holed, [30], [0, 1])[1] & 2
     assert attend(table[:, :2].contiguous(), [39], [0, 1])[1] & 2
+
+
+# -- gated recurrence ------------------------------------------------------------------------------
+@pytest.mark.parametrize("heads, dk, dv, lead", ((2, 64, 64, 4), (1, 128, 128, 4), (1, 160, 100, 4), (2, 12, 260, 8), (1, 168, 36, 1), (3, 6, 8, 4)))
+@pytest.mark.parametrize("counts", ([128], [129, 200, 3], [191, 1, 192, 130]))
+def test_gated_recurrence_chunks(native, heads, dk, dv, lead, counts):
+    """One stretch of 128 channels or columns and more, rows that start on 16 bytes and rows that do not,
+    sub-chunks that are whole and that are cut; gates from nearly zero to one, from states that are not zero."""
+    gen = torch.Generator().manual_seed(heads * 100 + dk + dv)
+    qk, v, n = heads * dk, heads * dv, sum(counts)
+    rand = lambda *shape: torch.randn(*shape, generator=gen)  # noqa: E731
+    width = (lead + 2 * qk + v + 3) // 4 * 4
+    proj = rand(n, width)
+    proj[:, lead + qk : lead + 2 * qk] *= 4.0
+    proj[5::7, lead + qk : lead + 2 * qk] = -40.0            # gates at their lower bound
+    lower, bias, norm = torch.rand(qk, generator=gen) * 0.5, rand(qk), 1 + 0.2 * rand(dv)
+    lower[: qk // 2] = 0.0
+    state = rand(len(counts) + 1, heads, dk, dv)
+    cu = [0]
+    for c in counts:
+        cu.append(cu[-1] + c)
+    ints = lambda values: torch.tensor(values, dtype=torch.int32, device=DEV)  # noqa: E731
+    got_state, out, status = state.to(DEV), torch.empty(n, v, device=DEV), status_word()
+    native.gated_recurrence(proj.to(DEV), lead, lead + qk, lead + 2 * qk, bias.to(DEV), lower.to(DEV), norm.to(DEV), 1e-5, got_state,
+                            ints(list(range(len(counts)))), ints(cu), out, len(counts), status, max_new=max(counts))
+    assert int(status.item()) == 0
+    rows = proj.double()
+    q = torch.nn.functional.silu(rows[:, lead : lead + qk]).view(n, heads, dk)
+    f = (lower.double() + (1 - lower.double()) * torch.sigmoid(rows[:, lead + qk : lead + 2 * qk] + bias.double())).view(n, heads, dk)
+    val = rows[:, lead + 2 * qk : lead + 2 * qk + v].view(n, heads, dv)
+    for e in range(len(counts)):
+        s = state[e].double()
+        want = torch.empty(counts[e], heads, dv, dtype=torch.float64)
+        for i, t in enumerate(range(cu[e], cu[e + 1])):
+            s = f[t][:, :, None] * s + (1 - f[t])[:, :, None] * val[t][:, None, :]
+            want[i] = torch.einsum("hdv,hd->hv", s, q[t])
+        want = (want * torch.rsqrt((want * want).mean(-1, keepdim=True) + 1e-5) * norm.double()).reshape(counts[e], v)
+        assert float((out[cu[e] : cu[e + 1]].cpu().double() - want).abs().max()) <= 2e-5 * max(1.0, float(want.abs().max()))
+        assert float((got_state[e].cpu().double() - s).abs().max()) <= 1e-5 * max(1.0, float(s.abs().max()))
+    assert torch.equal(got_state[-1].cpu(), state[-1])       # the row of no entry
