@@ -164,3 +164,39 @@ def test_gated_recurrence_chunks(native, heads, dk, dv, lead, counts):
         assert float((out[cu[e] : cu[e + 1]].cpu().double() - want).abs().max()) <= 2e-5 * max(1.0, float(want.abs().max()))
         assert float((got_state[e].cpu().double() - s).abs().max()) <= 1e-5 * max(1.0, float(s.abs().max()))
     assert torch.equal(got_state[-1].cpu(), state[-1])       # the row of no entry
+
+
+# -- delta rule's inputs ---------------------------------------------------------------------------
+@pytest.mark.parametrize("taps, dk, dv", ((2, 64, 64), (3, 32, 20), (4, 128, 128), (4, 40, 64), (4, 6, 10), (5, 64, 64)))
+@pytest.mark.parametrize("counts", ([256], [1, 2, 3, 270, 1], [100, 100, 57]))
+def test_delta_prepare_of_many_tokens(native, taps, dk, dv, counts):
+    """Runs of tokens that begin and end inside entries, entries shorter than the taps between them."""
+    gen = torch.Generator().manual_seed(taps * 100 + dk)
+    heads, kv, n = 4, 2, sum(counts)
+    channels = 2 * kv * dk + heads * dv
+    rand = lambda *shape: torch.randn(*shape, generator=gen, dtype=torch.float64)  # noqa: E731
+    proj, conv, a_log, dt = rand(n, channels + heads * dv + 2 * heads), rand(channels, taps), rand(heads), rand(heads)
+    state = rand(len(counts) + 1, taps - 1, channels)
+    ints = lambda values: torch.tensor(values, dtype=torch.int32, device=DEV)  # noqa: E731
+    cu = [0]
+    for c in counts:
+        cu.append(cu[-1] + c)
+    want, want_state = torch.empty(n, channels, dtype=torch.float64), state.clone()
+    for e in range(len(counts)):
+        rows = torch.cat([state[e], proj[cu[e] : cu[e + 1], :channels]])
+        y = sum(rows[j : j + counts[e]] * conv[:, j] for j in range(taps))
+        y = y * torch.sigmoid(y)
+        for r in range(2 * kv):
+            part = y[:, r * dk : (r + 1) * dk]
+            part *= torch.rsqrt((part * part).sum(-1, keepdim=True) + 1e-6) * (dk ** -0.5 if r < kv else 1.0)
+        want[cu[e] : cu[e + 1]] = y
+        want_state[e] = rows[counts[e] :]
+    b, a = proj[:, channels + heads * dv : -heads], proj[:, -heads:]
+    want_gates = torch.stack([torch.sigmoid(b), -torch.exp(a_log) * torch.nn.functional.softplus(a + dt)], dim=-1)
+    dev = lambda t: t.float().to(DEV).contiguous()  # noqa: E731
+    out, gates, got_state = torch.empty(n, channels, device=DEV), torch.empty(n, heads, 2, device=DEV), dev(state)
+    native.delta_prepare(dev(proj), channels + heads * dv, channels + heads * dv + heads, dev(conv.T), got_state, ints(list(range(len(counts)))),
+                         ints(cu), ints([e for e, c in enumerate(counts) for _ in range(c)]), dev(a_log), dev(dt), kv, dk, heads, dv, out,
+                         gates, len(counts))
+    for mine, ref in ((out, want), (gates, want_gates), (got_state, want_state)):
+        assert float((mine.cpu() - ref).abs().max()) <= 2e-5 * max(1.0, float(ref.abs().max()))
