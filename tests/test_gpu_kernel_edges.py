@@ -6,7 +6,7 @@ from __future__ import annotations
 import pytest
 import torch
 
-from test_gpu_kernels import dense_attention, paged_layout, status_word
+from test_gpu_kernels import dense_attention, paged_layout, status_word, twin_uniform
 
 pytestmark = pytest.mark.gpu
 
@@ -200,3 +200,44 @@ def test_delta_prepare_of_many_tokens(native, taps, dk, dv, counts):
                          gates, len(counts))
     for mine, ref in ((out, want), (gates, want_gates), (got_state, want_state)):
         assert float((mine.cpu() - ref).abs().max()) <= 2e-5 * max(1.0, float(ref.abs().max()))
+
+
+# -- sampling -------------------------------------------------------------------------------------
+def drawn(row, temperature, top_k, top_p, u):
+    """(index, running sums, target): among equal values top-k keeps the lowest indices and top-p all or none."""
+    x = row.double() / temperature
+    x = x - x.max()
+    keep = torch.ones_like(x, dtype=torch.bool)
+    if top_k:
+        keep[:] = False
+        keep[torch.sort(x, descending=True, stable=True).indices[:top_k]] = True
+    if top_p < 1.0:
+        values, where = torch.unique(x[keep], return_inverse=True)
+        mass = torch.zeros_like(values).index_add_(0, where, torch.exp(x[keep]))
+        above = mass.flip(0).cumsum(0).flip(0) - mass            # of the larger values
+        keep &= x >= values[above <= top_p * mass.sum()].min()
+    weights = torch.where(keep, torch.exp(x), torch.zeros_like(x))
+    running, target = torch.cumsum(weights, 0), u * float(weights.sum())
+    index = int(torch.searchsorted(running, torch.tensor(target, dtype=torch.float64), right=True))
+    return min(index, int(torch.nonzero(weights > 0)[-1])), running, target
+
+
+@pytest.mark.parametrize("rows, vocab", ((1, 4096), (3, 16385), (40, 32768), (64, 151936), (5, 300000), (25, 300000), (2, 700001)))
+@pytest.mark.parametrize("top_k, top_p", ((0, 1.0), (37, 1.0), (0, 0.8), (50, 0.9)))
+def test_sampling_of_long_rows(native, rows, vocab, top_k, top_p):
+    """Slices that are kept in shared memory and slices that are not, rows in one block and in several; ties
+    at the k-th value.  A draw may differ only where its target lies within rounding of a boundary."""
+    gen = torch.Generator().manual_seed(rows + vocab)
+    base = torch.randn(vocab, generator=gen) * 2.0
+    base[torch.randint(0, vocab, (60,), generator=gen)] = 9.0
+    seeds = torch.arange(rows, dtype=torch.int64) * 31 + 3
+    out, status = torch.empty(rows, dtype=torch.int32, device=DEV), status_word()
+    dev = lambda value, dtype: torch.full((rows,), value, dtype=dtype, device=DEV)  # noqa: E731
+    native.sample(base[None].repeat(rows, 1).to(DEV), out, status, temperature=dev(0.8, torch.float32), top_k=dev(top_k, torch.int32),
+                  top_p=dev(top_p, torch.float32), min_p=dev(0.0, torch.float32), seeds=seeds.to(DEV),
+                  counters=torch.zeros(rows, dtype=torch.int64, device=DEV))
+    assert int(status.item()) == 0
+    for r in range(min(rows, 4)):
+        want, running, target = drawn(base, 0.8, top_k, top_p, twin_uniform(int(seeds[r]), 0))
+        if int(out[r]) != want:
+            assert float((running - target).abs().min()) < 1e-5 * float(running[-1]), (r, int(out[r]), want)
