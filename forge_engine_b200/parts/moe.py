@@ -152,13 +152,17 @@ class RoutedMLP(FeedForward):
         return shapes
 
     def tile_rows(self, slots: int) -> int:
-        """Rows of a row tile of the tcgen05 products: few rows per expert (decoding) take
-        the narrow tiles, whose rings are deepest."""
+        """Rows of a row tile of the tcgen05 products: few rows per expert (decoding) take the narrow tiles,
+        whose rings are deepest; more take the tile that most experts fill once, because every further row tile
+        reads the expert's weights again.  Whole layer, 16 experts of 4,864 (of 2,432) at width 2,560, us with
+        tiles of 32 / 64 / 128 rows: 32 rows an expert 261 / 258 / 302 (147 / 154 / 183), 40 rows 282 / 279 / 305
+        (155 / 154 / 184), 75 rows 405 / 309 / 315 (211 / 177 / 188), 87 rows 429 / 359 / 325 (229 / 197 / 190),
+        125 rows 549 / 413 / 371 (285 / 233 / 203)."""
         wish = int(os.environ.get("FORGE_ENGINE_MOE_TILE", "0"))
         if wish in (16, 32, 64, 128):
             return wish
         per_expert = slots / self.experts
-        return 16 if per_expert <= 16 else 32 if per_expert <= 32 else 64 if per_expert <= 96 else 128
+        return 16 if per_expert <= 16 else 32 if per_expert <= 36 else 64 if per_expert <= 80 else 128
 
     def forward(self, x, add=None):
         """``add`` (32-bit [N, width]) is added to the update, in the kernel that sums a token's rows."""
