@@ -310,7 +310,9 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
                       tok0 + (row0 + x * TC5_ROWS) / p.groups, q_full);
     }
     const int pages_per_tile = TC5_KEYS / p.page_size;          // <= 32: a lane per page
-    const int rows_in_cache = p.num_pages * p.nkv * p.page_size;
+    const int page_rows = p.head_cols > 0 ? p.page_size : p.nkv * p.page_size, head_rows = p.head_cols > 0 ? 0 : p.page_size;
+    const int head_col = kvh * p.head_cols;
+    const int rows_in_cache = p.num_pages * page_rows;
     bool ok = true;
     for (int i = 0; i < n_tiles && ok; ++i) {
       const int ks = i % TC5_K_STAGES, vs = i % TC5_V_STAGES;
@@ -319,7 +321,7 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       int row = rows_in_cache;            // outside the tensor: zeros
       if (lane < pages_per_tile && key < key_end) {
         const int page = logical < p.max_pages ? table[logical] : -1;
-        if (page >= 0 && page < p.num_pages) row = (page * p.nkv + kvh) * p.page_size;
+        if (page >= 0 && page < p.num_pages) row = page * page_rows + kvh * head_rows;
         else if (key + p.page_size > key_lo) atomicOr(p.status, FE_STATUS_BAD_PAGE);
       }
       const int offset = lane * p.page_size * 128;
@@ -334,14 +336,14 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       if (lane < pages_per_tile) {
 #pragma unroll
         for (int blk = 0; blk < D / 64; ++blk)
-          tma_load_2d(k_tiles + ks * TC5_KV_BYTES + blk * (TC5_KEYS * 128) + offset, &map_k, blk * 64, row, k_full + ks);
+          tma_load_2d(k_tiles + ks * TC5_KV_BYTES + blk * (TC5_KEYS * 128) + offset, &map_k, head_col + blk * 64, row, k_full + ks);
       }
       // values
       if (lane == 0) mbar_expect_tx(v_full + vs, TC5_KV_BYTES);
       if (lane < pages_per_tile) {
 #pragma unroll
         for (int blk = 0; blk < D / 64; ++blk)
-          tma_load_2d(v_tiles + vs * TC5_KV_BYTES + blk * (TC5_KEYS * 128) + offset, &map_v, blk * 64, row, v_full + vs);
+          tma_load_2d(v_tiles + vs * TC5_KV_BYTES + blk * (TC5_KEYS * 128) + offset, &map_v, head_col + blk * 64, row, v_full + vs);
       }
     }
   } else if (warp == 1) {
@@ -543,9 +545,10 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       const int token = row / p.groups, g = row - token * p.groups;
       if (p.gate != nullptr && p.gate_dim == 0 && row_valid)
         inv *= 1.f / (1.f + expf(-p.gate[(size_t)(tok0 + token) * p.gate_stride + kvh * p.groups + g]));
-      bf16* dst = p.out + ((size_t)(tok0 + token) * num_q_heads + kvh * p.groups + g) * D;
+      const int out_dim = p.out_dim > 0 ? p.out_dim : D;
+      bf16* dst = p.out + ((size_t)(tok0 + token) * num_q_heads + kvh * p.groups + g) * out_dim;
 #pragma unroll 1
-      for (int c = 0; c < D; c += 32) {
+      for (int c = 0; c < out_dim; c += 32) {
         float o[32];
         tc5_ld32(o_addr + c, o);
         if (row_valid) {
@@ -588,6 +591,18 @@ int make_query_map(CUtensorMap* map, const void* q, int q_stride, int tokens, in
   const CUresult r = g_encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(q), dims, strides, box,
                                     elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                                     CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : 20000 + (int)r;
+}
+
+// Tensor map of `rows` rows of `columns` elements, `row_elems` apart.  Box: 64 columns x one key tile.
+int make_rows_map(CUtensorMap* map, const void* base, int columns, int rows, long long row_elems) {
+  if (g_encode_tiled == nullptr) return FE_ERR_BAD_SHAPE;
+  cuuint64_t dims[2] = {(cuuint64_t)columns, (cuuint64_t)rows};
+  cuuint64_t strides[1] = {(cuuint64_t)row_elems * 2};
+  cuuint32_t box[2] = {64u, (cuuint32_t)TC5_KEYS}, elem[2] = {1, 1};
+  const CUresult r = g_encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, elem,
+                                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : 20000 + (int)r;
 }
 

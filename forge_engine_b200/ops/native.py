@@ -110,6 +110,7 @@ def _declare(handle: ctypes.CDLL) -> None:
         "fe_retention_scratch": [i, i, i, i, i, i],
         "fe_rglru": [p, ll, i, i, p, p, i, p, p, i, p, p, p, p, p, p, p, i, p, p, p, p, i, i, i, i, i, i, p, p, p],
         "fe_rglru_scratch": [i, i, i],
+        "fe_latent_rows": [p, i, p, i, i, i, p, i, p, p, p, p],
         "fe_rglru_one_launch": [i, i],
         "fe_gemm_tc5_qkv_rope": [p, p, p, p, i, i, i, p, p, f, p, p, p, p, p, p, i, i, i, i, i, i, p, p],
     }
@@ -200,6 +201,45 @@ def attention_prefill_tc5(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch
              int(window or 0), int(chunk or 0), int(keep_first or 0), float(scale), ptr(gate), gate_stride, d if gate_per_element else 0, int(row_lo),
              ptr(distance_bias), 0 if distance_bias is None else int(distance_bias.shape[1]), float(softcap or 0.0),
              ptr(sinks), ptr(status), stream()), "attention_prefill_tc5")
+
+
+EXPANDED_DIM = 128         # head size of the expanded prefill attention: keys and values are padded to it with zeros
+
+
+def latent_rows(cache: torch.Tensor, block_table: torch.Tensor, where: torch.Tensor, ctx_lens: torch.Tensor, out: torch.Tensor,
+                status: torch.Tensor) -> None:
+    """Rows 128 j .. 128 j + 127 of ``out`` [blocks * 128, width] (bfloat16): the cached vectors at positions
+    where[j, 1].. of entry where[j, 0]; zero before position where[j, 2] and past the entry's ``ctx_lens``.  ``cache`` [pages, 1, page_size, width]."""
+    _dense(cache, "cache"), _dense(block_table, "block_table"), _dense(where, "where"), _dense(out, "out")
+    num_pages, heads, page_size, width = cache.shape
+    assert heads == 1 and cache.dtype == out.dtype == torch.bfloat16 and where.dtype == ctx_lens.dtype == torch.int32
+    assert where.shape[1] == 3 and out.shape == (where.shape[0] * PREFILL_TC5_KEYS, width)
+    check(lib().fe_latent_rows(ptr(cache), width, ptr(block_table), block_table.shape[1], page_size, num_pages, ptr(where),
+                               where.shape[0], ptr(ctx_lens), ptr(out), ptr(status), stream()), "latent_rows")
+
+
+def attention_prefill_expanded(q: torch.Tensor, kv: torch.Tensor, out: torch.Tensor, table: torch.Tensor, cu_tokens: torch.Tensor,
+                               starts: torch.Tensor, n_entries: int, max_new: int, heads: int, out_dim: int, window: int | None,
+                               scale: float, row_lo: int, sinks: torch.Tensor | None, status: torch.Tensor) -> None:
+    """The tcgen05 prefill attention over keys and values expanded for this step: ``q`` [N, heads * 128], ``kv``
+    [rows, 2 * heads * 128] (a token's keys of all heads, then its values; padded with zeros), ``table`` [entries, L]:
+    which stretch of 128 rows holds positions 128 j .. of an entry (-1: none).  ``out`` [N, heads * out_dim] is written
+    for entries of more than ``row_lo`` new tokens."""
+    _dense(q, "q"), _dense(kv, "kv"), _dense(out, "out"), _dense(table, "table")
+    d = EXPANDED_DIM
+    n, rows = q.shape[0], kv.shape[0]
+    assert q.dtype == kv.dtype == out.dtype == torch.bfloat16 and table.dtype == torch.int32
+    assert q.shape[1] == heads * d and kv.shape[1] == 2 * heads * d and rows % PREFILL_TC5_KEYS == 0 and out.shape == (n, heads * out_dim)
+    assert sinks is None or (sinks.dtype == torch.float32 and sinks.is_cuda and sinks.is_contiguous() and sinks.numel() == heads)
+    fn = getattr(_attention_handle(d), f"fe_attention_prefill_expanded_d{d}")
+    if not getattr(fn, "_declared", False):
+        p, i, f, ll = c_void_p, c_int, c_float, ctypes.c_longlong
+        fn.argtypes = [p, i, p, i, p, p, ll, p, i, i, i, p, p, i, i, i, i, f, i, p, p, p]
+        fn.restype = c_int
+        fn._declared = True
+    check(fn(ptr(q), heads * d, ptr(out), int(out_dim), ptr(kv), ptr(kv) + heads * d * 2, 2 * heads * d, ptr(table), table.shape[1],
+             rows // PREFILL_TC5_KEYS, heads, ptr(cu_tokens), ptr(starts), int(n_entries), int(max_new), n, int(window or 0),
+             float(scale), int(row_lo), ptr(sinks), ptr(status), stream()), "attention_prefill_expanded")
 
 
 def _attention_handle(head_dim: int):

@@ -7,11 +7,16 @@ RMS-normalised, are the latent c, the last rot_dim, rotated, are a key part that
 share.  Head h's key is [W_uk,h c | shared part], its value W_uv,h c.  Only c and the shared
 part are kept in the cache: one vector of kv_rank + rot_dim per token for all heads.
 
-The expansion is never carried out for cached tokens.  Since q_h . (W_uk,h c) =
+In decoding and short portions the expansion is never carried out.  Since q_h . (W_uk,h c) =
 (W_uk,h^T q_h) . c, the step's queries are taken through W_uk,h^T once (kv_rank numbers per
 head), attention then runs with one shared "kv head" whose key is the cached vector itself
 and whose value is its first kv_rank elements, and the weighted sum of latents is expanded by
 W_uv,h afterwards.  A step's cost does not depend on how many heads read the cache.
+
+For a long prompt portion that is the dearer way: a query against a key then takes 2 kv_rank + rot_dim
+multiply-adds per head instead of head_dim + rot_dim + v_head_dim.  There the portion's context is taken
+out of its pages, expanded for all heads by one product (the shared part rides along through an identity
+block) and read by the tcgen05 prefill kernel, keys and values padded to 128.
 
 A layer with ``kv_from`` has no W_dkv and reads the cache of the layer named there.
 
@@ -22,6 +27,8 @@ the softmax's denominator once, as a weight on no key and no value.
 
 from __future__ import annotations
 
+import os
+
 import torch
 
 from ..cache.manager import CacheNeeds, PagedKVSpec
@@ -29,6 +36,15 @@ from ..config.specs import local_name
 from ..ops import native
 from .base import BuildContext, CacheView, Mixer, WeightInfo, build_part, register_part
 from .linear import Linear, fused_rows
+
+
+# Portions of more than EXPAND_FROM tokens are expanded, in steps of more than EXPAND_STEP tokens.  Which
+# rows of a step's expansion belong to whom depends on every entry's length, so such a step could not be
+# replayed for another one: the line is the most tokens a replayed step has (engine/graphs.py).  1,500
+# tokens after 500 (32 heads, 64 + 32 / 64, rank 256): 464 us in the absorbed form, 65 us with the
+# expansion; 128 tokens are where a head's 128-row tile is full.
+EXPAND_FROM = 128
+EXPAND_STEP = max(512, int(os.environ.get("FORGE_ENGINE_GRAPH_TOKENS", "512")))
 
 
 class LatentAttention(Mixer):
@@ -62,15 +78,80 @@ class LatentAttention(Mixer):
         if getattr(spec, "sink", False):
             self.sinks = weights[name("sink")].to(device=ctx.device, dtype=torch.float32).contiguous()
         self.plan_key = ("latent_attention", self.h, self.kv_rank, self.r, self.window)
+        self.expanded = None
+        wide = native.EXPANDED_DIM
+        # the expanded form: both sizes fit the kernel's head, outputs are stored 32 at a time
+        if (self.d + self.r <= wide and self.dv <= wide and self.dv % 32 == 0 and spec.scale > 0 and (self.kv_rank + self.r) % 8 == 0
+                and native.general_mma_takes(ctx.dtype, self.kv_rank + self.r, self.kv_rank)
+                and all(t.dtype == torch.bfloat16 for t in (self.up_q.weight, self.uk_t, self.uv))):
+            # [2 heads x 128, kv_rank + rot_dim]: a head's key rows (expansion, then the identity on the
+            # shared part), then its value rows; rows of zeros pad both to 128
+            both = torch.zeros((2, self.h, wide, self.kv_rank + self.r), dtype=torch.bfloat16, device=self.uv.device)
+            both[0, :, : self.d, : self.kv_rank] = self.uk_t.transpose(1, 2)
+            both[0, :, self.d : self.d + self.r, self.kv_rank :] = torch.eye(self.r, dtype=torch.bfloat16, device=self.uv.device)
+            both[1, :, : self.dv, : self.kv_rank] = self.uv
+            queries = torch.zeros((self.h, wide, self.q_rank), dtype=torch.bfloat16, device=self.uv.device)
+            queries[:, : self.d + self.r] = self.up_q.weight.view(self.h, self.d + self.r, self.q_rank)
+            self.expanded = (Linear(both.view(2 * self.h * wide, -1), status=ctx.status),
+                             Linear(queries.view(self.h * wide, -1), status=ctx.status))
 
     def plan_step(self, entries: list, page_size: int, plans: dict) -> None:
-        """The host's decision for a step of ``entries`` ((slot, cached, new) each): how many
-        blocks share the keys of one tile of query rows (layers of one geometry share it)."""
+        """The host's decision for a step of ``entries`` ((slot, cached, new) each; layers of one
+        geometry share it): how many blocks share the keys of one tile of query rows (None: no entry
+        takes the absorbed form), and (cached, new) of the entries if some are expanded."""
         if self.plan_key not in plans:
-            splits = 1
-            if native.general_mma_takes(self.ctx.dtype, self.kv_rank + self.r, self.kv_rank):
-                splits = native.general_splits(entries, self.h, 1, self.window)
-            plans[self.plan_key] = splits
+            short, expanded = list(entries), None
+            if self.expanded is not None and sum(count for _, _, count in entries) > EXPAND_STEP:
+                short = [e for e in entries if e[2] <= EXPAND_FROM]
+                if len(short) < len(entries):
+                    expanded = tuple((start, count) for _, start, count in entries)
+            splits = 1 if short else None
+            if short and native.general_mma_takes(self.ctx.dtype, self.kv_rank + self.r, self.kv_rank):
+                splits = native.general_splits(short, self.h, 1, self.window)
+            plans[self.plan_key] = (splits, expanded)
+
+    def _stretches(self, spans: tuple, batch):
+        """Where the expanded entries' contexts lie in the step's expansion, worked out once a step: int32 on
+        the device, (entry, first position, first position needed) per stretch of 128 rows and [entries, L]
+        the stretch of positions 128 j .. (-1: none)."""
+        key = (self.plan_key, "stretches")
+        if key not in batch.shared:
+            size = native.PREFILL_TC5_KEYS
+            where, tables = [], []
+            for entry, (start, count) in enumerate(spans):
+                row = []
+                if count > EXPAND_FROM:
+                    needed = max(0, start - self.window + 1) if self.window else 0
+                    first = needed // size
+                    last = -(-(start + count) // size)
+                    row = [-1] * first + [len(where) + j for j in range(last - first)]
+                    where += [(entry, size * j, needed) for j in range(first, last)]
+                tables.append(row)
+            width = max(len(row) for row in tables)
+            flat = [v for stretch in where for v in stretch] + [v for row in tables for v in row + [-1] * (width - len(row))]
+            device = torch.tensor(flat, dtype=torch.int32).pin_memory().to(self.ctx.device, non_blocking=True)
+            batch.shared[key] = device[: 3 * len(where)].view(-1, 3), device[3 * len(where) :].view(len(spans), width)
+        return batch.shared[key]
+
+    def _attend_expanded(self, c_q, spans: tuple, batch, latent_cache, table, angles, heads) -> None:
+        """The expanded entries' rows of ``heads`` [N, heads * v_head_dim]."""
+        n, h, d, r, wide = c_q.shape[0], self.h, self.d, self.r, native.EXPANDED_DIM
+        expand, up_q = self.expanded
+        with self.ctx.section("mixer.qkv_rope_cache"):
+            q = up_q(c_q)
+            native.qkv_prepare(
+                q=q[:, d:], q_heads=h, q_dim=r, q_head_stride=wide, q_rot_off=0,
+                q_out=q, q_out_strides=(h * wide, wide), q_out_offset=d,
+                table=angles, rot_dims=self.rot_dims, interleaved=self.position.interleaved,
+                positions=batch.positions, token_entry=batch.token_entry, status=self.ctx.status,
+            )
+            where, stretches = self._stretches(spans, batch)
+            rows = torch.empty((where.shape[0] * native.PREFILL_TC5_KEYS, self.kv_rank + r), dtype=torch.bfloat16, device=c_q.device)
+            native.latent_rows(latent_cache, table, where, batch.ctx_lens, rows, self.ctx.status)
+            kv = expand(rows)
+        with self.ctx.section("mixer.attention"):
+            native.attention_prefill_expanded(q, kv, heads, stretches, batch.cu_tokens, batch.starts, batch.n_entries, batch.max_new,
+                                              h, self.dv, self.window, self.spec.scale, EXPAND_FROM, self.sinks, self.ctx.status)
 
     @classmethod
     def weight_shapes(cls, spec) -> dict:
@@ -130,8 +211,23 @@ class LatentAttention(Mixer):
                 k_cache=latent_cache, block_table=table, positions=batch.positions, token_entry=batch.token_entry,
                 status=self.ctx.status,
             )
+        heads = torch.empty((n, h, dv), dtype=dtype, device=x.device)
+        if self.plan_key not in batch.plans:
+            self.plan_step(batch.entries, latent_cache.shape[2], batch.plans)
+        splits, expanded = batch.plans[self.plan_key]
+        if splits is not None:
+            self._attend_absorbed(c_q, splits, expanded is not None, batch, latent_cache, table, angles, heads)
+        if expanded is not None:
+            self._attend_expanded(c_q, expanded, batch, latent_cache, table, angles, heads.view(n, h * dv))
+        return heads.view(n, h * dv)
+
+    def _attend_absorbed(self, c_q, splits: int, some_expanded: bool, batch, latent_cache, table, angles, heads) -> None:
+        """All rows of ``heads`` [N, heads, v_head_dim], or with ``some_expanded`` those of the other entries
+        (and anything in theirs)."""
+        n, h, d, r, rank = c_q.shape[0], self.h, self.d, self.r, self.kv_rank
+        with self.ctx.section("mixer.qkv_rope_cache"):
             q = self.up_q(c_q)                                     # [N, heads * (d + r)]
-            q_eff = torch.empty((n, h, rank + r), dtype=dtype, device=x.device)
+            q_eff = torch.empty((n, h, rank + r), dtype=c_q.dtype, device=c_q.device)
             # rotated parts of the queries straight to where attention reads them
             native.qkv_prepare(
                 q=q[:, d:], q_heads=h, q_dim=r, q_head_stride=d + r, q_rot_off=0,
@@ -141,19 +237,15 @@ class LatentAttention(Mixer):
             )
             # the other parts through the transposed key expansion
             self._per_head(q.view(n, h, d + r)[:, :, :d], self.uk_t, q_eff[:, :, :rank])
-        mixed = torch.empty((n, h, rank), dtype=dtype, device=x.device)
-        if self.plan_key not in batch.plans:
-            self.plan_step(batch.entries, latent_cache.shape[2], batch.plans)
+        mixed = torch.empty((n, h, rank), dtype=c_q.dtype, device=c_q.device)
         with self.ctx.section("mixer.attention"):
             native.attention_general(q_eff, (h * (rank + r), rank + r), latent_cache, rank + r, latent_cache, rank,
                                      mixed, (h * rank, rank), table, batch.positions, batch.token_entry, h, None, self.window,
                                      self.spec.scale, self.ctx.status,
                                      entries=(batch.cu_tokens, batch.starts, batch.n_entries, batch.max_new),
-                                     splits=batch.plans[self.plan_key], sinks=self.sinks)
-        heads = torch.empty((n, h, dv), dtype=dtype, device=x.device)
+                                     splits=splits, sinks=self.sinks, row_hi=EXPAND_FROM * h if some_expanded else 0)
         with self.ctx.section("mixer.expand"):
             self._per_head(mixed, self.uv, heads)
-        return heads.view(n, h * dv)
 
 
 register_part("latent_attention", LatentAttention, replace=True)

@@ -241,3 +241,86 @@ def test_sampling_of_long_rows(native, rows, vocab, top_k, top_p):
         want, running, target = drawn(base, 0.8, top_k, top_p, twin_uniform(int(seeds[r]), 0))
         if int(out[r]) != want:
             assert float((running - target).abs().min()) < 1e-5 * float(running[-1]), (r, int(out[r]), want)
+
+
+# -- attention over cached latents -------------------------------------------------------------------
+@pytest.mark.parametrize("window, sink", ((None, False), (200, True), (40, False)))
+@pytest.mark.parametrize("heads, dim, rot, vdim, rank", ((3, 64, 32, 64, 64), (2, 96, 32, 128, 48), (4, 16, 16, 32, 32)))
+def test_expanded_latent_attention(native, monkeypatch, window, sink, heads, dim, rot, vdim, rank):
+    """Portions of 129 tokens and more beside shorter ones, keys and values expanded, against the absorbed form
+    of the same layer and against 64 bits."""
+    import dataclasses
+
+    from forge_engine_b200.config.registry import read_model_config
+    from forge_engine_b200.engine import ModelRunner, StepEntry
+    from forge_engine_b200.engine.batch import build_batch
+    from forge_engine_b200.parts import latent_attention as part
+
+    width, q_rank = 128, 64
+    raw = {"architecture": "Zofadra", "vocab": 32, "width": width, "norm": {"eps": 1e-5}, "layers": [{"type": "latent_attention", "mixer": {
+        "heads": heads, "dim": dim, "rot_dim": rot, "vdim": vdim, "q_rank": q_rank, "kv_rank": rank,
+        "rot": {"base": 1e4, "dims": rot}, "scale": (dim + rot) ** -0.5}}]}
+    arch, _, spec = read_model_config(raw)
+    layer = spec.layers[0]
+    spec = dataclasses.replace(spec, layers=(dataclasses.replace(layer, mixer=dataclasses.replace(layer.mixer, window=window, sink=sink)),))
+    gen = torch.Generator().manual_seed(heads + dim)
+    weights = {name: ((1 + 0.1 * torch.randn(info.shape, generator=gen)) if "norm" in name else
+                      torch.randn(info.shape, generator=gen) * (info.shape[-1] ** -0.5 if len(info.shape) > 1 else 1.0)).bfloat16().to(DEV)
+               for name, info in arch.expected_tensors(spec).items()}
+    counts, starts = [130, 5, 257, 1, 400], [0, 60, 37, 9, 250]
+    x = torch.randn((sum(counts), width), generator=gen).bfloat16().to(DEV)
+    before = torch.randn((max(starts), rank + rot), generator=gen).bfloat16().to(DEV)
+    results = {}
+    for name, step in (("expanded", 512), ("absorbed", 1 << 30)):
+        monkeypatch.setattr(part, "EXPAND_STEP", step)
+        runner = ModelRunner.from_tensors(spec, dict(weights), dtype="bfloat16", device=DEV, page_size=16, num_pages=128, max_requests=6,
+                                          architecture=arch)
+        cache = runner.cache
+        for i, start in enumerate(starts):
+            runner.begin(i)
+            if start:
+                cache.reserve(i, start)
+                cache.advance(i, start)
+                pages = cache.request(i).tables[0].pages
+                for p in range(start):
+                    if pages[p // 16] >= 0:
+                        cache.kv_of_run(0)[0][pages[p // 16], 0, p % 16] = before[p]
+        entries = [StepEntry(i, [0] * c) for i, c in enumerate(counts)]
+        for i, (start, count) in enumerate(zip(starts, counts)):
+            cache.reserve(i, start + count)
+        batch = build_batch(entries, cache, DEV)
+        results[name] = runner.model.blocks[0].mixer.attend(x, batch, cache.view(0)).clone()
+        assert batch.plans[runner.model.blocks[0].mixer.plan_key][1] == (tuple(zip(starts, counts)) if name == "expanded" else None)
+        runner.check_status()
+    w = {k.split(".mix.")[-1]: v.double().cpu() for k, v in weights.items()}
+    rms = lambda t, g: t * torch.rsqrt((t * t).mean(-1, keepdim=True) + 1e-5) * g  # noqa: E731
+
+    def turned(t, positions):
+        angle = positions.double()[:, None] * 1e4 ** (-torch.arange(0, rot, 2, dtype=torch.float64) / rot)
+        cos, sin = torch.cos(angle), torch.sin(angle)
+        if t.dim() == 3:
+            cos, sin = cos[:, None], sin[:, None]
+        a, b = t[..., 0::2], t[..., 1::2]
+        return torch.stack((a * cos - b * sin, b * cos + a * sin), dim=-1).flatten(-2)
+
+    at = 0
+    for start, count in zip(starts, counts):
+        h = x[at : at + count].double().cpu()
+        positions = torch.arange(start, start + count)
+        q = (rms(h @ w["dq"].T, w["dq.norm"]) @ w["uq"].T).view(count, heads, dim + rot)
+        q = torch.cat((q[..., :dim], turned(q[..., dim:], positions)), dim=-1)
+        both = h @ w["dkv"].T
+        own = torch.cat((rms(both[:, :rank], w["dkv.norm"]), turned(both[:, rank:], positions)), dim=-1)
+        latents = torch.cat((before[:start].double().cpu(), own))
+        keys = torch.cat(((latents[:, :rank] @ w["uk"].T).view(-1, heads, dim), latents[:, None, rank:].expand(-1, heads, -1)), dim=-1)
+        values = (latents[:, :rank] @ w["uv"].T).view(-1, heads, vdim)
+        scores = torch.einsum("thd,shd->hts", q, keys) * (dim + rot) ** -0.5
+        distance = positions[:, None] - torch.arange(start + count)[None, :]
+        hidden = (distance < 0) | ((distance >= window) if window else torch.zeros_like(distance, dtype=torch.bool))
+        e = torch.exp(scores.masked_fill(hidden, float("-inf")))
+        total = e.sum(-1, keepdim=True) + (torch.exp(w["sink"])[:, None, None] if sink else 0.0)
+        want = torch.einsum("hts,shd->thd", e / total, values).reshape(count, -1)
+        for name, got in results.items():
+            off = float((got[at : at + count].double().cpu() - want).norm() / want.norm())
+            assert off < 1e-2, (name, start, count, off)
+        at += count
