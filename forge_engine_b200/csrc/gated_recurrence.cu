@@ -35,9 +35,11 @@
 //   then the head's norm and the store.
 // All factors are products of gates: there is no division by a decay anywhere (a gate may be as small
 // as its lower bound allows), and everything stays 32-bit; against the token-by-token walk only the order
-// of additions differs.  What a token costs is 2 dk dv multiply-adds as register tiles of 4 x 4 to 8 x 8
-// (the walk takes five operations per state element and reads two operands of each from shared memory).
-#include "common.cuh"
+// of additions differs.  What a token costs is 2 dk dv multiply-adds (the walk takes five operations per state
+// element and reads two operands of each from shared memory); the products run on the tensor cores with
+// both operands split (mma_split.cuh), because the multiply-add units are bound by what shared memory
+// delivers to them long before their own rate.
+#include "mma_split.cuh"
 
 #define GR_CHUNK 16
 #define GR_MAX_KPT 32
@@ -75,7 +77,10 @@ __device__ __forceinline__ void gr_copy16(void* dst, const void* src, bool valid
                ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(valid ? 16 : 0) : "memory");
 }
 __device__ __forceinline__ void gr_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void gr_wait_one() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
+template <int PENDING>
+__device__ __forceinline__ void gr_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory"); }
+__device__ __forceinline__ void gr_store2(float* p, float a, float b) { *reinterpret_cast<float2*>(p) = make_float2(a, b); }
+__device__ __forceinline__ void gr_store2(bf16* p, float a, float b) { *reinterpret_cast<__nv_bfloat162*>(p) = __floats2bfloat162_rn(a, b); }
 __device__ __forceinline__ float gr_sigmoid(float x) { return 1.f / (1.f + expf(-x)); }
 
 template <typename TO, int KPT>
@@ -174,14 +179,6 @@ __device__ __forceinline__ float gr_sum16(float (&x)[16], int lane) {
   return x[0] + __shfl_xor_sync(0xffffffffu, x[0], 1);
 }
 
-__device__ __forceinline__ void gr_outer(float (&acc)[4][4], const float4 a, const float4 b) {
-  const float x[4] = {a.x, a.y, a.z, a.w}, y[4] = {b.x, b.y, b.z, b.w};
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(x[i], y[j], acc[i][j]);
-}
-
 // One chunk of a long entry (see the head of this file).  Tokens past the entry's end have f = 1 and
 // q = k = v = 0.
 __global__ void __launch_bounds__(256, 2) gated_recurrence_chunk_kernel(GatedRecurrence p, int aligned) {
@@ -193,7 +190,8 @@ __global__ void __launch_bounds__(256, 2) gated_recurrence_chunk_kernel(GatedRec
   if (entry_count < p.long_from || chunk * GR_LONG_CHUNK >= entry_count) return;
   const int first = entry_first + chunk * GR_LONG_CHUNK, count = min(GR_LONG_CHUNK, entry_count - chunk * GR_LONG_CHUNK);
   const int dk = p.dk, dv = p.dv;
-  const int dp = min(p.dkp, GR_SLICE) + 4, vp = min(dv, GR_SLICE) + 4;   // pitches: rows of 16 bytes in different banks
+  // pitches: a fragment's rows (q, k) and its columns (v) fall into different banks
+  const int dp = min(p.dkp, GR_SLICE) + 4, vp = min(dv, GR_SLICE) + 8;
   float* fs = smem;                              // [64][dp]: gates, then what is left of k
   float* qs = fs + GR_LONG_CHUNK * dp;           // [64][dp]; when q is done, vs [64][vp]
   float* vs = qs;
@@ -206,6 +204,8 @@ __global__ void __launch_bounds__(256, 2) gated_recurrence_chunk_kernel(GatedRec
   for (int d0 = 0; d0 < dk; d0 += GR_SLICE) {
     const int nd = min(GR_SLICE, dk - d0), ndp = (nd + 3) & ~3;
     __syncthreads();
+    // four channels behind the last are read as part of a fragment
+    for (int i = tid; i < GR_LONG_CHUNK * 4; i += 256) fs[(i >> 2) * dp + ndp + (i & 3)] = qs[(i >> 2) * dp + ndp + (i & 3)] = 0.f;
     if (aligned) {
       // four channels a thread, all loads of four rows on their way before the first is used
       const int quads = ndp >> 2, step = 256 / 32;      // a warp takes a row (up to 32 quads)
@@ -316,31 +316,27 @@ __global__ void __launch_bounds__(256, 2) gated_recurrence_chunk_kernel(GatedRec
       }
     }
     __syncthreads();
-    // sub-chunks `apart` apart: A's blocks of 16 x 16, 64 threads each; q then takes the gates of the
+    // sub-chunks `apart` apart: A's blocks of 16 x 16, two warps each; q then takes the gates of the
     // sub-chunk it has just been multiplied with
+    const int fg = lane >> 2, fq = lane & 3;           // this lane's row and column in a fragment
 #pragma unroll 1
     for (int apart = 1; apart < GR_SUBS; ++apart) {
-      const int block = tid >> 6;
+      const int block = warp >> 1, side = (warp & 1) * 8;
       if (block < GR_SUBS - apart) {
-        const int r = (tid & 63) >> 3, c = tid & 7;
-        const float* q0 = qs + ((apart + block) * GR_SUB + r) * dp;
-        const float* k0 = fs + (block * GR_SUB + c) * dp;
-        float sum[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+        const float* q0 = qs + ((apart + block) * GR_SUB + fg) * dp + fq;
+        const float* k0 = fs + (block * GR_SUB + side + fg) * dp + fq;
+        float sum[4] = {0.f, 0.f, 0.f, 0.f}, small[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 4
-        for (int d = 0; d < ndp; d += 4) {
-          float a[2][4], b[2][4];
-          load4(q0 + d, a[0]), load4(q0 + 8 * dp + d, a[1]), load4(k0 + d, b[0]), load4(k0 + 8 * dp + d, b[1]);
-#pragma unroll
-          for (int e = 0; e < 4; ++e)
-#pragma unroll
-            for (int i = 0; i < 2; ++i)
-#pragma unroll
-              for (int j = 0; j < 2; ++j) sum[i][j] = fmaf(a[i][e], b[j][e], sum[i][j]);
+        for (int d = 0; d < ndp; d += 8) {
+          SplitA fa;
+          SplitB fb;
+          split_load_a(fa, q0 + d, dp, 1);
+          split_load_b(fb, k0 + d, 1);
+          split_mma(sum, small, fa, fb);
         }
 #pragma unroll
-        for (int i = 0; i < 2; ++i)
-#pragma unroll
-          for (int j = 0; j < 2; ++j) as[((apart + block) * GR_SUB + r + 8 * i) * GR_AP + block * GR_SUB + c + 8 * j] += sum[i][j];
+        for (int i = 0; i < 4; ++i)
+          as[((apart + block) * GR_SUB + fg + 8 * (i >> 1)) * GR_AP + block * GR_SUB + side + 2 * fq + (i & 1)] += sum[i] + small[i];
       }
       __syncthreads();
       if (lane * 4 < ndp) {
@@ -377,7 +373,6 @@ __global__ void __launch_bounds__(256, 2) gated_recurrence_chunk_kernel(GatedRec
       p.chunk_decay[at * dk + d0 + d] = b;
     }
     // the chunk's own end state
-    const int ty = tid >> 4, tx = tid & 15;
     for (int v0 = 0; v0 < dv; v0 += GR_SLICE) {
       const int nv = min(GR_SLICE, dv - v0);
       __syncthreads();
@@ -403,57 +398,45 @@ __global__ void __launch_bounds__(256, 2) gated_recurrence_chunk_kernel(GatedRec
         }
       }
       __syncthreads();
-      const bool d_lo = ty * 4 < ndp, d_hi = ty * 4 + 64 < ndp, v_lo = tx * 4 < nv, v_hi = tx * 4 + 64 < nv;
-      float acc[2][2][4][4];
+      // a warp takes 32 channels and 32 columns at a time
+      const int m0 = (warp >> 1) * 32;
+      for (int c0 = (warp & 1) * 32; c0 < nv && m0 < ndp; c0 += 64) {
+        float sum[2][4][4], small[2][4][4];
 #pragma unroll
-      for (int a = 0; a < 2; ++a)
+        for (int a = 0; a < 2; ++a)
 #pragma unroll
-        for (int b = 0; b < 2; ++b)
+          for (int b = 0; b < 4; ++b)
 #pragma unroll
-          for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) acc[a][b][i][j] = 0.f;
-      const float* kd = fs + ty * 4;
-      const float* vd = vs + tx * 4;
-      const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (ndp > 64 && nv > 64) {
+            for (int i = 0; i < 4; ++i) sum[a][b][i] = small[a][b][i] = 0.f;
+        const float* ka = fs + fq * dp + m0 + fg;
+        const float* vb = vs + fq * vp + c0 + fg;
 #pragma unroll 2
-        for (int s = 0; s < GR_LONG_CHUNK; ++s) {
-          const float4 k0 = *reinterpret_cast<const float4*>(kd + s * dp), k1 = d_hi ? *reinterpret_cast<const float4*>(kd + s * dp + 64) : zero;
-          const float4 x0 = *reinterpret_cast<const float4*>(vd + s * vp), x1 = v_hi ? *reinterpret_cast<const float4*>(vd + s * vp + 64) : zero;
-          gr_outer(acc[0][0], k0, x0);
-          gr_outer(acc[0][1], k0, x1);
-          gr_outer(acc[1][0], k1, x0);
-          gr_outer(acc[1][1], k1, x1);
+        for (int t = 0; t < GR_LONG_CHUNK; t += 8) {
+          SplitA fa[2];
+          split_load_a(fa[0], ka + t * dp, 1, dp);
+          split_load_a(fa[1], ka + t * dp + 16, 1, dp);
+#pragma unroll
+          for (int b = 0; b < 4; ++b) {
+            SplitB fb;
+            split_load_b(fb, vb + t * vp + 8 * b, vp);
+            split_mma(sum[0][b], small[0][b], fa[0], fb);
+            split_mma(sum[1][b], small[1][b], fa[1], fb);
+          }
         }
-      } else if (ndp > 64) {
-#pragma unroll 2
-        for (int s = 0; s < GR_LONG_CHUNK; ++s) {
-          const float4 k0 = *reinterpret_cast<const float4*>(kd + s * dp), k1 = d_hi ? *reinterpret_cast<const float4*>(kd + s * dp + 64) : zero;
-          const float4 x0 = v_lo ? *reinterpret_cast<const float4*>(vd + s * vp) : zero;
-          gr_outer(acc[0][0], k0, x0);
-          gr_outer(acc[1][0], k1, x0);
-        }
-      } else {
-#pragma unroll 2
-        for (int s = 0; s < GR_LONG_CHUNK; ++s) {
-          const float4 k0 = d_lo ? *reinterpret_cast<const float4*>(kd + s * dp) : zero;
-          const float4 x0 = v_lo ? *reinterpret_cast<const float4*>(vd + s * vp) : zero, x1 = v_hi ? *reinterpret_cast<const float4*>(vd + s * vp + 64) : zero;
-          gr_outer(acc[0][0], k0, x0);
-          gr_outer(acc[0][1], k0, x1);
-        }
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int d = m0 + 16 * a + 8 * h + fg;
+            if (d >= nd) continue;
+            float* dst = p.chunk_state + (at * dk + d0 + d) * dv + v0;
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+              const int c = c0 + 8 * b + 2 * fq;
+              if (c < nv) *reinterpret_cast<float2*>(dst + c) = make_float2(sum[a][b][2 * h] + small[a][b][2 * h], sum[a][b][2 * h + 1] + small[a][b][2 * h + 1]);
+            }
+          }
       }
-#pragma unroll
-      for (int a = 0; a < 2; ++a)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int d = ty * 4 + 64 * a + i;
-          if (d >= nd) continue;
-          float* dst = p.chunk_state + (at * dk + d0 + d) * dv + v0;
-#pragma unroll
-          for (int b = 0; b < 2; ++b)
-            if (tx * 4 + 64 * b < nv) store4(dst + tx * 4 + 64 * b, acc[a][b][i]);
-        }
     }
   }
   __syncthreads();
@@ -511,14 +494,17 @@ __global__ void __launch_bounds__(128) gated_recurrence_scan_kernel(GatedRecurre
 }
 
 // o = [q D | A] [S_start; V] for the 64 tokens of a chunk, then the head's norm.  Both operands pass
-// through shared memory in stretches of 32 rows of the right one; thread (ty, tx) of 8 x 16 keeps tokens
-// ty, ty + 8, .. of the columns 4 tx .. and 64 + 4 tx .. of a pass of 128 columns (dv is a multiple of 4).
-// Where dv takes more than one pass the rows wait in shared memory for the norm.
+// through shared memory in stretches of 32 rows of the right one; a warp takes 32 tokens and 32 columns of a
+// pass of 128 columns (dv is a multiple of 4).  Where dv takes more than one pass the rows wait in shared
+// memory for the norm.
 #define GR_FK 32
 #define GR_FX (GR_FK + 4)
+__host__ __device__ static inline int gr_finish_pitch(int dv) { return ((dv < GR_SLICE ? dv : GR_SLICE) + 31) / 32 * 32 + 8; }
+__host__ __device__ static inline int gr_finish_stages(int dv) { return dv <= GR_SLICE ? 3 : 2; }
 template <typename TO>
-__global__ void __launch_bounds__(128, 2) gated_recurrence_finish_kernel(GatedRecurrence p, int v_aligned) {
+__global__ void __launch_bounds__(256, 2) gated_recurrence_finish_kernel(GatedRecurrence p, int v_aligned) {
   extern __shared__ __align__(16) float smem[];
+  __shared__ float part[4][GR_LONG_CHUNK];
   pdl_trigger();
   pdl_wait();
   const int head = blockIdx.x, entry = blockIdx.y, chunk = blockIdx.z;
@@ -526,134 +512,136 @@ __global__ void __launch_bounds__(128, 2) gated_recurrence_finish_kernel(GatedRe
   if (entry_count < p.long_from || chunk * GR_LONG_CHUNK >= entry_count) return;
   const int first = entry_first + chunk * GR_LONG_CHUNK, count = min(GR_LONG_CHUNK, entry_count - chunk * GR_LONG_CHUNK);
   const int dk = p.dk, dv = p.dv;
-  const int wide = min(dv, GR_SLICE);
-  const int stage_floats = GR_LONG_CHUNK * GR_FX + GR_FK * wide;
-  float* os = smem + 2 * stage_floats;          // [64][dv], only where dv > 128
-  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+  const int pitch = gr_finish_pitch(dv), stages = gr_finish_stages(dv);
+  const int stage_floats = GR_LONG_CHUNK * GR_FX + GR_FK * pitch;
+  float* os = smem + stages * stage_floats;          // [64][dv], only where dv > 128
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, fg = lane >> 2, fq = lane & 3;
+  const int m0 = (warp >> 2) * 32, n0 = (warp & 3) * 32;
   const size_t at = (size_t)gr_chunk_slot(entry_first, entry, chunk) * p.heads + head;
-  const float* qb = p.qb + ((size_t)first * p.heads + head) * p.dkp;
-  const float* within = p.within + at * GR_LONG_CHUNK * GR_LONG_CHUNK;
   const float* start = p.chunk_state + at * dk * dv;
   const float* values = p.proj + (size_t)first * p.ld + p.v_off + (size_t)head * dv;
   const int q_steps = (p.dkp + GR_FK - 1) / GR_FK, steps = q_steps + (count + GR_FK - 1) / GR_FK;
+  // what this thread copies of a stretch: eight numbers of a row of the left operand, every eighth four of a row
+  // of the right one
+  const int xt = tid >> 2, xk = (tid & 3) * 8, yk = tid >> 3, yc = (tid & 7) * 4;
+  const bool row = xt < count;
+  const float* x_q = p.qb + ((size_t)(first + (row ? xt : 0)) * p.heads + head) * p.dkp + xk;
+  const float* x_a = p.within + at * GR_LONG_CHUNK * GR_LONG_CHUNK + xt * GR_LONG_CHUNK + xk;
 
   auto stage = [&](int step, int v0, int nv) {
-    float* xs = smem + (step & 1) * stage_floats;
-    float* ys = xs + GR_LONG_CHUNK * GR_FX;
+    float* xs = smem + (step % stages) * stage_floats;
+    float* ys = xs + GR_LONG_CHUNK * GR_FX + yk * pitch + yc;
     const bool state = step < q_steps;
     const int k0 = (state ? step : step - q_steps) * GR_FK;
-    for (int i = tid; i < GR_LONG_CHUNK * (GR_FK / 4); i += 128) {
-      const int t = i / (GR_FK / 4), k = (i % (GR_FK / 4)) * 4;
-      const float* src = state ? qb + (size_t)t * p.heads * p.dkp + k0 + k : within + t * GR_LONG_CHUNK + k0 + k;
-      const bool valid = t < count && (!state || k0 + k < p.dkp);
-      gr_copy16(xs + t * GR_FX + k, valid ? src : within, valid);
-    }
-    for (int i = tid; i < GR_FK * (nv / 4); i += 128) {
-      const int k = i / (nv / 4), c = (i % (nv / 4)) * 4;
-      const bool valid = state ? k0 + k < dk : k0 + k < count;
-      const float* src = !valid ? start : state ? start + (size_t)(k0 + k) * dv + v0 + c : values + (size_t)(k0 + k) * p.ld + v0 + c;
+    const float* src = (state ? x_q : x_a) + k0;
+    float* to = xs + xt * GR_FX + xk;
+    gr_copy16(to, src, row && (!state || k0 + xk < p.dkp));
+    gr_copy16(to + 4, src + 4, row && (!state || k0 + xk + 4 < p.dkp));
+    const bool valid = state ? k0 + yk < dk : k0 + yk < count;
+    const float* from = !valid ? start : (state ? start + (size_t)(k0 + yk) * dv : values + (size_t)(k0 + yk) * p.ld) + v0 + yc;
+#pragma unroll
+    for (int j = 0; j < GR_SLICE / 32; ++j) {
+      if (yc + 32 * j >= nv) break;
       if (state || v_aligned) {
-        gr_copy16(ys + k * wide + c, src, valid);
+        gr_copy16(ys + 32 * j, valid ? from + 32 * j : from, valid);
       } else {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) ys[k * wide + c + e] = valid ? src[e] : 0.f;
+        for (int e = 0; e < 4; ++e) ys[32 * j + e] = valid ? from[32 * j + e] : 0.f;
       }
     }
-    gr_commit();
   };
 
   for (int v0 = 0; v0 < dv; v0 += GR_SLICE) {
     const int nv = min(GR_SLICE, dv - v0);
-    const bool has0 = tx * 4 < nv, has1 = tx * 4 + 64 < nv;
-    float acc[2][2][4][4];
+    float sum[2][4][4], small[2][4][4];
 #pragma unroll
-    for (int h = 0; h < 2; ++h)
+    for (int a = 0; a < 2; ++a)
 #pragma unroll
-      for (int b = 0; b < 2; ++b)
+      for (int b = 0; b < 4; ++b)
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) acc[h][b][i][j] = 0.f;
+        for (int i = 0; i < 4; ++i) sum[a][b][i] = small[a][b][i] = 0.f;
     __syncthreads();
-    stage(0, v0, nv);
+    for (int s = 0; s + 1 < stages; ++s) {
+      if (s < steps) stage(s, v0, nv);
+      gr_commit();
+    }
     for (int step = 0; step < steps; ++step) {
-      if (step + 1 < steps) stage(step + 1, v0, nv);
-      else gr_commit();
-      gr_wait_one();
-      __syncthreads();
-      const float* xs = smem + (step & 1) * stage_floats + ty * GR_FX;
-      const float* ys = smem + (step & 1) * stage_floats + GR_LONG_CHUNK * GR_FX + tx * 4;
+      if (stages == 3) gr_wait<1>();
+      else gr_wait<0>();
+      __syncthreads();               // this stretch has landed; everyone is done with the one before it
+      if (step + stages - 1 < steps) stage(step + stages - 1, v0, nv);
+      gr_commit();
       // the first 32 tokens come before all tokens of the second stretch of V: A is zero there
-      const bool second = step > q_steps;
+      if (n0 < nv && (m0 > 0 || step <= q_steps)) {
+        const float* xs = smem + (step % stages) * stage_floats + (m0 + fg) * GR_FX + fq;
+        const float* ys = smem + (step % stages) * stage_floats + GR_LONG_CHUNK * GR_FX + fq * pitch + n0 + fg;
 #pragma unroll 2
-      for (int k = 0; k < GR_FK; k += 4) {
-        float x[2][4][4];                         // tokens ty + 8 i, and 32 further
+        for (int k = 0; k < GR_FK; k += 8) {
+          SplitA fa[2];
+          split_load_a(fa[0], xs + k, GR_FX, 1);
+          split_load_a(fa[1], xs + 16 * GR_FX + k, GR_FX, 1);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          if (!second) load4(xs + 8 * i * GR_FX + k, x[0][i]);
-          load4(xs + (8 * i + 32) * GR_FX + k, x[1][i]);
-        }
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float4 late = make_float4(x[1][0][e], x[1][1][e], x[1][2][e], x[1][3][e]);
-          float4 y0 = make_float4(0.f, 0.f, 0.f, 0.f), y1 = y0;
-          if (has0) y0 = *reinterpret_cast<const float4*>(ys + (k + e) * wide);
-          if (has1) y1 = *reinterpret_cast<const float4*>(ys + (k + e) * wide + 64);
-          gr_outer(acc[1][0], late, y0);
-          if (nv > 64) gr_outer(acc[1][1], late, y1);
-          if (!second) {
-            const float4 early = make_float4(x[0][0][e], x[0][1][e], x[0][2][e], x[0][3][e]);
-            gr_outer(acc[0][0], early, y0);
-            if (nv > 64) gr_outer(acc[0][1], early, y1);
+          for (int b = 0; b < 4; ++b) {
+            SplitB fb;
+            split_load_b(fb, ys + k * pitch + 8 * b, pitch);
+            split_mma(sum[0][b], small[0][b], fa[0], fb);
+            split_mma(sum[1][b], small[1][b], fa[1], fb);
           }
         }
       }
-      __syncthreads();
     }
-    if (dv <= GR_SLICE) {
-      float w[2][4];
 #pragma unroll
-      for (int b = 0; b < 2; ++b)
+    for (int a = 0; a < 2; ++a)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) w[b][j] = tx * 4 + 64 * b < nv ? p.norm_w[tx * 4 + 64 * b + j] : 0.f;
+      for (int b = 0; b < 4; ++b)
 #pragma unroll
-      for (int h = 0; h < 2; ++h)
+        for (int i = 0; i < 4; ++i) sum[a][b][i] = n0 + 8 * b + 2 * fq < nv ? sum[a][b][i] + small[a][b][i] : 0.f;
+    if (dv > GR_SLICE) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          float sq = 0.f;
+      for (int a = 0; a < 2; ++a)
 #pragma unroll
-          for (int b = 0; b < 2; ++b)
+        for (int b = 0; b < 4; ++b)
+          if (n0 + 8 * b + 2 * fq < nv)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) sq = fmaf(acc[h][b][i][j], acc[h][b][i][j], sq);
+            for (int h = 0; h < 2; ++h)
+              *reinterpret_cast<float2*>(os + (m0 + 16 * a + 8 * h + fg) * dv + v0 + n0 + 8 * b + 2 * fq) =
+                  make_float2(sum[a][b][2 * h], sum[a][b][2 * h + 1]);
+      continue;
+    }
 #pragma unroll
-          for (int o = 8; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
-          const float inv = 1.f / sqrtf(sq / (float)dv + p.eps);
-          const int t = 32 * h + 8 * i + ty;
-          if (t >= count) continue;
+    for (int a = 0; a < 2; ++a)
 #pragma unroll
-          for (int b = 0; b < 2; ++b) {
-            const int c = tx * 4 + 64 * b;
-            if (c >= nv) continue;
-            float o[4];
+      for (int h = 0; h < 2; ++h) {
+        float sq = 0.f;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) o[j] = acc[h][b][i][j] * inv * w[b][j];
-            store4((TO*)p.out + ((size_t)(first + t) * p.heads + head) * dv + c, o);
-          }
+        for (int b = 0; b < 4; ++b) {
+          sq = fmaf(sum[a][b][2 * h], sum[a][b][2 * h], sq);
+          sq = fmaf(sum[a][b][2 * h + 1], sum[a][b][2 * h + 1], sq);
         }
-    } else {
+        sq += __shfl_xor_sync(0xffffffffu, sq, 1);
+        sq += __shfl_xor_sync(0xffffffffu, sq, 2);
+        if (fq == 0) part[warp & 3][m0 + 16 * a + 8 * h + fg] = sq;
+      }
+    __syncthreads();
 #pragma unroll
-      for (int h = 0; h < 2; ++h)
+    for (int a = 0; a < 2; ++a)
 #pragma unroll
-        for (int b = 0; b < 2; ++b)
-          if (tx * 4 + 64 * b < nv)
+      for (int h = 0; h < 2; ++h) {
+        const int t = m0 + 16 * a + 8 * h + fg;
+        if (t >= count) continue;
+        const float inv = 1.f / sqrtf((part[0][t] + part[1][t] + part[2][t] + part[3][t]) / (float)dv + p.eps);
+        TO* dst = (TO*)p.out + ((size_t)(first + t) * p.heads + head) * dv;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) store4(os + (32 * h + 8 * i + ty) * dv + v0 + tx * 4 + 64 * b, acc[h][b][i]);
-    }
+        for (int b = 0; b < 4; ++b) {
+          const int c = n0 + 8 * b + 2 * fq;
+          if (c >= nv) continue;
+          gr_store2(dst + c, sum[a][b][2 * h] * inv * p.norm_w[c], sum[a][b][2 * h + 1] * inv * p.norm_w[c + 1]);
+        }
+      }
   }
   if (dv <= GR_SLICE) return;
   __syncthreads();
-  const int warp = tid >> 5, lane = tid & 31, warps = blockDim.x >> 5;
-  for (int r = warp; r < count; r += warps) {
+  for (int r = warp; r < count; r += 8) {
     float sq = 0.f;
     for (int c = lane; c < dv; c += 32) sq = fmaf(os[r * dv + c], os[r * dv + c], sq);
     const float inv = 1.f / sqrtf(warp_sum(sq) / (float)dv + p.eps);
@@ -679,12 +667,12 @@ static int gr_column_threads(int dk, int dv) {
 
 // Shared memory of the chunk kernels.
 static size_t gr_chunk_smem(int dk, int dv) {
-  const int dkp = (dk + 3) & ~3, dp = (dkp < GR_SLICE ? dkp : GR_SLICE) + 4, vp = (dv < GR_SLICE ? dv : GR_SLICE) + 4;
+  const int dkp = (dk + 3) & ~3, dp = (dkp < GR_SLICE ? dkp : GR_SLICE) + 4, vp = (dv < GR_SLICE ? dv : GR_SLICE) + 8;
   return sizeof(float) * ((size_t)GR_LONG_CHUNK * (dp + (dp > vp ? dp : vp) + GR_AP) + GR_SUBS * dp);
 }
 static size_t gr_finish_smem(int dv) {
-  const int wide = dv < GR_SLICE ? dv : GR_SLICE;
-  return sizeof(float) * ((size_t)2 * (GR_LONG_CHUNK * GR_FX + GR_FK * wide) + (dv > GR_SLICE ? (size_t)GR_LONG_CHUNK * dv : 0));
+  return sizeof(float) * ((size_t)gr_finish_stages(dv) * (GR_LONG_CHUNK * GR_FX + GR_FK * gr_finish_pitch(dv)) +
+                          (dv > GR_SLICE ? (size_t)GR_LONG_CHUNK * dv : 0));
 }
 
 // 32-bit floats of scratch the chunk-parallel kernels need for a step of `tokens` tokens in
@@ -762,12 +750,12 @@ FE_EXPORT int fe_gated_recurrence(const float* proj, long long ld, int q_off, in
   if (out_dtype == FE_DTYPE_F32) {
     if (finish_smem > 48 * 1024)
       cudaFuncSetAttribute(gated_recurrence_finish_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)finish_smem);
-    rc = fe_launch_dependent(gated_recurrence_finish_kernel<float>, dim3(heads, entries, chunks), dim3(128), finish_smem, stream, p,
+    rc = fe_launch_dependent(gated_recurrence_finish_kernel<float>, dim3(heads, entries, chunks), dim3(256), finish_smem, stream, p,
                              v_aligned);
   } else {
     if (finish_smem > 48 * 1024)
       cudaFuncSetAttribute(gated_recurrence_finish_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)finish_smem);
-    rc = fe_launch_dependent(gated_recurrence_finish_kernel<bf16>, dim3(heads, entries, chunks), dim3(128), finish_smem, stream, p,
+    rc = fe_launch_dependent(gated_recurrence_finish_kernel<bf16>, dim3(heads, entries, chunks), dim3(256), finish_smem, stream, p,
                              v_aligned);
   }
   return rc ? rc : fe_last_error();
