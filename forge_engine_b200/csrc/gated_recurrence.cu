@@ -336,7 +336,7 @@ __global__ void __launch_bounds__(256, 2) gated_recurrence_chunk_kernel(GatedRec
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i)
-          as[((apart + block) * GR_SUB + fg + 8 * (i >> 1)) * GR_AP + block * GR_SUB + side + 2 * fq + (i & 1)] += sum[i] + small[i];
+          as[((apart + block) * GR_SUB + fg + 8 * (i >> 1)) * GR_AP + block * GR_SUB + side + 2 * fq + (i & 1)] += split_join(sum[i], small[i]);
       }
       __syncthreads();
       if (lane * 4 < ndp) {
@@ -433,7 +433,7 @@ __global__ void __launch_bounds__(256, 2) gated_recurrence_chunk_kernel(GatedRec
 #pragma unroll
             for (int b = 0; b < 4; ++b) {
               const int c = c0 + 8 * b + 2 * fq;
-              if (c < nv) *reinterpret_cast<float2*>(dst + c) = make_float2(sum[a][b][2 * h] + small[a][b][2 * h], sum[a][b][2 * h + 1] + small[a][b][2 * h + 1]);
+              if (c < nv) *reinterpret_cast<float2*>(dst + c) = make_float2(split_join(sum[a][b][2 * h], small[a][b][2 * h]), split_join(sum[a][b][2 * h + 1], small[a][b][2 * h + 1]));
             }
           }
       }
@@ -595,7 +595,7 @@ __global__ void __launch_bounds__(256, 2) gated_recurrence_finish_kernel(GatedRe
 #pragma unroll
       for (int b = 0; b < 4; ++b)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) sum[a][b][i] = n0 + 8 * b + 2 * fq < nv ? sum[a][b][i] + small[a][b][i] : 0.f;
+        for (int i = 0; i < 4; ++i) sum[a][b][i] = n0 + 8 * b + 2 * fq < nv ? split_join(sum[a][b][i], small[a][b][i]) : 0.f;
     if (dv > GR_SLICE) {
 #pragma unroll
       for (int a = 0; a < 2; ++a)
