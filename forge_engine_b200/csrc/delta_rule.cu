@@ -19,6 +19,7 @@
 //                   the chunks with two products each (u, and the state it leads to); then
 //                     o_t = e^(c_t) S^T q_t + sum_(j <= t) e^(c_t - c_j) (q_t . k_j) u_j.
 #include "state_recurrence.cuh"
+#include "mma_split.cuh"
 
 // ---------------------------------------------------------------------------
 // delta_prepare
@@ -353,23 +354,26 @@ struct Delta {
 };
 
 // W and U of one chunk of one head: the triangular system solved for the columns of beta e^c k
-// and beta v, sixteen rows at a time.  A block of rows first loses what the rows before it give (a
-// small product), then a thread per column solves the 16 x 16 triangle in registers and stores the
-// result, also for the blocks below.
+// and beta v, sixteen rows at a time.  A block of rows first loses what the rows before it give, then a
+// thread per column solves the 16 x 16 triangle in registers and stores the result, also for the blocks
+// below.  The products (L itself, and a block's from the rows before it) run on the tensor cores, both
+// operands split: 2,048 tokens of 32 heads of 64 channels take 68 us, 80 as tiles of multiply-adds; what
+// remains is the triangles, one row after the other, and the loads before them.
 #define DS_THREADS 256
+// Columns of the right sides: k in fours, then v, in eights altogether.
+__host__ __device__ static inline int ds_columns(int dk, int dv) { return (((dk + 3) & ~3) + dv + 7) & ~7; }
 __global__ void __launch_bounds__(DS_THREADS) delta_solve_kernel(const Delta m, const StateRun p) {
   extern __shared__ __align__(16) float smem[];
-  pdl_trigger();
   pdl_wait();
   ChunkAt at;
   if (!sr_locate(p, &at)) return;
   const int head = blockIdx.x, dk = p.dk, dv = p.dv, tid = threadIdx.x;
-  const int v0 = (dk + 3) & ~3, ldx = v0 + ((dv + 3) & ~3);      // columns of k, then of v
+  const int v0 = (dk + 3) & ~3, columns = ds_columns(dk, dv), ldx = columns + 8, dk8 = (dk + 7) & ~7;      // columns of k, then of v
   __shared__ double c[SR_LONG];
   __shared__ float bt[SR_LONG], be[SR_LONG];
   float* lt = smem;                          // [SR_LONG columns j][SR_TP rows t]: L transposed
   float* X = lt + SR_LONG * SR_TP;           // [SR_LONG][ldx]
-  float* kt = X + SR_LONG * ldx;             // [dk][SR_TP]
+  float* kt = X + SR_LONG * ldx;             // [dk8][SR_TP]; rows past dk are zero
   if (tid < 32) {
     double sums[2];
     m.chunk_sums(p, head, at, sums);
@@ -388,6 +392,7 @@ __global__ void __launch_bounds__(DS_THREADS) delta_solve_kernel(const Delta m, 
   }
   const Rows keys = m.keys(p, head, at), values{p.v + (size_t)at.first * p.v_ld + (size_t)head * dv, p.v_ld};
   sr_stage_transposed(kt, keys, dk, at.count);
+  for (int i = tid; i < (dk8 - dk) * SR_TP; i += DS_THREADS) kt[dk * SR_TP + i] = 0.f;
   __syncthreads();
   // the right sides: rows of beta e^c k and beta v, zero past the last token and between the two
   const int warp = tid >> 5, lane = tid & 31;
@@ -396,48 +401,49 @@ __global__ void __launch_bounds__(DS_THREADS) delta_solve_kernel(const Delta m, 
     const float a = be[t], b = bt[t];
     float* x = X + t * ldx;
     for (int d = lane; d < v0; d += 32) x[d] = d < dk ? a * kt[d * SR_TP + t] : 0.f;
-    for (int d = lane; d < ldx - v0; d += 32) x[v0 + d] = has && d < dv ? b * values.row(t)[d] : 0.f;
+    for (int d = lane; d < columns - v0; d += 32) x[v0 + d] = has && d < dv ? b * values.row(t)[d] : 0.f;
   }
+  const int fg = lane >> 2, fq = lane & 3;
   {
-    const int row = 4 * (tid & 15), col = 4 * (tid >> 4);
-    float a[4][4] = {};
-    if (col <= row + 3) sr_mm44(a, kt, SR_TP, kt, SR_TP, dk, row, col);
+    const int m0 = (warp >> 2) * 32, n0 = (warp & 3) * 16;
+    OutTile s;
+    s.clear();
+    if (n0 <= m0 + 31) s.add(kt + fq * SR_TP + m0 + fg, kt + fq * SR_TP + n0 + fg, SR_TP, dk8);
 #pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      float l[4];
+    for (int a = 0; a < 2; ++a)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int t = row + e;
-        l[e] = col + b < t ? a[e][b] * bt[t] * expf((float)(c[t] - c[col + b])) : 0.f;
-      }
-      store4(lt + (col + b) * SR_TP + row, l);
-    }
+      for (int b = 0; b < 2; ++b)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int t = m0 + 16 * a + 8 * (i >> 1) + fg, j = n0 + 8 * b + 2 * fq + (i & 1);
+          lt[j * SR_TP + t] = j < t ? s.at(a, b, i >> 1, i & 1) * bt[t] * expf((float)(c[t] - c[j])) : 0.f;
+        }
   }
   const size_t cell = m.cell(p, at, head);
   for (int r0 = 0; r0 < SR_LONG; r0 += 16) {
     __syncthreads();
     if (r0 > 0) {
-      const int row = r0 + 4 * (tid & 3);
-      for (int col = 2 * (tid >> 2); col < ldx; col += DS_THREADS / 2) {
-        float acc[4][2] = {};
-#pragma unroll 8
-        for (int j = 0; j < r0; ++j) {
-          const float4 l = *reinterpret_cast<const float4*>(lt + j * SR_TP + row);
-          const float2 x = *reinterpret_cast<const float2*>(X + j * ldx + col);
-          acc[0][0] = fmaf(l.x, x.x, acc[0][0]), acc[0][1] = fmaf(l.x, x.y, acc[0][1]);
-          acc[1][0] = fmaf(l.y, x.x, acc[1][0]), acc[1][1] = fmaf(l.y, x.y, acc[1][1]);
-          acc[2][0] = fmaf(l.z, x.x, acc[2][0]), acc[2][1] = fmaf(l.z, x.y, acc[2][1]);
-          acc[3][0] = fmaf(l.w, x.x, acc[3][0]), acc[3][1] = fmaf(l.w, x.y, acc[3][1]);
+      for (int n0 = 8 * warp; n0 < columns; n0 += DS_THREADS / 4) {
+        float sum[4] = {0.f, 0.f, 0.f, 0.f}, small[4] = {0.f, 0.f, 0.f, 0.f};
+        const float* l = lt + fq * SR_TP + r0 + fg;
+        const float* x = X + fq * ldx + n0 + fg;
+#pragma unroll 2
+        for (int j = 0; j < r0; j += 8) {
+          SplitA fa;
+          SplitB fb;
+          split_load_a(fa, l + j * SR_TP, 1, SR_TP);
+          split_load_b(fb, x + j * ldx, ldx);
+          split_mma(sum, small, fa, fb);
         }
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          float2* x2 = reinterpret_cast<float2*>(X + (row + e) * ldx + col);
-          *x2 = make_float2(x2->x - acc[e][0], x2->y - acc[e][1]);
+        for (int h = 0; h < 2; ++h) {
+          float2* x2 = reinterpret_cast<float2*>(X + (r0 + 8 * h + fg) * ldx + n0 + 2 * fq);
+          *x2 = make_float2(x2->x - split_join(sum[2 * h], small[2 * h]), x2->y - split_join(sum[2 * h + 1], small[2 * h + 1]));
         }
       }
       __syncthreads();
     }
-    for (int i = tid; i < ldx; i += DS_THREADS) {
+    for (int i = tid; i < columns; i += DS_THREADS) {
       float x[16];
 #pragma unroll
       for (int t = 0; t < 16; ++t) x[t] = X[(r0 + t) * ldx + i];
@@ -466,28 +472,18 @@ __global__ void __launch_bounds__(DS_THREADS) delta_solve_kernel(const Delta m, 
 }
 
 // The chain over an entry's chunks for one head and COLS value columns: u = U - W S, then
-// S <- e^(c_end) S + sum_j k_j (e^(c_end - c_j) u_j)^T.  The state's columns stay in shared memory;
-// the next chunk's W and keys are on their way while a chunk is worked on.  Thread (rg, cg) of
-// 16 x COLS / 2 owns four rows and two columns of a product; two such groups of threads take half of
-// a product's depth each, the second one's share is added by (W S) or after (the state) the first's.
-template <int COLS>
-__device__ __forceinline__ void dc_mm42(float (&acc)[4][2], const float* xt, int ldx, const float* y, int depth, int row, int col) {
-#pragma unroll 8
-  for (int k = 0; k < depth; ++k) {
-    const float4 x = *reinterpret_cast<const float4*>(xt + k * ldx + row);
-    const float2 b = *reinterpret_cast<const float2*>(y + k * COLS + col);
-    acc[0][0] = fmaf(x.x, b.x, acc[0][0]), acc[0][1] = fmaf(x.x, b.y, acc[0][1]);
-    acc[1][0] = fmaf(x.y, b.x, acc[1][0]), acc[1][1] = fmaf(x.y, b.y, acc[1][1]);
-    acc[2][0] = fmaf(x.z, b.x, acc[2][0]), acc[2][1] = fmaf(x.z, b.y, acc[2][1]);
-    acc[3][0] = fmaf(x.w, b.x, acc[3][0]), acc[3][1] = fmaf(x.w, b.y, acc[3][1]);
-  }
-}
-
-template <int COLS>
+// S <- e^(c_end) S + sum_j k_j (e^(c_end - c_j) u_j)^T.  What bounds it is one chunk's two products after the
+// other, so they run on the tensor cores with both operands split (mma_split.cuh): a warp takes 16 x 8
+// outputs, reads 48 numbers a lane where a 4 x 2 tile of multiply-adds read 192, and a chunk has two
+// barriers.  The state's columns stay in registers, as the warps' pieces of the second product, and in shared
+// memory for the first; the next chunk's W and keys, and what a lane needs of it besides, are on their way
+// while a chunk is worked on.  2,048 tokens, 32 heads of 64 channels: 102 us, 179 with multiply-adds.
+#define DC_WP (SR_LONG + 8)          // pitches: the rows of a fragment fall into different banks
+template <int KD, int COLS>
 __global__ void __launch_bounds__(16 * COLS) delta_chain_kernel(const Delta m, const StateRun p, int* status) {
   extern __shared__ __align__(16) float smem[];
-  pdl_trigger();
   pdl_wait();
+  constexpr int KP = 64 * KD + 8, SP = COLS + 8, THREADS = 16 * COLS, WARPS = THREADS / 32;
   const int head = blockIdx.x, entry = blockIdx.y, col0 = blockIdx.z * COLS, tid = threadIdx.x;
   const int first = p.cu_tokens[entry], count = p.cu_tokens[entry + 1] - first;
   if (count < p.long_from) return;
@@ -496,35 +492,50 @@ __global__ void __launch_bounds__(16 * COLS) delta_chain_kernel(const Delta m, c
     if (tid == 0 && blockIdx.z == 0) atomicOr(status, FE_STATUS_BAD_PAGE);
     return;
   }
-  const int dk = p.dk, dv = p.dv, kp = (dk + 63) / 64 * 64;
-  const int cols = min(COLS, dv - col0), half = dk * SR_LONG + SR_LONG * kp;
-  float* S = smem;                           // [kp][COLS]
-  float* us = S + kp * COLS;                 // [SR_LONG][COLS], weighted
-  float* share = us + SR_LONG * COLS;        // [SR_LONG][COLS]: the second group's part of W S
-  float* buffers = share + SR_LONG * COLS;   // 2 x (W transposed [dk][SR_LONG], keys [SR_LONG][kp])
-  const int group = tid / (8 * COLS), mine = tid - group * 8 * COLS;
-  const int row = 4 * (mine & 15), col = 2 * (mine >> 4);
-  const int d_from = group == 0 ? 0 : dk / 2, d_count = group == 0 ? dk / 2 : dk - dk / 2;
-  float* st = p.state + ((size_t)slot * p.heads + head) * dk * dv + col0;
-  for (int i = tid; i < kp * COLS; i += blockDim.x) {
-    const int d = i / COLS, c = i - d * COLS;
-    S[i] = (d < dk && c < cols) ? st[(size_t)d * dv + c] : 0.f;
-  }
-  for (int i = tid; i < 2 * half; i += blockDim.x) buffers[i] = 0.f;      // key channels past dk stay zero
+  const int dk = p.dk, dv = p.dv, dk8 = (dk + 7) & ~7, half = dk8 * DC_WP + SR_LONG * KP;
+  float* S = smem;                           // [64 KD][SP]
+  float* us = S + 64 * KD * SP;              // [SR_LONG][SP], weighted
+  float* buffers = us + SR_LONG * SP;        // 2 x (W transposed [dk8][DC_WP], keys [SR_LONG][KP])
+  const int lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
+  const int t0 = 16 * (warp & 3) + g, n0 = 8 * (warp >> 2);        // first row and columns of this warp's pieces
+  const int col = col0 + n0 + 2 * q;                               // this lane's two columns
+  const bool in0 = col < dv, in1 = col + 1 < dv, pair = in1 && (dv & 1) == 0;
+  auto load2 = [&](const float* at, float& a, float& b) {
+    if (pair) { const float2 x = *reinterpret_cast<const float2*>(at); a = x.x, b = x.y; }
+    else { a = in0 ? at[0] : 0.f, b = in1 ? at[1] : 0.f; }
+  };
+  auto store2 = [&](float* at, float a, float b) {
+    if (pair) { *reinterpret_cast<float2*>(at) = make_float2(a, b); }
+    else { if (in0) at[0] = a; if (in1) at[1] = b; }
+  };
+  float* st = p.state + ((size_t)slot * p.heads + head) * dk * dv + col;
+  float s[KD][2][2];                         // rows 64 kd + t0, + 8 of the state
+#pragma unroll
+  for (int kd = 0; kd < KD; ++kd)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int d = 64 * kd + t0 + 8 * h;
+      s[kd][h][0] = s[kd][h][1] = 0.f;
+      if (d < dk) load2(st + (size_t)d * dv, s[kd][h][0], s[kd][h][1]);
+      *reinterpret_cast<float2*>(S + d * SP + n0 + 2 * q) = make_float2(s[kd][h][0], s[kd][h][1]);
+    }
+  for (int i = tid; i < 2 * half; i += THREADS) buffers[i] = 0.f;      // channels past dk stay zero
   __syncthreads();
   const int chunks = (count + SR_LONG - 1) / SR_LONG;
-  const int lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
   const size_t cell0 = (size_t)sr_slot(first, entry, 0) * p.heads + head;
   const Rows keys{m.k_row(p, head, first), m.ld};
   const bool wide = keys.wide(dk);
   auto fetch = [&](int chunk, float* buf) {
-    const float* w = m.w + (cell0 + (size_t)chunk * p.heads) * dk * SR_LONG;
-    for (int i = 4 * tid; i < dk * SR_LONG; i += 4 * blockDim.x) sr_copy16(buf + i, w + i);
-    const int have = min(SR_LONG, count - chunk * SR_LONG);
-    float* ks = buf + dk * SR_LONG;
-    for (int t = warp; t < SR_LONG; t += warps) {
-      float* dst = ks + t * kp;
-      if (t >= have) {
+    const float* w = m.w + (cell0 + (size_t)chunk * p.heads) * dk * SR_LONG + (tid & 15) * 4;
+    float* to = buf + (tid & 15) * 4;
+#pragma unroll 4
+    for (int d = tid >> 4; d < dk; d += THREADS / 16) sr_copy16(to + d * DC_WP, w + d * SR_LONG);
+    const int rows = min(SR_LONG, count - chunk * SR_LONG);
+    float* ks = buf + dk8 * DC_WP;
+#pragma unroll 4
+    for (int t = warp; t < SR_LONG; t += WARPS) {
+      float* dst = ks + t * KP;
+      if (t >= rows) {
         for (int d = lane; d < dk; d += 32) dst[d] = 0.f;
       } else if (wide) {
         for (int d = 4 * lane; d < dk; d += 128) sr_copy16(dst + d, keys.row(chunk * SR_LONG + t) + d);
@@ -534,92 +545,100 @@ __global__ void __launch_bounds__(16 * COLS) delta_chain_kernel(const Delta m, c
     }
     sr_copy_commit();
   };
+  float x[2][2], w[2], keep;                 // U, its weights and the state's decay over the chunk
+  auto ask = [&](int chunk) {
+    const size_t cell = cell0 + (size_t)chunk * p.heads;
+    const float* decays = m.decays + cell * (SR_LONG + 4);
+    keep = decays[SR_LONG];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      w[h] = decays[t0 + 8 * h];
+      load2(m.u + (cell * SR_LONG + t0 + 8 * h) * dv + col, x[h][0], x[h][1]);
+    }
+  };
   fetch(0, buffers);
+  ask(0);
   for (int chunk = 0; chunk < chunks; ++chunk) {
     const size_t cell = cell0 + (size_t)chunk * p.heads;
     const float* buf = buffers + (chunk & 1) * half;
-    float* u = m.u + (cell * SR_LONG + row) * dv + col0 + col;
-    const float* decays = m.decays + cell * (SR_LONG + 4);
-    float x[4][2], w[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      w[e] = decays[row + e];
-#pragma unroll
-      for (int b = 0; b < 2; ++b) x[e][b] = group == 0 && col + b < cols ? u[(size_t)e * dv + b] : 0.f;
-    }
-    const float keep = decays[SR_LONG];
+    if (chunk + 1 == chunks) pdl_trigger();    // state_out's blocks would only lie beside this one's till then
     sr_copy_wait<0>();
-    __syncthreads();
+    __syncthreads();           // this chunk's tiles have landed, the state is whole; everyone is done with the other buffer
     if (chunk + 1 < chunks) fetch(chunk + 1, buffers + ((chunk + 1) & 1) * half);
-    float a[4][2] = {};
-    dc_mm42<COLS>(a, buf + d_from * SR_LONG, SR_LONG, S + d_from * COLS, d_count, row, col);
-    if (group == 1) {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) *reinterpret_cast<float2*>(share + (row + e) * COLS + col) = make_float2(a[e][0], a[e][1]);
-    }
     // the state before the chunk, for state_out
-    float* dst = m.before + cell * dk * dv + col0;
-    for (int i = tid; i < dk * COLS; i += blockDim.x) {
-      const int d = i / COLS, c = i - d * COLS;
-      if (c < cols) dst[(size_t)d * dv + c] = S[i];
-    }
-    __syncthreads();
-    if (group == 0) {
+    float* before = m.before + cell * dk * dv + col;
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float2 more = *reinterpret_cast<const float2*>(share + (row + e) * COLS + col);
-        x[e][0] -= a[e][0] + more.x;
-        x[e][1] -= a[e][1] + more.y;
-        *reinterpret_cast<float2*>(us + (row + e) * COLS + col) = make_float2(x[e][0] * w[e], x[e][1] * w[e]);
+    for (int kd = 0; kd < KD; ++kd)
 #pragma unroll
-        for (int b = 0; b < 2; ++b)
-          if (col + b < cols) u[(size_t)e * dv + b] = x[e][b];
+      for (int h = 0; h < 2; ++h) {
+        const int d = 64 * kd + t0 + 8 * h;
+        if (d < dk) store2(before + (size_t)d * dv, s[kd][h][0], s[kd][h][1]);
+      }
+    {
+      float sum[4] = {0.f, 0.f, 0.f, 0.f}, small[4] = {0.f, 0.f, 0.f, 0.f};
+      const float* a = buf + q * DC_WP + t0;
+      const float* b = S + q * SP + n0 + g;
+#pragma unroll 8
+      for (int d = 0; d < dk8; d += 8) {
+        SplitA fa;
+        SplitB fb;
+        split_load_a(fa, a + d * DC_WP, 1, DC_WP);
+        split_load_b(fb, b + d * SP, SP);
+        split_mma(sum, small, fa, fb);
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        x[h][0] -= split_join(sum[2 * h], small[2 * h]);
+        x[h][1] -= split_join(sum[2 * h + 1], small[2 * h + 1]);
+        *reinterpret_cast<float2*>(us + (t0 + 8 * h) * SP + n0 + 2 * q) = make_float2(x[h][0] * w[h], x[h][1] * w[h]);
+        store2(m.u + (cell * SR_LONG + t0 + 8 * h) * dv + col, x[h][0], x[h][1]);
       }
     }
+    const float decay = keep;
     __syncthreads();
-    const float* ks = buf + dk * SR_LONG;
-    const int t_from = group * (SR_LONG / 2);
-    for (int d0 = 0; d0 < kp; d0 += 64) {
-      float b[4][2] = {};
-      dc_mm42<COLS>(b, ks + t_from * kp + d0, kp, us + t_from * COLS, SR_LONG / 2, row, col);
-      if (group == 0) {
+    if (chunk + 1 < chunks) ask(chunk + 1);
+    const float* b = us + q * SP + n0 + g;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          float2* s2 = reinterpret_cast<float2*>(S + (d0 + row + e) * COLS + col);
-          const float2 old = *s2;
-          *s2 = make_float2(fmaf(keep, old.x, b[e][0]), fmaf(keep, old.y, b[e][1]));
-        }
+    for (int kd = 0; kd < KD; ++kd) {
+      float sum[4] = {0.f, 0.f, 0.f, 0.f}, small[4] = {0.f, 0.f, 0.f, 0.f};
+      const float* a = buf + dk8 * DC_WP + q * KP + 64 * kd + t0;
+#pragma unroll
+      for (int t = 0; t < SR_LONG; t += 8) {
+        SplitA fa;
+        SplitB fb;
+        split_load_a(fa, a + t * KP, 1, KP);
+        split_load_b(fb, b + t * SP, SP);
+        split_mma(sum, small, fa, fb);
       }
-      __syncthreads();
-      if (group == 1) {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          float2* s2 = reinterpret_cast<float2*>(S + (d0 + row + e) * COLS + col);
-          const float2 old = *s2;
-          *s2 = make_float2(old.x + b[e][0], old.y + b[e][1]);
-        }
+      for (int h = 0; h < 2; ++h) {
+        s[kd][h][0] = fmaf(decay, s[kd][h][0], split_join(sum[2 * h], small[2 * h]));
+        s[kd][h][1] = fmaf(decay, s[kd][h][1], split_join(sum[2 * h + 1], small[2 * h + 1]));
+        *reinterpret_cast<float2*>(S + (64 * kd + t0 + 8 * h) * SP + n0 + 2 * q) = make_float2(s[kd][h][0], s[kd][h][1]);
       }
     }
   }
-  __syncthreads();
-  for (int i = tid; i < dk * COLS; i += blockDim.x) {
-    const int d = i / COLS, c = i - d * COLS;
-    if (c < cols) st[(size_t)d * dv + c] = S[i];
-  }
+#pragma unroll
+  for (int kd = 0; kd < KD; ++kd)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int d = 64 * kd + t0 + 8 * h;
+      if (d < dk) store2(st + (size_t)d * dv, s[kd][h][0], s[kd][h][1]);
+    }
 }
 
 static size_t delta_solve_smem(int dk, int dv) {
-  const size_t ldx = (size_t)((dk + 3) / 4 * 4) + (dv + 3) / 4 * 4;
-  return sizeof(float) * ((size_t)SR_LONG * SR_TP + SR_LONG * ldx + (size_t)dk * SR_TP);
+  return sizeof(float) * ((size_t)SR_LONG * SR_TP + (size_t)SR_LONG * (ds_columns(dk, dv) + 8) + (size_t)(dk + 7) / 8 * 8 * SR_TP);
 }
 // Value columns of a block of delta_chain: few where the heads are small, so that there are more blocks.
 static int delta_chain_cols(int dv) { return dv <= 64 ? 16 : 32; }
 static size_t delta_chain_smem(int dk, int cols) {
-  const size_t kp = (size_t)(dk + 63) / 64 * 64;
-  return sizeof(float) * (kp * cols + (size_t)2 * SR_LONG * cols + 2 * ((size_t)dk * SR_LONG + SR_LONG * kp));
+  const size_t kp = (size_t)(dk + 63) / 64 * 64, dk8 = (size_t)(dk + 7) / 8 * 8, sp = cols + 8;
+  return sizeof(float) * ((kp + SR_LONG) * sp + 2 * (dk8 * DC_WP + SR_LONG * (kp + 8)));
 }
 static bool delta_chunk_takes(int dk, int dv) {
-  return chunk_takes(dk, dv, true) && delta_solve_smem(dk, dv) <= 200 * 1024 && delta_chain_smem(dk, delta_chain_cols(dv)) <= 200 * 1024;
+  return dk <= 192 && chunk_takes(dk, dv, true) && delta_solve_smem(dk, dv) <= 218 * 1024 &&
+         delta_chain_smem(dk, delta_chain_cols(dv)) <= 226 * 1024;
 }
 
 FE_EXPORT long long fe_delta_rule_scratch(int tokens, int entries, int heads, int dk, int dv, int max_new) {
@@ -655,16 +674,28 @@ FE_EXPORT int fe_delta_rule(const float* qkv, long long ld, const float* gates, 
   cudaFuncSetAttribute(delta_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   rc = fe_launch_dependent(delta_solve_kernel, dim3(heads, entries, chunks), dim3(DS_THREADS), smem, stream, m, p);
   if (rc) return rc;
+  // delta_chain is not launched as a dependent: its blocks, fewer than the SMs or not many more, would take their
+  // places while delta_solve's last blocks leave theirs, two on one SM and none on the next (143 us for a chain
+  // over 2,048 tokens that takes 102 us spread evenly).
   const int cols = delta_chain_cols(dv);
   smem = delta_chain_smem(dk, cols);
   const dim3 chain(heads, entries, (dv + cols - 1) / cols);
-  if (cols == 16) {
-    cudaFuncSetAttribute(delta_chain_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    rc = fe_launch_dependent(delta_chain_kernel<16>, chain, dim3(256), smem, stream, m, p, status);
-  } else {
-    cudaFuncSetAttribute(delta_chain_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    rc = fe_launch_dependent(delta_chain_kernel<32>, chain, dim3(512), smem, stream, m, p, status);
-  }
+#define DC_LAUNCH(KD, COLS)                                                                                       \
+  do {                                                                                                            \
+    cudaFuncSetAttribute(delta_chain_kernel<KD, COLS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);   \
+    delta_chain_kernel<KD, COLS><<<chain, 16 * COLS, smem, stream>>>(m, p, status);                               \
+    rc = fe_last_error();                                                                                         \
+  } while (0)
+#define DC_BY_DK(COLS)                 \
+  do {                                 \
+    if (dk <= 64) DC_LAUNCH(1, COLS);  \
+    else if (dk <= 128) DC_LAUNCH(2, COLS); \
+    else DC_LAUNCH(3, COLS);           \
+  } while (0)
+  if (cols == 16) DC_BY_DK(16);
+  else DC_BY_DK(32);
+#undef DC_BY_DK
+#undef DC_LAUNCH
   if (rc) return rc;
   rc = launch_out(m, p, out_dtype, entries, chunks, stream);
   return rc ? rc : fe_last_error();

@@ -214,8 +214,7 @@ __global__ void __launch_bounds__(256) memory_sums_kernel(const Memory m, const 
 
 // One thread per element of (S, n) walks an entry's chunks.
 __global__ void __launch_bounds__(256) memory_scan_kernel(const Memory m, const StateRun p, int* status) {
-  pdl_trigger();
-  pdl_wait();
+  pdl_wait();                // no trigger: state_out's shared memory finds no room on an SM beside this kernel's blocks
   const int head = blockIdx.x, entry = blockIdx.y;
   const int first = p.cu_tokens[entry], count = p.cu_tokens[entry + 1] - first;
   if (count < p.long_from) return;

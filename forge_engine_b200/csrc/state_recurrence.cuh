@@ -16,17 +16,17 @@
 // chunk kernels - portions of SR_LONG_FROM tokens or more run in chunks of SR_LONG tokens: what a
 //   chunk adds and how it decays what came before is worked out for all chunks side by side, the
 //   states are chained (or, where the chain is a product, walked chunk by chunk), and state_out
-//   takes the outputs of all chunks side by side as small 32-bit products from shared memory.
+//   takes the outputs of all chunks side by side as small products from shared memory.
 //
 // Everything is 32-bit; sums of log decays inside a chunk are 64-bit, so that the exponential of
 // a difference of two of them keeps its precision however far both have fallen.
 #pragma once
-#include "common.cuh"
+#include "mma_split.cuh"
 
 #define SR_CHUNK 16          // tokens staged at a time by the walk
 #define SR_LONG 64           // tokens of a chunk of the chunk-parallel form
 #define SR_LONG_FROM 96      // tokens from which on an entry takes that form
-#define SR_TP (SR_LONG + 4)  // pitch of a transposed tile [channel][token]
+#define SR_TP (SR_LONG + 8)  // pitch of a transposed tile [channel][token]: the rows of a fragment in different banks
 
 struct StateRun {
   float* state;            // [rows, heads, dk, dv]
@@ -51,6 +51,8 @@ __device__ __forceinline__ float sr_gate(float z, int act) {
   const float s = 1.f / (1.f + expf(-z));
   return act == 0 ? z * s : s;
 }
+__device__ __forceinline__ void sr_store2(float* p, float a, float b) { *reinterpret_cast<float2*>(p) = make_float2(a, b); }
+__device__ __forceinline__ void sr_store2(bf16* p, float a, float b) { *reinterpret_cast<__nv_bfloat162*>(p) = __floats2bfloat162_rn(a, b); }
 __device__ __forceinline__ float sr_softplus(float z) { return fmaxf(z, 0.f) + log1pf(expf(-fabsf(z))); }
 
 // Sum over the ds neighbouring lanes of a column.
@@ -361,8 +363,9 @@ __device__ __forceinline__ void sr_stage_transposed(float* dst, const Rows& src,
   }
 }
 
-// Columns c0 .. c0 + 63 of `count` of `rows` rows of `width` numbers as a tile dst[row * 64 + column];
+// Columns c0 .. c0 + 63 of `count` of `rows` rows of `width` numbers as a tile dst[row * PITCH + column];
 // zero past the last row and the last column.
+template <int PITCH = 64>
 __device__ __forceinline__ void sr_stage_columns(float* dst, const Rows& src, int rows, int count, int c0, int width) {
   const int step = blockDim.x;
   if (src.wide(width)) {
@@ -377,7 +380,7 @@ __device__ __forceinline__ void sr_stage_columns(float* dst, const Rows& src, in
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const int i = i0 + j * step;
-        if (i < items) reinterpret_cast<float4*>(dst)[i] = x[j];
+        if (i < items) *reinterpret_cast<float4*>(dst + (i >> 4) * PITCH + (i & 15) * 4) = x[j];
       }
     }
     return;
@@ -393,7 +396,7 @@ __device__ __forceinline__ void sr_stage_columns(float* dst, const Rows& src, in
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int i = i0 + j * step;
-      if (i < items) dst[i] = x[j];
+      if (i < items) dst[(i >> 6) * PITCH + (i & 63)] = x[j];
     }
   }
 }
@@ -428,7 +431,42 @@ __device__ __forceinline__ void sr_running_max(double& a, double& b) {
 //                     per token, what the scores weigh, the state before the chunk per key channel,
 //                     what the chunk's own tokens give (without SCORES)
 //   NORMALISER        whether rows are divided by max(|sum|, floor_t) + 1e-6 (M's `start_norm`)
-// 256 threads: thread (rg, cg) owns rows 4 rg .. and, in pass n, columns 64 n + 4 cg ..
+// 256 threads: a warp takes 32 tokens and, in pass n, 16 of the columns 64 n ..; the products run on the
+// tensor cores with both operands split (mma_split.cuh), since multiply-adds fed from shared memory in tiles of
+// 4 x 4 are bound by what it delivers.  Retention over 1,024 tokens, 16 heads of 128 channels, all kernels: 98 us
+// against 114, 32 heads of 64: 62 against 70; its error against 64 bits falls from 2.6e-7 to 2.0e-7 and from
+// 2.2e-7 to 1.9e-7.  The delta rule over 2,048 tokens, 32 heads of 64: 80 us of this kernel against 85, bound by
+// the latency of the tiles' loads, which nothing overlaps within a block.
+struct OutTile {            // a warp's 32 x 16 outputs
+  float sum[2][2][4], small[2][2][4];
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int a = 0; a < 2; ++a)
+#pragma unroll
+      for (int b = 0; b < 2; ++b)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sum[a][b][i] = small[a][b][i] = 0.f;
+  }
+  // += X^T Y over `depth` rows (a multiple of 8) of both: x at this lane's place in [k][token], y in [k][column]
+  __device__ __forceinline__ void add(const float* x, const float* y, int ldy, int depth) {
+#pragma unroll 2
+    for (int k = 0; k < depth; k += 8) {
+      SplitA fa[2];
+      split_load_a(fa[0], x + k * SR_TP, 1, SR_TP);
+      split_load_a(fa[1], x + k * SR_TP + 16, 1, SR_TP);
+#pragma unroll
+      for (int b = 0; b < 2; ++b) {
+        SplitB fb;
+        split_load_b(fb, y + k * ldy + 8 * b, ldy);
+        split_mma(sum[0][b], small[0][b], fa[0], fb);
+        split_mma(sum[1][b], small[1][b], fa[1], fb);
+      }
+    }
+  }
+  __device__ __forceinline__ float at(int a, int b, int h, int e) const { return split_join(sum[a][b][2 * h + e], small[a][b][2 * h + e]); }
+};
+
+#define SR_OP (64 + 8)       // pitch of a tile of 64 columns
 template <class M, typename TO, int NP>
 __global__ void __launch_bounds__(256) state_out_kernel(const M m, const StateRun p) {
   extern __shared__ __align__(16) float smem[];
@@ -436,120 +474,134 @@ __global__ void __launch_bounds__(256) state_out_kernel(const M m, const StateRu
   pdl_wait();
   ChunkAt at;
   if (!sr_locate(p, &at)) return;
-  const int head = blockIdx.x, dk = p.dk, dv = p.dv, tid = threadIdx.x;
+  const int head = blockIdx.x, dk = p.dk, dv = p.dv, tid = threadIdx.x, dk8 = (dk + 7) & ~7;
   __shared__ double rt[SR_LONG], ct[SR_LONG];
   __shared__ float ea[SR_LONG], fl[SR_LONG], den[SR_LONG];
-  __shared__ float part[16][SR_LONG];
-  float* qt = smem;                              // [dk][SR_TP]
-  float* as = qt + dk * SR_TP;                   // [SR_LONG tokens j][SR_TP tokens t] (SCORES only)
-  float* tile = as + (M::SCORES ? SR_LONG * SR_TP : 0);   // keys [dk][SR_TP], then tiles of 64 columns
-  const int rg = tid & 15, cg = tid >> 4, row = 4 * rg;
+  __shared__ float part[4][SR_LONG];
+  float* qt = smem;                              // [dk8][SR_TP]; rows past dk are zero
+  float* as = qt + dk8 * SR_TP;                  // [SR_LONG tokens j][SR_TP tokens t] (SCORES only)
+  float* tile = as + (M::SCORES ? SR_LONG * SR_TP : 0);   // keys [dk8][SR_TP], then tiles of 64 columns
+  const int warp = tid >> 5, lane = tid & 31, fg = lane >> 2, fq = lane & 3;
+  const int m0 = (warp >> 2) * 32, n0 = (warp & 3) * 16;
+  const float* x_at = qt + fq * SR_TP + m0 + fg;
   sr_stage_transposed(qt, m.queries(p, head, at), dk, at.count, m.query_mul());
-  if constexpr (M::SCORES) sr_stage_transposed(tile, m.keys(p, head, at), dk, at.count);
+  for (int i = tid; i < (dk8 - dk) * SR_TP; i += 256) qt[dk * SR_TP + i] = 0.f;
+  if constexpr (M::SCORES) {
+    sr_stage_transposed(tile, m.keys(p, head, at), dk, at.count);
+    for (int i = tid; i < (dk8 - dk) * SR_TP; i += 256) tile[dk * SR_TP + i] = 0.f;
+  }
   if (tid < 32) m.out_begin(p, head, at, rt, ct, ea, fl);
   __syncthreads();
   if constexpr (M::SCORES) {
-    float a[4][4] = {};
-    if (4 * cg <= row + 3) sr_mm44(a, qt, SR_TP, tile, SR_TP, dk, row, 4 * cg);
+    OutTile s;
+    s.clear();
+    if (n0 <= m0 + 31) s.add(x_at, tile + fq * SR_TP + n0 + fg, SR_TP, dk8);
 #pragma unroll
-    for (int b = 0; b < 4; ++b) {
-      const int j = 4 * cg + b;
-      float w[4];
+    for (int a = 0; a < 2; ++a)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int t = row + e;
-        w[e] = (j <= t && t < at.count) ? a[e][b] * expf((float)(rt[t] + ct[j])) : 0.f;
-      }
-      store4(as + j * SR_TP + row, w);
-    }
+      for (int b = 0; b < 2; ++b)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int t = m0 + 16 * a + 8 * (i >> 1) + fg, j = n0 + 8 * b + 2 * fq + (i & 1);
+          as[j * SR_TP + t] = (j <= t && t < at.count) ? s.at(a, b, i >> 1, i & 1) * expf((float)(rt[t] + ct[j])) : 0.f;
+        }
     __syncthreads();
     if constexpr (M::NORMALISER) {
       // four threads a token: the sum of its weights and its query against the start normaliser
       const int t = tid >> 2, g = tid & 3;
-      const float* n0 = m.start_norm(p, head, at);
+      const float* nrm = m.start_norm(p, head, at);
       float own = 0.f, old = 0.f;
 #pragma unroll 4
       for (int j = g; j < SR_LONG; j += 4) own += as[j * SR_TP + t];
 #pragma unroll 4
-      for (int d = g; d < dk; d += 4) old = fmaf(qt[d * SR_TP + t], n0[d], old);
+      for (int d = g; d < dk; d += 4) old = fmaf(qt[d * SR_TP + t], nrm[d], old);
       own = sr_column_sum(fmaf(ea[t], old, own), 4);
       if (g == 0) den[t] = 1.f / (fmaxf(fabsf(own), fl[t]) + 1e-6f);
     }
   }
-  float acc[NP][4][4];
-  float ss[4] = {0.f, 0.f, 0.f, 0.f};
+  float acc[NP][2][2][4];
+  float ss[2][2] = {};
 #pragma unroll
   for (int n = 0; n < NP; ++n) {
-    const int c0 = 64 * n, col = c0 + 4 * cg;
-    float own[4][4] = {}, old[4][4] = {};
+    const int c0 = 64 * n;
+    OutTile own, old;
+    own.clear();
+    old.clear();
     if constexpr (M::SCORES) {
       __syncthreads();
-      sr_stage_columns(tile, m.others(p, head, at), SR_LONG, at.count, c0, dv);
+      sr_stage_columns<SR_OP>(tile, m.others(p, head, at), SR_LONG, at.count, c0, dv);
       __syncthreads();
-      sr_mm44(own, as, SR_TP, tile, 64, min(at.count, row + 4), row, 4 * cg);
+      own.add(as + fq * SR_TP + m0 + fg, tile + fq * SR_OP + n0 + fg, SR_OP, min((at.count + 7) & ~7, m0 + 32));
     }
     __syncthreads();
-    sr_stage_columns(tile, m.starts(p, head, at), dk, dk, c0, dv);
+    sr_stage_columns<SR_OP>(tile, m.starts(p, head, at), dk8, dk, c0, dv);
     __syncthreads();
-    sr_mm44(old, qt, SR_TP, tile, 64, dk, row, 4 * cg);
+    old.add(x_at, tile + fq * SR_OP + n0 + fg, SR_OP, dk8);
 #pragma unroll
-    for (int a = 0; a < 4; ++a) {
-      const int t = row + a;
+    for (int a = 0; a < 2; ++a)
 #pragma unroll
-      for (int b = 0; b < 4; ++b) {
-        float x = fmaf(ea[t], old[a][b], own[a][b]);
-        if constexpr (!M::SCORES) x += (t < at.count && col + b < dv) ? m.locals(p, head, at).row(t)[col + b] : 0.f;
-        if constexpr (M::NORMALISER) x *= den[t];
-        acc[n][a][b] = x;
-        ss[a] = fmaf(x, x, ss[a]);
-      }
-    }
+      for (int b = 0; b < 2; ++b)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int h = i >> 1, t = m0 + 16 * a + 8 * h + fg, c = c0 + n0 + 8 * b + 2 * fq + (i & 1);
+          float x = fmaf(ea[t], old.at(a, b, h, i & 1), own.at(a, b, h, i & 1));
+          if constexpr (!M::SCORES) x += (t < at.count && c < dv) ? m.locals(p, head, at).row(t)[c] : 0.f;
+          if constexpr (M::NORMALISER) x *= den[t];
+          acc[n][a][b][i] = x;
+          ss[a][h] = fmaf(x, x, ss[a][h]);
+        }
   }
 #pragma unroll
-  for (int a = 0; a < 4; ++a) part[cg][row + a] = ss[a];
+  for (int a = 0; a < 2; ++a)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float sum = ss[a][h];
+      sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+      sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+      if (fq == 0) part[warp & 3][m0 + 16 * a + 8 * h + fg] = sum;
+    }
   __syncthreads();
   const float* w = p.norm_w == nullptr ? nullptr : p.norm_w + (size_t)head * p.norm_stride;
-  const bool wide = (dv & 3) == 0 && (p.norm_stride & 3) == 0 && (p.gate_ld & 3) == 0 &&
-                    (((uintptr_t)p.norm_w | (uintptr_t)p.gate | (uintptr_t)p.out) & 15) == 0;
+  const bool wide = (dv & 1) == 0 && (p.norm_stride & 1) == 0 && (p.gate_ld & 1) == 0 &&
+                    (((uintptr_t)p.norm_w | (uintptr_t)p.gate | (uintptr_t)p.out) & 7) == 0;
 #pragma unroll
-  for (int a = 0; a < 4; ++a) {
-    const int t = row + a;
-    if (t >= at.count) continue;
-    float sum = 0.f;
+  for (int a = 0; a < 2; ++a)
 #pragma unroll
-    for (int g = 0; g < 16; ++g) sum += part[g][t];
-    const float inv = 1.f / sqrtf(sum / (float)dv + p.eps);
-    const float* g = p.gate + (size_t)(at.first + t) * p.gate_ld + (size_t)head * dv;
-    TO* dst = (TO*)p.out + ((size_t)(at.first + t) * p.heads + head) * dv;
+    for (int h = 0; h < 2; ++h) {
+      const int t = m0 + 16 * a + 8 * h + fg;
+      if (t >= at.count) continue;
+      const float inv = 1.f / sqrtf((part[0][t] + part[1][t] + part[2][t] + part[3][t]) / (float)dv + p.eps);
+      const float* gate = p.gate + (size_t)(at.first + t) * p.gate_ld + (size_t)head * dv;
+      TO* dst = (TO*)p.out + ((size_t)(at.first + t) * p.heads + head) * dv;
 #pragma unroll
-    for (int n = 0; n < NP; ++n) {
-      const int c = 64 * n + 4 * cg;
-      if (wide) {
-        if (c >= dv) continue;
-        float wv[4] = {1.f, 1.f, 1.f, 1.f}, gv[4], y[4];
-        if (w != nullptr) load4(w + c, wv);
-        load4(g + c, gv);
+      for (int n = 0; n < NP; ++n)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) y[b] = acc[n][a][b] * inv * wv[b] * sr_gate(gv[b], p.gate_act);
-        store4(dst + c, y);
-      } else {
-#pragma unroll
-        for (int b = 0; b < 4; ++b)
-          if (c + b < dv) dst[c + b] = from_float<TO>(acc[n][a][b] * inv * (w == nullptr ? 1.f : w[c + b]) * sr_gate(g[c + b], p.gate_act));
-      }
+        for (int b = 0; b < 2; ++b) {
+          const int c = 64 * n + n0 + 8 * b + 2 * fq;
+          const float x0 = acc[n][a][b][2 * h] * inv, x1 = acc[n][a][b][2 * h + 1] * inv;
+          if (wide) {
+            if (c >= dv) continue;
+            float2 wv = make_float2(1.f, 1.f);
+            if (w != nullptr) wv = *reinterpret_cast<const float2*>(w + c);
+            const float2 gv = *reinterpret_cast<const float2*>(gate + c);
+            sr_store2(dst + c, x0 * wv.x * sr_gate(gv.x, p.gate_act), x1 * wv.y * sr_gate(gv.y, p.gate_act));
+          } else {
+            if (c < dv) dst[c] = from_float<TO>(x0 * (w == nullptr ? 1.f : w[c]) * sr_gate(gate[c], p.gate_act));
+            if (c + 1 < dv) dst[c + 1] = from_float<TO>(x1 * (w == nullptr ? 1.f : w[c + 1]) * sr_gate(gate[c + 1], p.gate_act));
+          }
+        }
     }
-  }
 }
 
 static size_t state_out_smem(int dk, bool scores) {
-  const size_t keys = scores ? (size_t)dk * SR_TP : 0, cols = (size_t)dk * 64;
-  size_t tile = keys > cols ? keys : cols;
-  if (scores && tile < SR_LONG * 64) tile = SR_LONG * 64;
-  return sizeof(float) * ((size_t)dk * SR_TP + (scores ? SR_LONG * SR_TP : 0) + tile);
+  const size_t dk8 = (size_t)(dk + 7) / 8 * 8;
+  size_t tile = scores ? dk8 * SR_TP : dk8 * SR_OP;
+  if (scores && tile < SR_LONG * SR_OP) tile = SR_LONG * SR_OP;
+  return sizeof(float) * (dk8 * SR_TP + (scores ? SR_LONG * SR_TP : 0) + tile);
 }
 
 // Sizes the chunk kernels take; others are walked whatever their length.
-static bool chunk_takes(int dk, int dv, bool scores) { return dv <= 256 && state_out_smem(dk, scores) <= 200 * 1024; }
+static bool chunk_takes(int dk, int dv, bool scores) { return dv <= 256 && state_out_smem(dk, scores) <= 218 * 1024; }
 
 template <class M>
 static int launch_out(const M& m, const StateRun& p, int out_dtype, int entries, int chunks, cudaStream_t stream) {

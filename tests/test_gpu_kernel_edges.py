@@ -166,6 +166,46 @@ def test_gated_recurrence_chunks(native, heads, dk, dv, lead, counts):
     assert torch.equal(got_state[-1].cpu(), state[-1])       # the row of no entry
 
 
+# -- delta rule: chunks ---------------------------------------------------------------------------
+@pytest.mark.parametrize("kv_heads, heads, dk, dv", ((1, 2, 64, 64), (2, 2, 72, 40), (1, 1, 128, 128), (1, 2, 192, 36), (2, 4, 6, 10), (1, 1, 13, 5), (1, 1, 65, 129)))
+@pytest.mark.parametrize("counts", ([96], [97, 160, 3], [191, 1, 192, 130]))
+def test_delta_rule_chunks(native, kv_heads, heads, dk, dv, counts):
+    """Heads that fill the fragments' eights and heads that do not (odd ones among them), chunks that are whole
+    and that are cut, entries that are walked between them; from states that are not zero."""
+    gen = torch.Generator().manual_seed(heads * 100 + dk + dv)
+    n, qk = sum(counts), kv_heads * dk
+    rand = lambda *shape: torch.randn(*shape, generator=gen)  # noqa: E731
+    unit = lambda x: x / x.norm(dim=-1, keepdim=True)  # noqa: E731
+    q, k, v = unit(rand(n, kv_heads, dk)) * dk**-0.5, unit(rand(n, kv_heads, dk)), rand(n, heads, dv)
+    qkv = torch.cat((q.reshape(n, qk), k.reshape(n, qk), v.reshape(n, -1)), dim=1)
+    gates = torch.stack((torch.rand(n, heads, generator=gen), -2.0 * torch.rand(n, heads, generator=gen) ** 4), dim=-1)
+    gates[7::31, :, 1] = -60.0                               # the state all but forgotten
+    gate, norm, state = rand(n, heads * dv), 1 + 0.2 * rand(dv), rand(len(counts) + 1, heads, dk, dv)
+    cu = [0]
+    for c in counts:
+        cu.append(cu[-1] + c)
+    ints = lambda values: torch.tensor(values, dtype=torch.int32, device=DEV)  # noqa: E731
+    got_state, out, status = state.to(DEV), torch.empty(n, heads * dv, device=DEV), status_word()
+    native.delta_rule(qkv.to(DEV), gates.to(DEV), gate.to(DEV), norm.to(DEV), 1e-3, got_state, ints(list(range(len(counts)))),
+                      ints(cu), out, kv_heads, len(counts), max(counts), status)
+    assert int(status.item()) == 0
+    group = lambda x: x.double().repeat_interleave(heads // kv_heads, dim=1)  # noqa: E731
+    q, k, v, beta, g = group(q), group(k), v.double(), gates[..., 0].double(), gates[..., 1].double().exp()
+    for e in range(len(counts)):
+        s = state[e].double()
+        want = torch.empty(counts[e], heads, dv, dtype=torch.float64)
+        for i, t in enumerate(range(cu[e], cu[e + 1])):
+            s = g[t][:, None, None] * s
+            u = beta[t][:, None] * (v[t] - torch.einsum("hkv,hk->hv", s, k[t]))
+            s = s + k[t][:, :, None] * u[:, None, :]
+            want[i] = torch.einsum("hkv,hk->hv", s, q[t])
+        want = (want * torch.rsqrt((want * want).mean(-1, keepdim=True) + 1e-3) * norm.double()).reshape(counts[e], -1)
+        want *= torch.nn.functional.silu(gate[cu[e] : cu[e + 1]].double())
+        assert float((out[cu[e] : cu[e + 1]].cpu().double() - want).abs().max()) <= 2e-5 * max(1.0, float(want.abs().max()))
+        assert float((got_state[e].cpu().double() - s).abs().max()) <= 1e-5 * max(1.0, float(s.abs().max()))
+    assert torch.equal(got_state[-1].cpu(), state[-1])       # the row of no entry
+
+
 # -- delta rule's inputs ---------------------------------------------------------------------------
 @pytest.mark.parametrize("taps, dk, dv", ((2, 64, 64), (3, 32, 20), (4, 128, 128), (4, 40, 64), (4, 6, 10), (5, 64, 64)))
 @pytest.mark.parametrize("counts", ([256], [1, 2, 3, 270, 1], [100, 100, 57]))
