@@ -1279,11 +1279,11 @@ FE_EXPORT int SYM(fe_attention_prefill_expanded_d)(const void* q, int q_stride, 
   if (!rc) rc = make_rows_map(&mk, k, heads * D, pages * TC5_KEYS, row_elems);
   if (!rc) rc = make_rows_map(&mv, v, heads * D, pages * TC5_KEYS, row_elems);
   if (rc) return rc;
-  const cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc5_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC5_SMEM);
+  const cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc5_kernel<false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC5_SMEM);
   if (e != cudaSuccess) return (int)e;
   const int query_blocks = (max_new + TC5_BLOCK_ROWS - 1) / TC5_BLOCK_ROWS;
   if (query_blocks > 65535) return FE_ERR_TOO_LARGE;
-  rc = fe_launch_dependent(attn_prefill_tc5_kernel<false>, dim3(heads, entries, query_blocks), dim3(TC5_THREADS), TC5_SMEM, stream, mq, mk, mv, p);
+  rc = fe_launch_dependent(attn_prefill_tc5_kernel<false, false, true>, dim3(heads, entries, query_blocks), dim3(TC5_THREADS), TC5_SMEM, stream, mq, mk, mv, p);
   return rc ? rc : fe_last_error();
 }
 

@@ -32,7 +32,7 @@ constexpr int TC5_THREADS = 320;
 constexpr int TC5_K_STAGES = 2;      // key tiles in flight
 constexpr int TC5_V_STAGES = 3;      // value tiles in flight: a value tile is needed a whole step after its keys
 constexpr int TC5_TMEM_COLS = 512;
-constexpr int TC5_COL_S = 0;         // + 128 x: 128 columns of 32-bit scores; P over the first 64
+constexpr int TC5_COL_S = 0;         // + 128 x: 128 columns of 32-bit scores; P over the first 64 (its remainder over the others)
 constexpr int TC5_COL_O = 256;       // + 128 x: D columns of 32-bit output accumulators
 constexpr float TC5_RESCALE_STEP = 8.f;   // in log2 units
 
@@ -215,7 +215,9 @@ __device__ __forceinline__ float tc5_tanh(float x) {
 // DIST_BIAS: with a learned bias by distance (AttnParams::dist_bias); SOFTCAP: scores capped by
 // cap tanh(score / cap) (AttnParams::cap_over_scale).  Each an instantiation of its own, so that
 // the plain one keeps its registers.
-template <bool DIST_BIAS, bool SOFTCAP = false>
+// REST: the weights go into the value product as two bfloat16 numbers, the rounded weight and the rounded
+// remainder (P fills half of its scores' columns, the remainder the other half), as in the general kernels.
+template <bool DIST_BIAS, bool SOFTCAP = false, bool REST = false>
 __global__ void __launch_bounds__(TC5_THREADS, 1)
 attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                         const __grid_constant__ CUtensorMap map_v, AttnParams p) {
@@ -399,6 +401,11 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
 #pragma unroll
             for (int kk = 1; kk < TC5_KEYS / 16; ++kk)
               tc5_mma_ts_acc(o_dst, p_src + kk * 8, vb + (uint64_t)(kk * (2048 >> 4)), idesc_pv);
+            if constexpr (REST) {
+#pragma unroll
+              for (int kk = 0; kk < TC5_KEYS / 16; ++kk)
+                tc5_mma_ts_acc(o_dst, p_src + TC5_KEYS / 2 + kk * 8, vb + (uint64_t)(kk * (2048 >> 4)), idesc_pv);
+            }
             ++done[x];
           }
           if (more && active(x, i + 1)) {
@@ -495,7 +502,7 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       uint64_t sum_a = tc5_pair(0.f, 0.f), sum_b = sum_a;
 #pragma unroll
       for (int c = 0; c < TC5_KEYS / 32; ++c) {
-        unsigned packed[16];
+        unsigned packed[16], rest[REST ? 16 : 1];
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           float e0, e1;
@@ -504,9 +511,12 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
           if (j & 1) sum_b = tc5_add2(sum_b, tc5_pair(e0, e1));
           else sum_a = tc5_add2(sum_a, tc5_pair(e0, e1));
           packed[j] = pack_bf16(e0, e1);
+          if constexpr (REST)
+            rest[j] = pack_bf16(e0 - __uint_as_float(packed[j] << 16), e1 - __uint_as_float(packed[j] & 0xffff0000u));
         }
         // P over the scores' own columns: this row's scores are all in registers by now
         tc5_st16(s_addr + c * 16, packed);
+        if constexpr (REST) tc5_st16(s_addr + TC5_KEYS / 2 + c * 16, rest);
       }
       float sum0, sum1;
       tc5_unpair(tc5_add2(sum_a, sum_b), sum0, sum1);

@@ -41,8 +41,8 @@ from .linear import Linear, fused_rows
 # Portions of more than EXPAND_FROM tokens are expanded, in steps of more than EXPAND_STEP tokens.  Which
 # rows of a step's expansion belong to whom depends on every entry's length, so such a step could not be
 # replayed for another one: the line is the most tokens a replayed step has (engine/graphs.py).  1,500
-# tokens after 500 (32 heads, 64 + 32 / 64, rank 256): 464 us in the absorbed form, 52 us after
-# the expansion, which takes 34 us itself; 128 tokens are where a head's 128-row tile is full.
+# tokens after 500 (32 heads, 64 + 32 / 64, rank 256): the mixer takes 575 us in the absorbed
+# form (464 of them attention), 196 to 204 expanded; 128 tokens are where a head's 128-row tile is full.
 EXPAND_FROM = 128
 EXPAND_STEP = max(512, int(os.environ.get("FORGE_ENGINE_GRAPH_TOKENS", "512")))
 
