@@ -77,7 +77,6 @@ class LatentAttention(Mixer):
         self.sinks = None
         if getattr(spec, "sink", False):
             self.sinks = weights[name("sink")].to(device=ctx.device, dtype=torch.float32).contiguous()
-        self.plan_key = ("latent_attention", self.h, self.kv_rank, self.r, self.window)
         self.expanded = None
         wide = native.EXPANDED_DIM
         # the expanded form: both sizes fit the kernel's head, outputs are stored 32 at a time
@@ -94,6 +93,8 @@ class LatentAttention(Mixer):
             queries[:, : self.d + self.r] = self.up_q.weight.view(self.h, self.d + self.r, self.q_rank)
             self.expanded = (Linear(both.view(2 * self.h * wide, -1), status=ctx.status),
                              Linear(queries.view(self.h * wide, -1), status=ctx.status))
+        # layers share a step's plan only where all of them can carry it out
+        self.plan_key = ("latent_attention", self.h, self.kv_rank, self.r, self.window, self.expanded is not None)
 
     def plan_step(self, entries: list, page_size: int, plans: dict) -> None:
         """The host's decision for a step of ``entries`` ((slot, cached, new) each; layers of one

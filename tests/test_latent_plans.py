@@ -1,0 +1,42 @@
+"""What latent attention layers decide on the host for a step."""
+
+from __future__ import annotations
+
+import itertools
+
+import pytest
+import torch
+
+from forge_engine_b200.config.registry import read_model_config
+from forge_engine_b200.parts.base import BuildContext
+from forge_engine_b200.parts.latent_attention import LatentAttention
+
+
+def mixers(layers, heads=2, rank=32, rot=32, q_rank=16, width=32, wide=()):
+    """A mixer per (dim, vdim) of ``layers``, with weights on the CPU; layers ``wide`` store their key expansion
+    in 32 bits."""
+    raw = {"architecture": "Zofadra", "vocab": 32, "width": width, "norm": {"eps": 1e-5}, "layers": [
+        {"type": "latent_attention", "mixer": {"heads": heads, "dim": dim, "rot_dim": rot, "vdim": vdim, "q_rank": q_rank, "kv_rank": rank,
+                                               "rot": {"base": 1e4, "dims": rot}, "scale": (dim + rot) ** -0.5}} for dim, vdim in layers]}
+    _, _, spec = read_model_config(raw)
+    made = []
+    for i, layer in enumerate(spec.layers):
+        weights = {name: torch.zeros(info.shape, dtype=torch.float32 if i in wide and name.endswith("uk") else torch.bfloat16)
+                   for name, info in LatentAttention.weight_shapes(layer.mixer).items()}
+        made.append(LatentAttention(layer.mixer, weights, BuildContext(torch.bfloat16, torch.device("cpu"), None)))
+    return made
+
+
+@pytest.mark.parametrize("sizes, wide", (([(64, 64), (128, 128), (96, 48)], ()), ([(64, 64), (64, 64)], (1,))))
+def test_a_layer_is_given_a_plan_it_can_carry_out(sizes, wide):
+    """Layers of the same heads, rank and rotated part, of which some cannot expand keys and values (heads too
+    wide, values not in thirty-twos, a matrix stored in 32 bits), in every order: a plan expands entries where
+    the layer can, and only there."""
+    can = [dim + 32 <= 128 and vdim <= 128 and vdim % 32 == 0 and i not in wide for i, (dim, vdim) in enumerate(sizes)]
+    for order in itertools.permutations(range(len(sizes))):
+        made, plans = mixers([sizes[i] for i in order], wide=[order.index(i) for i in wide]), {}
+        for mixer in made:
+            mixer.plan_step([(0, 0, 600)], 16, plans)
+        for i, mixer in zip(order, made):
+            assert (mixer.expanded is not None) == can[i]
+            assert (plans[mixer.plan_key][1] is not None) == can[i], order
