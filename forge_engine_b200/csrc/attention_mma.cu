@@ -1253,13 +1253,12 @@ FE_EXPORT int SYM(fe_attention_prefill_tc5_d)(const void* q, int q_stride, void*
 // token t's keys of all heads, `row_elems` elements after row t - 1, head h's D of them from column h * D
 // on; "page" j of the table is rows 128 j .. 128 j + 127, rows past an entry's last token are zero.  Every
 // head has its own keys.  out is [tokens, heads * out_dim]: the first out_dim of a head's D sums (a multiple
-// of 32).  Entries with more than `row_lo` new tokens.
+// of 32).
 FE_EXPORT int SYM(fe_attention_prefill_expanded_d)(const void* q, int q_stride, void* out, int out_dim, const void* k, const void* v,
                                                    long long row_elems, const int* table, int max_pages, int pages, int heads,
                                                    const int* cu_tokens, const int* starts, int entries, int max_new, int total_tokens,
-                                                   int window, float scale, int row_lo, const float* sinks, int* status,
-                                                   cudaStream_t stream) {
-  if (entries <= 0 || max_new <= row_lo) return 0;
+                                                   int window, float scale, const float* sinks, int* status, cudaStream_t stream) {
+  if (entries <= 0 || max_new <= 0) return 0;
   if (window < 0 || scale <= 0.f || (D != 128 && D != 64) || out_dim <= 0 || out_dim > D || out_dim % 32 || row_elems < (long long)heads * D)
     return FE_ERR_BAD_SHAPE;
   if (!ensure_encode()) return FE_ERR_BAD_SHAPE;
@@ -1271,7 +1270,7 @@ FE_EXPORT int SYM(fe_attention_prefill_expanded_d)(const void* q, int q_stride, 
   p.block_table = table; p.max_pages = max_pages; p.page_size = TC5_KEYS; p.num_pages = pages;
   p.nkv = heads; p.groups = 1; p.cu_tokens = cu_tokens; p.starts = starts;
   p.window = window; p.scale_log2 = scale * 1.4426950408889634f; p.status = status;
-  p.row_lo = row_lo; p.row_hi = 0x7fffffff;
+  p.row_lo = 0; p.row_hi = 0x7fffffff;
   p.num_splits = 1; p.ws_acc = nullptr; p.ws_ml = nullptr; p.ws_count = nullptr; p.cluster_merge = 0;
   p.sinks = sinks; p.head_cols = D; p.out_dim = out_dim;
   CUtensorMap mk, mv, mq;

@@ -220,11 +220,10 @@ def latent_rows(cache: torch.Tensor, block_table: torch.Tensor, where: torch.Ten
 
 def attention_prefill_expanded(q: torch.Tensor, kv: torch.Tensor, out: torch.Tensor, table: torch.Tensor, cu_tokens: torch.Tensor,
                                starts: torch.Tensor, n_entries: int, max_new: int, heads: int, out_dim: int, window: int | None,
-                               scale: float, row_lo: int, sinks: torch.Tensor | None, status: torch.Tensor) -> None:
+                               scale: float, sinks: torch.Tensor | None, status: torch.Tensor) -> None:
     """The tcgen05 prefill attention over keys and values expanded for this step: ``q`` [N, heads * 128], ``kv``
     [rows, 2 * heads * 128] (a token's keys of all heads, then its values; padded with zeros), ``table`` [entries, L]:
-    which stretch of 128 rows holds positions 128 j .. of an entry (-1: none).  ``out`` [N, heads * out_dim] is written
-    for entries of more than ``row_lo`` new tokens."""
+    which stretch of 128 rows holds positions 128 j .. of an entry (-1: none).  ``out`` [N, heads * out_dim]."""
     _dense(q, "q"), _dense(kv, "kv"), _dense(out, "out"), _dense(table, "table")
     d = EXPANDED_DIM
     n, rows = q.shape[0], kv.shape[0]
@@ -234,12 +233,12 @@ def attention_prefill_expanded(q: torch.Tensor, kv: torch.Tensor, out: torch.Ten
     fn = getattr(_attention_handle(d), f"fe_attention_prefill_expanded_d{d}")
     if not getattr(fn, "_declared", False):
         p, i, f, ll = c_void_p, c_int, c_float, ctypes.c_longlong
-        fn.argtypes = [p, i, p, i, p, p, ll, p, i, i, i, p, p, i, i, i, i, f, i, p, p, p]
+        fn.argtypes = [p, i, p, i, p, p, ll, p, i, i, i, p, p, i, i, i, i, f, p, p, p]
         fn.restype = c_int
         fn._declared = True
     check(fn(ptr(q), heads * d, ptr(out), int(out_dim), ptr(kv), ptr(kv) + heads * d * 2, 2 * heads * d, ptr(table), table.shape[1],
              rows // PREFILL_TC5_KEYS, heads, ptr(cu_tokens), ptr(starts), int(n_entries), int(max_new), n, int(window or 0),
-             float(scale), int(row_lo), ptr(sinks), ptr(status), stream()), "attention_prefill_expanded")
+             float(scale), ptr(sinks), ptr(status), stream()), "attention_prefill_expanded")
 
 
 def _attention_handle(head_dim: int):

@@ -45,6 +45,80 @@ from .linear import Linear, fused_rows
 # form (464 of them attention), 196 to 204 expanded; 128 tokens are where a head's 128-row tile is full.
 EXPAND_FROM = 128
 EXPAND_STEP = max(512, int(os.environ.get("FORGE_ENGINE_GRAPH_TOKENS", "512")))
+# A step that holds other entries too runs both forms, each on the rows of its own entries, and the host launches
+# a layer's mixer almost twice (about 100 us more): there the portions are expanded only where the absorbed
+# attention over them takes longer than that.  Its operations, two per multiply-add, at about 1.4e14 a second.
+# Steps of 6 layers of width 2,560, 32 heads, us a layer, absorbed / both: rank 256, 8 decoding and 510 tokens
+# (4.5e9) 433 / 468, 8 and 700 (8.5e9) 486 / 501, 48 and 1,000 (1.7e10) 675 / 598, 100 and 500 after 2,000 (3.9e10)
+# 927 / 726; rank 512, 100 and 430 (6.4e9) 767 / 794, 16 and twice 257 (2.2e10) 566 / 496; width 1,024, 16
+# heads, 8 and 700 (4.3e9) 364 / 453, 100 and 500 after 2,000 (2.0e10) 654 / 682.
+EXPAND_BESIDE = 2e10
+
+
+class _Rows:
+    """Entries of a step that take the same form, as a batch of their own: which rows of the step are theirs (None:
+    all, a slice, or an index), and the integers of that batch."""
+
+    def __init__(self, batch) -> None:
+        """All entries of the step."""
+        self.tokens = self.of_table = None
+        self.n_tokens, self.n_entries, self.max_new = batch.n_tokens, batch.n_entries, batch.max_new
+        self.cu_tokens, self.starts, self.positions, self.token_entry = batch.cu_tokens, batch.starts, batch.positions, batch.token_entry
+
+    def pick(self, batch, spans: tuple, chosen: list, flat: list) -> list:
+        """Keep the entries ``chosen`` (in order) of the step's ``spans`` ((cached, new) each).  What the device has
+        to be sent is appended to ``flat``; answers where it lies there, for ``sent``."""
+        first, cu, ends = [], [0], 0
+        for _, count in spans:
+            first.append(ends)
+            ends += count
+        for e in chosen:
+            cu.append(cu[-1] + spans[e][1])
+        self.n_tokens, self.n_entries, self.max_new = cu[-1], len(chosen), max(spans[e][1] for e in chosen)
+        lists = [cu]
+        if chosen[-1] - chosen[0] + 1 == len(chosen):             # neighbours: their rows are a range
+            self.tokens, self.of_table = slice(first[chosen[0]], first[chosen[0]] + cu[-1]), slice(chosen[0], chosen[-1] + 1)
+        else:
+            lists += [[t for e in chosen for t in range(first[e], first[e] + spans[e][1])], chosen,
+                      [i for i, e in enumerate(chosen) for _ in range(spans[e][1])]]
+        return [_place(flat, values) for values in lists]
+
+    def sent(self, batch, flat: torch.Tensor, places: list) -> None:
+        lists = [flat[a:b] for a, b in places]
+        self.cu_tokens = lists[0]
+        if len(lists) > 1:
+            self.tokens, self.of_table, self.token_entry = lists[1].long(), lists[2], lists[3]
+        else:
+            self.token_entry = batch.token_entry[self.tokens] - self.of_table.start
+        self.starts, self.positions = self._take(batch.starts, self.of_table), self._take(batch.positions, self.tokens)
+
+    @staticmethod
+    def _take(x: torch.Tensor, which) -> torch.Tensor:
+        return x if which is None else x[which] if isinstance(which, slice) else x.index_select(0, which)
+
+    def of(self, x: torch.Tensor) -> torch.Tensor:
+        """Their rows of ``x`` [tokens, ...]."""
+        return self._take(x, self.tokens)
+
+    def table(self, table: torch.Tensor) -> torch.Tensor:
+        """Their rows of a block table [entries, pages]."""
+        return self._take(table, self.of_table)
+
+    def room(self, x: torch.Tensor) -> torch.Tensor:
+        """Where their rows of ``x`` are worked out; ``put`` then stores them."""
+        return x.new_empty((self.n_tokens, *x.shape[1:])) if isinstance(self.tokens, torch.Tensor) else self.of(x)
+
+    def put(self, x: torch.Tensor, room: torch.Tensor) -> None:
+        if isinstance(self.tokens, torch.Tensor):
+            x.index_copy_(0, self.tokens, room)
+
+
+def _place(flat: list, values: list) -> tuple:
+    """Append ``values`` to ``flat``, where the next ones begin on a 16-byte boundary again; where they lie."""
+    begin = len(flat)
+    flat += values
+    flat += [0] * (-len(flat) % 4)
+    return begin, begin + len(values)
 
 
 class LatentAttention(Mixer):
@@ -103,56 +177,79 @@ class LatentAttention(Mixer):
         if self.plan_key not in plans:
             short, expanded = list(entries), None
             if self.expanded is not None and sum(count for _, _, count in entries) > EXPAND_STEP:
-                short = [e for e in entries if e[2] <= EXPAND_FROM]
-                if len(short) < len(entries):
+                long = [e for e in entries if e[2] > EXPAND_FROM]
+                if long and (len(long) == len(entries) or 2 * self.h * (2 * self.kv_rank + self.r) * self._pairs(long) > EXPAND_BESIDE):
+                    short = [e for e in entries if e[2] <= EXPAND_FROM]
                     expanded = tuple((start, count) for _, start, count in entries)
             splits = 1 if short else None
             if short and native.general_mma_takes(self.ctx.dtype, self.kv_rank + self.r, self.kv_rank):
                 splits = native.general_splits(short, self.h, 1, self.window)
             plans[self.plan_key] = (splits, expanded)
 
-    def _stretches(self, spans: tuple, batch):
-        """Where the expanded entries' contexts lie in the step's expansion, worked out once a step: int32 on
-        the device, (entry, first position, first position needed) per stretch of 128 rows and [entries, L]
+    def _pairs(self, entries: list) -> int:
+        """How many (query, key) pairs a head works on for the new tokens of ``entries``."""
+        total = 0
+        for _, start, count in entries:
+            whole = max(0, min(count, (self.window or start + count) - start))      # queries that see every earlier token
+            total += whole * start + whole * (whole + 1) // 2 + (count - whole) * (self.window or 0)
+        return total
+
+    def _forms(self, spans: tuple, batch) -> tuple:
+        """The step's rows by the form they take, worked out once a step: (those that take the absorbed one or
+        None, those that are expanded, where the latter's contexts lie in the expansion).  That is, int32 on the
+        device, (entry, first position, first position needed) per stretch of 128 rows, and [expanded entries, L]
         the stretch of positions 128 j .. (-1: none)."""
-        key = (self.plan_key, "stretches")
-        if key not in batch.shared:
-            size = native.PREFILL_TC5_KEYS
-            where, tables = [], []
-            for entry, (start, count) in enumerate(spans):
-                row = []
-                if count > EXPAND_FROM:
-                    needed = max(0, start - self.window + 1) if self.window else 0
-                    first = needed // size
-                    last = -(-(start + count) // size)
-                    row = [-1] * first + [len(where) + j for j in range(last - first)]
-                    where += [(entry, size * j, needed) for j in range(first, last)]
-                tables.append(row)
-            width = max(len(row) for row in tables)
-            flat = [v for stretch in where for v in stretch] + [v for row in tables for v in row + [-1] * (width - len(row))]
-            device = torch.tensor(flat, dtype=torch.int32).pin_memory().to(self.ctx.device, non_blocking=True)
-            batch.shared[key] = device[: 3 * len(where)].view(-1, 3), device[3 * len(where) :].view(len(spans), width)
+        key = (self.plan_key, "forms")
+        if key in batch.shared:
+            return batch.shared[key]
+        size = native.PREFILL_TC5_KEYS
+        short, long, where, tables = [], [], [], []
+        for entry, (start, count) in enumerate(spans):
+            if count <= EXPAND_FROM:
+                short.append(entry)
+                continue
+            long.append(entry)
+            needed = max(0, start - self.window + 1) if self.window else 0
+            first, last = needed // size, -(-(start + count) // size)
+            stretch = len(where) // 3
+            tables.append([-1] * first + list(range(stretch, stretch + last - first)))
+            for j in range(first, last):
+                where += (entry, size * j, needed)
+        width = max(map(len, tables))
+        flat: list = []
+        at = _place(flat, where)
+        of_entry = _place(flat, [v for row in tables for v in row + [-1] * (width - len(row))])
+        parts = [(None, None), (_Rows(batch), None)]
+        if short:
+            parts = [(rows, rows.pick(batch, spans, chosen, flat)) for rows, chosen in ((_Rows(batch), short), (_Rows(batch), long))]
+        device = torch.tensor(flat, dtype=torch.int32).pin_memory().to(self.ctx.device, non_blocking=True)
+        for rows, places in parts:
+            if places is not None:
+                rows.sent(batch, device, places)
+        batch.shared[key] = parts[0][0], parts[1][0], (device[at[0] : at[1]].view(-1, 3), device[of_entry[0] : of_entry[1]].view(len(long), width))
         return batch.shared[key]
 
-    def _attend_expanded(self, c_q, spans: tuple, batch, latent_cache, table, angles, heads) -> None:
-        """The expanded entries' rows of ``heads`` [N, heads * v_head_dim]."""
-        n, h, d, r, wide = c_q.shape[0], self.h, self.d, self.r, native.EXPANDED_DIM
+    def _attend_expanded(self, c_q, rows: _Rows, stretches: tuple, batch, latent_cache, table, angles, heads) -> None:
+        """The rows ``rows`` of ``heads`` [N, heads, v_head_dim]."""
+        h, d, r, dv, wide = self.h, self.d, self.r, self.dv, native.EXPANDED_DIM
         expand, up_q = self.expanded
         with self.ctx.section("mixer.qkv_rope_cache"):
-            q = up_q(c_q)
+            q = up_q(rows.of(c_q))
             native.qkv_prepare(
                 q=q[:, d:], q_heads=h, q_dim=r, q_head_stride=wide, q_rot_off=0,
                 q_out=q, q_out_strides=(h * wide, wide), q_out_offset=d,
-                table=angles, rot_dims=self.rot_dims, interleaved=self.position.interleaved,
-                positions=batch.positions, token_entry=batch.token_entry, status=self.ctx.status,
+                table=rows.of(angles), rot_dims=self.rot_dims, interleaved=self.position.interleaved,
+                positions=rows.positions, token_entry=rows.token_entry, status=self.ctx.status,
             )
-            where, stretches = self._stretches(spans, batch)
-            rows = torch.empty((where.shape[0] * native.PREFILL_TC5_KEYS, self.kv_rank + r), dtype=torch.bfloat16, device=c_q.device)
-            native.latent_rows(latent_cache, table, where, batch.ctx_lens, rows, self.ctx.status)
-            kv = expand(rows)
+            where, of_entry = stretches
+            latents = torch.empty((where.shape[0] * native.PREFILL_TC5_KEYS, self.kv_rank + r), dtype=torch.bfloat16, device=c_q.device)
+            native.latent_rows(latent_cache, table, where, batch.ctx_lens, latents, self.ctx.status)
+            kv = expand(latents)
         with self.ctx.section("mixer.attention"):
-            native.attention_prefill_expanded(q, kv, heads, stretches, batch.cu_tokens, batch.starts, batch.n_entries, batch.max_new,
-                                              h, self.dv, self.window, self.spec.scale, EXPAND_FROM, self.sinks, self.ctx.status)
+            out = rows.room(heads)
+            native.attention_prefill_expanded(q, kv, out.view(rows.n_tokens, h * dv), of_entry, rows.cu_tokens, rows.starts, rows.n_entries,
+                                              rows.max_new, h, dv, self.window, self.spec.scale, self.sinks, self.ctx.status)
+            rows.put(heads, out)
 
     @classmethod
     def weight_shapes(cls, spec) -> dict:
@@ -215,38 +312,42 @@ class LatentAttention(Mixer):
         heads = torch.empty((n, h, dv), dtype=dtype, device=x.device)
         if self.plan_key not in batch.plans:
             self.plan_step(batch.entries, latent_cache.shape[2], batch.plans)
-        splits, expanded = batch.plans[self.plan_key]
-        if splits is not None:
-            self._attend_absorbed(c_q, splits, expanded is not None, batch, latent_cache, table, angles, heads)
-        if expanded is not None:
-            self._attend_expanded(c_q, expanded, batch, latent_cache, table, angles, heads.view(n, h * dv))
+        splits, spans = batch.plans[self.plan_key]
+        if spans is None:
+            self._attend_absorbed(c_q, splits, _Rows(batch), latent_cache, table, angles, heads)
+        else:
+            short, long, stretches = self._forms(spans, batch)
+            if short is not None:
+                self._attend_absorbed(c_q, splits, short, latent_cache, table, angles, heads)
+            self._attend_expanded(c_q, long, stretches, batch, latent_cache, table, angles, heads)
         return heads.view(n, h * dv)
 
-    def _attend_absorbed(self, c_q, splits: int, some_expanded: bool, batch, latent_cache, table, angles, heads) -> None:
-        """All rows of ``heads`` [N, heads, v_head_dim], or with ``some_expanded`` those of the other entries
-        (and anything in theirs)."""
-        n, h, d, r, rank = c_q.shape[0], self.h, self.d, self.r, self.kv_rank
+    def _attend_absorbed(self, c_q, splits: int, rows: _Rows, latent_cache, table, angles, heads) -> None:
+        """The rows ``rows`` of ``heads`` [N, heads, v_head_dim]."""
+        n, h, d, r, rank = rows.n_tokens, self.h, self.d, self.r, self.kv_rank
         with self.ctx.section("mixer.qkv_rope_cache"):
-            q = self.up_q(c_q)                                     # [N, heads * (d + r)]
+            q = self.up_q(rows.of(c_q))                            # [n, heads * (d + r)]
             q_eff = torch.empty((n, h, rank + r), dtype=c_q.dtype, device=c_q.device)
             # rotated parts of the queries straight to where attention reads them
             native.qkv_prepare(
                 q=q[:, d:], q_heads=h, q_dim=r, q_head_stride=d + r, q_rot_off=0,
                 q_out=q_eff, q_out_strides=(h * (rank + r), rank + r), q_out_offset=rank,
-                table=angles, rot_dims=self.rot_dims, interleaved=self.position.interleaved,
-                positions=batch.positions, token_entry=batch.token_entry, status=self.ctx.status,
+                table=rows.of(angles), rot_dims=self.rot_dims, interleaved=self.position.interleaved,
+                positions=rows.positions, token_entry=rows.token_entry, status=self.ctx.status,
             )
             # the other parts through the transposed key expansion
             self._per_head(q.view(n, h, d + r)[:, :, :d], self.uk_t, q_eff[:, :, :rank])
         mixed = torch.empty((n, h, rank), dtype=c_q.dtype, device=c_q.device)
         with self.ctx.section("mixer.attention"):
             native.attention_general(q_eff, (h * (rank + r), rank + r), latent_cache, rank + r, latent_cache, rank,
-                                     mixed, (h * rank, rank), table, batch.positions, batch.token_entry, h, None, self.window,
+                                     mixed, (h * rank, rank), rows.table(table), rows.positions, rows.token_entry, h, None, self.window,
                                      self.spec.scale, self.ctx.status,
-                                     entries=(batch.cu_tokens, batch.starts, batch.n_entries, batch.max_new),
-                                     splits=splits, sinks=self.sinks, row_hi=EXPAND_FROM * h if some_expanded else 0)
+                                     entries=(rows.cu_tokens, rows.starts, rows.n_entries, rows.max_new),
+                                     splits=splits, sinks=self.sinks)
         with self.ctx.section("mixer.expand"):
-            self._per_head(mixed, self.uv, heads)
+            out = rows.room(heads)
+            self._per_head(mixed, self.uv, out)
+            rows.put(heads, out)
 
 
 register_part("latent_attention", LatentAttention, replace=True)

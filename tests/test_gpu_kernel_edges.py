@@ -313,6 +313,7 @@ def test_expanded_latent_attention(native, monkeypatch, window, sink, heads, dim
     results = {}
     for name, step in (("expanded", 512), ("absorbed", 1 << 30)):
         monkeypatch.setattr(part, "EXPAND_STEP", step)
+        monkeypatch.setattr(part, "EXPAND_BESIDE", 0.0)
         runner = ModelRunner.from_tensors(spec, dict(weights), dtype="bfloat16", device=DEV, page_size=16, num_pages=128, max_requests=6,
                                           architecture=arch)
         cache = runner.cache

@@ -40,3 +40,25 @@ def test_a_layer_is_given_a_plan_it_can_carry_out(sizes, wide):
         for i, mixer in zip(order, made):
             assert (mixer.expanded is not None) == can[i]
             assert (plans[mixer.plan_key][1] is not None) == can[i], order
+
+
+@pytest.mark.parametrize("window", (None, 1, 40, 200, 1000))
+def test_pairs_of_queries_and_keys(window):
+    mixer = object.__new__(LatentAttention)
+    mixer.window = window
+    for start in (0, 1, 39, 40, 41, 500):
+        for count in (1, 2, 39, 40, 41, 300):
+            want = sum(min(start + i + 1, window or 10**9) for i in range(count))
+            assert mixer._pairs([(0, start, count)]) == want, (start, count)
+
+
+@pytest.mark.parametrize("decoders, portions, expands", ((0, [(0, 600)], True), (0, [(0, 300), (0, 300)], True), (0, [(0, 512)], False),
+                                                         (8, [(0, 700)], False), (100, [(0, 430)], False), (48, [(2000, 1000)], True)))
+def test_portions_beside_other_entries_are_expanded_where_that_pays_for_both_forms(decoders, portions, expands):
+    """32 heads of rank 256: a step without short entries expands above 512 tokens; beside decoding requests
+    the portions' attention has to be long enough to pay for the second set of launches."""
+    mixer, = mixers([(64, 64)], heads=32, rank=256)
+    entries, plans = [(i, 2000, 1) for i in range(decoders)] + [(99, s, n) for s, n in portions], {}
+    mixer.plan_step(entries, 16, plans)
+    splits, spans = plans[mixer.plan_key]
+    assert (spans is not None) == expands and (splits is None) == (expands and not decoders)
