@@ -86,9 +86,10 @@ struct AttnParams {
   // products, so it is given cap / scale and scale / cap
   float cap_over_scale = 0.f, scale_over_cap = 0.f;
   // above zero: keys and values lie as rows of one token for all heads, head h's from column head_cols * h
-  // on (a page is page_size such rows), and rows of the output hold out_dim elements per head
+  // on (a page is page_size such rows), and rows of the output hold out_dim elements for each of out_heads heads
   int head_cols = 0;
   int out_dim = 0;
+  int out_heads = 0;
 };
 
 __device__ __forceinline__ unsigned smem_addr(const void* p) {
@@ -1249,34 +1250,34 @@ FE_EXPORT int SYM(fe_attention_prefill_tc5_d)(const void* q, int q_stride, void*
   return rc ? rc : fe_last_error();
 }
 
-// The same kernel over keys and values that were expanded for this step: row t of k (and of v) holds
-// token t's keys of all heads, `row_elems` elements after row t - 1, head h's D of them from column h * D
-// on; "page" j of the table is rows 128 j .. 128 j + 127, rows past an entry's last token are zero.  Every
-// head has its own keys.  out is [tokens, heads * out_dim]: the first out_dim of a head's D sums (a multiple
-// of 32).
-FE_EXPORT int SYM(fe_attention_prefill_expanded_d)(const void* q, int q_stride, void* out, int out_dim, const void* k, const void* v,
-                                                   long long row_elems, const int* table, int max_pages, int pages, int heads,
+// The same kernel over keys and values that were expanded for this step: row t of kv holds token t's D
+// keys and then its D values of each of `heads` heads; "page" j of the table is rows 128 j .. 128 j + 127, rows
+// past an entry's last token are zero.  Every head has its own keys.  out is [tokens, out_heads * out_dim], written
+// for these heads: the first out_dim of a head's D sums (a multiple of 32).
+FE_EXPORT int SYM(fe_attention_prefill_expanded_d)(const void* q, int q_stride, void* out, int out_dim, int out_heads, const void* kv,
+                                                   const int* table, int max_pages, int pages, int heads,
                                                    const int* cu_tokens, const int* starts, int entries, int max_new, int total_tokens,
                                                    int window, float scale, const float* sinks, int* status, cudaStream_t stream) {
   if (entries <= 0 || max_new <= 0) return 0;
-  if (window < 0 || scale <= 0.f || (D != 128 && D != 64) || out_dim <= 0 || out_dim > D || out_dim % 32 || row_elems < (long long)heads * D)
+  if (window < 0 || scale <= 0.f || (D != 128 && D != 64) || out_dim <= 0 || out_dim > D || out_dim % 32 || out_heads < heads)
     return FE_ERR_BAD_SHAPE;
   if (!ensure_encode()) return FE_ERR_BAD_SHAPE;
   if (entries > 65535 || heads > 65535 || (long long)pages * TC5_KEYS > 0x7fffffff) return FE_ERR_TOO_LARGE;
-  if ((((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)out) & 15) || q_stride % 8 || row_elems % 8) return FE_ERR_BAD_ALIGN;
+  if ((((uintptr_t)q | (uintptr_t)kv | (uintptr_t)out) & 15) || q_stride % 8) return FE_ERR_BAD_ALIGN;
   AttnParams p;
   p.q = (const bf16*)q; p.q_stride = q_stride; p.out = (bf16*)out;
-  p.k = (const bf16*)k; p.v = (const bf16*)v;
+  p.k = (const bf16*)kv; p.v = p.k + D;
   p.block_table = table; p.max_pages = max_pages; p.page_size = TC5_KEYS; p.num_pages = pages;
   p.nkv = heads; p.groups = 1; p.cu_tokens = cu_tokens; p.starts = starts;
   p.window = window; p.scale_log2 = scale * 1.4426950408889634f; p.status = status;
   p.row_lo = 0; p.row_hi = 0x7fffffff;
   p.num_splits = 1; p.ws_acc = nullptr; p.ws_ml = nullptr; p.ws_count = nullptr; p.cluster_merge = 0;
-  p.sinks = sinks; p.head_cols = D; p.out_dim = out_dim;
+  p.sinks = sinks; p.head_cols = 2 * D; p.out_dim = out_dim; p.out_heads = out_heads;
   CUtensorMap mk, mv, mq;
   int rc = make_query_map(&mq, q, q_stride, total_tokens, heads, 1);
-  if (!rc) rc = make_rows_map(&mk, k, heads * D, pages * TC5_KEYS, row_elems);
-  if (!rc) rc = make_rows_map(&mv, v, heads * D, pages * TC5_KEYS, row_elems);
+  const int columns = heads * 2 * D;
+  if (!rc) rc = make_rows_map(&mk, p.k, columns, pages * TC5_KEYS, columns);
+  if (!rc) rc = make_rows_map(&mv, p.v, columns - D, pages * TC5_KEYS, columns);
   if (rc) return rc;
   const cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc5_kernel<false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC5_SMEM);
   if (e != cudaSuccess) return (int)e;

@@ -551,7 +551,7 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       if (p.sinks != nullptr && row_valid)
         l += exp2f(p.sinks[kvh * p.groups + row % p.groups] * 1.4426950408889634f - m_used);
       float inv = l > 0.f ? 1.f / l : 0.f;
-      const int num_q_heads = p.nkv * p.groups;
+      const int num_q_heads = p.out_heads > 0 ? p.out_heads : p.nkv * p.groups;
       const int token = row / p.groups, g = row - token * p.groups;
       if (p.gate != nullptr && p.gate_dim == 0 && row_valid)
         inv *= 1.f / (1.f + expf(-p.gate[(size_t)(tok0 + token) * p.gate_stride + kvh * p.groups + g]));

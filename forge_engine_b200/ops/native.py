@@ -222,21 +222,23 @@ def attention_prefill_expanded(q: torch.Tensor, kv: torch.Tensor, out: torch.Ten
                                starts: torch.Tensor, n_entries: int, max_new: int, heads: int, out_dim: int, window: int | None,
                                scale: float, sinks: torch.Tensor | None, status: torch.Tensor) -> None:
     """The tcgen05 prefill attention over keys and values expanded for this step: ``q`` [N, heads * 128], ``kv``
-    [rows, 2 * heads * 128] (a token's keys of all heads, then its values; padded with zeros), ``table`` [entries, L]:
-    which stretch of 128 rows holds positions 128 j .. of an entry (-1: none).  ``out`` [N, heads * out_dim]."""
-    _dense(q, "q"), _dense(kv, "kv"), _dense(out, "out"), _dense(table, "table")
+    [rows, heads * 2 * 128] (a token's keys and then its values of a head, padded with zeros), ``table`` [entries, L]:
+    which stretch of 128 rows holds positions 128 j .. of an entry (-1: none).  ``out`` [N, heads * out_dim].  ``q`` and
+    ``out`` may be column slices of tensors of more heads."""
+    _dense(kv, "kv"), _dense(table, "table")
     d = EXPANDED_DIM
     n, rows = q.shape[0], kv.shape[0]
     assert q.dtype == kv.dtype == out.dtype == torch.bfloat16 and table.dtype == torch.int32
     assert q.shape[1] == heads * d and kv.shape[1] == 2 * heads * d and rows % PREFILL_TC5_KEYS == 0 and out.shape == (n, heads * out_dim)
+    assert q.stride(1) == out.stride(1) == 1 and out.stride(0) % out_dim == 0
     assert sinks is None or (sinks.dtype == torch.float32 and sinks.is_cuda and sinks.is_contiguous() and sinks.numel() == heads)
     fn = getattr(_attention_handle(d), f"fe_attention_prefill_expanded_d{d}")
     if not getattr(fn, "_declared", False):
-        p, i, f, ll = c_void_p, c_int, c_float, ctypes.c_longlong
-        fn.argtypes = [p, i, p, i, p, p, ll, p, i, i, i, p, p, i, i, i, i, f, p, p, p]
+        p, i, f = c_void_p, c_int, c_float
+        fn.argtypes = [p, i, p, i, i, p, p, i, i, i, p, p, i, i, i, i, f, p, p, p]
         fn.restype = c_int
         fn._declared = True
-    check(fn(ptr(q), heads * d, ptr(out), int(out_dim), ptr(kv), ptr(kv) + heads * d * 2, 2 * heads * d, ptr(table), table.shape[1],
+    check(fn(ptr(q), int(q.stride(0)), ptr(out), int(out_dim), int(out.stride(0)) // int(out_dim), ptr(kv), ptr(table), table.shape[1],
              rows // PREFILL_TC5_KEYS, heads, ptr(cu_tokens), ptr(starts), int(n_entries), int(max_new), n, int(window or 0),
              float(scale), ptr(sinks), ptr(status), stream()), "attention_prefill_expanded")
 

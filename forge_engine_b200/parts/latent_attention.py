@@ -38,12 +38,19 @@ from .base import BuildContext, CacheView, Mixer, WeightInfo, build_part, regist
 from .linear import Linear, fused_rows
 
 
-# Portions of more than EXPAND_FROM tokens are expanded, in steps of more than EXPAND_STEP tokens.  Which
+# Portions of more than EXPAND_FROM tokens (EXPAND_FROM_CHEAP where rank and rotated part are small) are expanded, in steps of more than EXPAND_STEP tokens.  Which
 # rows of a step's expansion belong to whom depends on every entry's length, so such a step could not be
 # replayed for another one: the line is the most tokens a replayed step has (engine/graphs.py).  1,500
 # tokens after 500 (32 heads, 64 + 32 / 64, rank 256): the mixer takes 575 us in the absorbed
 # form (464 of them attention), 196 to 204 expanded; 128 tokens are where a head's 128-row tile is full.
-EXPAND_FROM = 128
+# Kernels of the mixer, absorbed / expanded, us, 129 tokens after 0, 2,000, 16,000 and 60,000 cached ones (32 heads,
+# width 2,560): rank 512 (+ 64) 66 / 43, 338 / 103, 2227 / 512, 8177 / 1774; rank 256 (+ 32) 55 / 41, 195 / 93, 1163 / 470,
+# 4214 / 1623; rank 64 41 / 39, 103 / 86, 527 / 447, 1863 / 1542; rank 32 39 / 37, 88 / 85, 426 / 434, 1488 / 1499; rank 16
+# 39 / 39, 82 / 86, 388 / 438, 1348 / 1510.  The expansion's multiply-adds run several times as fast as those of the
+# absorbed attention, so the context hardly moves the line; the rank does where a query against a key is cheap:
+# up to 64 multiply-adds a head the line lies at 384 tokens (rank 16: 256 tokens after 4,000 131 / 144, 400 after
+# 8,000 288 / 261).
+EXPAND_FROM, EXPAND_FROM_CHEAP, EXPAND_CHEAP = 128, 384, 64
 EXPAND_STEP = max(512, int(os.environ.get("FORGE_ENGINE_GRAPH_TOKENS", "512")))
 # A step that holds other entries too runs both forms, each on the rows of its own entries, and the host launches
 # a layer's mixer almost twice (about 100 us more): there the portions are expanded only where the absorbed
@@ -53,6 +60,9 @@ EXPAND_STEP = max(512, int(os.environ.get("FORGE_ENGINE_GRAPH_TOKENS", "512")))
 # 927 / 726; rank 512, 100 and 430 (6.4e9) 767 / 794, 16 and twice 257 (2.2e10) 566 / 496; width 1,024, 16
 # heads, 8 and 700 (4.3e9) 364 / 453, 100 and 500 after 2,000 (2.0e10) 654 / 682.
 EXPAND_BESIDE = 2e10
+# Keys and values of all heads take 512 bytes a head and token of context, up to this many at a time: heads beyond
+# go through the same buffer after them (one head at least, which is about what the cached latents take).
+EXPAND_BYTES = 1 << 30
 
 
 class _Rows:
@@ -157,16 +167,16 @@ class LatentAttention(Mixer):
         if (self.d + self.r <= wide and self.dv <= wide and self.dv % 32 == 0 and spec.scale > 0 and (self.kv_rank + self.r) % 8 == 0
                 and native.general_mma_takes(ctx.dtype, self.kv_rank + self.r, self.kv_rank)
                 and all(t.dtype == torch.bfloat16 for t in (self.up_q.weight, self.uk_t, self.uv))):
-            # [2 heads x 128, kv_rank + rot_dim]: a head's key rows (expansion, then the identity on the
+            # [heads x 2 x 128, kv_rank + rot_dim]: a head's key rows (expansion, then the identity on the
             # shared part), then its value rows; rows of zeros pad both to 128
-            both = torch.zeros((2, self.h, wide, self.kv_rank + self.r), dtype=torch.bfloat16, device=self.uv.device)
-            both[0, :, : self.d, : self.kv_rank] = self.uk_t.transpose(1, 2)
-            both[0, :, self.d : self.d + self.r, self.kv_rank :] = torch.eye(self.r, dtype=torch.bfloat16, device=self.uv.device)
-            both[1, :, : self.dv, : self.kv_rank] = self.uv
+            both = torch.zeros((self.h, 2, wide, self.kv_rank + self.r), dtype=torch.bfloat16, device=self.uv.device)
+            both[:, 0, : self.d, : self.kv_rank] = self.uk_t.transpose(1, 2)
+            both[:, 0, self.d : self.d + self.r, self.kv_rank :] = torch.eye(self.r, dtype=torch.bfloat16, device=self.uv.device)
+            both[:, 1, : self.dv, : self.kv_rank] = self.uv
             queries = torch.zeros((self.h, wide, self.q_rank), dtype=torch.bfloat16, device=self.uv.device)
             queries[:, : self.d + self.r] = self.up_q.weight.view(self.h, self.d + self.r, self.q_rank)
-            self.expanded = (Linear(both.view(2 * self.h * wide, -1), status=ctx.status),
-                             Linear(queries.view(self.h * wide, -1), status=ctx.status))
+            self.expanded = (both.view(2 * self.h * wide, -1).t(), Linear(queries.view(self.h * wide, -1), status=ctx.status))
+        self.expand_from = EXPAND_FROM_CHEAP if 2 * self.kv_rank + self.r <= EXPAND_CHEAP else EXPAND_FROM
         # layers share a step's plan only where all of them can carry it out
         self.plan_key = ("latent_attention", self.h, self.kv_rank, self.r, self.window, self.expanded is not None)
 
@@ -177,14 +187,19 @@ class LatentAttention(Mixer):
         if self.plan_key not in plans:
             short, expanded = list(entries), None
             if self.expanded is not None and sum(count for _, _, count in entries) > EXPAND_STEP:
-                long = [e for e in entries if e[2] > EXPAND_FROM]
+                long = [e for e in entries if e[2] > self.expand_from]
                 if long and (len(long) == len(entries) or 2 * self.h * (2 * self.kv_rank + self.r) * self._pairs(long) > EXPAND_BESIDE):
-                    short = [e for e in entries if e[2] <= EXPAND_FROM]
+                    short = [e for e in entries if e[2] <= self.expand_from]
                     expanded = tuple((start, count) for _, start, count in entries)
             splits = 1 if short else None
             if short and native.general_mma_takes(self.ctx.dtype, self.kv_rank + self.r, self.kv_rank):
                 splits = native.general_splits(short, self.h, 1, self.window)
             plans[self.plan_key] = (splits, expanded)
+
+    def _heads_at_once(self, rows: int) -> int:
+        """Heads whose keys and values of ``rows`` tokens are held at a time, in stretches that are about equal."""
+        most = max(1, EXPAND_BYTES // (rows * 2 * native.EXPANDED_DIM * 2))
+        return -(-self.h // -(-self.h // most))
 
     def _pairs(self, entries: list) -> int:
         """How many (query, key) pairs a head works on for the new tokens of ``entries``."""
@@ -205,7 +220,7 @@ class LatentAttention(Mixer):
         size = native.PREFILL_TC5_KEYS
         short, long, where, tables = [], [], [], []
         for entry, (start, count) in enumerate(spans):
-            if count <= EXPAND_FROM:
+            if count <= self.expand_from:
                 short.append(entry)
                 continue
             long.append(entry)
@@ -244,12 +259,21 @@ class LatentAttention(Mixer):
             where, of_entry = stretches
             latents = torch.empty((where.shape[0] * native.PREFILL_TC5_KEYS, self.kv_rank + r), dtype=torch.bfloat16, device=c_q.device)
             native.latent_rows(latent_cache, table, where, batch.ctx_lens, latents, self.ctx.status)
-            kv = expand(latents)
-        with self.ctx.section("mixer.attention"):
-            out = rows.room(heads)
-            native.attention_prefill_expanded(q, kv, out.view(rows.n_tokens, h * dv), of_entry, rows.cu_tokens, rows.starts, rows.n_entries,
-                                              rows.max_new, h, dv, self.window, self.spec.scale, self.sinks, self.ctx.status)
-            rows.put(heads, out)
+        room = rows.room(heads)
+        out, most = room.view(rows.n_tokens, h * dv), self._heads_at_once(latents.shape[0])
+        if most == h:
+            turns = [(h, expand, q, out, self.sinks)]
+        else:
+            turns = [(min(h, a + most) - a, expand[:, 2 * wide * a : 2 * wide * (a + most)], q[:, wide * a : wide * (a + most)],
+                      out[:, dv * a : dv * (a + most)], None if self.sinks is None else self.sinks[a : a + most]) for a in range(0, h, most)]
+        for n_heads, weight, queries, into, sinks in turns:
+            with self.ctx.section("mixer.qkv_rope_cache"):
+                kv = torch.mm(latents, weight)
+            with self.ctx.section("mixer.attention"):
+                native.attention_prefill_expanded(queries, kv, into, of_entry, rows.cu_tokens, rows.starts, rows.n_entries, rows.max_new,
+                                                  n_heads, dv, self.window, self.spec.scale, sinks, self.ctx.status)
+            del kv
+        rows.put(heads, room)
 
     @classmethod
     def weight_shapes(cls, spec) -> dict:

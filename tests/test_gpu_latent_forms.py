@@ -2,6 +2,8 @@
 
 from __future__ import annotations
 
+import dataclasses
+
 import pytest
 import torch
 
@@ -16,14 +18,16 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
 
 
-def latent_runner(seed, heads=3, dim=64, rot=32, vdim=64, rank=64, q_rank=64, width=128, pages=128, requests=8):
+def latent_runner(seed, heads=3, dim=64, rot=32, vdim=64, rank=64, q_rank=64, width=128, pages=128, requests=8, sink=False):
     raw = {"architecture": "Zofadra", "vocab": 32, "width": width, "norm": {"eps": 1e-5}, "layers": [{"type": "latent_attention", "mixer": {
         "heads": heads, "dim": dim, "rot_dim": rot, "vdim": vdim, "q_rank": q_rank, "kv_rank": rank,
         "rot": {"base": 1e4, "dims": rot}, "scale": (dim + rot) ** -0.5}}]}
     arch, _, spec = read_model_config(raw)
+    layer = spec.layers[0]
+    spec = dataclasses.replace(spec, layers=(dataclasses.replace(layer, mixer=dataclasses.replace(layer.mixer, sink=sink)),))
     gen = torch.Generator().manual_seed(seed)
     weights = {name: ((1 + 0.1 * torch.randn(info.shape, generator=gen)) if "norm" in name else
-                      torch.randn(info.shape, generator=gen) * info.shape[-1] ** -0.5).bfloat16().to(DEV)
+                      torch.randn(info.shape, generator=gen) * (info.shape[-1] ** -0.5 if len(info.shape) > 1 else 1.0)).bfloat16().to(DEV)
                for name, info in arch.expected_tensors(spec).items()}
     return ModelRunner.from_tensors(spec, weights, dtype="bfloat16", device=DEV, page_size=16, num_pages=pages, max_requests=requests, architecture=arch)
 
@@ -61,7 +65,7 @@ def test_rows_go_through_one_form(starts, counts, monkeypatch):
     monkeypatch.setattr(mixer, "up_q", note("absorbed", mixer.up_q))
     monkeypatch.setattr(mixer, "expanded", (mixer.expanded[0], note("expanded", mixer.expanded[1])))
     got = mixer.attend(x, batch, runner.cache.view(0)).double()
-    short = sum(c for c in counts if c <= part.EXPAND_FROM)
+    short = sum(c for c in counts if c <= mixer.expand_from)
     assert rows == {"absorbed": [short] * 3, "expanded": [sum(counts) - short]}
     monkeypatch.setattr(part, "EXPAND_STEP", 1 << 30)
     batch.plans.clear(), batch.shared.clear()
@@ -69,3 +73,23 @@ def test_rows_go_through_one_form(starts, counts, monkeypatch):
     runner.check_status()
     for a, b in zip(got.split(counts), want.split(counts)):
         assert float((a - b).norm() / b.norm()) < 2e-2
+
+
+@pytest.mark.parametrize("sink", (False, True))
+@pytest.mark.parametrize("heads, at_once", ((3, 2), (5, 1), (8, 3)))
+def test_heads_take_turns(heads, at_once, sink, monkeypatch):
+    """Keys and values held for some heads at a time give what they give for all at once, up to the order of the
+    sums of the product that expands them (its results are bfloat16 numbers: 2^-8 of them)."""
+    starts, counts = [90, 700], [300, 260]
+    runner = latent_runner(heads, heads=heads, sink=sink)
+    x = torch.randn((sum(counts), 128), generator=torch.Generator().manual_seed(1)).bfloat16().to(DEV)
+    batch = cached(runner, starts, counts, 2)
+    mixer = runner.model.blocks[0].mixer
+    whole = mixer.attend(x, batch, runner.cache.view(0)).double()
+    rows, calls = 128 * (4 + 8), []
+    monkeypatch.setattr(part, "EXPAND_BYTES", at_once * rows * 512)
+    monkeypatch.setattr(native, "attention_prefill_expanded", lambda *a, call=native.attention_prefill_expanded: (calls.append(a[8]), call(*a))[1])
+    parts = mixer.attend(x, batch, runner.cache.view(0)).double()
+    runner.check_status()
+    assert sum(calls) == heads and len(calls) > 1 and max(calls) <= at_once
+    assert float((parts - whole).norm() / whole.norm()) < 2.0**-8

@@ -62,3 +62,25 @@ def test_portions_beside_other_entries_are_expanded_where_that_pays_for_both_for
     mixer.plan_step(entries, 16, plans)
     splits, spans = plans[mixer.plan_key]
     assert (spans is not None) == expands and (splits is None) == (expands and not decoders)
+
+
+@pytest.mark.parametrize("rank, rot, least", ((16, 32, 385), (32, 16, 129), (32, 32, 129), (256, 32, 129)))
+def test_portions_are_expanded_from_a_length_that_depends_on_the_rank(rank, rot, least):
+    mixer, = mixers([(64, 64)], rank=rank, rot=rot)
+    for count, spans in ((least - 1, None), (least, ((60, least),) * 8)):
+        plans = {}
+        mixer.plan_step([(i, 60, count) for i in range(8)], 16, plans)
+        assert plans[mixer.plan_key][1] == spans
+
+
+@pytest.mark.parametrize("heads", (1, 3, 32, 128))
+def test_expanded_keys_and_values_are_held_within_bounds(heads):
+    """Whatever the contexts of a step add up to, the keys and values held at a time take at most 1 GiB, or one
+    head's; every head has its turn, in stretches that differ by less than one head's share."""
+    mixer = object.__new__(LatentAttention)
+    mixer.h = heads
+    for rows in (128, 4096, 65536, 480 * 1024, 1 << 20, 1 << 22):
+        most = mixer._heads_at_once(rows)
+        assert 1 <= most <= heads and (most == 1 or most * rows * 512 <= 1 << 30)
+        turns = -(-heads // most)
+        assert most == -(-heads // turns) and (turns == 1 or rows * 512 * -(-heads // (turns - 1)) > 1 << 30)
