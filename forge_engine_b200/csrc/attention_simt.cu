@@ -41,7 +41,8 @@ struct Simt {
   float scale;
   void* out;
   int num_q_heads, groups, spans, row_tiles;
-  float* partial;           // [unit][kv head][row tile][span][row][D + 2]
+  int unit0;                // of this launch: the units go through the workspace in slices
+  float* partial;           // [unit of the slice][kv head][row tile][span][row][D + 2]
   int* status;
 };
 
@@ -107,7 +108,7 @@ __global__ void __launch_bounds__(SPAN_THREADS) attention_simt_span_kernel(const
   __shared__ int ok[SPAN_STAGES][SPAN_KEYS];
   pdl_trigger();
   pdl_wait();
-  const int D = p.cache.head_dim, unit = blockIdx.x, span = blockIdx.z, kvh = blockIdx.y / p.row_tiles, tile = blockIdx.y % p.row_tiles;
+  const int D = p.cache.head_dim, unit = p.unit0 + (int)blockIdx.z, span = blockIdx.x, kvh = blockIdx.y / p.row_tiles, tile = blockIdx.y % p.row_tiles;
   int token = unit, entry;
   if (p.cu_tokens != nullptr) {
     token = p.cu_tokens[unit];
@@ -209,7 +210,7 @@ __global__ void __launch_bounds__(SPAN_THREADS) attention_simt_span_kernel(const
       }
     }
   }
-  float* part = p.partial + ((((size_t)unit * gridDim.y + blockIdx.y) * p.spans + span) * R) * (D + 2);
+  float* part = p.partial + ((((size_t)blockIdx.z * gridDim.y + blockIdx.y) * p.spans + span) * R) * (D + 2);
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     if (r < rows) {
@@ -236,7 +237,7 @@ __global__ void __launch_bounds__(128) attention_simt_merge_kernel(const Simt p,
   __shared__ float best;
   pdl_trigger();
   pdl_wait();
-  const int D = p.cache.head_dim, unit = blockIdx.x, head = blockIdx.y;
+  const int D = p.cache.head_dim, unit = p.unit0 + (int)blockIdx.x, head = blockIdx.y;
   int token = unit;
   if (p.cu_tokens != nullptr) {
     token = p.cu_tokens[unit];
@@ -247,7 +248,7 @@ __global__ void __launch_bounds__(128) attention_simt_merge_kernel(const Simt p,
   const int from = lo / SPAN, to = min(pos / SPAN, p.spans - 1);
   const int kvh = head / p.groups, within = head - kvh * p.groups;
   const size_t stride = (size_t)R * (D + 2);
-  const float* part = p.partial + (((size_t)unit * (p.cache.num_kv_heads * p.row_tiles) + kvh * p.row_tiles + within / R) * p.spans) * stride +
+  const float* part = p.partial + (((size_t)blockIdx.x * (p.cache.num_kv_heads * p.row_tiles) + kvh * p.row_tiles + within / R) * p.spans) * stride +
                       (size_t)(within % R) * (D + 2);
   if (threadIdx.x < 32) {
     float top = -INFINITY;
@@ -277,7 +278,7 @@ __global__ void __launch_bounds__(TILE_THREADS) attention_simt_tile_kernel(const
   __shared__ int ok[TILE_KEYS];
   pdl_trigger();
   pdl_wait();
-  const int D = p.cache.head_dim, entry = blockIdx.z, kvh = blockIdx.y;
+  const int D = p.cache.head_dim, entry = p.unit0 + (int)blockIdx.z, kvh = blockIdx.y;
   const int token0 = p.cu_tokens[entry], count = p.cu_tokens[entry + 1] - token0;
   if (count <= 1) return;
   const int total = count * p.groups, tiles = (total + TILE_ROWS - 1) / TILE_ROWS;
@@ -430,28 +431,54 @@ int launch(K kernel, dim3 grid, int threads, size_t smem, cudaStream_t stream, c
 
 int rows_of(int groups) { return groups <= 2 ? 2 : groups <= 4 ? 4 : groups <= 8 ? 8 : 16; }
 
+// Floats of a unit's partial results, and how many units go through the workspace at once: all of them up to
+// 128 MB (48 requests of 16 heads of 128 at 32,768 positions), then slices of them one after the other, so that one
+// long request among many does not ask for its spans that many times.
+constexpr long long SIMT_WORKSPACE = 1ll << 25;
+long long unit_floats(int num_q_heads, int num_kv_heads, int head_dim, long long spans) {
+  const int groups = num_q_heads / num_kv_heads, R = rows_of(groups);
+  return (long long)num_kv_heads * ((groups + R - 1) / R) * spans * R * (head_dim + 2);
+}
+int units_at_once(int units, long long floats) {
+  const long long most = SIMT_WORKSPACE / floats;
+  return (int)(most < 1 ? 1 : most > 65535 ? (units < 65535 ? units : 65535) : most < units ? most : units);
+}
+long long spans_of(int max_pages, int page_size) {
+  const long long spans = ((long long)max_pages * page_size + SPAN - 1) / SPAN;
+  return spans < 1 ? 1 : spans;
+}
+
 template <typename T, int DMAX>
-int run_spans(const Simt& p, cudaStream_t stream) {
+int run_spans(Simt p, cudaStream_t stream) {
   const int R = rows_of(p.groups), D = p.cache.head_dim;
   const size_t smem = (size_t)R * D * 4 + SPAN_STAGES * SPAN_KEYS * ((size_t)2 * D * sizeof(T) + 16);
-  const dim3 grid(p.units, p.cache.num_kv_heads * p.row_tiles, p.spans);
-  int code;
-  if (R == 2) code = launch(attention_simt_span_kernel<T, 2, DMAX>, grid, SPAN_THREADS, smem, stream, p);
-  else if (R == 4) code = launch(attention_simt_span_kernel<T, 4, DMAX>, grid, SPAN_THREADS, smem, stream, p);
-  else if (R == 8) code = launch(attention_simt_span_kernel<T, 8, DMAX>, grid, SPAN_THREADS, smem, stream, p);
-  else code = launch(attention_simt_span_kernel<T, 16, DMAX>, grid, SPAN_THREADS, smem, stream, p);
-  if (code) return code;
-  return launch(attention_simt_merge_kernel<T>, dim3(p.units, p.num_q_heads), 128, 0, stream, p, R);
+  const int slice = units_at_once(p.units, unit_floats(p.num_q_heads, p.cache.num_kv_heads, D, p.spans));
+  int code = 0;
+  for (; p.unit0 < p.units && code == 0; p.unit0 += slice) {
+    const int units = p.units - p.unit0 < slice ? p.units - p.unit0 : slice;
+    const dim3 grid(p.spans, p.cache.num_kv_heads * p.row_tiles, units);
+    if (R == 2) code = launch(attention_simt_span_kernel<T, 2, DMAX>, grid, SPAN_THREADS, smem, stream, p);
+    else if (R == 4) code = launch(attention_simt_span_kernel<T, 4, DMAX>, grid, SPAN_THREADS, smem, stream, p);
+    else if (R == 8) code = launch(attention_simt_span_kernel<T, 8, DMAX>, grid, SPAN_THREADS, smem, stream, p);
+    else code = launch(attention_simt_span_kernel<T, 16, DMAX>, grid, SPAN_THREADS, smem, stream, p);
+    if (code == 0) code = launch(attention_simt_merge_kernel<T>, dim3(units, p.num_q_heads), 128, 0, stream, p, R);
+  }
+  return code;
 }
 
 template <typename T>
-int run_tiles(const Simt& p, int max_new, cudaStream_t stream) {
+int run_tiles(Simt p, int max_new, cudaStream_t stream) {
   const int D = p.cache.head_dim;
   const size_t smem = (size_t)4 * TILE_ROWS * (D + 4 + P_PITCH) + (size_t)TILE_KEYS * (2 * D * sizeof(T) + 16);
-  const dim3 grid((unsigned)(((long long)max_new * p.groups + TILE_ROWS - 1) / TILE_ROWS), p.cache.num_kv_heads, p.units);
-  if (D <= 64) return launch(attention_simt_tile_kernel<T, 64>, grid, TILE_THREADS, smem, stream, p);
-  if (D <= 128) return launch(attention_simt_tile_kernel<T, 128>, grid, TILE_THREADS, smem, stream, p);
-  return launch(attention_simt_tile_kernel<T, 256>, grid, TILE_THREADS, smem, stream, p);
+  int code = 0;
+  for (; p.unit0 < p.units && code == 0; p.unit0 += 65535) {
+    const dim3 grid((unsigned)(((long long)max_new * p.groups + TILE_ROWS - 1) / TILE_ROWS), p.cache.num_kv_heads,
+                    p.units - p.unit0 < 65535 ? p.units - p.unit0 : 65535);
+    if (D <= 64) code = launch(attention_simt_tile_kernel<T, 64>, grid, TILE_THREADS, smem, stream, p);
+    else if (D <= 128) code = launch(attention_simt_tile_kernel<T, 128>, grid, TILE_THREADS, smem, stream, p);
+    else code = launch(attention_simt_tile_kernel<T, 256>, grid, TILE_THREADS, smem, stream, p);
+  }
+  return code;
 }
 
 template <typename T>
@@ -467,12 +494,15 @@ int run(const Simt& p, int n_tokens, int max_new, cudaStream_t stream) {
 
 }  // namespace
 
-// Floats of workspace for `units` single tokens whose block tables are `max_pages` wide.
+// For `units` single tokens whose block tables are `max_pages` wide: how many of them are worked on at
+// once, and the floats of workspace those take.
+FE_EXPORT int fe_attention_simt_units(int units, int num_q_heads, int num_kv_heads, int head_dim, int max_pages, int page_size) {
+  if (units <= 0 || num_kv_heads <= 0 || num_q_heads <= 0 || num_q_heads % num_kv_heads) return 0;
+  return units_at_once(units, unit_floats(num_q_heads, num_kv_heads, head_dim, spans_of(max_pages, page_size)));
+}
 FE_EXPORT long long fe_attention_simt_scratch(int units, int num_q_heads, int num_kv_heads, int head_dim, int max_pages, int page_size) {
-  if (units <= 0 || num_kv_heads <= 0 || num_q_heads % num_kv_heads) return 0;
-  const int groups = num_q_heads / num_kv_heads, R = rows_of(groups);
-  const long long spans = ((long long)max_pages * page_size + SPAN - 1) / SPAN;
-  return (long long)units * num_kv_heads * ((groups + R - 1) / R) * spans * R * (head_dim + 2);
+  const int slice = fe_attention_simt_units(units, num_q_heads, num_kv_heads, head_dim, max_pages, page_size);
+  return slice == 0 ? 0 : slice * unit_floats(num_q_heads, num_kv_heads, head_dim, spans_of(max_pages, page_size));
 }
 
 // `cu_tokens` [units + 1] says which tokens each unit (an entry: row u of the block table, positions
@@ -489,14 +519,13 @@ FE_EXPORT int fe_attention_simt(const void* q, int q_stride, int dtype, const vo
   if (num_kv_heads <= 0 || num_q_heads % num_kv_heads || num_q_heads > 65535) return FE_ERR_BAD_SHAPE;
   if (((uintptr_t)k_cache | (uintptr_t)v_cache) & 15) return FE_ERR_BAD_ALIGN;
   if (cu_tokens == nullptr) units = n_tokens;
-  if (cu_tokens != nullptr && units > 65535) return FE_ERR_TOO_LARGE;
   PagedKV cache{k_cache, v_cache, block_table, max_pages, page_size, num_pages, num_kv_heads, head_dim};
   const int groups = num_q_heads / num_kv_heads, R = rows_of(groups);
-  const long long spans = ((long long)max_pages * page_size + SPAN - 1) / SPAN;
+  const long long spans = spans_of(max_pages, page_size);
   const int row_tiles = (groups + R - 1) / R;
-  if (spans > 65535 || (long long)num_kv_heads * row_tiles > 65535) return FE_ERR_TOO_LARGE;
+  if (spans > 0x7fffffff || (long long)num_kv_heads * row_tiles > 65535) return FE_ERR_TOO_LARGE;
   Simt p{q, q_stride, cache, positions, token_entry, cu_tokens, units, window, scale, out, num_q_heads, groups,
-         (int)spans, row_tiles, workspace, status};
+         (int)spans, row_tiles, 0, workspace, status};
   if (dtype == FE_DTYPE_F32) return run<float>(p, n_tokens, max_new, stream);
   if (dtype == FE_DTYPE_BF16) return run<bf16>(p, n_tokens, max_new, stream);
   return FE_ERR_BAD_DTYPE;

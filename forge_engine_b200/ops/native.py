@@ -90,6 +90,7 @@ def _declare(handle: ctypes.CDLL) -> None:
         "fe_rope_table": [p, p, i, i, f, p, p],
         "fe_attention_simt": [p, i, i, p, p, p, i, i, i, p, p, p, i, i, i, f, p, i, i, i, i, p, p, p],
         "fe_attention_simt_scratch": [i, i, i, i, i, i],
+        "fe_attention_simt_units": [i, i, i, i, i, i],
         "fe_gemm_simt": [p, i, p, i, p, p, i, i, i, i, i, p],
         "fe_sample": [p, i, i, p, p, p, p, p, p, p, p, p],
         "fe_gemm_tc5": [p, p, p, p, i, i, i, i, i, p, p, p, f, f, p],
@@ -1470,10 +1471,12 @@ def attention_simt(
     n = out.shape[0]
     assert out.shape[1] == num_q_heads * head_dim and out.dtype == q.dtype == k_cache.dtype
     cu_tokens, units, max_new = (None, n, 1) if entries is None else entries
-    workspace = None
+    workspace, slices = None, 0
     if max_new <= 1 or units > 1 or n <= 1:            # some token may come by itself
-        floats = lib().fe_attention_simt_scratch(int(units), num_q_heads, nkv, head_dim, block_table.shape[1], page_size)
-        workspace = _attention_workspace(q.device, max(1, floats))
+        sizes = (int(units), num_q_heads, nkv, head_dim, block_table.shape[1], page_size)
+        # the call's own, so that runs on several streams do not share it
+        workspace = torch.empty(max(1, lib().fe_attention_simt_scratch(*sizes)), dtype=torch.float32, device=q.device)
+        slices = -(-int(units) // max(1, lib().fe_attention_simt_units(*sizes)))
     check(
         lib().fe_attention_simt(
             ptr(q), int(q_stride), code(q), ptr(k_cache), ptr(v_cache), ptr(block_table),
@@ -1484,7 +1487,7 @@ def attention_simt(
         "attention_simt",
     )
     global LAUNCHES
-    LAUNCHES += (2 if workspace is not None else 0) + (1 if cu_tokens is not None and max_new > 1 else 0) - 1
+    LAUNCHES += 2 * slices + (1 if cu_tokens is not None and max_new > 1 else 0) - 1
 
 
 _balanced_blocks: dict = {}

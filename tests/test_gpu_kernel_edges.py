@@ -126,6 +126,31 @@ def test_attention_marks_missing_pages_and_keeps_later_infinities_out(native):
     assert attend(table[:, :2].contiguous(), [39], [0, 1])[1] & 2
 
 
+def test_attention_keeps_its_partial_results_to_itself(native, monkeypatch):
+    """Runs on several streams share no buffer, and many single tokens beside one long block table take a bounded
+    one: they go through it in slices, with the same results."""
+    nq, nkv, d, page = 4, 2, 64, 16
+    lengths = [1 + 37 * i for i in range(40)]
+    k_cache, v_cache, table, _, _ = paged_layout(lengths, page, nkv, d, torch.float32, seed=2)
+    q = torch.randn((40, nq * d), generator=torch.Generator().manual_seed(3)).to(DEV)
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)  # noqa: E731
+    wide = torch.full((40, 32768), -1, dtype=torch.int32, device=DEV)
+    wide[:, : table.shape[1]] = table
+    monkeypatch.setattr(native, "_attention_workspace", None)
+    status, outs = status_word(), []
+    for t in (table, wide):
+        sizes = (nq, nkv, d, t.shape[1], page)
+        assert native.lib().fe_attention_simt_scratch(40, *sizes) <= 1 << 25
+        assert (native.lib().fe_attention_simt_units(40, *sizes) < 40) == (t is wide)
+        for entries in (None, (ints(list(range(41))), 40, 1)):
+            out, before = torch.empty((40, nq * d), device=DEV), native.LAUNCHES
+            native.attention_simt(q, nq * d, k_cache, v_cache, t, ints([n - 1 for n in lengths]), ints(list(range(40))), None, 0.125, out, nq,
+                                  status, entries=entries)
+            assert native.LAUNCHES - before == 2 * -(-40 // native.lib().fe_attention_simt_units(40, *sizes))
+            outs.append(out)
+    assert int(status.item()) == 0 and all(torch.equal(out, outs[0]) for out in outs[1:])
+
+
 # -- gated recurrence ------------------------------------------------------------------------------
 @pytest.mark.parametrize("heads, dk, dv, lead", ((2, 64, 64, 4), (1, 128, 128, 4), (1, 160, 100, 4), (2, 12, 260, 8), (1, 168, 36, 1), (3, 6, 8, 4)))
 @pytest.mark.parametrize("counts", ([128], [129, 200, 3], [191, 1, 192, 130]))
