@@ -10,15 +10,17 @@
 //
 // attention_simt_span: single tokens (decoding, or a caller that names no entries).  A block takes
 //   the query heads of one kv head (up to 16) over one span of 128 key positions, whose keys and
-//   values pass through a ring in shared memory; attention_simt_merge adds a token's spans up in
+//   values pass through a ring in shared memory; attention_simt_merge folds a token's spans in
 //   order.  Bound by the bytes of keys and values; the spans are what keeps the chip busy at few
 //   requests.
 // attention_simt_tile: entries of several tokens.  A block takes 32 rows (token, query head) of one
 //   kv head over all their keys in tiles of 64, as two small FFMA products from shared memory.
 //
-// Spans and tiles are counted from position 0, every sum runs over positions (or elements of a
-// head: even and odd ones apart) in ascending order, and which kernel a token takes depends on how
-// many its entry brings: nothing depends on what else is in the batch.
+// A row's bits depend on nothing but its token and the keys it sees: not on what else is in the batch, nor on
+// how its portion was cut.  Both kernels take a span's keys, counted from position 0, in thirty-twos with one
+// running maximum, sum over positions (or elements of a head: even and odd ones apart) in ascending order,
+// and fold the spans one after the other (fold_factors).  In the tile kernel that takes a second set of sums: 500
+// tokens of 16 heads of 128 146 us, 137 without; single tokens 18.6 against 19.3 (4 after 700 cached ones).
 #include "attention_common.cuh"
 
 namespace {
@@ -69,6 +71,33 @@ __device__ __forceinline__ void pairs4(const bf16* p, uint64_t (&out)[2]) {
   const uint2 raw = *reinterpret_cast<const uint2*>(p);
   out[0] = (uint64_t)(raw.x << 16) | ((uint64_t)(raw.x & 0xffff0000u) << 32);
   out[1] = (uint64_t)(raw.y << 16) | ((uint64_t)(raw.y & 0xffff0000u) << 32);
+}
+
+// Sums (or maxima) of eight numbers over 16 neighbouring lanes, for all of them, in the order of warp_sum's last
+// four steps: half of the numbers go to the partner at a time, and come back whole.
+template <bool MAX>
+__device__ __forceinline__ void reduce8(float (&x)[8], int lane) {
+#pragma unroll
+  for (int half = 4, bit = 8; half > 0; half >>= 1, bit >>= 1) {
+    const bool upper = (lane & bit) != 0;
+#pragma unroll
+    for (int i = 0; i < half; ++i) {
+      const float send = upper ? x[i] : x[i + half], keep = upper ? x[i + half] : x[i];
+      const float got = __shfl_xor_sync(0xffffffffu, send, bit);
+      x[i] = MAX ? fmaxf(keep, got) : keep + got;
+    }
+  }
+  const float got = __shfl_xor_sync(0xffffffffu, x[0], 1), mine = MAX ? fmaxf(x[0], got) : x[0] + got;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) x[i] = __shfl_sync(0xffffffffu, mine, (lane & 16) | (i << 1));
+}
+
+// A span (maximum m) joins those before it (maximum top): their sums take `old`, its own `mine`.
+__device__ __forceinline__ void fold_factors(float& top, float m, float& old, float& mine) {
+  const float t = fmaxf(top, m);
+  old = top == -INFINITY ? 0.f : expf(top - t);
+  mine = m == -INFINITY ? 0.f : expf(m - t);
+  top = t;
 }
 
 // Where key position `key` of an entry lies, in elements of the cache; -1 (and a status bit) without a page.
@@ -172,11 +201,11 @@ __global__ void __launch_bounds__(SPAN_THREADS) attention_simt_span_kernel(const
           fma2(dot, a[0], b[0]);
           fma2(dot, a[1], b[1]);
         }
-        const float score = ok[s][lane] ? sum2(dot) * p.scale : -INFINITY;
+        const float score = ok[s][lane] ? __fmul_rn(sum2(dot), p.scale) : -INFINITY;
         const float top = fmaxf(m[i], warp_max(score));
         const float e = score == -INFINITY ? 0.f : expf(score - top);
         const float c = m[i] == -INFINITY ? 0.f : expf(m[i] - top);
-        l[i] = l[i] * c + warp_sum(e);
+        l[i] = fmaf(l[i], c, warp_sum(e));
         m[i] = top;
         ps[r][lane] = e;
         if (lane == 0) corr[r] = c;
@@ -234,7 +263,6 @@ __global__ void __launch_bounds__(SPAN_THREADS) attention_simt_span_kernel(const
 // One block per (query head, unit): its spans in ascending order.
 template <typename T>
 __global__ void __launch_bounds__(128) attention_simt_merge_kernel(const Simt p, int R) {
-  __shared__ float best;
   pdl_trigger();
   pdl_wait();
   const int D = p.cache.head_dim, unit = p.unit0 + (int)blockIdx.x, head = blockIdx.y;
@@ -250,22 +278,15 @@ __global__ void __launch_bounds__(128) attention_simt_merge_kernel(const Simt p,
   const size_t stride = (size_t)R * (D + 2);
   const float* part = p.partial + (((size_t)blockIdx.x * (p.cache.num_kv_heads * p.row_tiles) + kvh * p.row_tiles + within / R) * p.spans) * stride +
                       (size_t)(within % R) * (D + 2);
-  if (threadIdx.x < 32) {
-    float top = -INFINITY;
-    for (int s = from + (int)threadIdx.x; s <= to; s += 32) top = fmaxf(top, part[s * stride + D]);
-    top = warp_max(top);
-    if (threadIdx.x == 0) best = top;
-  }
-  __syncthreads();
-  const float top = best;
   T* out = (T*)p.out + ((size_t)token * p.num_q_heads + head) * D;
   for (int d = threadIdx.x; d < D; d += blockDim.x) {
-    float num = 0.f, den = 0.f;
+    float num = 0.f, den = 0.f, top = -INFINITY;
 #pragma unroll 4
     for (int s = from; s <= to; ++s) {
-      const float m = part[s * stride + D], f = m == -INFINITY ? 0.f : expf(m - top);
-      num = fmaf(part[s * stride + d], f, num);
-      den = fmaf(part[s * stride + D + 1], f, den);
+      float old, mine;
+      fold_factors(top, part[s * stride + D], old, mine);
+      num = fmaf(part[s * stride + d], mine, __fmul_rn(num, old));
+      den = fmaf(part[s * stride + D + 1], mine, __fmul_rn(den, old));
     }
     out[d] = from_float<T>(den > 0.f ? num / den : 0.f);
   }
@@ -305,15 +326,16 @@ __global__ void __launch_bounds__(TILE_THREADS) attention_simt_tile_kernel(const
   const int* table = p.cache.block_table + (size_t)entry * p.cache.max_pages;
   const int low = p.positions[token0 + row0 / p.groups], high = p.positions[token0 + (min(row0 + TILE_ROWS, total) - 1) / p.groups];
   const int lo = p.window > 0 ? max(0, low - p.window + 1) : 0;
-  float m[4], l[4], acc[4][CG][4];
+  // of the span at hand, and of the spans before it
+  float m[4], l[4], acc[4][CG][4], top[4], den[4], num[4][CG][4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    m[i] = -INFINITY;
-    l[i] = 0.f;
+    m[i] = top[i] = -INFINITY;
+    l[i] = den[i] = 0.f;
 #pragma unroll
     for (int g = 0; g < CG; ++g)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) acc[i][g][e] = 0.f;
+      for (int e = 0; e < 4; ++e) acc[i][g][e] = num[i][g][e] = 0.f;
   }
   for (int first = lo / TILE_KEYS * TILE_KEYS; first <= high; first += TILE_KEYS) {
     __syncthreads();
@@ -340,39 +362,48 @@ __global__ void __launch_bounds__(TILE_THREADS) attention_simt_tile_kernel(const
 #pragma unroll
           for (int j = 0; j < 4; ++j) fma2(dot[i][j], a[i][e], b[j][e]);
     }
+    // by row and thirty-two of keys: maxima, corrections of what came before, sums
+    float score[4][4], most[8], corr[2][4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      float score[4], top = m[i];
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const int key = first + tx + 16 * j;
-        score[j] = ok[tx + 16 * j] && key >= from[i] && key <= upto[i] ? sum2(dot[i][j]) * p.scale : -INFINITY;
-        top = fmaxf(top, score[j]);
+        score[i][j] = ok[tx + 16 * j] && key >= from[i] && key <= upto[i] ? __fmul_rn(sum2(dot[i][j]), p.scale) : -INFINITY;
+        if (j & 1) most[2 * i + j / 2] = fmaxf(score[i][j - 1], score[i][j]);
       }
+    reduce8<true>(most, threadIdx.x & 31);
 #pragma unroll
-      for (int o = 8; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
-      const float c = m[i] == -INFINITY ? 0.f : expf(m[i] - top);
-      float sum = 0.f;
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float e = score[j] == -INFINITY ? 0.f : expf(score[j] - top);
-        ps[(ty * 4 + i) * P_PITCH + tx + 16 * j] = e;
-        sum += e;
+      for (int h = 0; h < 2; ++h) {
+        const float now = fmaxf(m[i], most[2 * i + h]);
+        corr[h][i] = m[i] == -INFINITY ? 0.f : expf(m[i] - now);
+        m[i] = now;
+        float e[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          e[j] = score[i][2 * h + j] == -INFINITY ? 0.f : expf(score[i][2 * h + j] - now);
+          ps[(ty * 4 + i) * P_PITCH + 32 * h + 16 * j + tx] = e[j];
+        }
+        most[2 * i + h] = e[0] + e[1];
       }
+    reduce8<false>(most, threadIdx.x & 31);
 #pragma unroll
-      for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-      l[i] = l[i] * c + sum;
-      m[i] = top;
-#pragma unroll
-      for (int g = 0; g < CG; ++g)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) acc[i][g][e] *= c;
-    }
+    for (int i = 0; i < 4; ++i) l[i] = fmaf(fmaf(l[i], corr[0][i], most[2 * i]), corr[1][i], most[2 * i + 1]);
     __syncwarp();                    // a row's probabilities are written and read by the same warp
     // Where some row of the tile does not see some key, that key's value is taken as zero for it: a
     // zero probability would not keep an infinity out.
     const bool edge = first < max(0, p.window > 0 ? high - p.window + 1 : 0) || first + TILE_KEYS - 1 > low;
     for (int key = 0; key < TILE_KEYS; key += 4) {
+      if (key % 32 == 0) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int g = 0; g < CG; ++g)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[i][g][e] *= key == 0 ? corr[0][i] : corr[1][i];
+      }
       float e[4][4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) load4(ps + (ty * 4 + i) * P_PITCH + key, e[i]);
@@ -401,6 +432,23 @@ __global__ void __launch_bounds__(TILE_THREADS) attention_simt_tile_kernel(const
         }
       }
     }
+    if ((first + TILE_KEYS) % SPAN == 0 || first + TILE_KEYS > high) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float old, mine;
+        fold_factors(top[i], m[i], old, mine);
+        den[i] = fmaf(l[i], mine, __fmul_rn(den[i], old));
+        m[i] = -INFINITY;
+        l[i] = 0.f;
+#pragma unroll
+        for (int g = 0; g < CG; ++g)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            num[i][g][e] = fmaf(acc[i][g][e], mine, __fmul_rn(num[i][g][e], old));
+            acc[i][g][e] = 0.f;
+          }
+      }
+    }
   }
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -413,7 +461,7 @@ __global__ void __launch_bounds__(TILE_THREADS) attention_simt_tile_kernel(const
       if (d < D) {
         float o[4];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) o[c] = l[i] > 0.f ? acc[i][g][c] / l[i] : 0.f;
+        for (int c = 0; c < 4; ++c) o[c] = den[i] > 0.f ? num[i][g][c] / den[i] : 0.f;
         store4(out + d, o);
       }
     }

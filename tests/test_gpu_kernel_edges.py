@@ -126,6 +126,34 @@ def test_attention_marks_missing_pages_and_keeps_later_infinities_out(native):
     assert attend(table[:, :2].contiguous(), [39], [0, 1])[1] & 2
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("nq, nkv, d, window", [(4, 2, 64, None), (6, 1, 40, 50), (4, 4, 256, 130), (9, 3, 72, 300)])
+def test_attention_of_a_portion_cut_in_any_way(native, dtype, nq, nkv, d, window):
+    """A prompt in one portion, in two, as single tokens and as tokens without entries: the same bits."""
+    length, page = 333, 16
+    k_cache, v_cache, table, _, _ = paged_layout([length], page, nkv, d, dtype, seed=d)
+    q = torch.randn((length, nq * d), generator=torch.Generator().manual_seed(4)).to(dtype).to(DEV)
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)  # noqa: E731
+    status = status_word()
+
+    def attend(first, last, cu=None):
+        out = torch.empty((last - first, nq * d), dtype=dtype, device=DEV)
+        rows = table if cu is None else table.expand(len(cu) - 1, -1).contiguous()
+        entry = [0] * (last - first) if cu is None else [e for e in range(len(cu) - 1) for _ in range(cu[e + 1] - cu[e])]
+        native.attention_simt(q[first:last].contiguous(), nq * d, k_cache, v_cache, rows, ints(list(range(first, last))), ints(entry), window,
+                              d ** -0.5, out, nq, status, entries=None if cu is None else
+                              (ints(cu), len(cu) - 1, max(b - a for a, b in zip(cu, cu[1:]))))
+        return out
+
+    whole = attend(0, length, [0, length])
+    assert torch.equal(attend(0, length), whole)
+    assert torch.equal(attend(0, length, list(range(length + 1))), whole)
+    for cut in (1, 64, 127, 200, length - 1):
+        assert torch.equal(torch.cat((attend(0, cut, [0, cut]), attend(cut, length, [0, length - cut]))), whole), cut
+        assert torch.equal(attend(0, length, [0, cut, length]), whole), cut
+    assert int(status.item()) == 0
+
+
 def test_attention_keeps_its_partial_results_to_itself(native, monkeypatch):
     """Runs on several streams share no buffer, and many single tokens beside one long block table take a bounded
     one: they go through it in slices, with the same results."""
