@@ -38,6 +38,7 @@ struct Product {
   const float* bias;
   void* y;
   int y_dtype, n, o, k, accumulate;
+  int* status;           // null: none
   long long ldx, ldy, batch_x, batch_w, batch_y;   // blockIdx.z: one product of a batch (a head)
 };
 
@@ -179,8 +180,15 @@ __global__ void __launch_bounds__(TY * TX) gemm_simt_tile_kernel(const Product p
 #define GSK_KT 128
 #define GSK_MAX_STAGES 8
 #define GSK_LOADERS 4
+// Usually tc5::WAIT_LIMIT and no stretch; see fe_gemm_simt_set_test_fault.
+struct Fault {
+  unsigned wait_limit;
+  int skip_stretch;
+};
+Fault g_test_fault{tc5::WAIT_LIMIT, -1};
+
 template <typename TX, typename TW, int COLS, int LC, int R>
-__global__ void __launch_bounds__(32 * (GSK_LOADERS + 8)) gemm_simt_rows_kernel(const Product p, int stages) {
+__global__ void __launch_bounds__(32 * (GSK_LOADERS + 8)) gemm_simt_rows_kernel(const Product p, int stages, const Fault fault) {
   constexpr int PX = GSK_KT + 16 / (int)sizeof(TX), PW = GSK_KT + 16 / (int)sizeof(TW);
   constexpr int ROWS = R * (32 / LC);           // rows of x a warp takes
   extern __shared__ __align__(16) unsigned char smem[];
@@ -220,7 +228,7 @@ __global__ void __launch_bounds__(32 * (GSK_LOADERS + 8)) gemm_simt_rows_kernel(
       const int k0 = step * GSK_KT;
       if (step >= stages) {
         int ok = 1;
-        if (lane == 0) ok = tc5::mbar_wait(&empty[s], phase, &abort_flag) ? 1 : 0;
+        if (lane == 0) ok = tc5::mbar_wait(&empty[s], phase, &abort_flag, fault.wait_limit) ? 1 : 0;
         if (!__shfl_sync(0xffffffffu, ok, 0)) break;
       }
       const TW* from = w + k0;
@@ -240,7 +248,7 @@ __global__ void __launch_bounds__(32 * (GSK_LOADERS + 8)) gemm_simt_rows_kernel(
           xfrom += x_step;
           xto += SX * PX;
         }
-      gs_arrive_copied(&full[s]);
+      if (step != fault.skip_stretch) gs_arrive_copied(&full[s]);
       if (++s == stages) s = 0, phase ^= 1u;
     }
     gs_commit();
@@ -255,7 +263,7 @@ __global__ void __launch_bounds__(32 * (GSK_LOADERS + 8)) gemm_simt_rows_kernel(
     unsigned phase = 0;
     for (int step = 0; step < steps; ++step) {
       const int kt = min(GSK_KT, p.k - step * GSK_KT);
-      ok = tc5::mbar_wait(&full[s], phase, &abort_flag);
+      ok = tc5::mbar_wait(&full[s], phase, &abort_flag, fault.wait_limit);
       if (!ok) break;
       const TW* wt = ws + (s * COLS + lc) * PW;
       const TX* xt = xs + (s * rows + mine) * PX;
@@ -294,8 +302,9 @@ __global__ void __launch_bounds__(32 * (GSK_LOADERS + 8)) gemm_simt_rows_kernel(
       if (lane == 0) gs_arrive(&empty[s]);
       if (++s == stages) s = 0, phase ^= 1u;
     }
+    if (!ok && lane == 0 && p.status) atomicOr(p.status, FE_STATUS_WAIT_TIMEOUT);
     if (col0 + lc < p.o) {
-      // after a wait that ran out the outputs are NaN, which the sampler reports
+      // after a wait that ran out the outputs are NaN
 #pragma unroll
       for (int i = 0; i < R; ++i)
         if (mine + i < p.n) gs_store(p, ok ? acc[i] : __int_as_float(0x7fffffff), mine + i, col0 + lc);
@@ -328,7 +337,7 @@ int launch_rows(const Product& p, int batch, cudaStream_t stream) {
   const size_t stage = COLS * (GSK_KT * sizeof(TW) + 16) + (size_t)groups * ROWS * (GSK_KT * sizeof(TX) + 16);
   const int stages = (int)std::min<size_t>(GSK_MAX_STAGES, std::max<size_t>(2, 110 * 1024 / stage));
   dim3 grid((p.o + COLS - 1) / COLS, 1, batch);
-  return launch_sized(gemm_simt_rows_kernel<TX, TW, COLS, LC, R>, grid, 32 * (workers + GSK_LOADERS), stages * stage, stream, p, stages);
+  return launch_sized(gemm_simt_rows_kernel<TX, TW, COLS, LC, R>, grid, 32 * (workers + GSK_LOADERS), stages * stage, stream, p, stages, g_test_fault);
 }
 
 // Which kernel: all of them give the same bits.
@@ -375,12 +384,19 @@ int launch_coded(int x_dtype, int w_dtype, const Product& p, int batch, cudaStre
 
 }  // namespace
 
+// For tests of the bounded waits only: later launches of the kernel for few rows poll at most `wait_limit` times per
+// wait (0: the usual bound) and their loaders do not report stretch `skip_stretch` of k (-1: none), so that the
+// block gives up, sets FE_STATUS_WAIT_TIMEOUT and returns.  Call with (0, -1) to go back to normal.
+FE_EXPORT void fe_gemm_simt_set_test_fault(unsigned wait_limit, int skip_stretch) {
+  g_test_fault = Fault{wait_limit ? wait_limit : tc5::WAIT_LIMIT, skip_stretch};
+}
+
 FE_EXPORT int fe_gemm_simt(const void* x, int x_dtype, const void* w, int w_dtype, const float* bias,
                            void* y, int y_dtype, int n, int o, int k, int accumulate,
-                           cudaStream_t stream) {
+                           int* status, cudaStream_t stream) {
   if (n <= 0 || o <= 0) return 0;
   if (k <= 0) return FE_ERR_BAD_SHAPE;
-  return launch_coded(x_dtype, w_dtype, Product{x, w, bias, y, y_dtype, n, o, k, accumulate, k, o, 0, 0, 0}, 1, stream);
+  return launch_coded(x_dtype, w_dtype, Product{x, w, bias, y, y_dtype, n, o, k, accumulate, status, k, o, 0, 0, 0}, 1, stream);
 }
 
 // `batch` products at once (one per head): product b reads x + b * batch_x (rows ldx apart),
@@ -388,9 +404,9 @@ FE_EXPORT int fe_gemm_simt(const void* x, int x_dtype, const void* w, int w_dtyp
 // in elements.
 FE_EXPORT int fe_gemm_simt_batched(const void* x, int x_dtype, const void* w, int w_dtype, void* y, int y_dtype,
                                    int n, int o, int k, int batch, long long ldx, long long ldy, long long batch_x,
-                                   long long batch_w, long long batch_y, cudaStream_t stream) {
+                                   long long batch_w, long long batch_y, int* status, cudaStream_t stream) {
   if (n <= 0 || o <= 0 || batch <= 0) return 0;
   if (k <= 0 || ldx < k || ldy < o) return FE_ERR_BAD_SHAPE;
-  return launch_coded(x_dtype, w_dtype, Product{x, w, nullptr, y, y_dtype, n, o, k, 0, ldx, ldy, batch_x, batch_w, batch_y},
+  return launch_coded(x_dtype, w_dtype, Product{x, w, nullptr, y, y_dtype, n, o, k, 0, status, ldx, ldy, batch_x, batch_w, batch_y},
                       batch, stream);
 }

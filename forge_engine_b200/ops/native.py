@@ -80,7 +80,7 @@ def _declare(handle: ctypes.CDLL) -> None:
         "fe_linear_recurrence": [p, i, i, i, i, i, i, p, p, p, p, p, i, i, i, i, i, p],
         "fe_linear_recurrence_chunked": [p, i, i, i, i, i, i, p, p, p, p, p, p, i, i, i, i, i, i, p],
         "fe_linear_recurrence_chunks": [i, i],
-        "fe_gemm_simt_batched": [p, i, p, i, p, i, i, i, i, i, ll, ll, ll, ll, ll, p],
+        "fe_gemm_simt_batched": [p, i, p, i, p, i, i, i, i, i, ll, ll, ll, ll, ll, p, p],
         "fe_add_rmsnorm": [p, p, i, p, p, i, p, p, ll, i, i, f, i, p],
         "fe_weighted_sum": [p, p, f, f, p, ll, p],
         "fe_norm_pair": [p, p, p, p, p, i, i, f, f, p],
@@ -91,7 +91,7 @@ def _declare(handle: ctypes.CDLL) -> None:
         "fe_attention_simt": [p, i, i, p, p, p, i, i, i, p, p, p, i, i, i, f, p, i, i, i, i, p, p, p],
         "fe_attention_simt_scratch": [i, i, i, i, i, i],
         "fe_attention_simt_units": [i, i, i, i, i, i],
-        "fe_gemm_simt": [p, i, p, i, p, p, i, i, i, i, i, p],
+        "fe_gemm_simt": [p, i, p, i, p, p, i, i, i, i, i, p, p],
         "fe_sample": [p, i, i, p, p, p, p, p, p, p, p, p],
         "fe_gemm_tc5": [p, p, p, p, i, i, i, i, i, p, p, p, f, f, p],
         "fe_gemm_tc5_grouped": [p, p, p, i, i, i, i, i, i, i, p, p, p, f, f, p, p],
@@ -1056,10 +1056,10 @@ def linear_recurrence(
     )
 
 
-def gemm_simt_batched(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
+def gemm_simt_batched(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, status: torch.Tensor | None = None) -> None:
     """out[n, b, :] = x[n, b, :] @ w[b].T with plain 32-bit FMAs, for x [n, batch, k] and out
     [n, batch, o] that may be strided in their first two extents, and w [batch, o, k]
-    contiguous."""
+    contiguous.  ``status`` as in ``gemm_simt``."""
     _dense(w, "w")
     n, batch, k = x.shape
     o = w.shape[1]
@@ -1067,7 +1067,7 @@ def gemm_simt_batched(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> No
     check(
         lib().fe_gemm_simt_batched(ptr(x), code(x), ptr(w), code(w), ptr(out), code(out), n, o, k, batch,
                                    int(x.stride(0)), int(out.stride(0)), int(x.stride(1)), o * k, int(out.stride(1)),
-                                   stream()),
+                                   ptr(status), stream()),
         "gemm_simt_batched",
     )
 
@@ -1576,8 +1576,10 @@ def gemm_simt(
     out: torch.Tensor,
     bias: torch.Tensor | None = None,
     accumulate: bool = False,
+    status: torch.Tensor | None = None,
 ) -> None:
-    """out = x @ w.T (+ bias) (+ out) with plain 32-bit FMAs; w is [out, in]."""
+    """out = x @ w.T (+ bias) (+ out) with plain 32-bit FMAs; w is [out, in].  A wait that runs out inside the kernel
+    for few rows sets its bit in the device word ``status`` and leaves NaN."""
     _dense(x, "x"), _dense(w, "w"), _dense(out, "out")
     n, k = x.shape
     o = w.shape[0]
@@ -1585,9 +1587,17 @@ def gemm_simt(
     assert bias is None or (bias.dtype == torch.float32 and bias.numel() == o)
     check(
         lib().fe_gemm_simt(ptr(x), code(x), ptr(w), code(w), ptr(bias), ptr(out), code(out), n, o, k,
-                           1 if accumulate else 0, stream()),
+                           1 if accumulate else 0, ptr(status), stream()),
         "gemm_simt",
     )
+
+
+def gemm_simt_set_test_fault(wait_limit: int = 0, skip_stretch: int = -1) -> None:
+    """For tests of the bounded waits: later ``gemm_simt`` launches for few rows poll at most ``wait_limit`` times per
+    wait (0: the usual bound) and do not report stretch ``skip_stretch`` of 128 k (-1: none)."""
+    fn = lib().fe_gemm_simt_set_test_fault
+    fn.argtypes, fn.restype = [ctypes.c_uint, c_int], None
+    fn(int(wait_limit), int(skip_stretch))
 
 
 TC5_STORE_BF16, TC5_STORE_F32, TC5_ADD_F32, TC5_SILU_MUL = 0, 1, 2, 3

@@ -309,7 +309,7 @@ class LatentAttention(Mixer):
         if x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and x.shape[0] > native.TC5_MAX_ROWS:
             out.copy_(torch.bmm(x.transpose(0, 1), w.transpose(1, 2)).transpose(0, 1))
         else:
-            native.gemm_simt_batched(x, w, out)
+            native.gemm_simt_batched(x, w, out, status=self.ctx.status)
 
     def attend(self, x, batch, cache: CacheView):
         n, h, d, r, dv, rank = x.shape[0], self.h, self.d, self.r, self.dv, self.kv_rank

@@ -100,7 +100,7 @@ class WKV(Mixer):
             native.gemm_tc5_grouped(x.reshape(4 * n, self.width), self.proj, out.view(4 * n, self.size), native.TC5_STORE_F32,
                                     self._grouped_plan(n, x.device), native.tc5_tile(n), 4, self.ctx.status)
         else:
-            native.gemm_simt_batched(x.transpose(0, 1), self.proj, out.transpose(0, 1))
+            native.gemm_simt_batched(x.transpose(0, 1), self.proj, out.transpose(0, 1), status=self.ctx.status)
         return out
 
     def forward(self, mixed, batch, cache: CacheView):

@@ -64,6 +64,36 @@ def test_batched_product_with_strided_rows(native, n):
     assert float((out[:, :, o:] - 7.0).abs().max()) == 0.0
 
 
+@pytest.mark.parametrize("n, o, k", ((1, 100, 1024), (4, 300, 1152), (16, 9000, 2048)))
+def test_a_wait_that_runs_out_is_reported(native, n, o, k):
+    """Loaders that do not report a stretch of k: the block gives up after a few polls, the status word says so and
+    the rows are NaN; the next call is sound again."""
+    gen = torch.Generator().manual_seed(o)
+    x, w = (torch.randn(shape, generator=gen).to(DEV) for shape in ((n, k), (o, k)))
+    good, bad, again = (torch.empty((n, o), device=DEV) for _ in range(3))
+    status = status_word()
+    native.gemm_simt(x, w, good, status=status)
+    assert int(status.item()) == 0
+    try:
+        native.gemm_simt_set_test_fault(2000, 2)
+        native.gemm_simt(x, w, bad, status=status)
+        torch.cuda.synchronize()
+    finally:
+        native.gemm_simt_set_test_fault()
+    assert int(status.item()) == 8 and not bool(torch.isfinite(bad).any())
+    native.gemm_simt(x, w, again, status=status_word())
+    assert torch.equal(again, good)
+
+
+def test_layers_give_products_their_status_word(native, monkeypatch):
+    from forge_engine_b200.parts.linear import Linear
+
+    seen, status = [], status_word()
+    monkeypatch.setattr(native, "gemm_simt", lambda *args, status=None, **kw: seen.append(status))
+    Linear(torch.randn(8, 16, device=DEV), status=status)(torch.randn(2, 16, device=DEV))
+    assert len(seen) == 1 and seen[0] is status
+
+
 # -- 32-bit attention --------------------------------------------------------------------------------
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("nq, nkv, d, page, window", [
