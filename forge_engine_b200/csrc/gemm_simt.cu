@@ -21,6 +21,9 @@ __device__ __forceinline__ void gs_copy16(void* dst, const void* src, bool valid
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(tc5::smem_u32(dst)), "l"(src), "r"(valid ? 16 : 0)
                : "memory");
 }
+__device__ __forceinline__ void gs_copy4(void* dst, const void* src, bool valid) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(tc5::smem_u32(dst)), "l"(src), "r"(valid ? 4 : 0) : "memory");
+}
 __device__ __forceinline__ void gs_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int PENDING>
 __device__ __forceinline__ void gs_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory"); }
@@ -59,12 +62,13 @@ __device__ __forceinline__ void gs_store(const Product& p, float v, int r, int c
 #define GS_BK 32
 #define GS_STAGES 3
 
-// What a thread copies of one operand's stages: rows row, row + STEP, ... of ROWS, one 16-byte piece of
-// each; zeros stand where a row or a k does not exist.  VEC: rows start on 16-byte boundaries and k is a
-// multiple of 16 bytes.
+// What a thread copies of one operand's stages: rows row, row + STEP, ... of ROWS, one piece of each; zeros
+// stand where a row or a k does not exist.  A piece is 16 bytes with VEC: rows start on 16-byte boundaries and
+// k is a multiple of 16 bytes.  Otherwise it is one number, a warp's 32 of them neighbours: 32-bit ones by
+// cp.async too, bfloat16 ones through registers.
 template <typename T, int ROWS, int THREADS, bool VEC>
 struct Stager {
-  static constexpr int CH = 16 / (int)sizeof(T), PER_ROW = GS_BK / CH, PITCH = GS_BK + CH;
+  static constexpr int CH = VEC ? 16 / (int)sizeof(T) : 1, PER_ROW = GS_BK / CH, PITCH = GS_BK + 16 / (int)sizeof(T);
   static constexpr int STEP = THREADS / PER_ROW, COPIES = (ROWS + STEP - 1) / STEP;
   const T* base;         // something to point at where nothing is read
   const T* src;
@@ -86,13 +90,10 @@ struct Stager {
 #pragma unroll
     for (int u = 0; u < COPIES; ++u) {
       if (ROWS % STEP == 0 || (int)threadIdx.x / PER_ROW + u * STEP < ROWS) {
-        if (VEC) {
-          const bool valid = u < rows && k0 + kk < k;
-          gs_copy16(to + u * STEP * PITCH, valid ? from : base, valid);
-        } else {
-#pragma unroll
-          for (int e = 0; e < CH; ++e) to[u * STEP * PITCH + e] = u < rows && k0 + kk + e < k ? from[e] : from_float<T>(0.f);
-        }
+        const bool valid = u < rows && k0 + kk < k;
+        if (VEC) gs_copy16(to + u * STEP * PITCH, valid ? from : base, valid);
+        else if (sizeof(T) == 4) gs_copy4(to + u * STEP * PITCH, valid ? from : base, valid);
+        else to[u * STEP * PITCH] = valid ? *from : from_float<T>(0.f);
       }
       from += step;
     }
@@ -349,7 +350,15 @@ int launch_typed(const Product& p, int batch, cudaStream_t stream) {
   };
   const bool vec = whole(p.x, p.ldx, batch > 1 ? p.batch_x : 0, p.k, sizeof(TX)) &&
                    whole(p.w, p.k, batch > 1 ? p.batch_w : 0, p.k, sizeof(TW));
-  if (!vec) return launch_tile<TX, TW, 4, 4, 8, 8, false>(p, batch, stream);
+  const long long big = (long long)((p.o + 63) / 64) * ((p.n + 63) / 64) * batch;
+  if (!vec) {
+    // Rows that do not start on 16 bytes, 32-bit operands, us (one number a copy, 64 x 64 or 32 x 32 tiles by this
+    // rule / 32 x 32 always, filled through registers / 64 x 64 by 256 threads, the kernel before both): 16 x 4,096 x
+    // 1,023 27 / 35 / 58, 64 x 4,096 x 1,023 45 / 71 / 60, 500 x 1,024 x 3,071 170 / 318 / 181, 500 x 4,096 x 1,023
+    // 130 / 216 / 164, 2,000 x 4,096 x 1,023 434 / 783 / 568.
+    if (p.n > 32 && (big >= 296 || (p.n <= 64 && big >= 64))) return launch_tile<TX, TW, 8, 4, 8, 16, false>(p, batch, stream);
+    return launch_tile<TX, TW, 4, 4, 8, 8, false>(p, batch, stream);
+  }
   // Few rows: as many columns a block as still give every SM one.  Measured with 32-bit operands, us
   // (8 / 16 / 32 columns): 4 x 1,024 x 3,072 14.7 / 16.0 / 16.8, 4 x 4,096 x 1,024 9.1 / 7.9 / 9.6,
   // 4 x 32,000 x 1,024 43 / 44 / 36; 16 x 1,024 x 3,072 23.0 / 25.7 / 26.7, 16 x 4,096 x 1,024 18.4 / 13.4 / 16.6,
@@ -367,7 +376,6 @@ int launch_typed(const Product& p, int batch, cudaStream_t stream) {
   // Many rows: tiles of 64 x 64 by 128 threads (8 x 4 each) where they fill the SMs twice, else of
   // 32 x 32 by 64 threads: 500 x 1,024 x 3,072 165 us against 211, 2,000 x 4,096 x 1,024 415 against 371 (45 TFLOP/s),
   // 64 x 4,096 x 1,024 43 against 37; 256 threads with 4 x 4 each, as before, 227 and 412.
-  const long long big = (long long)((p.o + 63) / 64) * ((p.n + 63) / 64) * batch;
   if (big >= 296 || (p.n <= 64 && big >= 64)) return launch_tile<TX, TW, 8, 4, 8, 16, true>(p, batch, stream);
   return launch_tile<TX, TW, 4, 4, 8, 8, true>(p, batch, stream);
 }

@@ -64,6 +64,18 @@ def test_batched_product_with_strided_rows(native, n):
     assert float((out[:, :, o:] - 7.0).abs().max()) == 0.0
 
 
+@pytest.mark.parametrize("xd, wd", [(torch.float32, torch.float32), (torch.float32, torch.bfloat16), (torch.bfloat16, torch.float32), (torch.bfloat16, torch.bfloat16)])
+@pytest.mark.parametrize("n, o, k", ((33, 2100, 65), (65, 4200, 31), (130, 9000, 33), (500, 1300, 127), (40, 64, 1)))
+def test_product_of_rows_off_16_bytes(native, xd, wd, n, o, k):
+    """Odd depths in both tile sizes, one operand or both a number at a time."""
+    gen = torch.Generator().manual_seed(n + k)
+    x, w = torch.randn((n, k), generator=gen).to(xd).to(DEV), torch.randn((o, k), generator=gen).to(wd).to(DEV)
+    got = torch.empty((n, o), device=DEV)
+    native.gemm_simt(x, w, got)
+    bound = (x.double().abs() @ w.double().abs().t()) * (k + 1) * 2.0**-24
+    assert bool(((got.double() - x.double() @ w.double().t()).abs() <= bound).all())
+
+
 @pytest.mark.parametrize("n, o, k", ((1, 100, 1024), (4, 300, 1152), (16, 9000, 2048)))
 def test_a_wait_that_runs_out_is_reported(native, n, o, k):
     """Loaders that do not report a stretch of k: the block gives up after a few polls, the status word says so and
