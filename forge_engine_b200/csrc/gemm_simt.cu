@@ -61,41 +61,69 @@ __device__ __forceinline__ void gs_store(const Product& p, float v, int r, int c
 // columns tx + TX j of the block's tile.
 #define GS_BK 32
 #define GS_STAGES 3
+#define GS_PITCH (GS_BK + 4)
 
 // What a thread copies of one operand's stages: rows row, row + STEP, ... of ROWS, one piece of each; zeros
 // stand where a row or a k does not exist.  A piece is 16 bytes with VEC: rows start on 16-byte boundaries and
-// k is a multiple of 16 bytes.  Otherwise it is one number, a warp's 32 of them neighbours: 32-bit ones by
-// cp.async too, bfloat16 ones through registers.
+// k is a multiple of 16 bytes.  Otherwise it is one number, a warp's 32 of them neighbours.  Tiles hold 32-bit
+// numbers: 32-bit operands go there by cp.async, bfloat16 ones through registers, asked for a stage earlier (read
+// from shared memory as they were, they would be widened once per output: 500 x 1,024 x 3,072 with
+// bfloat16 rows, weights or both 213, 220 and 240 us, 187, 184 and 208 this way).
 template <typename T, int ROWS, int THREADS, bool VEC>
 struct Stager {
-  static constexpr int CH = VEC ? 16 / (int)sizeof(T) : 1, PER_ROW = GS_BK / CH, PITCH = GS_BK + 16 / (int)sizeof(T);
+  static constexpr bool HELD = sizeof(T) == 2;
+  static constexpr int CH = VEC ? 16 / (int)sizeof(T) : 1, PER_ROW = GS_BK / CH;
   static constexpr int STEP = THREADS / PER_ROW, COPIES = (ROWS + STEP - 1) / STEP;
   const T* base;         // something to point at where nothing is read
   const T* src;
   long long step;
   int kk, rows;          // rows of this thread's that exist
-  T* dst;
-  __device__ __forceinline__ Stager(T* tile, const T* from, long long ld, int row0, int limit) : base(from) {
+  float* dst;
+  uint4 held[HELD && VEC ? COPIES : 1];
+  T one[HELD && !VEC ? COPIES : 1];
+  __device__ __forceinline__ Stager(float* tile, const T* from, long long ld, int row0, int limit) : base(from) {
     const int row = threadIdx.x / PER_ROW;
     kk = (threadIdx.x % PER_ROW) * CH;
     src = base + (size_t)min(row0 + row, limit - 1) * ld + kk;
     step = STEP * ld;
     const int have = min(limit - row0, ROWS) - row;
     rows = have <= 0 ? 0 : (have + STEP - 1) / STEP;
-    dst = tile + row * PITCH + kk;
+    dst = tile + row * GS_PITCH + kk;
   }
-  __device__ __forceinline__ void copy(int stage, int k0, int k) const {
-    T* to = dst + stage * (ROWS * PITCH);
+  // 32-bit operands: stage `stage` is on its way.  bfloat16 ones: held for put().
+  __device__ __forceinline__ void get(int stage, int k0, int k) {
+    float* to = dst + stage * (ROWS * GS_PITCH);
     const T* from = src + k0;
 #pragma unroll
     for (int u = 0; u < COPIES; ++u) {
       if (ROWS % STEP == 0 || (int)threadIdx.x / PER_ROW + u * STEP < ROWS) {
         const bool valid = u < rows && k0 + kk < k;
-        if (VEC) gs_copy16(to + u * STEP * PITCH, valid ? from : base, valid);
-        else if (sizeof(T) == 4) gs_copy4(to + u * STEP * PITCH, valid ? from : base, valid);
-        else to[u * STEP * PITCH] = valid ? *from : from_float<T>(0.f);
+        if constexpr (HELD && VEC) held[u] = valid ? *reinterpret_cast<const uint4*>(from) : make_uint4(0u, 0u, 0u, 0u);
+        else if constexpr (HELD) one[u] = valid ? *from : from_float<T>(0.f);
+        else if constexpr (VEC) gs_copy16(to + u * STEP * GS_PITCH, valid ? from : base, valid);
+        else gs_copy4(to + u * STEP * GS_PITCH, valid ? from : base, valid);
       }
       from += step;
+    }
+  }
+  __device__ __forceinline__ void put(int stage) const {
+    if constexpr (HELD) {
+      float* to = dst + stage * (ROWS * GS_PITCH);
+#pragma unroll
+      for (int u = 0; u < COPIES; ++u) {
+        if (ROWS % STEP == 0 || (int)threadIdx.x / PER_ROW + u * STEP < ROWS) {
+          if constexpr (VEC) {
+            const unsigned w[4] = {held[u].x, held[u].y, held[u].z, held[u].w};
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+              *reinterpret_cast<float4*>(to + u * STEP * GS_PITCH + 4 * e) =
+                  make_float4(__uint_as_float(w[2 * e] << 16), __uint_as_float(w[2 * e] & 0xffff0000u),
+                              __uint_as_float(w[2 * e + 1] << 16), __uint_as_float(w[2 * e + 1] & 0xffff0000u));
+          } else {
+            to[u * STEP * GS_PITCH] = to_float(one[u]);
+          }
+        }
+      }
     }
   }
 };
@@ -103,15 +131,15 @@ struct Stager {
 template <typename TX_, typename TW_, int TM, int TN, int TY, int TX, bool VEC>
 __global__ void __launch_bounds__(TY * TX) gemm_simt_tile_kernel(const Product p) {
   constexpr int BM = TM * TY, BN = TN * TX, THREADS = TY * TX;
-  constexpr int PX = GS_BK + 16 / (int)sizeof(TX_), PW = GS_BK + 16 / (int)sizeof(TW_);
+  constexpr int PX = GS_PITCH, PW = GS_PITCH;
   extern __shared__ __align__(16) unsigned char smem[];
-  TX_* xs = (TX_*)smem;
-  TW_* ws = (TW_*)(smem + (size_t)GS_STAGES * BM * PX * sizeof(TX_));
+  float* xs = (float*)smem;
+  float* ws = xs + GS_STAGES * BM * PX;
   pdl_trigger();
   pdl_wait();
   const int row0 = blockIdx.y * BM, col0 = blockIdx.x * BN;
-  const Stager<TX_, BM, THREADS, VEC> get_x(xs, (const TX_*)p.x + (size_t)blockIdx.z * p.batch_x, p.ldx, row0, p.n);
-  const Stager<TW_, BN, THREADS, VEC> get_w(ws, (const TW_*)p.w + (size_t)blockIdx.z * p.batch_w, p.k, col0, p.o);
+  Stager<TX_, BM, THREADS, VEC> x_in(xs, (const TX_*)p.x + (size_t)blockIdx.z * p.batch_x, p.ldx, row0, p.n);
+  Stager<TW_, BN, THREADS, VEC> w_in(ws, (const TW_*)p.w + (size_t)blockIdx.z * p.batch_w, p.k, col0, p.o);
   const int ty = threadIdx.x / TX, tx = threadIdx.x % TX;
   float acc[TM][TN];
 #pragma unroll
@@ -123,8 +151,9 @@ __global__ void __launch_bounds__(TY * TX) gemm_simt_tile_kernel(const Product p
 #pragma unroll
   for (int s = 0; s < GS_STAGES - 1; ++s) {
     if (s < steps) {
-      get_x.copy(s, s * GS_BK, p.k);
-      get_w.copy(s, s * GS_BK, p.k);
+      x_in.get(s, s * GS_BK, p.k);
+      w_in.get(s, s * GS_BK, p.k);
+      if (s == 0) x_in.put(0), w_in.put(0);
     }
     gs_commit();
   }
@@ -132,15 +161,16 @@ __global__ void __launch_bounds__(TY * TX) gemm_simt_tile_kernel(const Product p
   for (int step = 0; step < steps; ++step) {
     gs_wait<GS_STAGES - 2>();
     __syncthreads();
-    const int next = step + GS_STAGES - 1;
+    const int next = step + GS_STAGES - 1, after = stage + 1 == GS_STAGES ? 0 : stage + 1;
+    if (step + 1 < steps) x_in.put(after), w_in.put(after);       // what is held of the stage after this one
     if (next < steps) {
       const int to = stage == 0 ? GS_STAGES - 1 : stage - 1;
-      get_x.copy(to, next * GS_BK, p.k);
-      get_w.copy(to, next * GS_BK, p.k);
+      x_in.get(to, next * GS_BK, p.k);
+      w_in.get(to, next * GS_BK, p.k);
     }
     gs_commit();
-    const TX_* xt = xs + stage * BM * PX + ty * PX;
-    const TW_* wt = ws + stage * BN * PW + tx * PW;
+    const float* xt = xs + stage * BM * PX + ty * PX;
+    const float* wt = ws + stage * BN * PW + tx * PW;
     float a[2][TM][4], b[2][TN][4];          // the next four k are read while these four are summed
 #pragma unroll
     for (int i = 0; i < TM; ++i) load4(xt + i * TY * PX, a[0][i]);
@@ -161,7 +191,7 @@ __global__ void __launch_bounds__(TY * TX) gemm_simt_tile_kernel(const Product p
 #pragma unroll
           for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[u & 1][i][e], b[u & 1][j][e], acc[i][j]);
     }
-    stage = stage + 1 == GS_STAGES ? 0 : stage + 1;
+    stage = after;
   }
 #pragma unroll
   for (int i = 0; i < TM; ++i) {
@@ -325,7 +355,7 @@ int launch_sized(K kernel, dim3 grid, int threads, size_t smem, cudaStream_t str
 template <typename TX_, typename TW_, int TM, int TN, int TY, int TX, bool VEC>
 int launch_tile(const Product& p, int batch, cudaStream_t stream) {
   constexpr int BM = TM * TY, BN = TN * TX;
-  const size_t smem = (size_t)GS_STAGES * (BM * (GS_BK * sizeof(TX_) + 16) + BN * (GS_BK * sizeof(TW_) + 16));
+  const size_t smem = (size_t)GS_STAGES * (BM + BN) * GS_PITCH * sizeof(float);
   dim3 grid((p.o + BN - 1) / BN, (p.n + BM - 1) / BM, batch);
   if (grid.y > 65535) return FE_ERR_TOO_LARGE;
   return launch_sized(gemm_simt_tile_kernel<TX_, TW_, TM, TN, TY, TX, VEC>, grid, TY * TX, smem, stream, p);
