@@ -20,6 +20,8 @@
 // sum in index order exceeds target.
 #include "common.cuh"
 
+#include <atomic>
+
 #define FE_STATUS_BAD_LOGITS 16
 #define SMP_THREADS 1024
 #define MASS_SCALE 1099511627776.0f  // 2^40
@@ -504,6 +506,60 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
 #undef SHIFTED
 }
 
+// Shared memory of a block's slice, and the most of it that fits an SM beside the histograms' 35 KB.
+#define SMP_SLICE_MOST (190 * 1024)
+static size_t slice_bytes(int vocab, int parts) { return ((size_t)slice_at((vocab + parts - 1) / parts) + 1) * sizeof(float); }
+
+// Clusters of `parts` blocks that run at once.  A block has an SM to itself (1,024 threads of 62 registers), and a
+// cluster's blocks lie in one group of SMs: 148, 74, 33 and 15 clusters of 1, 2, 4 and 8 on a whole B200.
+static int resident_clusters(int parts) {
+  static std::atomic<int> known[16][4];
+  int device = 0, slot = parts == 1 ? 0 : parts == 2 ? 1 : parts == 4 ? 2 : 3;
+  if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 16) return 148 / parts;
+  int count = known[device][slot].load(std::memory_order_relaxed);
+  if (count > 0) return count;
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3(parts, 1);
+  config.blockDim = dim3(SMP_THREADS);
+  cudaLaunchAttribute attribute[1];
+  attribute[0].id = cudaLaunchAttributeClusterDimension;
+  attribute[0].val.clusterDim.x = parts;
+  attribute[0].val.clusterDim.y = 1;
+  attribute[0].val.clusterDim.z = 1;
+  config.attrs = attribute;
+  config.numAttrs = 1;
+  if (cudaOccupancyMaxActiveClusters(&count, sample_kernel, &config) != cudaSuccess || count < 1) {
+    cudaGetLastError();
+    count = 148 / parts;
+  }
+  known[device][slot].store(count, std::memory_order_relaxed);
+  return count;
+}
+
+// How many blocks share a row: the number for which the rounds of clusters that run at once, times what a
+// block's slice takes, is least.  A slice takes 30 us and 1.4 us per 1,000 logits where it is kept in shared
+// memory, 45 and 1.85 where every pass reads it again, from L2 (3.3 where the rows at hand do not fit there); top-k 50
+// and top-p 0.95.  Measured, 1 / 2 / 4 / 8 blocks a row, us: 8 rows of
+// 151,936 330 / 187 / 88 / 64, 16 rows 326 / 187 / 86 / 122, 40 rows 327 / 186 / 168 / 185, 64 rows 328 / 188 /
+// 172 / 302, 128 rows 333 / 368 / 336 / 544; 40 rows of 32,000 70 / 51 / 76 / 118, 256 rows 135 / 191 / 300 / 663; 64 rows
+// of 300,000 611 / 337 / 372 / 436, 128 rows 1047 / 715 / 757 / 815.
+static int sample_parts(int rows, int vocab) {
+  int best = 1;
+  double least = 0.0;
+  for (int parts = 1; parts <= 8 && (parts == 1 || vocab >= parts * 4096); parts *= 2) {
+    const int resident = resident_clusters(parts), rounds = (rows + resident - 1) / resident;
+    const double slice = (double)((vocab + parts - 1) / parts);
+    const bool in_l2 = (double)(rows < resident ? rows : resident) * vocab * 4.0 < 110e6;
+    const double time = rounds * (slice_bytes(vocab, parts) <= SMP_SLICE_MOST ? 30.0 + 1.4e-3 * slice
+                                                                              : 45.0 + (in_l2 ? 1.85e-3 : 3.3e-3) * slice);
+    if (parts == 1 || time < least) best = parts, least = time;
+  }
+  return best;
+}
+
+// What the rule above decides, for its test.
+FE_EXPORT int fe_sample_parts(int rows, int vocab) { return sample_parts(rows, vocab); }
+
 FE_EXPORT int fe_sample(const float* logits, int rows, int vocab, const float* temperature,
                         const int* top_k, const float* top_p, const float* min_p,
                         const unsigned long long* seeds, const unsigned long long* counters,
@@ -511,15 +567,15 @@ FE_EXPORT int fe_sample(const float* logits, int rows, int vocab, const float* t
   if (rows <= 0) return 0;
   if (vocab <= 0) return FE_ERR_BAD_SHAPE;
   if (rows > 65535) return FE_ERR_TOO_LARGE;
-  // a row's vocabulary over up to 8 blocks (one cluster) of at least 4,096 logits each, while the blocks of
-  // all rows still run at once (two fit on each of the 148 SMs) or a slice does not fit an SM twice
-  auto slice_bytes = [&](int parts) { return ((size_t)slice_at((vocab + parts - 1) / parts) + 1) * sizeof(float); };
-  const size_t half = 80 * 1024, whole = 190 * 1024;        // beside the histograms' 32 KB
+  // A row's vocabulary over up to 8 blocks (one cluster) of at least 4,096 logits each.
   int parts = 1;
-  while (parts < 8 && vocab >= parts * 2 * 4096 &&
-         (rows * parts * 2 <= 296 || (temperature != nullptr && slice_bytes(parts) > half))) parts *= 2;
-  size_t smem = temperature == nullptr ? 0 : slice_bytes(parts);
-  if (smem > half && (smem > whole || rows * parts > 148)) smem = 0;
+  size_t smem = 0;
+  if (temperature == nullptr) {
+    while (parts < 8 && rows * parts * 2 <= 296 && vocab >= parts * 2 * 4096) parts *= 2;
+  } else {
+    parts = sample_parts(rows, vocab);
+    if (slice_bytes(vocab, parts) <= SMP_SLICE_MOST) smem = slice_bytes(vocab, parts);
+  }
   if (smem > 0) {
     const cudaError_t set = cudaFuncSetAttribute(sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (set != cudaSuccess) return (int)set;

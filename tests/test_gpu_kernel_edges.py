@@ -357,6 +357,15 @@ def drawn(row, temperature, top_k, top_p, u):
     return min(index, int(torch.nonzero(weights > 0)[-1])), running, target
 
 
+def test_blocks_of_a_row_run_at_once(native):
+    """A block has an SM to itself and clusters fit only whole: the rows of a call are cut so that they take no more rounds
+    than they have to."""
+    parts = native.lib().fe_sample_parts
+    assert [parts(n, 151936) for n in (1, 8, 24, 28, 64, 128)] == [8, 8, 4, 4, 4, 1]
+    assert [parts(n, 32000) for n in (1, 16, 28, 40, 70, 128, 256)] == [4, 4, 4, 2, 2, 1, 1]
+    assert [parts(n, 300000) for n in (12, 28, 64, 128)] == [8, 8, 2, 2] and parts(1, 8191) == 1 and parts(1, 8192) == 2
+
+
 @pytest.mark.parametrize("rows, vocab", ((1, 4096), (3, 16385), (40, 32768), (64, 151936), (5, 300000), (25, 300000), (2, 700001)))
 @pytest.mark.parametrize("top_k, top_p", ((0, 1.0), (37, 1.0), (0, 0.8), (50, 0.9)))
 def test_sampling_of_long_rows(native, rows, vocab, top_k, top_p):
