@@ -357,8 +357,9 @@ struct Delta {
 // and beta v, sixteen rows at a time.  A block of rows first loses what the rows before it give, then a
 // thread per column solves the 16 x 16 triangle in registers and stores the result, also for the blocks
 // below.  The products (L itself, and a block's from the rows before it) run on the tensor cores, both
-// operands split: 2,048 tokens of 32 heads of 64 channels take 68 us, 80 as tiles of multiply-adds; what
-// remains is the triangles, one row after the other, and the loads before them.
+// operands split; what remains is the triangles, one row after the other, and the loads before them.  Solve, chain and
+// outputs of 2,048 tokens, 32 heads of 64 channels: 307 us, 371 with tiles of multiply-adds; 3 prompts of 1,000 to 666 tokens,
+// heads of 128: 971 and 1,062; outputs' error against 64 bits 1.3e-7 and 1.9e-7, 1.3e-7 and 2.3e-7.
 #define DS_THREADS 256
 // Columns of the right sides: k in fours, then v, in eights altogether.
 __host__ __device__ static inline int ds_columns(int dk, int dv) { return (((dk + 3) & ~3) + dv + 7) & ~7; }
@@ -477,7 +478,7 @@ __global__ void __launch_bounds__(DS_THREADS) delta_solve_kernel(const Delta m, 
 // outputs, reads 48 numbers a lane where a 4 x 2 tile of multiply-adds read 192, and a chunk has two
 // barriers.  The state's columns stay in registers, as the warps' pieces of the second product, and in shared
 // memory for the first; the next chunk's W and keys, and what a lane needs of it besides, are on their way
-// while a chunk is worked on.  2,048 tokens, 32 heads of 64 channels: 102 us, 179 with multiply-adds.
+// while a chunk is worked on.
 #define DC_WP (SR_LONG + 8)          // pitches: the rows of a fragment fall into different banks
 template <int KD, int COLS>
 __global__ void __launch_bounds__(16 * COLS) delta_chain_kernel(const Delta m, const StateRun p, int* status) {
@@ -675,8 +676,8 @@ FE_EXPORT int fe_delta_rule(const float* qkv, long long ld, const float* gates, 
   rc = fe_launch_dependent(delta_solve_kernel, dim3(heads, entries, chunks), dim3(DS_THREADS), smem, stream, m, p);
   if (rc) return rc;
   // delta_chain is not launched as a dependent: its blocks, fewer than the SMs or not many more, would take their
-  // places while delta_solve's last blocks leave theirs, two on one SM and none on the next (143 us for a chain
-  // over 2,048 tokens that takes 102 us spread evenly).
+  // places while delta_solve's last blocks leave theirs, two on one SM and none on the next (measured with two tf32
+  // numbers an operand: 143 us for a chain over 2,048 tokens that took 102 us spread evenly).
   const int cols = delta_chain_cols(dv);
   smem = delta_chain_smem(dk, cols);
   const dim3 chain(heads, entries, (dv + cols - 1) / cols);

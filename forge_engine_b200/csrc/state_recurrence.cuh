@@ -433,10 +433,10 @@ __device__ __forceinline__ void sr_running_max(double& a, double& b) {
 //   NORMALISER        whether rows are divided by max(|sum|, floor_t) + 1e-6 (M's `start_norm`)
 // 256 threads: a warp takes 32 tokens and, in pass n, 16 of the columns 64 n ..; the products run on the
 // tensor cores with both operands split (mma_split.cuh), since multiply-adds fed from shared memory in tiles of
-// 4 x 4 are bound by what it delivers.  Retention over 1,024 tokens, 16 heads of 128 channels, all kernels: 98 us
-// against 114, 32 heads of 64: 62 against 70; its error against 64 bits falls from 2.6e-7 to 2.0e-7 and from
-// 2.2e-7 to 1.9e-7.  The delta rule over 2,048 tokens, 32 heads of 64: 80 us of this kernel against 85, bound by
-// the latency of the tiles' loads, which nothing overlaps within a block.
+// 4 x 4 are bound by what it delivers.  Retention over 1,024 tokens, 16 heads of 128 channels, all kernels: 109 us
+// against 115, 32 heads of 64: 69 against 69, 8 heads of 256: 261 against 313; its error against 64 bits falls from 2.6e-7
+// to 1.6e-7 and from 2.2e-7 to 1.6e-7.  Bound by the instructions that split the operands and the latency of the tiles'
+// loads, which nothing overlaps within a block.
 struct OutTile {            // a warp's 32 x 16 outputs
   float sum[2][2][4], small[2][2][4];
   __device__ __forceinline__ void clear() {
