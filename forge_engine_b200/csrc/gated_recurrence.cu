@@ -571,6 +571,39 @@ __global__ void __launch_bounds__(256, 2) gated_recurrence_finish_kernel(GatedRe
       __syncthreads();               // this stretch has landed; everyone is done with the one before it
       if (step + stages - 1 < steps) stage(step + stages - 1, v0, nv);
       gr_commit();
+      if (step >= q_steps) {
+        // What is too loud to be split joins by multiply-adds, and only the tokens that see it: its products with
+        // the zeros of A would not be zero.
+        float* ys = smem + (step % stages) * stage_floats + GR_LONG_CHUNK * GR_FX;
+        bool loud = false;
+        const int quads = nv >> 2;
+        for (int i = tid; i < GR_FK * quads; i += 256) {
+          float x[4];
+          load4(ys + (i / quads) * pitch + (i % quads) * 4, x);
+          loud |= split_loud(x[0]) || split_loud(x[1]) || split_loud(x[2]) || split_loud(x[3]);
+        }
+        if (__syncthreads_or(loud)) {
+          const float* xs = ys - GR_LONG_CHUNK * GR_FX;
+#pragma unroll
+          for (int a = 0; a < 2; ++a)
+#pragma unroll
+            for (int b = 0; b < 4; ++b)
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const int t = m0 + 16 * a + 8 * (i >> 1) + fg, c = n0 + 8 * b + 2 * fq + (i & 1);
+                if (c >= nv) continue;
+#pragma unroll 1
+                for (int s = 0; s < GR_FK && s + GR_FK * (step - q_steps) <= t; ++s)
+                  if (split_loud(ys[s * pitch + c])) sum[a][b][i] = fmaf(xs[t * GR_FX + s], ys[s * pitch + c], sum[a][b][i]);
+              }
+          __syncthreads();
+          for (int i = tid; i < GR_FK * nv; i += 256) {
+            float& x = ys[(i / nv) * pitch + i % nv];
+            if (split_loud(x)) x = 0.f;
+          }
+          __syncthreads();
+        }
+      }
       // the first 32 tokens come before all tokens of the second stretch of V: A is zero there
       if (n0 < nv && (m0 > 0 || step <= q_steps)) {
         const float* xs = smem + (step % stages) * stage_floats + (m0 + fg) * GR_FX + fq;

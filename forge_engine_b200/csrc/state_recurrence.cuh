@@ -364,10 +364,11 @@ __device__ __forceinline__ void sr_stage_transposed(float* dst, const Rows& src,
 }
 
 // Columns c0 .. c0 + 63 of `count` of `rows` rows of `width` numbers as a tile dst[row * PITCH + column];
-// zero past the last row and the last column.
+// zero past the last row and the last column.  Whether one of this thread's is too loud to be split.
 template <int PITCH = 64>
-__device__ __forceinline__ void sr_stage_columns(float* dst, const Rows& src, int rows, int count, int c0, int width) {
+__device__ __forceinline__ bool sr_stage_columns(float* dst, const Rows& src, int rows, int count, int c0, int width) {
   const int step = blockDim.x;
+  bool loud = false;
   if (src.wide(width)) {
     const int items = rows * 16;
     for (int i0 = threadIdx.x; i0 < items; i0 += 4 * step) {
@@ -376,6 +377,7 @@ __device__ __forceinline__ void sr_stage_columns(float* dst, const Rows& src, in
       for (int j = 0; j < 4; ++j) {
         const int i = i0 + j * step, r = i >> 4, c = c0 + (i & 15) * 4;
         x[j] = (r < count && c < width) ? *reinterpret_cast<const float4*>(src.row(r) + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+        loud |= split_loud(x[j].x) || split_loud(x[j].y) || split_loud(x[j].z) || split_loud(x[j].w);
       }
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -383,7 +385,7 @@ __device__ __forceinline__ void sr_stage_columns(float* dst, const Rows& src, in
         if (i < items) *reinterpret_cast<float4*>(dst + (i >> 4) * PITCH + (i & 15) * 4) = x[j];
       }
     }
-    return;
+    return loud;
   }
   const int items = rows * 64;
   for (int i0 = threadIdx.x; i0 < items; i0 += 4 * step) {
@@ -392,6 +394,7 @@ __device__ __forceinline__ void sr_stage_columns(float* dst, const Rows& src, in
     for (int j = 0; j < 4; ++j) {
       const int i = i0 + j * step, r = i >> 6, c = c0 + (i & 63);
       x[j] = (r < count && c < width) ? src.row(r)[c] : 0.f;
+      loud |= split_loud(x[j]);
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -399,6 +402,7 @@ __device__ __forceinline__ void sr_stage_columns(float* dst, const Rows& src, in
       if (i < items) dst[(i >> 6) * PITCH + (i & 63)] = x[j];
     }
   }
+  return loud;
 }
 
 // Inclusive running sum / maximum over 64 numbers held by a warp: element lane in `a`, element
@@ -446,6 +450,16 @@ struct OutTile {            // a warp's 32 x 16 outputs
       for (int b = 0; b < 2; ++b)
 #pragma unroll
         for (int i = 0; i < 4; ++i) sum[a][b][i] = small[a][b][i] = 0.f;
+  }
+  // the sum of number i (all 16: rows' halves a, columns' halves b, as in `sum`)
+  __device__ __forceinline__ void set(int i, float x) {
+#pragma unroll
+    for (int a = 0; a < 2; ++a)
+#pragma unroll
+      for (int b = 0; b < 2; ++b)
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (i == 8 * a + 4 * b + e) sum[a][b][e] = x;
   }
   // += X^T Y over `depth` rows (a multiple of 8) of both: x at this lane's place in [k][token], y in [k][column]
   __device__ __forceinline__ void add(const float* x, const float* y, int ldy, int depth) {
@@ -529,8 +543,23 @@ __global__ void __launch_bounds__(256) state_out_kernel(const M m, const StateRu
     old.clear();
     if constexpr (M::SCORES) {
       __syncthreads();
-      sr_stage_columns<SR_OP>(tile, m.others(p, head, at), SR_LONG, at.count, c0, dv);
-      __syncthreads();
+      if (__syncthreads_or(sr_stage_columns<SR_OP>(tile, m.others(p, head, at), SR_LONG, at.count, c0, dv))) {
+        // what is too loud to be split joins by multiply-adds, and only the tokens that see it
+#pragma unroll 1
+        for (int i = 0; i < 16; ++i) {
+          const int a = i >> 3, b = (i >> 2) & 1, t = m0 + 16 * a + 8 * ((i >> 1) & 1) + fg, c = n0 + 8 * b + 2 * fq + (i & 1);
+          float x = 0.f;
+          for (int j = 0; j <= t; ++j)
+            if (split_loud(tile[j * SR_OP + c])) x = fmaf(as[j * SR_TP + t], tile[j * SR_OP + c], x);
+          own.set(i, x);
+        }
+        __syncthreads();
+        for (int i = tid; i < SR_LONG * 64; i += 256) {
+          float& x = tile[(i >> 6) * SR_OP + (i & 63)];
+          if (split_loud(x)) x = 0.f;
+        }
+        __syncthreads();
+      }
       own.add(as + fq * SR_TP + m0 + fg, tile + fq * SR_OP + n0 + fg, SR_OP, min((at.count + 7) & ~7, m0 + 32));
     }
     __syncthreads();

@@ -301,6 +301,51 @@ def test_delta_rule_chunks(native, kv_heads, heads, dk, dv, counts):
     assert torch.equal(got_state[-1].cpu(), state[-1])       # the row of no entry
 
 
+# -- values that are not finite --------------------------------------------------------------------
+@pytest.mark.parametrize("loud", (float("inf"), float("nan"), 3.4e38))
+@pytest.mark.parametrize("name, dk, dv", (("gated", 64, 64), ("gated", 12, 100), ("gated", 12, 260), ("delta", 64, 64), ("delta", 72, 130),
+                                          ("retention", 64, 64), ("retention", 40, 200), ("memory", 64, 64), ("memory", 24, 72)))
+def test_a_loud_value_reaches_no_earlier_token(native, name, dk, dv, loud):
+    """A value that is infinite, no number, or rounds to infinity as a bfloat16 number, late in a chunk: the rows of the
+    tokens before it, and of other heads, are what they are without it, bit for bit."""
+    heads, n = 2, 200
+    gen = torch.Generator().manual_seed(dk + dv)
+    rand = lambda *shape: torch.randn(*shape, generator=gen)  # noqa: E731
+    ints = lambda values: torch.tensor(values, dtype=torch.int32, device=DEV)  # noqa: E731
+    qk, v = heads * dk, heads * dv
+    proj, gate, norm, gates = rand(n, 2 * qk + 2 * v + 2 * heads), rand(n, v), torch.ones(v, device=DEV), torch.rand(n, heads, 2, generator=gen)
+    proj[:, : 2 * qk] *= dk**-0.5
+    gates[..., 1] *= -0.2
+
+    def run(values):
+        p = proj.clone()
+        p[:, 2 * qk : 2 * qk + v] = values
+        p, state, status = p.to(DEV), torch.zeros(2, heads, dk, dv, device=DEV), status_word()
+        out, slots, cu = torch.empty(n, v, device=DEV), ints([0]), ints([0, n])
+        if name == "gated":
+            native.gated_recurrence(p, 0, qk, 2 * qk, None, torch.zeros(qk, device=DEV), norm[:dv], 1e-5, state, slots, cu, out, 1, status, max_new=n)
+        elif name == "delta":
+            native.delta_rule(p[:, : 2 * qk + v].contiguous(), gates.to(DEV), gate.to(DEV), norm[:dv], 1e-5, state, slots, cu, out, heads, 1, n, status)
+        elif name == "retention":
+            native.retention(p, (0, qk, 2 * qk, 2 * qk + v), 1.0, torch.full((heads,), 0.97, device=DEV), None, 0, False, None, 1e-5, state, slots,
+                             cu, out, 1, n, status)
+        else:
+            native.matrix_memory(p, (0, qk, 2 * qk, 2 * qk + v, 2 * qk + 2 * v, 2 * qk + 2 * v + heads), torch.full((heads,), -2.0, device=DEV),
+                                 torch.full((heads,), 3.0, device=DEV), 15.0, 1.0, norm, 1e-5, state, torch.zeros(2, heads, dk, device=DEV),
+                                 torch.zeros(2, heads, device=DEV), slots, cu, out, 1, n, status)
+        assert int(status.item()) == 0
+        return out.view(n, heads, dv)
+
+    values = rand(n, v)
+    clean = run(values)
+    for at in (31, 50, 64, 127, 140):
+        spoilt = values.clone()
+        spoilt[at, dv // 2] = loud
+        got = run(spoilt)
+        assert torch.equal(got[:at], clean[:at]) and torch.equal(got[:, 1], clean[:, 1]), at
+        assert not torch.equal(got[at, 0], clean[at, 0])
+
+
 # -- delta rule's inputs ---------------------------------------------------------------------------
 @pytest.mark.parametrize("taps, dk, dv", ((2, 64, 64), (3, 32, 20), (4, 128, 128), (4, 40, 64), (4, 6, 10), (5, 64, 64)))
 @pytest.mark.parametrize("counts", ([256], [1, 2, 3, 270, 1], [100, 100, 57]))
