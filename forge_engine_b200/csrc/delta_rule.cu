@@ -19,7 +19,6 @@
 //                   the chunks with two products each (u, and the state it leads to); then
 //                     o_t = e^(c_t) S^T q_t + sum_(j <= t) e^(c_t - c_j) (q_t . k_j) u_j.
 #include "state_recurrence.cuh"
-#include "mma_split.cuh"
 
 // ---------------------------------------------------------------------------
 // delta_prepare
@@ -637,6 +636,8 @@ static size_t delta_chain_smem(int dk, int cols) {
   const size_t kp = (size_t)(dk + 63) / 64 * 64, dk8 = (size_t)(dk + 7) / 8 * 8, sp = cols + 8;
   return sizeof(float) * ((kp + SR_LONG) * sp + 2 * (dk8 * DC_WP + SR_LONG * (kp + 8)));
 }
+// Keys of up to 176 numbers with 16 columns a block and up to 152 with 32: what shared memory holds of a chunk and the
+// next one.  (The instantiations would reach 192.)
 static bool delta_chunk_takes(int dk, int dv) {
   return dk <= 192 && chunk_takes(dk, dv, true) && delta_solve_smem(dk, dv) <= 218 * 1024 &&
          delta_chain_smem(dk, delta_chain_cols(dv)) <= 226 * 1024;

@@ -262,13 +262,15 @@ def test_gated_recurrence_chunks(native, heads, dk, dv, lead, counts):
 
 
 # -- delta rule: chunks ---------------------------------------------------------------------------
-@pytest.mark.parametrize("kv_heads, heads, dk, dv", ((1, 2, 64, 64), (2, 2, 72, 40), (1, 1, 128, 128), (1, 2, 192, 36), (2, 4, 6, 10), (1, 1, 13, 5), (1, 1, 65, 129)))
+@pytest.mark.parametrize("kv_heads, heads, dk, dv", ((1, 2, 64, 64), (2, 2, 72, 40), (1, 1, 128, 128), (1, 2, 160, 36), (1, 1, 176, 64), (1, 1, 152, 100), (2, 4, 6, 10), (1, 1, 13, 5), (1, 1, 65, 129)))
 @pytest.mark.parametrize("counts", ([96], [97, 160, 3], [191, 1, 192, 130]))
 def test_delta_rule_chunks(native, kv_heads, heads, dk, dv, counts):
     """Heads that fill the fragments' eights and heads that do not (odd ones among them), chunks that are whole
     and that are cut, entries that are walked between them; from states that are not zero."""
     gen = torch.Generator().manual_seed(heads * 100 + dk + dv)
     n, qk = sum(counts), kv_heads * dk
+    room = native.lib().fe_delta_rule_scratch
+    assert room(n, len(counts), heads, dk, dv, max(counts)) > room(n, len(counts), heads, dk, dv, 1)      # not all of them walked
     rand = lambda *shape: torch.randn(*shape, generator=gen)  # noqa: E731
     unit = lambda x: x / x.norm(dim=-1, keepdim=True)  # noqa: E731
     q, k, v = unit(rand(n, kv_heads, dk)) * dk**-0.5, unit(rand(n, kv_heads, dk)), rand(n, heads, dv)
