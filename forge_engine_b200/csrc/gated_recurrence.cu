@@ -181,6 +181,9 @@ __device__ __forceinline__ float gr_sum16(float (&x)[16], int lane) {
 
 // One chunk of a long entry (see the head of this file).  Tokens past the entry's end have f = 1 and
 // q = k = v = 0.
+// R: channels a lane of the sub-chunks' own blocks holds, in a slice, as few as the head needs.  32 heads of 64, 2,048
+// tokens, all kernels: 216 us with two, 225 with four; 32 heads of 16, 1,000 tokens: 77 us with one, 89 with four.
+template <int R>
 __global__ void __launch_bounds__(256, 2) gated_recurrence_chunk_kernel(GatedRecurrence p, int aligned) {
   extern __shared__ __align__(16) float smem[];
   pdl_trigger();
@@ -261,16 +264,16 @@ __global__ void __launch_bounds__(256, 2) gated_recurrence_chunk_kernel(GatedRec
 #pragma unroll 1
       for (int pass = 0; pass < 8 / AT; ++pass) {
         const int s0 = (warp & 1) * 8 + pass * AT;
-        float w[AT][GR_SLICE / 32], sums[AT][GR_SUB];
+        float w[AT][R], sums[AT][GR_SUB];
 #pragma unroll
         for (int k = 0; k < AT; ++k)
 #pragma unroll
-          for (int r = 0; r < GR_SLICE / 32; ++r) w[k][r] = 0.f;
+          for (int r = 0; r < R; ++r) w[k][r] = 0.f;
 #pragma unroll
         for (int t = 0; t < GR_SUB; ++t) {
-          float f[GR_SLICE / 32], q[GR_SLICE / 32];
+          float f[R], q[R];
 #pragma unroll
-          for (int r = 0; r < GR_SLICE / 32; ++r) {
+          for (int r = 0; r < R; ++r) {
             const bool has = lane + 32 * r < ndp;
             f[r] = has ? fs[(base + t) * dp + lane + 32 * r] : 1.f;
             q[r] = has ? qs[(base + t) * dp + lane + 32 * r] : 0.f;
@@ -279,7 +282,7 @@ __global__ void __launch_bounds__(256, 2) gated_recurrence_chunk_kernel(GatedRec
           for (int k = 0; k < AT; ++k) {
             float sum = 0.f;
 #pragma unroll
-            for (int r = 0; r < GR_SLICE / 32; ++r) {
+            for (int r = 0; r < R; ++r) {
               w[k][r] = t == s0 + k ? 1.f - f[r] : w[k][r] * f[r];
               sum = fmaf(q[r], w[k][r], sum);
             }
@@ -770,11 +773,11 @@ FE_EXPORT int fe_gated_recurrence(const float* proj, long long ld, int q_off, in
   const int chunks = (max_new + GR_LONG_CHUNK - 1) / GR_LONG_CHUNK;
   if (chunks > 65535) return FE_ERR_TOO_LARGE;
   const size_t chunk_smem = gr_chunk_smem(dk, dv);
-  if (chunk_smem > 48 * 1024)
-    cudaFuncSetAttribute(gated_recurrence_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)chunk_smem);
+  auto chunk_kernel = dk <= 32 ? gated_recurrence_chunk_kernel<1> : dk <= 64 ? gated_recurrence_chunk_kernel<2> : gated_recurrence_chunk_kernel<GR_SLICE / 32>;
+  if (chunk_smem > 48 * 1024) cudaFuncSetAttribute(chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)chunk_smem);
   const int v_aligned = ((uintptr_t)proj & 15) == 0 && ld % 4 == 0 && v_off % 4 == 0;
   const int aligned = v_aligned && q_off % 4 == 0 && f_off % 4 == 0 && dk % 4 == 0 && (((uintptr_t)lower | (uintptr_t)f_bias) & 15) == 0;
-  rc = fe_launch_dependent(gated_recurrence_chunk_kernel, dim3(heads, entries, chunks), dim3(256), chunk_smem, stream, p, aligned);
+  rc = fe_launch_dependent(chunk_kernel, dim3(heads, entries, chunks), dim3(256), chunk_smem, stream, p, aligned);
   if (rc) return rc;
   rc = fe_launch_dependent(gated_recurrence_scan_kernel, dim3(heads, entries, (dk * dv + 511) / 512), dim3(128), 0, stream,
                            p, status);
