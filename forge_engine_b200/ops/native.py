@@ -1511,8 +1511,9 @@ def _attention_counters(device, pairs: int) -> torch.Tensor:
 
 
 def _attention_workspace(device, floats: int) -> torch.Tensor:
-    """Partial results of split decode attention.  One buffer per device serves every layer:
-    a layer's attention has combined its parts before the next layer's begins."""
+    """Partial results of split decode attention (bfloat16).  One buffer per device serves every layer:
+    a layer's attention has combined its parts before the next layer's begins.  Steps of several runners of one
+    device must therefore follow one another on the device, not run side by side on streams of their own."""
     return _scratch.get("attention workspace", device, floats, torch.float32, 1 << 22)
 
 
