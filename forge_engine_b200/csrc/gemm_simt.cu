@@ -1,9 +1,10 @@
-// y[n, o] = sum_k x[n, k] * w[o, k] (+ bias[o]) (+ y[n, o])   -- plain FFMA, no tensor cores.
+// y[n, o] = sum_k x[n, k] * w[o, k] (+ bias[o]) (+ y[n, o])   -- in 32 bits.
 //
 // This is the matrix product of the true 32-bit path and of any tensor whose
 // checkpoint dtype is float32.  Both operands are K-major, like nn.Linear's
-// [out, in] weight (src/forge_engine/qwen3.py:113-122).  Each output element is
-// summed over k in ascending order by one thread, in both kernels below, so a row's result
+// [out, in] weight (src/forge_engine/qwen3.py:113-122).  Deep products of 32-bit operands go to the tensor
+// cores (gemm_split.cuh); for the others each output element is summed over k in ascending order by one
+// thread, in both kernels below.  Which of the two does not depend on the number of rows, so a row's result
 // does not depend on how many other rows are in the call, nor on the tile.
 //
 // Tiles of both operands lie in shared memory as they lie in memory, rows of k with 16 bytes
@@ -56,6 +57,19 @@ __device__ __forceinline__ void gs_store(const Product& p, float v, int r, int c
     *dst = from_float<bf16>(p.accumulate ? v + to_float(*dst) : v);
   }
 }
+
+// Usually tc5::WAIT_LIMIT and no stretch; see fe_gemm_simt_set_test_fault.
+struct Fault {
+  unsigned wait_limit;
+  int skip_stretch;
+};
+Fault g_test_fault{tc5::WAIT_LIMIT, -1};
+
+}  // namespace
+
+#include "gemm_split.cuh"
+
+namespace {
 
 // Many rows: TY x TX threads keep TM x TN outputs each; thread (ty, tx) the rows ty + TY i and the
 // columns tx + TX j of the block's tile.
@@ -211,13 +225,6 @@ __global__ void __launch_bounds__(TY * TX) gemm_simt_tile_kernel(const Product p
 #define GSK_KT 128
 #define GSK_MAX_STAGES 8
 #define GSK_LOADERS 4
-// Usually tc5::WAIT_LIMIT and no stretch; see fe_gemm_simt_set_test_fault.
-struct Fault {
-  unsigned wait_limit;
-  int skip_stretch;
-};
-Fault g_test_fault{tc5::WAIT_LIMIT, -1};
-
 template <typename TX, typename TW, int COLS, int LC, int R>
 __global__ void __launch_bounds__(32 * (GSK_LOADERS + 8)) gemm_simt_rows_kernel(const Product p, int stages, const Fault fault) {
   constexpr int PX = GSK_KT + 16 / (int)sizeof(TX), PW = GSK_KT + 16 / (int)sizeof(TW);
@@ -371,15 +378,64 @@ int launch_rows(const Product& p, int batch, cudaStream_t stream) {
   return launch_sized(gemm_simt_rows_kernel<TX, TW, COLS, LC, R>, grid, 32 * (workers + GSK_LOADERS), stages * stage, stream, p, stages, g_test_fault);
 }
 
-// Which kernel: all of them give the same bits.
+template <int NT>
+int launch_split(const Product& p, int batch, int cuts, bool batched, cudaStream_t stream) {
+  const dim3 grid((unsigned)((p.o + 127) / 128) * cuts, (p.n + NT - 1) / NT, batch);
+  if (grid.y > 65535) return FE_ERR_TOO_LARGE;
+  const cudaError_t err = cudaFuncSetAttribute(gemm_split_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, gst_smem(NT));
+  if (err != cudaSuccess) return (int)err;
+  return fe_launch_dependent_shaped(gemm_split_kernel<NT>, grid, dim3(gst_workers(NT) + 32), gst_smem(NT), stream, dim3(cuts, 1, 1), p, cuts,
+                                    batched ? 1 : 0, g_test_fault);
+}
+
+// Rows of x a block takes, and into how many blocks (a cluster) k is cut: the number for which the time below is least.
+// Measured, us, w out of memory: by one block a tile 16 rows x 4,096 x 1,024 29, 1,024 x 2,048 47, 1,024 x 3,072 66 and by eight 18, 16
+// and 20; 128 rows of 500 x 4,096 x 1,024 45, 1,024 x 2,048 70, by four 78 and 31, by eight 113 and 51.  So a stretch takes
+// 1.15 to 1.6 us, a tile 10 to 19 besides; blocks beyond what the SMs hold start when others have ended (with up to 16 rows two
+// share an SM, and the time of a stretch).
+int split_cuts(int tile, long long tiles, int k) {
+  const int stretches = (k + GST_K - 1) / GST_K;
+  const double stretch = tile == 16 ? 1.15 : tile == 32 ? 1.2 : tile == 64 ? 1.3 : 1.6, again = tile == 16 ? 2.5 : tile == 128 ? 11.0 : 8.0;
+  const double fixed = tile == 16 ? 10.0 : tile == 32 ? 13.0 : tile == 64 ? 14.0 : 19.0;
+  int cuts = 1;
+  double least = 0.0;
+  for (int c = 1; c <= 8; c = c == 1 ? 4 : 2 * c) {
+    const int at_once = c == 8 ? 128 : c == 4 ? 136 : 148;        // clusters lie in one group of SMs
+    const double layers = (double)((tiles * c + at_once - 1) / at_once);
+    const double time = (c == 1 ? fixed : tile == 16 ? 12.5 : 16.0) + (stretches + c - 1) / c * stretch * layers + again * (layers - 1.0);
+    if (c == 1 || time < least) cuts = c, least = time;
+  }
+  return cuts;
+}
+
+int split_product(const Product& p, int batch, bool batched, cudaStream_t stream) {
+  const int tile = p.n <= 16 ? 16 : p.n <= 32 ? 32 : p.n <= 64 ? 64 : 128;
+  const int cuts = split_cuts(tile, (long long)((p.o + 127) / 128) * ((p.n + tile - 1) / tile) * batch, p.k);
+  switch (tile) {
+    case 16: return launch_split<16>(p, batch, cuts, batched, stream);
+    case 32: return launch_split<32>(p, batch, cuts, batched, stream);
+    case 64: return launch_split<64>(p, batch, cuts, batched, stream);
+    default: return launch_split<128>(p, batch, cuts, batched, stream);
+  }
+}
+
+// Which kernel: those below give the same bits.
 template <typename TX, typename TW>
-int launch_typed(const Product& p, int batch, cudaStream_t stream) {
+int launch_typed(const Product& p, int batch, bool batched, cudaStream_t stream) {
   if (batch > 65535) return FE_ERR_TOO_LARGE;
   auto whole = [](const void* base, long long ld, long long step, long long k, size_t item) {
     return ((uintptr_t)base & 15) == 0 && (ld * item) % 16 == 0 && (step * item) % 16 == 0 && (k * item) % 16 == 0;
   };
   const bool vec = whole(p.x, p.ldx, batch > 1 ? p.batch_x : 0, p.k, sizeof(TX)) &&
                    whole(p.w, p.k, batch > 1 ? p.batch_w : 0, p.k, sizeof(TW));
+  if constexpr (sizeof(TX) == 4 && sizeof(TW) == 4) {
+    // Deep rows of 32-bit numbers go to the tensor cores, however many there are, so that a row's bits do not depend on that.  us,
+    // the kernels below against those: 4 x 4,096 x 1,024 14 / 18, 4 x 1,024 x 3,072 18 / 20, 4 x 32,000 x 1,024 45 / 55 (in a decode step
+    // of 4 layers, where a product's weights are asked for ahead, 343 / 325 altogether), 16 x 32,000 x 1,024 72 / 57, 64 x 4,096 x 1,024
+    // 43 / 22, 500 x 4,096 x 1,024 119 / 45, 500 x 1,024 x 3,072 111 / 39, 1,024 x 32,000 x 1,024 1,437 / 560.  Shallower than 256
+    // a tile's fixed part is more than the sum (500 x 300 x 256 13 / 16).
+    if (vec && p.k >= GST_MIN_K && p.k < (1 << 22) && p.ldx < (1 << 22)) return split_product(p, batch, batched, stream);
+  }
   const long long big = (long long)((p.o + 63) / 64) * ((p.n + 63) / 64) * batch;
   if (!vec) {
     // Rows that do not start on 16 bytes, 32-bit operands, us (one number a copy, 64 x 64 or 32 x 32 tiles by this
@@ -410,13 +466,13 @@ int launch_typed(const Product& p, int batch, cudaStream_t stream) {
   return launch_tile<TX, TW, 4, 4, 8, 8, true>(p, batch, stream);
 }
 
-int launch_coded(int x_dtype, int w_dtype, const Product& p, int batch, cudaStream_t stream) {
+int launch_coded(int x_dtype, int w_dtype, const Product& p, int batch, bool batched, cudaStream_t stream) {
   if ((p.y_dtype | x_dtype | w_dtype) & ~1) return FE_ERR_BAD_DTYPE;
   switch (x_dtype * 2 + w_dtype) {
-    case 0: return launch_typed<float, float>(p, batch, stream);
-    case 1: return launch_typed<float, bf16>(p, batch, stream);
-    case 2: return launch_typed<bf16, float>(p, batch, stream);
-    default: return launch_typed<bf16, bf16>(p, batch, stream);
+    case 0: return launch_typed<float, float>(p, batch, batched, stream);
+    case 1: return launch_typed<float, bf16>(p, batch, batched, stream);
+    case 2: return launch_typed<bf16, float>(p, batch, batched, stream);
+    default: return launch_typed<bf16, bf16>(p, batch, batched, stream);
   }
 }
 
@@ -434,7 +490,7 @@ FE_EXPORT int fe_gemm_simt(const void* x, int x_dtype, const void* w, int w_dtyp
                            int* status, cudaStream_t stream) {
   if (n <= 0 || o <= 0) return 0;
   if (k <= 0) return FE_ERR_BAD_SHAPE;
-  return launch_coded(x_dtype, w_dtype, Product{x, w, bias, y, y_dtype, n, o, k, accumulate, status, k, o, 0, 0, 0}, 1, stream);
+  return launch_coded(x_dtype, w_dtype, Product{x, w, bias, y, y_dtype, n, o, k, accumulate, status, k, o, 0, 0, 0}, 1, false, stream);
 }
 
 // `batch` products at once (one per head): product b reads x + b * batch_x (rows ldx apart),
@@ -446,5 +502,5 @@ FE_EXPORT int fe_gemm_simt_batched(const void* x, int x_dtype, const void* w, in
   if (n <= 0 || o <= 0 || batch <= 0) return 0;
   if (k <= 0 || ldx < k || ldy < o) return FE_ERR_BAD_SHAPE;
   return launch_coded(x_dtype, w_dtype, Product{x, w, nullptr, y, y_dtype, n, o, k, 0, status, ldx, ldy, batch_x, batch_w, batch_y},
-                      batch, stream);
+                      batch, true, stream);
 }
