@@ -516,3 +516,63 @@ def test_expanded_latent_attention(native, monkeypatch, window, sink, heads, dim
             off = float((got[at : at + count].double().cpu() - want).norm() / want.norm())
             assert off < 1e-2, (name, start, count, off)
         at += count
+
+
+# -- deep 32-bit products on the tensor cores --------------------------------------------------------
+@pytest.mark.parametrize("o, k", ((1, 256), (127, 260), (129, 320), (300, 1028), (4224, 448), (2500, 3072)))
+def test_deep_product_of_any_number_of_rows(native, o, k):
+    """Row counts at the edges of the four tiles, depths with and without a rest of a stretch of 64 and with fewer stretches
+    than parts: a row's bits do not depend on the others (nor on how k is cut over blocks, which changes with them).  Bound: a
+    stretch's sum is off by its 24 additions in the tensor core (2^-23 of the sum of magnitudes each), the sums outside by
+    2^-24 each; along a random result far less, and less than one chain of multiply-adds (2.9e-7 at 256)."""
+    gen = torch.Generator().manual_seed(o + k)
+    w, rows = (torch.randn(shape, generator=gen).to(DEV) for shape in ((o, k), (300, k)))
+    bias = torch.randn(o, generator=gen).to(DEV)
+    want = rows.double() @ w.double().t()
+    bound = (rows.double().abs() @ w.double().abs().t()) * (24 * 2.0**-23 + (k // 64 + 10) * 2.0**-24) + 2.0**-22 * bias.double().abs()
+    whole = torch.empty((300, o), device=DEV)
+    native.gemm_simt(rows, w, whole)
+    assert float((whole.double() - want).norm() / want.norm()) < 2.5e-7
+    for n in (1, 16, 17, 32, 33, 64, 65, 128, 129):
+        got = torch.empty((n, o), device=DEV)
+        native.gemm_simt(rows[:n].contiguous(), w, got)
+        assert torch.equal(got, whole[:n]), n
+        added = torch.ones((n, o), device=DEV)
+        native.gemm_simt(rows[:n].contiguous(), w, added, bias, accumulate=True)
+        assert bool(((added.double() - 1.0 - bias.double() - want[:n]).abs() <= bound[:n] + 2.0**-22).all()), n
+
+
+def test_deep_batched_product_with_strided_rows(native):
+    gen = torch.Generator().manual_seed(3)
+    batch, o, k = 3, 140, 272
+    w = torch.randn((batch, o, k), generator=gen).to(DEV)
+    for n in (1, 20, 150):
+        x = torch.randn((n, batch, k + 8), generator=gen).to(DEV)[:, :, :k]
+        out = torch.full((n, batch, o + 3), 7.0, device=DEV)
+        native.gemm_simt_batched(x, w, out[:, :, :o])
+        want = torch.einsum("nbk,bok->nbo", x.double(), w.double())
+        assert float((out[:, :, :o].double() - want).norm() / want.norm()) < 2.5e-7
+        assert float((out[:, :, o:] - 7.0).abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("n", (3, 40, 200))
+def test_deep_product_of_values_that_are_not_finite(native, n):
+    """Infinities, NaN and numbers that round to infinity in 16 bits give what one chain of multiply-adds gives, and
+    reach no other row or column."""
+    gen = torch.Generator().manual_seed(n)
+    k, o = 512, 150
+    x, w = torch.randn((n, k), generator=gen), torch.randn((o, k), generator=gen)
+    clean = torch.empty((n, o), device=DEV)
+    native.gemm_simt(x.to(DEV), w.to(DEV), clean)
+    x[0, 5], x[1, 9], x[2, 1], w[7, 3], w[9, 2] = float("inf"), float("nan"), 3.4e38, float("-inf"), -3.4e38
+    got = torch.empty((n, o), device=DEV)
+    native.gemm_simt(x.to(DEV), w.to(DEV), got)
+    want = x.double() @ w.double().t()                       # 64 bits hold what overflows 32
+    got, clean = got.cpu(), clean.cpu()
+    keep = [c for c in range(o) if c not in (7, 9)]
+    assert torch.equal(got[3:, keep], clean[3:, keep])
+    assert bool(got[1].isnan().all()) and bool((got[0, keep] == want[0, keep]).all())
+    big = want[2, keep].abs() > 3.5e38
+    assert bool(torch.isinf(got[2, keep][big]).all()) and bool((got[3:, 7] == want[3:, 7]).all())
+    sound = want[2, keep].abs() < 3.3e38
+    assert float((got[2, keep][sound].double() / want[2, keep][sound] - 1).abs().max()) < 1e-5
