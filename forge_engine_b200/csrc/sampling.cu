@@ -15,6 +15,10 @@
 // it fits, so that only the first pass reads the logits; the digit that a pass decides on is found
 // by a warp.  (16 rows of 151,936, top-k 50 and top-p 0.95: 199 us with the slice read from L2 in
 // every pass and a single thread walking the 256 digits.)
+// With a top-k of up to 512 the passes are not taken: a bound from the threads' maxima leaves a few hundred elements, and
+// one block decides among them without a barrier of the cluster (the same 16 rows 93 us by passes, 34 this way; top-k 200 94 and
+// 38, 512 95 and 47; 64 rows 179 and 63; 16 rows of 32,000 43 and 26).  More than 1,024 elements above the bound (ties, or
+// the largest all in one block's slice) go through the passes.
 // The draw: u = uniform(seed, counter) from a counter hash (see fe_uniform below and
 // its Python twin), target = u * sum(weights of survivors), first index whose running
 // sum in index order exceeds target.
@@ -181,11 +185,149 @@ __device__ __forceinline__ int digit_of_mass(const unsigned int* n, const unsign
   return any ? __shfl_sync(0xffffffffu, largest, __ffs(any) - 1) : 0;
 }
 
+// What a row is sampled with.
+struct SampleRow {
+  float temperature, top_p, min_p;
+  int top_k;
+  unsigned long long seed, counter;
+};
+// Up to SMP_ROWS_BY_VALUE rows travel as an argument of the kernel (no copy to the device goes ahead of it), more as arrays there.
+#define SMP_ROWS_BY_VALUE 64
+struct SampleParams {
+  const float* temperature;     // null: 0
+  const int* top_k;
+  const float* top_p;
+  const float* min_p;
+  const unsigned long long* seeds;
+  const unsigned long long* counters;
+  int by_value;
+  SampleRow rows[SMP_ROWS_BY_VALUE];
+  __device__ __forceinline__ SampleRow of(int row) const {
+    if (by_value) return rows[row];
+    return SampleRow{temperature ? temperature[row] : 0.f, top_p ? top_p[row] : 1.f, min_p ? min_p[row] : 0.f, top_k ? top_k[row] : 0,
+                     seeds ? seeds[row] : 0ull, counters ? counters[row] : 0ull};
+  }
+};
+
+#define FEW_MOST 512                 // a top-k up to which the largest keys are collected
+
+// Top-k, top-p, min-p and the draw among `n` <= 1,024 elements that hold the row's k largest, in index order (s: shifted
+// logits, index: their places): the element drawn, or -1.  Thread t holds element t; `room`: 16 KB.  One block; the sums
+// are added up as by a cluster of `parts` blocks whose threads walk stretches of the row.
+__device__ int choose_of_few(const float* s_in, const int* index_in, int n, int k, float p, float mp, float u, int vocab, int parts,
+                             unsigned char* room, unsigned long long* scan_u, float* scan_f, int* scan_i, int* red_i) {
+  unsigned long long* mass = reinterpret_cast<unsigned long long*>(room);        // [512] of the k survivors
+  float* s_of = reinterpret_cast<float*>(mass + FEW_MOST);                        // [512]
+  float* w_of = s_of + FEW_MOST;
+  int* index_of = reinterpret_cast<int*>(w_of + FEW_MOST);
+  int* lives = index_of + FEW_MOST;
+  float* walked = reinterpret_cast<float*>(lives + FEW_MOST);                     // [1024] sums of a block's threads
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  // top-k: the k-th largest key, bit by bit; of the keys equal to it the first in index order
+  {
+    const bool have = tid < n;
+    const float s = have ? s_in[tid] : 0.f;
+    const unsigned int key = have ? float_key(s) : 0u;
+    unsigned int threshold = 0u;
+#pragma unroll 1
+    for (int bit = 31; bit >= 0; --bit) {
+      const unsigned int trial = threshold | (1u << bit);
+      if (__syncthreads_count(have && key >= trial) >= k) threshold = trial;
+    }
+    const int ties = k - __syncthreads_count(have && key > threshold);
+    int total;
+    const int before = block_exclusive_scan<int>(have && key == threshold ? 1 : 0, scan_i, &total);
+    const bool keep = have && (key > threshold || (key == threshold && before < ties));
+    const int at = block_exclusive_scan<int>(keep ? 1 : 0, scan_i, &total);
+    if (keep) { s_of[at] = s; index_of[at] = index_in[tid]; }
+    n = total;
+    __syncthreads();
+  }
+  const bool have = tid < n;
+  const float s = have ? s_of[tid] : 0.f, w = have ? expf(s) : 0.f;
+  const int index = have ? index_of[tid] : 0;
+  const unsigned int key = float_key(s);
+  bool live = have;
+  // top-p: the smallest key whose mass of strictly larger survivors is at most p of all
+  if (p < 1.f) {
+    const unsigned long long own = have ? (unsigned long long)(w * MASS_SCALE) : 0ull;
+    if (have) mass[tid] = own;
+    unsigned long long total;
+    block_exclusive_scan<unsigned long long>(own, scan_u, &total);
+    const unsigned long long limit = (unsigned long long)((double)p * (double)total);
+    unsigned long long above = 0ull;
+    if (have)
+      for (int j = 0; j < n; ++j)
+        if (float_key(s_of[j]) > key) above += mass[j];
+    unsigned int boundary = have && above <= limit ? key : 0xffffffffu;
+    boundary = __reduce_min_sync(0xffffffffu, boundary);
+    __syncthreads();
+    if (lane == 0) red_i[warp] = (int)boundary;
+    __syncthreads();
+    boundary = __reduce_min_sync(0xffffffffu, (unsigned int)red_i[lane]);
+    live = live && key >= boundary;
+  }
+  if (mp > 0.f) live = live && !(w < mp);
+  if (have) { w_of[tid] = w; lives[tid] = live ? 1 : 0; }
+  // the draw in index order: the first element of every (block, thread) stretch adds up the stretch
+  const int chunk = (vocab + parts - 1) / parts;
+  auto owner_of = [&](int i) {
+    const int block = i / chunk, first = block * chunk, last = min(vocab, first + chunk);
+    return block * SMP_THREADS + (i - first) / ((last - first + SMP_THREADS - 1) / SMP_THREADS);
+  };
+  const int owner = have ? owner_of(index) : -1;
+  __syncthreads();
+  const bool leads = have && (tid == 0 || owner_of(index_of[tid - 1]) != owner);
+  float sum = 0.f;
+  int end = tid, last = -1;
+  if (leads) {
+    do {
+      if (lives[end]) { sum += w_of[end]; last = end; }
+      ++end;
+    } while (end < n && owner_of(index_of[end]) == owner);
+  }
+  float total = 0.f, before = 0.f;
+  for (int r = 0; r < parts; ++r) {
+    const bool here = leads && owner / SMP_THREADS == r;
+    walked[tid] = 0.f;
+    __syncthreads();
+    if (here) walked[owner % SMP_THREADS] = sum;
+    __syncthreads();
+    const float mine = walked[tid];
+    float block_total;
+    const float upto = block_exclusive_scan<float>(mine, scan_f, &block_total);
+    walked[tid] = upto + total;
+    __syncthreads();
+    if (here) before = walked[owner % SMP_THREADS];
+    total += block_total;
+    __syncthreads();
+  }
+  const float target = u * total;
+  int best = last >= 0 && before <= target ? owner : -1;
+  best = __reduce_max_sync(0xffffffffu, best);
+  if (lane == 0) red_i[warp] = best;
+  __syncthreads();
+  best = __reduce_max_sync(0xffffffffu, red_i[lane]);
+  __syncthreads();
+  if (tid == 0) red_i[0] = -1;
+  __syncthreads();
+  if (leads && owner == best) {
+    float c = before;
+    int pick = last;
+    for (int j = tid; j < end; ++j) {
+      if (!lives[j]) continue;
+      c += w_of[j];
+      if (target < c) { pick = j; break; }
+    }
+    red_i[0] = index_of[pick];
+  }
+  __syncthreads();
+  return red_i[0];
+}
+
 __global__ void __launch_bounds__(SMP_THREADS)
-sample_kernel(const float* __restrict__ logits, int vocab, const float* __restrict__ temperature,
-              const int* __restrict__ top_k, const float* __restrict__ top_p,
-              const float* __restrict__ min_p, const unsigned long long* __restrict__ seeds,
-              const unsigned long long* __restrict__ counters, int* __restrict__ out, int* status, int keep_slice) {
+sample_kernel(const float* __restrict__ logits, int vocab, const __grid_constant__ SampleParams params,
+              int* __restrict__ out, int* status, int keep_slice) {
   extern __shared__ float slice[];                   // with keep_slice: this block's shifted logits
   __shared__ float red_v[32];
   __shared__ int red_i[32];
@@ -223,6 +365,7 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
     if (v != v || v == INFINITY) bad = true;
     if (v > best) { best = v; best_i = i; }
   }
+  const float own_max = best;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     const float ov = __shfl_xor_sync(0xffffffffu, best, o);
@@ -253,13 +396,75 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
   }
   turn ^= 1;
   if (arg == 0x7fffffff) arg = 0;
-  const float temp = temperature ? temperature[row] : 0.f;
+  const SampleRow wish = params.of(row);
+  const float temp = wish.temperature;
   if (temp <= 0.f || row_max == -INFINITY) {
     if (tid == 0 && part == 0) out[row] = arg;
     cluster_sync();        // nobody leaves while another block may still read its shared memory
     return;
   }
-  const float inv_t = 1.f / temp;
+  const float inv_t = 1.f / temp, p = wish.top_p, mp = wish.min_p, u = fe_uniform(wish.seed, wish.counter);
+  const int k = wish.top_k;
+
+  // ---- few wanted: the largest keys alone ----
+  // Two lower bounds of the row's k-th largest key (their upper 20 bits): the best block's k-th largest of its threads'
+  // maxima, and the worst block's (k / blocks)-th largest.  What reaches the larger of the two is collected in
+  // index order in the first block, which decides among it: the same survivors, and the same sums in the same
+  // order, as the passes over the whole row below.
+  if (keep_slice && k > 0 && k <= FEW_MOST && k < vocab) {
+    const unsigned int top_key = float_key((own_max - row_max) * inv_t);
+    const int fair = (k + parts - 1) / parts;
+    unsigned int bound = 0u, fair_bound = 0u;
+#pragma unroll 1
+    for (int bit = 31; bit >= 12; --bit) {
+      const unsigned int trial = bound | (1u << bit), fair_trial = fair_bound | (1u << bit);
+      if (__syncthreads_count(top_key >= trial) >= k) bound = trial;
+      if (__syncthreads_count(top_key >= fair_trial) >= fair) fair_bound = fair_trial;
+    }
+    if (tid == 0) { share[turn][0] = bound; share[turn][1] = fair_bound; }
+    cluster_sync();
+    for (int r = 0; r < parts; ++r) {
+      bound = max(bound, (unsigned int)peer_u64(&share[turn][0], r));
+      fair_bound = min(fair_bound, (unsigned int)peer_u64(&share[turn][1], r));
+    }
+    bound = max(bound, fair_bound);
+    turn ^= 1;
+    const int seg = (hi - lo + SMP_THREADS - 1) / SMP_THREADS;
+    const int begin = min(hi, lo + tid * seg), end = min(hi, begin + seg);
+    int mine = 0, total;
+    for (int i = begin; i < end; ++i) mine += float_key((slice[slice_at(i - lo)] - row_max) * inv_t) >= bound;
+    int at = block_exclusive_scan<int>(mine, scan_i, &total);
+    if (tid == 0) share[turn][0] = (unsigned long long)(unsigned int)total;
+    cluster_sync();
+    int all = 0;
+    for (int r = 0; r < parts; ++r) {
+      const int theirs = (int)(unsigned int)peer_u64(&share[turn][0], r);
+      if (r < part) at += theirs;
+      all += theirs;
+    }
+    turn ^= 1;
+    if (all <= SMP_THREADS) {
+      float* few_s = reinterpret_cast<float*>(group_n);        // [1024] shifted logits, [1024] indices
+      int* few_i = reinterpret_cast<int*>(group_n) + SMP_THREADS;
+      if (mine > 0) {
+        const unsigned int to_s = peer_address(few_s, 0), to_i = peer_address(few_i, 0);
+        for (int i = begin; i < end; ++i) {
+          const float s = (slice[slice_at(i - lo)] - row_max) * inv_t;
+          if (float_key(s) < bound) continue;
+          asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(to_s + 4u * (unsigned)at), "f"(s) : "memory");
+          asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(to_i + 4u * (unsigned)at), "r"(i) : "memory");
+          ++at;
+        }
+      }
+      cluster_sync();
+      if (part == 0) {
+        const int pick = choose_of_few(few_s, few_i, all, k, p, mp, u, vocab, parts, reinterpret_cast<unsigned char*>(group_m), scan_u, scan_f,
+                                       scan_i, red_i);
+        if (tid == 0) out[row] = pick < 0 ? arg : pick;
+      }
+      return;
+    }
+  }
   Survive keep{0u, 0x7fffffff, 0.f};
   if (keep_slice) {
     for (int i = lo + tid; i < hi; i += SMP_THREADS) slice[slice_at(i - lo)] = (slice[slice_at(i - lo)] - row_max) * inv_t;
@@ -295,7 +500,6 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
   } while (0)
 
   // ---- top-k: radix search for the k-th largest key ----
-  const int k = top_k ? top_k[row] : 0;
   if (k > 0 && k < vocab) {
     if (tid == 0) { sh_prefix = 0u; sh_remaining = k; }
     for (int shift = 24; shift >= 0; shift -= 8) {
@@ -366,7 +570,6 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
   }
 
   // ---- top-p: smallest key whose mass of strictly larger survivors is <= top_p * Z ----
-  const float p = top_p ? top_p[row] : 1.f;
   if (p < 1.f) {
     if (tid == 0) { sh_prefix = 0u; sh_mass_above = 0ull; }
     unsigned long long limit = 0ull;
@@ -443,7 +646,6 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
   }
 
   // ---- min-p: drop p_i < min_p * p_max  <=>  exp(x_i) < min_p (the largest has exp 1) ----
-  const float mp = min_p ? min_p[row] : 0.f;
   if (mp > 0.f) keep.min_w = mp;
 
   // ---- draw in index order ----
@@ -468,7 +670,6 @@ sample_kernel(const float* __restrict__ logits, int vocab, const float* __restri
   }
   turn ^= 1;
   before += earlier;
-  const float u = fe_uniform(seeds ? seeds[row] : 0ull, counters ? counters[row] : 0ull);
   const float target = u * total;
   // the last thread (in index order over the whole row) that has survivors and starts at or below target
   int cand = (last_survivor >= 0 && before <= target) ? part * SMP_THREADS + tid : -1;
@@ -560,17 +761,15 @@ static int sample_parts(int rows, int vocab) {
 // What the rule above decides, for its test.
 FE_EXPORT int fe_sample_parts(int rows, int vocab) { return sample_parts(rows, vocab); }
 
-FE_EXPORT int fe_sample(const float* logits, int rows, int vocab, const float* temperature,
-                        const int* top_k, const float* top_p, const float* min_p,
-                        const unsigned long long* seeds, const unsigned long long* counters,
-                        int* out, int* status, cudaStream_t stream) {
+static int launch_sample(const float* logits, int rows, int vocab, const SampleParams& params, bool drawn, int* out, int* status,
+                         cudaStream_t stream) {
   if (rows <= 0) return 0;
   if (vocab <= 0) return FE_ERR_BAD_SHAPE;
   if (rows > 65535) return FE_ERR_TOO_LARGE;
   // A row's vocabulary over up to 8 blocks (one cluster) of at least 4,096 logits each.
   int parts = 1;
   size_t smem = 0;
-  if (temperature == nullptr) {
+  if (!drawn) {
     while (parts < 8 && rows * parts * 2 <= 296 && vocab >= parts * 2 * 4096) parts *= 2;
   } else {
     parts = sample_parts(rows, vocab);
@@ -592,10 +791,25 @@ FE_EXPORT int fe_sample(const float* logits, int rows, int vocab, const float* t
   attribute[0].val.clusterDim.z = 1;
   config.attrs = attribute;
   config.numAttrs = parts > 1 ? 1 : 0;
-  const cudaError_t e = cudaLaunchKernelEx(&config, sample_kernel, logits, vocab, temperature, top_k, top_p, min_p,
-                                           seeds, counters, out, status, smem > 0 ? 1 : 0);
+  const cudaError_t e = cudaLaunchKernelEx(&config, sample_kernel, logits, vocab, params, out, status, smem > 0 ? 1 : 0);
   if (e != cudaSuccess) return (int)e;
   return fe_last_error();
+}
+
+FE_EXPORT int fe_sample(const float* logits, int rows, int vocab, const float* temperature,
+                        const int* top_k, const float* top_p, const float* min_p,
+                        const unsigned long long* seeds, const unsigned long long* counters,
+                        int* out, int* status, cudaStream_t stream) {
+  SampleParams params{temperature, top_k, top_p, min_p, seeds, counters, 0, {}};
+  return launch_sample(logits, rows, vocab, params, temperature != nullptr, out, status, stream);
+}
+
+// The same with the rows' parameters in host memory, SampleRow after SampleRow; at most SMP_ROWS_BY_VALUE of them.
+FE_EXPORT int fe_sample_rows(const float* logits, int rows, int vocab, const SampleRow* wishes, int* out, int* status, cudaStream_t stream) {
+  if (rows > SMP_ROWS_BY_VALUE) return FE_ERR_TOO_LARGE;
+  SampleParams params{nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 1, {}};
+  for (int r = 0; r < rows; ++r) params.rows[r] = wishes[r];
+  return launch_sample(logits, rows, vocab, params, true, out, status, stream);
 }
 
 // Host copy of the uniform, for the Python twin's self-check.

@@ -93,6 +93,7 @@ def _declare(handle: ctypes.CDLL) -> None:
         "fe_attention_simt_units": [i, i, i, i, i, i],
         "fe_gemm_simt": [p, i, p, i, p, p, i, i, i, i, i, p, p],
         "fe_sample": [p, i, i, p, p, p, p, p, p, p, p, p],
+        "fe_sample_rows": [p, i, i, ctypes.c_char_p, p, p, p],
         "fe_gemm_tc5": [p, p, p, p, i, i, i, i, i, p, p, p, f, f, p],
         "fe_gemm_tc5_grouped": [p, p, p, i, i, i, i, i, i, i, p, p, p, f, f, p, p],
         "fe_moe_gather": [p, i, i, i, i, p, p, p, p],
@@ -1857,3 +1858,15 @@ def sample(
                         ptr(seeds), ptr(counters), ptr(out), ptr(status), stream()),
         "sample",
     )
+
+
+SAMPLE_ROWS_BY_VALUE = 64      # rows whose parameters travel as an argument of the sampling kernel
+
+
+def sample_rows(logits: torch.Tensor, out: torch.Tensor, status: torch.Tensor, wishes: bytes) -> None:
+    """``sample`` with the parameters of every row packed on the host: temperature, top_p, min_p (32-bit floats), top_k
+    (32-bit, 0: none), seed, counter (64-bit) of one row after another, for at most ``SAMPLE_ROWS_BY_VALUE`` rows."""
+    _dense(logits, "logits")
+    rows, vocab = logits.shape
+    assert logits.dtype == torch.float32 and out.dtype == torch.int32 and out.numel() >= rows and len(wishes) == 32 * rows
+    check(lib().fe_sample_rows(ptr(logits), rows, vocab, wishes, ptr(out), ptr(status), stream()), "sample_rows")

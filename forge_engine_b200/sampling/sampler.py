@@ -7,12 +7,16 @@ Here all rows of a step are sampled by one kernel launch and read back by one co
 
 from __future__ import annotations
 
+import struct
 from typing import Sequence
 
 import torch
 
 from ..ops import native
 from .params import SamplingParams
+
+
+_MASK64 = (1 << 64) - 1
 
 
 def _to_signed64(value: int) -> int:
@@ -43,6 +47,13 @@ class Sampler:
         out = torch.empty(rows, dtype=torch.int32, device=self.device)
         if all(p.greedy for p in params):
             native.sample(logits, out, self.status)
+            return out
+        if rows <= native.SAMPLE_ROWS_BY_VALUE and all((p.top_k or 0) < 1 << 31 for p in params):
+            # the parameters go with the launch: three pinned copies ahead of it took 60 us of host time
+            fields = []
+            for p, seed, counter in zip(params, seeds, counters):
+                fields += (p.temperature, p.top_p, p.min_p, p.top_k or 0, seed & _MASK64, counter & _MASK64)
+            native.sample_rows(logits, out, self.status, struct.pack("=" + "3fi2Q" * rows, *fields))
             return out
         floats = torch.tensor(
             [[p.temperature for p in params], [p.top_p for p in params], [p.min_p for p in params]],

@@ -3,6 +3,8 @@ against 64-bit arithmetic on the same inputs."""
 
 from __future__ import annotations
 
+import struct
+
 import pytest
 import torch
 
@@ -576,3 +578,52 @@ def test_deep_product_of_values_that_are_not_finite(native, n):
     assert bool(torch.isinf(got[2, keep][big]).all()) and bool((got[3:, 7] == want[3:, 7]).all())
     sound = want[2, keep].abs() < 3.3e38
     assert float((got[2, keep][sound].double() / want[2, keep][sound] - 1).abs().max()) < 1e-5
+
+
+# -- the largest logits alone ------------------------------------------------------------------------
+def drawn_among(row, temperature, top_k, top_p, min_p, u):
+    """(index, distance of the target from the nearest boundary of the running sum, over the sum) in 64 bits: of equal
+    logits the first ones are kept by top-k and all of them by top-p."""
+    x = ((row - row.max()) * (1.0 / torch.tensor(temperature))).double()
+    order = torch.argsort(-x, stable=True)
+    keep = torch.zeros(len(x), dtype=torch.bool)
+    keep[order[:top_k]] = True
+    weights = torch.where(keep, torch.exp(x), 0.0)
+    if top_p < 1.0:
+        values, inverse = torch.unique(x, return_inverse=True)
+        mass = torch.zeros(len(values), dtype=torch.float64).index_add_(0, inverse, weights)
+        above = mass.flip(0).cumsum(0).flip(0) - mass
+        weights = torch.where(above[inverse] <= top_p * weights.sum(), weights, 0.0)
+    weights = torch.where(torch.exp(x) < min_p, 0.0, weights)
+    running = weights.cumsum(0)
+    target = u * running[-1]
+    index = min(int(torch.searchsorted(running, target, right=True)), int(weights.nonzero()[-1]))
+    return index, float((running - target).abs().min() / running[-1])
+
+
+@pytest.mark.parametrize("vocab", (300, 4097, 70001))
+@pytest.mark.parametrize("shape", ("normal", "ties", "sorted", "masked"))
+def test_sampling_among_the_largest(native, vocab, shape):
+    """Top-k at the ends of what is decided among the collected elements (512) and past it, with more elements above the
+    bound than there is room for (equal logits) and the largest all in one block's slice: the draw of 64-bit arithmetic.
+    Only a target within rounding (1e-5 of the sum) of a boundary of the running sum may differ."""
+    gen = torch.Generator().manual_seed(vocab)
+    logits = torch.randn((12, vocab), generator=gen) * 2.0
+    if shape == "ties":
+        logits = logits.round()
+    if shape == "sorted":
+        logits = logits.sort(dim=1, descending=True).values.contiguous()
+    if shape == "masked":
+        logits[torch.rand(logits.shape, generator=gen) < 0.99] = float("-inf")
+        logits[:, 0] = 1.0
+    top_k = [1, 2, 50, 200, 511, 512, 513, 20, 20, 50, 50, 1024]
+    top_p = [1.0, 1.0, 0.95, 0.9, 1.0, 0.99, 0.9, 1.0, 0.5, 1e-6, 1.0, 0.9]
+    min_p = [0.0] * 7 + [0.05, 0.0, 0.0, 0.3, 0.0]
+    asked = [(0.8, min(k, vocab), p, m) for k, p, m in zip(top_k, top_p, min_p)]
+    wishes = b"".join(struct.pack("=3fi2Q", t, p, m, k, 11 + r, 2**40 + r) for r, (t, k, p, m) in enumerate(asked))
+    out, status = torch.empty(12, dtype=torch.int32, device=DEV), status_word()
+    native.sample_rows(logits.to(DEV), out, status, wishes)
+    assert int(status.item()) == 0
+    for r, got in enumerate(out.tolist()):
+        want, gap = drawn_among(logits[r], *asked[r], twin_uniform(11 + r, 2**40 + r))
+        assert got == want or gap < 1e-5, (r, got, want, gap)
