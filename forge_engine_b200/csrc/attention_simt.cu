@@ -14,13 +14,15 @@
 //   order.  Bound by the bytes of keys and values; the spans are what keeps the chip busy at few
 //   requests.
 // attention_simt_tile: entries of several tokens.  A block takes 32 rows (token, query head) of one
-//   kv head over all their keys in tiles of 64, as two small FFMA products from shared memory.
+//   kv head over all their keys in tiles of 64, as two small FFMA products from shared memory; where that leaves
+//   the chip idle, over one span of them, and attention_simt_fold folds a row's spans.  Bound by instructions (two
+//   blocks of 8 warps an SM issue in 53 % of the cycles; with 4 warps of twice the rows 30 %).
 //
 // A row's bits depend on nothing but its token and the keys it sees: not on what else is in the batch, nor on
 // how its portion was cut.  Both kernels take a span's keys, counted from position 0, in thirty-twos with one
 // running maximum, sum over positions (or elements of a head: even and odd ones apart) in ascending order,
-// and fold the spans one after the other (fold_factors).  In the tile kernel that takes a second set of sums: 500
-// tokens of 16 heads of 128 146 us, 137 without; single tokens 18.6 against 19.3 (4 after 700 cached ones).
+// and fold the spans one after the other (fold_factors).  500 tokens of 16 heads of 128 take 108 us in a layer (150 by 4 warps
+// a block, all spans of a row by one block and the value product without pairs of columns).
 #include "attention_common.cuh"
 
 namespace {
@@ -29,7 +31,8 @@ constexpr int SPAN = 128;          // key positions of a block of the span kerne
 constexpr int SPAN_KEYS = 32;      // of one stage of its ring
 constexpr int SPAN_STAGES = 3;
 constexpr int SPAN_THREADS = 128;
-constexpr int TILE_ROWS = 32, TILE_KEYS = 64, TILE_THREADS = 128;
+constexpr int TILE_ROWS = 32, TILE_KEYS = 64, TILE_THREADS = 256;
+constexpr int RT = TILE_ROWS / (TILE_THREADS / 16);      // rows of a thread
 constexpr int P_PITCH = TILE_KEYS + 4;
 
 struct Simt {
@@ -45,6 +48,7 @@ struct Simt {
   int num_q_heads, groups, spans, row_tiles;
   int unit0;                // of this launch: the units go through the workspace in slices
   float* partial;           // [unit of the slice][kv head][row tile][span][row][D + 2]
+  int n_tokens;
   int* status;
 };
 
@@ -59,6 +63,17 @@ __device__ __forceinline__ void wait() { asm volatile("cp.async.wait_group %0;" 
 __device__ __forceinline__ void fma2(uint64_t& acc, uint64_t a, uint64_t b) {
   asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
 }
+__device__ __forceinline__ uint64_t twice(float x) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ uint64_t scale2(uint64_t x, float by) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(x), "l"(twice(by)));
+  return r;
+}
+__device__ __forceinline__ float half2_of(uint64_t x, int which) { return __uint_as_float((unsigned)(which ? x >> 32 : x)); }
 __device__ __forceinline__ float sum2(uint64_t acc) {
   return __uint_as_float((unsigned)acc) + __uint_as_float((unsigned)(acc >> 32));
 }
@@ -73,12 +88,12 @@ __device__ __forceinline__ void pairs4(const bf16* p, uint64_t (&out)[2]) {
   out[1] = (uint64_t)(raw.y << 16) | ((uint64_t)(raw.y & 0xffff0000u) << 32);
 }
 
-// Sums (or maxima) of eight numbers over 16 neighbouring lanes, for all of them, in the order of warp_sum's last
+// Sums (or maxima) of four numbers over 16 neighbouring lanes, for all of them, in the order of warp_sum's last
 // four steps: half of the numbers go to the partner at a time, and come back whole.
 template <bool MAX>
-__device__ __forceinline__ void reduce8(float (&x)[8], int lane) {
+__device__ __forceinline__ void reduce4(float (&x)[4], int lane) {
 #pragma unroll
-  for (int half = 4, bit = 8; half > 0; half >>= 1, bit >>= 1) {
+  for (int half = 2, bit = 8; half > 0; half >>= 1, bit >>= 1) {
     const bool upper = (lane & bit) != 0;
 #pragma unroll
     for (int i = 0; i < half; ++i) {
@@ -87,9 +102,14 @@ __device__ __forceinline__ void reduce8(float (&x)[8], int lane) {
       x[i] = MAX ? fmaxf(keep, got) : keep + got;
     }
   }
-  const float got = __shfl_xor_sync(0xffffffffu, x[0], 1), mine = MAX ? fmaxf(x[0], got) : x[0] + got;
+  float mine = x[0];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) x[i] = __shfl_sync(0xffffffffu, mine, (lane & 16) | (i << 1));
+  for (int bit = 2; bit > 0; bit >>= 1) {
+    const float got = __shfl_xor_sync(0xffffffffu, mine, bit);
+    mine = MAX ? fmaxf(mine, got) : mine + got;
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) x[i] = __shfl_sync(0xffffffffu, mine, (lane & 16) | (i << 2));
 }
 
 // A span (maximum m) joins those before it (maximum top): their sums take `old`, its own `mine`.
@@ -292,19 +312,48 @@ __global__ void __launch_bounds__(128) attention_simt_merge_kernel(const Simt p,
   }
 }
 
-template <typename T, int DMAX>
+// Which entry of several tokens row tile `index` of the launch belongs to, and which of its tiles it is: a warp counts 32
+// entries at a time.  False past the last tile.
+__device__ __forceinline__ bool find_tile(const Simt& p, int index, int& entry, int& tile, int& tiles) {
+  const int lane = threadIdx.x & 31;
+  for (int base = 0, seen = 0; base < p.units; base += 32) {
+    const int e = base + lane;
+    const int count = e < p.units ? p.cu_tokens[e + 1] - p.cu_tokens[e] : 0;
+    const int mine = count > 1 ? (count * p.groups + TILE_ROWS - 1) / TILE_ROWS : 0;
+    int upto = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += t;
+    }
+    const unsigned past = __ballot_sync(0xffffffffu, index < seen + upto);
+    if (past) {
+      const int owner = __ffs(past) - 1;
+      entry = base + owner;
+      tiles = __shfl_sync(0xffffffffu, mine, owner);
+      tile = index - seen - (__shfl_sync(0xffffffffu, upto, owner) - tiles);
+      return true;
+    }
+    seen += __shfl_sync(0xffffffffu, upto, 31);
+  }
+  return false;
+}
+
+// SPLIT: the block takes one span of the keys (blockIdx.y = span * kv heads + kv head) and leaves its maxima and sums to
+// attention_simt_fold_kernel.
+template <typename T, int DMAX, bool SPLIT>
 __global__ void __launch_bounds__(TILE_THREADS) attention_simt_tile_kernel(const Simt p) {
   constexpr int CH = 16 / (int)sizeof(T), CG = DMAX / 64;      // groups of four output columns of a thread
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ int ok[TILE_KEYS];
   pdl_trigger();
   pdl_wait();
-  const int D = p.cache.head_dim, entry = p.unit0 + (int)blockIdx.z, kvh = blockIdx.y;
+  const int D = p.cache.head_dim, kvh = blockIdx.y % p.cache.num_kv_heads, span = blockIdx.y / p.cache.num_kv_heads;
+  int entry = 0, tile = 0, tiles = 0;
+  if (!find_tile(p, blockIdx.x, entry, tile, tiles)) return;
   const int token0 = p.cu_tokens[entry], count = p.cu_tokens[entry + 1] - token0;
-  if (count <= 1) return;
-  const int total = count * p.groups, tiles = (total + TILE_ROWS - 1) / TILE_ROWS;
-  if ((int)blockIdx.x >= tiles) return;
-  const int row0 = (tiles - 1 - (int)blockIdx.x) * TILE_ROWS;    // the tiles with the most keys first
+  const int total = count * p.groups;
+  const int row0 = (tiles - 1 - tile) * TILE_ROWS;    // the tiles with the most keys first
   const int qpitch = D + 4;
   float* qs = (float*)smem;                                     // [row][D + 4]
   float* ps = qs + TILE_ROWS * qpitch;                          // [row][key]
@@ -316,65 +365,73 @@ __global__ void __launch_bounds__(TILE_THREADS) attention_simt_tile_kernel(const
     const int token = token0 + row / p.groups, head = kvh * p.groups + row % p.groups;
     qs[r * qpitch + d] = row < total ? to_float(((const T*)p.q)[(size_t)token * p.q_stride + (size_t)head * D + d]) : 0.f;
   }
-  int from[4], upto[4];              // the positions this thread's rows see
+  int from[RT], upto[RT];              // the positions this thread's rows see
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int row = row0 + ty * 4 + i;
+  for (int i = 0; i < RT; ++i) {
+    const int row = row0 + ty * RT + i;
     upto[i] = row < total ? p.positions[token0 + row / p.groups] : -1;
     from[i] = p.window > 0 ? max(0, upto[i] - p.window + 1) : 0;
   }
   const int* table = p.cache.block_table + (size_t)entry * p.cache.max_pages;
-  const int low = p.positions[token0 + row0 / p.groups], high = p.positions[token0 + (min(row0 + TILE_ROWS, total) - 1) / p.groups];
+  const int low = p.positions[token0 + row0 / p.groups], last = p.positions[token0 + (min(row0 + TILE_ROWS, total) - 1) / p.groups];
   const int lo = p.window > 0 ? max(0, low - p.window + 1) : 0;
+  const int high = SPLIT ? min(last, span * SPAN + SPAN - 1) : last;
+  if (SPLIT && span == 0 && last >= p.spans * SPAN && threadIdx.x == 0) atomicOr(p.status, FE_STATUS_BAD_PAGE);   // past the block table
+  if (SPLIT && (high < span * SPAN || lo > high)) return;
   // of the span at hand, and of the spans before it
-  float m[4], l[4], acc[4][CG][4], top[4], den[4], num[4][CG][4];
+  float m[RT], l[RT], top[SPLIT ? 1 : RT], den[SPLIT ? 1 : RT], num[SPLIT ? 1 : RT][CG][4];
+  uint64_t acc[RT][CG][2];           // two neighbouring columns each
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    m[i] = top[i] = -INFINITY;
-    l[i] = den[i] = 0.f;
+  for (int i = 0; i < RT; ++i) {
+    m[i] = -INFINITY;
+    l[i] = 0.f;
+    if (!SPLIT) top[i] = -INFINITY, den[i] = 0.f;
 #pragma unroll
     for (int g = 0; g < CG; ++g)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) acc[i][g][e] = num[i][g][e] = 0.f;
+      for (int e = 0; e < 4; ++e) {
+        acc[i][g][e / 2] = 0;
+        if (!SPLIT) num[i][g][e] = 0.f;
+      }
   }
-  for (int first = lo / TILE_KEYS * TILE_KEYS; first <= high; first += TILE_KEYS) {
+  for (int first = max(lo, SPLIT ? span * SPAN : 0) / TILE_KEYS * TILE_KEYS; first <= high; first += TILE_KEYS) {
     __syncthreads();
     stage_keys<T, TILE_KEYS, TILE_THREADS>(p, table, kvh, first, lo, high, ks, vs, ok);
     commit();
     wait<0>();
     __syncthreads();
-    uint64_t dot[4][4];
+    uint64_t dot[RT][4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < RT; ++i)
 #pragma unroll
       for (int j = 0; j < 4; ++j) dot[i][j] = 0;
 #pragma unroll 4
     for (int d = 0; d < D; d += 4) {
-      uint64_t a[4][2], b[4][2];
+      uint64_t a[RT][2], b[4][2];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) pairs4(qs + (ty * 4 + i) * qpitch + d, a[i]);
+      for (int i = 0; i < RT; ++i) pairs4(qs + (ty * RT + i) * qpitch + d, a[i]);
 #pragma unroll
       for (int j = 0; j < 4; ++j) pairs4(ks + (tx + 16 * j) * (D + CH) + d, b[j]);
 #pragma unroll
       for (int e = 0; e < 2; ++e)
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < RT; ++i)
 #pragma unroll
           for (int j = 0; j < 4; ++j) fma2(dot[i][j], a[i][e], b[j][e]);
     }
     // by row and thirty-two of keys: maxima, corrections of what came before, sums
-    float score[4][4], most[8], corr[2][4];
+    float score[RT][4], most[2 * RT], corr[2][RT];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < RT; ++i)
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const int key = first + tx + 16 * j;
         score[i][j] = ok[tx + 16 * j] && key >= from[i] && key <= upto[i] ? __fmul_rn(sum2(dot[i][j]), p.scale) : -INFINITY;
         if (j & 1) most[2 * i + j / 2] = fmaxf(score[i][j - 1], score[i][j]);
       }
-    reduce8<true>(most, threadIdx.x & 31);
+    reduce4<true>(most, threadIdx.x & 31);
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < RT; ++i)
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const float now = fmaxf(m[i], most[2 * i + h]);
@@ -384,57 +441,51 @@ __global__ void __launch_bounds__(TILE_THREADS) attention_simt_tile_kernel(const
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
           e[j] = score[i][2 * h + j] == -INFINITY ? 0.f : expf(score[i][2 * h + j] - now);
-          ps[(ty * 4 + i) * P_PITCH + 32 * h + 16 * j + tx] = e[j];
+          ps[(ty * RT + i) * P_PITCH + 32 * h + 16 * j + tx] = e[j];
         }
         most[2 * i + h] = e[0] + e[1];
       }
-    reduce8<false>(most, threadIdx.x & 31);
+    reduce4<false>(most, threadIdx.x & 31);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) l[i] = fmaf(fmaf(l[i], corr[0][i], most[2 * i]), corr[1][i], most[2 * i + 1]);
+    for (int i = 0; i < RT; ++i) l[i] = fmaf(fmaf(l[i], corr[0][i], most[2 * i]), corr[1][i], most[2 * i + 1]);
     __syncwarp();                    // a row's probabilities are written and read by the same warp
-    // Where some row of the tile does not see some key, that key's value is taken as zero for it: a
+    // Where some row of the tile does not see some key, that key's value is left out for it: a
     // zero probability would not keep an infinity out.
-    const bool edge = first < max(0, p.window > 0 ? high - p.window + 1 : 0) || first + TILE_KEYS - 1 > low;
+    const bool edge = first < max(0, p.window > 0 ? last - p.window + 1 : 0) || first + TILE_KEYS - 1 > low;
     for (int key = 0; key < TILE_KEYS; key += 4) {
       if (key % 32 == 0) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < RT; ++i)
 #pragma unroll
           for (int g = 0; g < CG; ++g)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) acc[i][g][e] *= key == 0 ? corr[0][i] : corr[1][i];
+            for (int e = 0; e < 2; ++e) acc[i][g][e] = scale2(acc[i][g][e], key == 0 ? corr[0][i] : corr[1][i]);
       }
-      float e[4][4];
+      float e[RT][4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) load4(ps + (ty * 4 + i) * P_PITCH + key, e[i]);
+      for (int i = 0; i < RT; ++i) load4(ps + (ty * RT + i) * P_PITCH + key, e[i]);
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
+        uint64_t v[CG][2];
 #pragma unroll
-        for (int g = 0; g < CG; ++g) {
-          const int d = tx * 4 + 64 * g;
-          if (d < D) {
-            float v[4];
-            load4(vs + (key + u) * D + d, v);
-            if (!edge) {
+        for (int g = 0; g < CG; ++g)
+          if (tx * 4 + 64 * g < D) pairs4(vs + (key + u) * D + tx * 4 + 64 * g, v[g]);
+          else v[g][0] = v[g][1] = 0;
 #pragma unroll
-              for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < RT; ++i) {
+          if (!edge || (first + key + u >= from[i] && first + key + u <= upto[i])) {
+            const uint64_t both = twice(e[i][u]);
 #pragma unroll
-                for (int c = 0; c < 4; ++c) acc[i][g][c] = fmaf(e[i][u], v[c], acc[i][g][c]);
-            } else {
+            for (int g = 0; g < CG; ++g)
 #pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                const bool seen = first + key + u >= from[i] && first + key + u <= upto[i];
-#pragma unroll
-                for (int c = 0; c < 4; ++c) acc[i][g][c] = fmaf(e[i][u], seen ? v[c] : 0.f, acc[i][g][c]);
-              }
-            }
+              for (int c = 0; c < 2; ++c) fma2(acc[i][g][c], both, v[g][c]);
           }
         }
       }
     }
-    if ((first + TILE_KEYS) % SPAN == 0 || first + TILE_KEYS > high) {
+    if constexpr (!SPLIT) if ((first + TILE_KEYS) % SPAN == 0 || first + TILE_KEYS > high) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
+      for (int i = 0; i < RT; ++i) {
         float old, mine;
         fold_factors(top[i], m[i], old, mine);
         den[i] = fmaf(l[i], mine, __fmul_rn(den[i], old));
@@ -444,16 +495,25 @@ __global__ void __launch_bounds__(TILE_THREADS) attention_simt_tile_kernel(const
         for (int g = 0; g < CG; ++g)
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
-            num[i][g][e] = fmaf(acc[i][g][e], mine, __fmul_rn(num[i][g][e], old));
-            acc[i][g][e] = 0.f;
+            num[i][g][e] = fmaf(half2_of(acc[i][g][e / 2], e & 1), mine, __fmul_rn(num[i][g][e], old));
+            if (e & 1) acc[i][g][e / 2] = 0;
           }
       }
     }
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int row = row0 + ty * 4 + i;
+  for (int i = 0; i < RT; ++i) {
+    const int row = row0 + ty * RT + i;
     if (row >= total) continue;
+    if constexpr (SPLIT) {
+      const size_t rows = (size_t)p.n_tokens * p.groups, at = (size_t)blockIdx.y * rows + (size_t)token0 * p.groups + row;
+      float* sums = p.partial + at * D;
+#pragma unroll
+      for (int g = 0; g < CG; ++g)
+        if (tx * 4 + 64 * g < D) *reinterpret_cast<ulonglong2*>(sums + tx * 4 + 64 * g) = make_ulonglong2(acc[i][g][0], acc[i][g][1]);
+      if (tx == 0) *reinterpret_cast<float2*>(p.partial + (size_t)gridDim.y * rows * D + 2 * at) = make_float2(m[i], l[i]);
+      continue;
+    }
     T* out = (T*)p.out + ((size_t)(token0 + row / p.groups) * p.num_q_heads + kvh * p.groups + row % p.groups) * D;
 #pragma unroll
     for (int g = 0; g < CG; ++g) {
@@ -461,10 +521,45 @@ __global__ void __launch_bounds__(TILE_THREADS) attention_simt_tile_kernel(const
       if (d < D) {
         float o[4];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) o[c] = den[i] > 0.f ? num[i][g][c] / den[i] : 0.f;
+        for (int c = 0; c < 4; ++c) o[c] = den[SPLIT ? 0 : i] > 0.f ? num[SPLIT ? 0 : i][g][c] / den[SPLIT ? 0 : i] : 0.f;
         store4(out + d, o);
       }
     }
+  }
+}
+
+// What the split tile kernel left, a warp a row (token, query head): its spans in ascending order, as the tile kernel folds them.
+template <typename T>
+__global__ void __launch_bounds__(256) attention_simt_fold_kernel(const Simt p) {
+  pdl_trigger();
+  pdl_wait();
+  const int D = p.cache.head_dim, lane = threadIdx.x & 31, index = blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int token = index / p.num_q_heads, head = index % p.num_q_heads;
+  if (token >= p.n_tokens) return;
+  const int entry = p.token_entry[token];
+  if (p.cu_tokens[entry + 1] - p.cu_tokens[entry] <= 1) return;
+  const int pos = p.positions[token], lo = p.window > 0 ? max(0, pos - p.window + 1) : 0;
+  const int from = lo / SPAN, to = min(pos / SPAN, p.spans - 1), kvh = head / p.groups;
+  const size_t rows = (size_t)p.n_tokens * p.groups, row = (size_t)token * p.groups + head % p.groups;
+  const float* ml = p.partial + (size_t)p.spans * p.cache.num_kv_heads * rows * D;
+  T* out = (T*)p.out + ((size_t)token * p.num_q_heads + head) * D;
+  for (int d = lane * 4; d < D; d += 128) {
+    float num[4] = {0.f, 0.f, 0.f, 0.f}, den = 0.f, top = -INFINITY;
+#pragma unroll 4
+    for (int s = from; s <= to; ++s) {
+      const size_t at = ((size_t)s * p.cache.num_kv_heads + kvh) * rows + row;
+      const float2 has = *reinterpret_cast<const float2*>(ml + 2 * at);
+      float part[4], old, mine;
+      load4(p.partial + at * D + d, part);
+      fold_factors(top, has.x, old, mine);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) num[e] = fmaf(part[e], mine, __fmul_rn(num[e], old));
+      den = fmaf(has.y, mine, __fmul_rn(den, old));
+    }
+    float o[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) o[e] = den > 0.f ? num[e] / den : 0.f;
+    store4(out + d, o);
   }
 }
 
@@ -514,26 +609,37 @@ int run_spans(Simt p, cudaStream_t stream) {
   return code;
 }
 
-template <typename T>
-int run_tiles(Simt p, int max_new, cudaStream_t stream) {
+// Whether entries of several tokens are cut into spans of their keys: while their row tiles are fewer than 400 blocks (the
+// chip holds 296, two an SM) and what the spans leave fits the workspace.  16 heads of 128, us, whole / in spans: 500 tokens (264
+// blocks) 132 / 118, 40 after 900 cached ones (32) 148 / 52, 100 after 5,000 (64) 720 / 298, 700 after 400 (360) 353 / 318,
+// 700 (360) 181 / 183, 1,000 (512) 323 / 337.
+long long tile_floats(int n_tokens, int num_q_heads, int num_kv_heads, int head_dim, long long spans, int units) {
+  const long long tiles = ((long long)n_tokens * (num_q_heads / num_kv_heads) + TILE_ROWS - 1) / TILE_ROWS + units;
+  const long long floats = (long long)n_tokens * num_q_heads * spans * (head_dim + 2);
+  return spans < 2 || tiles * num_kv_heads >= 400 || floats > SIMT_WORKSPACE || spans * num_kv_heads > 65535 ? 0 : floats;
+}
+
+template <typename T, bool SPLIT>
+int run_tiles(const Simt& p, cudaStream_t stream) {
   const int D = p.cache.head_dim;
   const size_t smem = (size_t)4 * TILE_ROWS * (D + 4 + P_PITCH) + (size_t)TILE_KEYS * (2 * D * sizeof(T) + 16);
-  int code = 0;
-  for (; p.unit0 < p.units && code == 0; p.unit0 += 65535) {
-    const dim3 grid((unsigned)(((long long)max_new * p.groups + TILE_ROWS - 1) / TILE_ROWS), p.cache.num_kv_heads,
-                    p.units - p.unit0 < 65535 ? p.units - p.unit0 : 65535);
-    if (D <= 64) code = launch(attention_simt_tile_kernel<T, 64>, grid, TILE_THREADS, smem, stream, p);
-    else if (D <= 128) code = launch(attention_simt_tile_kernel<T, 128>, grid, TILE_THREADS, smem, stream, p);
-    else code = launch(attention_simt_tile_kernel<T, 256>, grid, TILE_THREADS, smem, stream, p);
-  }
-  return code;
+  // tiles of all entries one after the other; an entry's last one may be short
+  const dim3 grid((unsigned)(((long long)p.n_tokens * p.groups + TILE_ROWS - 1) / TILE_ROWS + p.units), p.cache.num_kv_heads * (SPLIT ? p.spans : 1));
+  int code;
+  if (D <= 64) code = launch(attention_simt_tile_kernel<T, 64, SPLIT>, grid, TILE_THREADS, smem, stream, p);
+  else if (D <= 128) code = launch(attention_simt_tile_kernel<T, 128, SPLIT>, grid, TILE_THREADS, smem, stream, p);
+  else code = launch(attention_simt_tile_kernel<T, 256, SPLIT>, grid, TILE_THREADS, smem, stream, p);
+  if (code || !SPLIT) return code;
+  const long long rows = (long long)p.n_tokens * p.num_q_heads;
+  return launch(attention_simt_fold_kernel<T>, dim3((unsigned)((rows + 7) / 8)), 256, 0, stream, p);
 }
 
 template <typename T>
 int run(const Simt& p, int n_tokens, int max_new, cudaStream_t stream) {
   // units that bring several tokens, then those that bring one; a step of one prompt has none of these
   if (p.cu_tokens != nullptr && max_new > 1) {
-    const int code = run_tiles<T>(p, max_new, stream);
+    const bool split = tile_floats(n_tokens, p.num_q_heads, p.cache.num_kv_heads, p.cache.head_dim, p.spans, p.units) > 0;
+    const int code = split ? run_tiles<T, true>(p, stream) : run_tiles<T, false>(p, stream);
     if (code) return code;
     if (p.units == 1 && n_tokens > 1) return 0;
   }
@@ -551,6 +657,13 @@ FE_EXPORT int fe_attention_simt_units(int units, int num_q_heads, int num_kv_hea
 FE_EXPORT long long fe_attention_simt_scratch(int units, int num_q_heads, int num_kv_heads, int head_dim, int max_pages, int page_size) {
   const int slice = fe_attention_simt_units(units, num_q_heads, num_kv_heads, head_dim, max_pages, page_size);
   return slice == 0 ? 0 : slice * unit_floats(num_q_heads, num_kv_heads, head_dim, spans_of(max_pages, page_size));
+}
+
+// The floats of workspace that entries of several tokens take (0: none), for `n_tokens` tokens of `units` entries.
+FE_EXPORT long long fe_attention_simt_tile_scratch(int n_tokens, int units, int num_q_heads, int num_kv_heads, int head_dim, int max_pages,
+                                                   int page_size) {
+  if (num_kv_heads <= 0 || num_q_heads <= 0 || num_q_heads % num_kv_heads) return 0;
+  return tile_floats(n_tokens, num_q_heads, num_kv_heads, head_dim, spans_of(max_pages, page_size), units);
 }
 
 // `cu_tokens` [units + 1] says which tokens each unit (an entry: row u of the block table, positions
@@ -573,7 +686,7 @@ FE_EXPORT int fe_attention_simt(const void* q, int q_stride, int dtype, const vo
   const int row_tiles = (groups + R - 1) / R;
   if (spans > 0x7fffffff || (long long)num_kv_heads * row_tiles > 65535) return FE_ERR_TOO_LARGE;
   Simt p{q, q_stride, cache, positions, token_entry, cu_tokens, units, window, scale, out, num_q_heads, groups,
-         (int)spans, row_tiles, 0, workspace, status};
+         (int)spans, row_tiles, 0, workspace, n_tokens, status};
   if (dtype == FE_DTYPE_F32) return run<float>(p, n_tokens, max_new, stream);
   if (dtype == FE_DTYPE_BF16) return run<bf16>(p, n_tokens, max_new, stream);
   return FE_ERR_BAD_DTYPE;

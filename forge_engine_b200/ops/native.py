@@ -91,6 +91,7 @@ def _declare(handle: ctypes.CDLL) -> None:
         "fe_attention_simt": [p, i, i, p, p, p, i, i, i, p, p, p, i, i, i, f, p, i, i, i, i, p, p, p],
         "fe_attention_simt_scratch": [i, i, i, i, i, i],
         "fe_attention_simt_units": [i, i, i, i, i, i],
+        "fe_attention_simt_tile_scratch": [i, i, i, i, i, i, i],
         "fe_gemm_simt": [p, i, p, i, p, p, i, i, i, i, i, p, p],
         "fe_sample": [p, i, i, p, p, p, p, p, p, p, p, p],
         "fe_sample_rows": [p, i, i, ctypes.c_char_p, p, p, p],
@@ -121,7 +122,7 @@ def _declare(handle: ctypes.CDLL) -> None:
         fn.argtypes = argtypes
         fn.restype = c_int
     for name in ("fe_gated_recurrence_scratch", "fe_wkv_scratch", "fe_delta_rule_scratch", "fe_matrix_memory_scratch",
-                 "fe_retention_scratch", "fe_rglru_scratch", "fe_attention_simt_scratch"):
+                 "fe_retention_scratch", "fe_rglru_scratch", "fe_attention_simt_scratch", "fe_attention_simt_tile_scratch"):
         getattr(handle, name).restype = ctypes.c_longlong
     handle.fe_uniform_host.argtypes = [c_ulonglong, c_ulonglong]
     handle.fe_uniform_host.restype = c_float
@@ -1472,12 +1473,18 @@ def attention_simt(
     n = out.shape[0]
     assert out.shape[1] == num_q_heads * head_dim and out.dtype == q.dtype == k_cache.dtype
     cu_tokens, units, max_new = (None, n, 1) if entries is None else entries
-    workspace, slices = None, 0
+    workspace, slices, floats, folded = None, 0, 0, 0
+    sizes = (int(units), num_q_heads, nkv, head_dim, block_table.shape[1], page_size)
     if max_new <= 1 or units > 1 or n <= 1:            # some token may come by itself
-        sizes = (int(units), num_q_heads, nkv, head_dim, block_table.shape[1], page_size)
-        # the call's own, so that runs on several streams do not share it
-        workspace = torch.empty(max(1, lib().fe_attention_simt_scratch(*sizes)), dtype=torch.float32, device=q.device)
+        floats = max(1, lib().fe_attention_simt_scratch(*sizes))
         slices = -(-int(units) // max(1, lib().fe_attention_simt_units(*sizes)))
+    if cu_tokens is not None and max_new > 1:
+        # entries of several tokens; the kernels run one after the other and take the same floats
+        folded = lib().fe_attention_simt_tile_scratch(n, *sizes)
+        floats = max(floats, folded)
+    if floats:
+        # the call's own, so that runs on several streams do not share it
+        workspace = torch.empty(floats, dtype=torch.float32, device=q.device)
     check(
         lib().fe_attention_simt(
             ptr(q), int(q_stride), code(q), ptr(k_cache), ptr(v_cache), ptr(block_table),
@@ -1488,7 +1495,7 @@ def attention_simt(
         "attention_simt",
     )
     global LAUNCHES
-    LAUNCHES += 2 * slices + (1 if cu_tokens is not None and max_new > 1 else 0) - 1
+    LAUNCHES += 2 * slices + ((2 if folded else 1) if cu_tokens is not None and max_new > 1 else 0) - 1
 
 
 _balanced_blocks: dict = {}
