@@ -427,13 +427,15 @@ __global__ void __launch_bounds__(DS_THREADS) delta_solve_kernel(const Delta m, 
         float sum[4] = {0.f, 0.f, 0.f, 0.f}, small[4] = {0.f, 0.f, 0.f, 0.f};
         const float* l = lt + fq * SR_TP + r0 + fg;
         const float* x = X + fq * ldx + n0 + fg;
-#pragma unroll 2
-        for (int j = 0; j < r0; j += 8) {
-          SplitA fa;
-          SplitB fb;
+#pragma unroll 1
+        for (int j = 0; j < r0; j += 16) {
+          SplitA fa, fa2;
+          SplitB fb, fb2;
           split_load_a(fa, l + j * SR_TP, 1, SR_TP);
+          split_load_a(fa2, l + (j + 8) * SR_TP, 1, SR_TP);
           split_load_b(fb, x + j * ldx, ldx);
-          split_mma(sum, small, fa, fb);
+          split_load_b(fb2, x + (j + 8) * ldx, ldx);
+          split_mma(sum, small, fa, fa2, fb, fb2);
         }
 #pragma unroll
         for (int h = 0; h < 2; ++h) {

@@ -165,22 +165,111 @@ __global__ void __launch_bounds__(1024) gated_recurrence_kernel(GatedRecurrence 
 #define GR_SLICE 128                             // channels (or columns) worked on at a time
 #define GR_AP (GR_LONG_CHUNK + 4)
 
-// Sums of 16 values over the lanes of a warp; lane l gets the sum of value l / 2.
-__device__ __forceinline__ float gr_sum16(float (&x)[16], int lane) {
+// Sums of the last N of 16 values over the lanes of a warp; lane l gets the sum of value 16 - N + l N / 32.
+template <int N>
+__device__ __forceinline__ float gr_sums(float (&x)[16], int lane) {
+  constexpr int FROM = 16 - N;
+  int bit = 16;
 #pragma unroll
-  for (int half = 8, bit = 16; half > 0; half >>= 1, bit >>= 1) {
+  for (int half = N / 2; half > 0; half >>= 1, bit >>= 1) {
     const bool upper = (lane & bit) != 0;
 #pragma unroll
-    for (int i = 0; i < half; ++i) {
+    for (int i = FROM; i < FROM + half; ++i) {
       const float send = upper ? x[i] : x[i + half], keep = upper ? x[i + half] : x[i];
       x[i] = keep + __shfl_xor_sync(0xffffffffu, send, bit);
     }
   }
-  return x[0] + __shfl_xor_sync(0xffffffffu, x[0], 1);
+#pragma unroll
+  for (int b = 16 / N; b > 0; b >>= 1) x[FROM] += __shfl_xor_sync(0xffffffffu, x[FROM], b);
+  return x[FROM];
+}
+
+// R neighbouring channels of a lane: products in pairs.
+template <int R> struct GrChannels {
+  static constexpr int PAIRS = R / 2;
+  uint64_t v[PAIRS];
+  __device__ __forceinline__ void load(const float* p) {
+    if constexpr (R == 4) { const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(p); v[0] = x.x, v[1] = x.y; }
+    else v[0] = *reinterpret_cast<const uint64_t*>(p);
+  }
+  __device__ __forceinline__ void fill(float x) {
+#pragma unroll
+    for (int i = 0; i < PAIRS; ++i) asm("mov.b64 %0, {%1, %1};" : "=l"(v[i]) : "f"(x));
+  }
+  __device__ __forceinline__ void times(const GrChannels& o) {
+#pragma unroll
+    for (int i = 0; i < PAIRS; ++i) asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(v[i]) : "l"(o.v[i]));
+  }
+  __device__ __forceinline__ void one_minus(const GrChannels& o) {
+#pragma unroll
+    for (int i = 0; i < PAIRS; ++i) {
+      float a, b;
+      asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(o.v[i]));
+      asm("mov.b64 %0, {%1, %2};" : "=l"(v[i]) : "f"(1.f - a), "f"(1.f - b));
+    }
+  }
+  __device__ __forceinline__ void take(bool which, const GrChannels& o) {
+#pragma unroll
+    for (int i = 0; i < PAIRS; ++i) v[i] = which ? o.v[i] : v[i];
+  }
+  __device__ __forceinline__ float dot(const GrChannels& o) const {
+    uint64_t sum;
+    float a, b;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(sum) : "l"(v[0]), "l"(o.v[0]));
+    if constexpr (PAIRS == 2) asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(sum) : "l"(v[1]), "l"(o.v[1]));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(sum));
+    return a + b;
+  }
+};
+template <> struct GrChannels<1> {
+  float v;
+  __device__ __forceinline__ void load(const float* p) { v = *p; }
+  __device__ __forceinline__ void fill(float x) { v = x; }
+  __device__ __forceinline__ void times(const GrChannels& o) { v *= o.v; }
+  __device__ __forceinline__ void one_minus(const GrChannels& o) { v = 1.f - o.v; }
+  __device__ __forceinline__ void take(bool which, const GrChannels& o) { v = which ? o.v : v; }
+  __device__ __forceinline__ float dot(const GrChannels& o) const { return v * o.v; }
+};
+
+// Inside a sub-chunk: the columns of its tokens 4 PASS .. 4 PASS + 3, two of them by each of its two warps.  Token by
+// token from the first of the four on: w, what is left of each token's k, takes the gates, and q w gives the next row.
+template <int R, int PASS>
+__device__ __forceinline__ void gr_inside(const float* fs, const float* qs, int dp, float* as, int odd, int lane, bool has) {
+  const int s0 = 4 * PASS + 2 * odd;
+  GrChannels<R> w[2];
+  float sums[2][GR_SUB];
+  w[0].fill(0.f), w[1].fill(0.f);
+#pragma unroll
+  for (int t = 0; t < GR_SUB; ++t) {
+    sums[0][t] = sums[1][t] = 0.f;
+    if (t < 4 * PASS) continue;
+    GrChannels<R> f, q;
+    f.fill(1.f), q.fill(0.f);
+    if (has) f.load(fs + t * dp), q.load(qs + t * dp);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      w[k].times(f);
+      if (t < 4 * PASS + 4) {
+        GrChannels<R> own;
+        own.one_minus(f);
+        w[k].take(t == s0 + k, own);
+      }
+      sums[k][t] = q.dot(w[k]);
+    }
+  }
+  constexpr int N = PASS < 2 ? 16 : PASS == 2 ? 8 : 4;
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const float sum = gr_sums<N>(sums[k], lane);
+    const int t = 16 - N + lane * N / 32;
+    if (lane % (32 / N) == 0 && t >= s0 + k) as[t * GR_AP + s0 + k] += sum;
+  }
 }
 
 // One chunk of a long entry (see the head of this file).  Tokens past the entry's end have f = 1 and
-// q = k = v = 0.
+// q = k = v = 0.  Bound by the instructions issued: inside a sub-chunk no row before a column's token is worked out and
+// channels go in pairs, and the products between sub-chunks are one round of a warp each without barriers (before, a round and
+// two barriers per distance with q rewritten in between).  3 prompts of 1,000 to 666 tokens, 32 heads of 128: 253 us before, 195 now.
 // R: channels a lane of the sub-chunks' own blocks holds, in a slice, as few as the head needs.  32 heads of 64, 2,048
 // tokens, all kernels: 216 us with two, 225 with four; 32 heads of 16, 1,000 tokens: 77 us with one, 89 with four.
 template <int R>
@@ -258,44 +347,14 @@ __global__ void __launch_bounds__(256, 2) gated_recurrence_chunk_kernel(GatedRec
     }
     __syncthreads();
     {
-      // inside the sub-chunks: two warps each, two tokens s at a time, lanes over the channels
-      constexpr int AT = 2;
-      const int sub = warp >> 1, base = sub * GR_SUB;
-#pragma unroll 1
-      for (int pass = 0; pass < 8 / AT; ++pass) {
-        const int s0 = (warp & 1) * 8 + pass * AT;
-        float w[AT][R], sums[AT][GR_SUB];
-#pragma unroll
-        for (int k = 0; k < AT; ++k)
-#pragma unroll
-          for (int r = 0; r < R; ++r) w[k][r] = 0.f;
-#pragma unroll
-        for (int t = 0; t < GR_SUB; ++t) {
-          float f[R], q[R];
-#pragma unroll
-          for (int r = 0; r < R; ++r) {
-            const bool has = lane + 32 * r < ndp;
-            f[r] = has ? fs[(base + t) * dp + lane + 32 * r] : 1.f;
-            q[r] = has ? qs[(base + t) * dp + lane + 32 * r] : 0.f;
-          }
-#pragma unroll
-          for (int k = 0; k < AT; ++k) {
-            float sum = 0.f;
-#pragma unroll
-            for (int r = 0; r < R; ++r) {
-              w[k][r] = t == s0 + k ? 1.f - f[r] : w[k][r] * f[r];
-              sum = fmaf(q[r], w[k][r], sum);
-            }
-            sums[k][t] = sum;
-          }
-        }
-#pragma unroll
-        for (int k = 0; k < AT; ++k) {
-          const float sum = gr_sum16(sums[k], lane);
-          const int t = lane >> 1;
-          if ((lane & 1) == 0 && t >= s0 + k) as[(base + t) * GR_AP + base + s0 + k] += sum;
-        }
-      }
+      // inside the sub-chunks: two warps each, lanes over the channels
+      const int base = (warp >> 1) * GR_SUB, at_lane = base * dp + lane * R;
+      const bool has = lane * R < ndp;
+      float* own = as + base * GR_AP + base;
+      gr_inside<R, 0>(fs + at_lane, qs + at_lane, dp, own, warp & 1, lane, has);
+      gr_inside<R, 1>(fs + at_lane, qs + at_lane, dp, own, warp & 1, lane, has);
+      gr_inside<R, 2>(fs + at_lane, qs + at_lane, dp, own, warp & 1, lane, has);
+      gr_inside<R, 3>(fs + at_lane, qs + at_lane, dp, own, warp & 1, lane, has);
     }
     __syncthreads();
     // q with the gates from its sub-chunk's start on, k with those up to its sub-chunk's end
@@ -311,6 +370,7 @@ __global__ void __launch_bounds__(256, 2) gated_recurrence_chunk_kernel(GatedRec
         q[t * dp] *= b;
       }
       whole[sub * dp + d] = b;
+      if (d < 4) whole[sub * dp + ndp + d] = 1.f;      // the channels behind the last (see above)
       b = 1.f;
 #pragma unroll
       for (int t = GR_SUB - 1; t >= 0; --t) {
@@ -319,60 +379,103 @@ __global__ void __launch_bounds__(256, 2) gated_recurrence_chunk_kernel(GatedRec
       }
     }
     __syncthreads();
-    // sub-chunks `apart` apart: A's blocks of 16 x 16, two warps each; q then takes the gates of the
-    // sub-chunk it has just been multiplied with
+    // between two sub-chunks: A's six blocks of 16 x 16, a warp each; q takes the gates of the whole sub-chunks in
+    // between on its way
     const int fg = lane >> 2, fq = lane & 3;           // this lane's row and column in a fragment
-#pragma unroll 1
-    for (int apart = 1; apart < GR_SUBS; ++apart) {
-      const int block = warp >> 1, side = (warp & 1) * 8;
-      if (block < GR_SUBS - apart) {
-        const float* q0 = qs + ((apart + block) * GR_SUB + fg) * dp + fq;
-        const float* k0 = fs + (block * GR_SUB + side + fg) * dp + fq;
-        float sum[4] = {0.f, 0.f, 0.f, 0.f}, small[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 4
-        for (int d = 0; d < ndp; d += 8) {
-          SplitA fa;
-          SplitB fb;
-          split_load_a(fa, q0 + d, dp, 1);
-          split_load_b(fb, k0 + d, 1);
-          split_mma(sum, small, fa, fb);
+    if (warp < 6) {
+      const int to = warp < 1 ? 1 : warp < 3 ? 2 : 3, from = warp - to * (to - 1) / 2;
+      const float* q0 = qs + (to * GR_SUB + fg) * dp + fq;
+      const float* k0 = fs + (from * GR_SUB + fg) * dp + fq;
+      float sum[2][4], small[2][4];
+#pragma unroll
+      for (int b = 0; b < 2; ++b)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sum[b][i] = small[b][i] = 0.f;
+      auto gated = [&](SplitA& a, int d) {
+        float x[4] = {q0[d], q0[d + 4], q0[8 * dp + d], q0[8 * dp + d + 4]};
+        for (int sub = to - 1; sub > from; --sub) {
+          const float g0 = whole[sub * dp + d + fq], g1 = whole[sub * dp + d + fq + 4];
+          x[0] *= g0, x[1] *= g1, x[2] *= g0, x[3] *= g1;
         }
+        split_pair(x[0], x[1], a.part[0][0], a.part[1][0], a.part[2][0]);
+        split_pair(x[2], x[3], a.part[0][1], a.part[1][1], a.part[2][1]);
+      };
+      int d = 0;
+#pragma unroll 1
+      for (; d + 12 <= ndp; d += 16) {
+        SplitA fa, fa2;
+        gated(fa, d), gated(fa2, d + 8);
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+          SplitB fb, fb2;
+          split_load_b(fb, k0 + 8 * b * dp + d, 1);
+          split_load_b(fb2, k0 + 8 * b * dp + d + 8, 1);
+          split_mma(sum[b], small[b], fa, fa2, fb, fb2);
+        }
+      }
+      if (d < ndp) {
+        SplitA fa;
+        gated(fa, d);
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+          SplitB fb;
+          split_load_b(fb, k0 + 8 * b * dp + d, 1);
+          split_mma(sum[b], small[b], fa, fb);
+        }
+      }
+#pragma unroll
+      for (int b = 0; b < 2; ++b)
 #pragma unroll
         for (int i = 0; i < 4; ++i)
-          as[((apart + block) * GR_SUB + fg + 8 * (i >> 1)) * GR_AP + block * GR_SUB + side + 2 * fq + (i & 1)] += split_join(sum[i], small[i]);
-      }
-      __syncthreads();
-      if (lane * 4 < ndp) {
-        const int d = lane * 4;
-#pragma unroll 4
-        for (int t = warp; t < (GR_SUBS - apart) * GR_SUB; t += 8) {
-          float* q = qs + (apart * GR_SUB + t) * dp + d;
-          float a[4], g[4];
-          load4(q, a), load4(whole + (t / GR_SUB) * dp + d, g);
+          as[(to * GR_SUB + fg + 8 * (i >> 1)) * GR_AP + from * GR_SUB + 8 * b + 2 * fq + (i & 1)] += split_join(sum[b][i], small[b][i]);
+    }
+    // q with the gates from the chunk's start on
+    if (lane * 4 < ndp) {
+      const int d = lane * 4;
 #pragma unroll
-          for (int e = 0; e < 4; ++e) a[e] *= g[e];
-          store4(q, a);
+      for (int sub = 0; sub < GR_SUBS; ++sub) {
+        float g[GR_SUBS][4];
+#pragma unroll
+        for (int m = 0; m < sub; ++m) load4(whole + m * dp + d, g[m]);
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const int t = sub * GR_SUB + u * 8 + warp;
+          if (t >= count) continue;
+          float a[4];
+          load4(qs + t * dp + d, a);
+#pragma unroll
+          for (int m = sub - 1; m >= 0; --m)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) a[e] *= g[m][e];
+          store4(p.qb + ((size_t)(first + t) * p.heads + head) * p.dkp + d0 + d, a);
         }
       }
-      __syncthreads();
     }
-    if (lane * 4 < ndp) {
-#pragma unroll 4
-      for (int t = warp; t < count; t += 8) {
-        float a[4];
-        load4(qs + t * dp + lane * 4, a);
-        store4(p.qb + ((size_t)(first + t) * p.heads + head) * p.dkp + d0 + lane * 4, a);
+    __syncthreads();
+    // k with the gates up to the chunk's end: four tokens and four channels at a time
+    const int quads = ndp >> 2;
+    for (int i = tid; i < quads * (GR_SUBS - 1) * 4; i += 256) {
+      const int d = (i % quads) * 4, t = (i / quads) * 4, sub = t / GR_SUB;
+      float b[4] = {1.f, 1.f, 1.f, 1.f};
+      for (int m = GR_SUBS - 1; m > sub; --m) {
+        float g[4];
+        load4(whole + m * dp + d, g);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) b[e] *= g[e];
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        float k[4];
+        load4(fs + (t + u) * dp + d, k);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) k[e] *= b[e];
+        store4(fs + (t + u) * dp + d, k);
       }
     }
-    // k with the gates up to the chunk's end
     for (int d = tid; d < nd; d += 256) {
       float b = 1.f;
 #pragma unroll
-      for (int sub = GR_SUBS - 1; sub >= 0; --sub) {
-        if (sub < GR_SUBS - 1)
-          for (int t = 0; t < GR_SUB; ++t) fs[(sub * GR_SUB + t) * dp + d] *= b;
-        b *= whole[sub * dp + d];
-      }
+      for (int sub = GR_SUBS - 1; sub >= 0; --sub) b *= whole[sub * dp + d];
       p.chunk_decay[at * dk + d0 + d] = b;
     }
     // the chunk's own end state
@@ -413,17 +516,21 @@ __global__ void __launch_bounds__(256, 2) gated_recurrence_chunk_kernel(GatedRec
             for (int i = 0; i < 4; ++i) sum[a][b][i] = small[a][b][i] = 0.f;
         const float* ka = fs + fq * dp + m0 + fg;
         const float* vb = vs + fq * vp + c0 + fg;
-#pragma unroll 2
-        for (int t = 0; t < GR_LONG_CHUNK; t += 8) {
-          SplitA fa[2];
-          split_load_a(fa[0], ka + t * dp, 1, dp);
-          split_load_a(fa[1], ka + t * dp + 16, 1, dp);
+#pragma unroll 1
+        for (int t = 0; t < GR_LONG_CHUNK; t += 16) {
+          SplitA fa[2], fa2[2];
+#pragma unroll
+          for (int a = 0; a < 2; ++a) {
+            split_load_a(fa[a], ka + t * dp + 16 * a, 1, dp);
+            split_load_a(fa2[a], ka + (t + 8) * dp + 16 * a, 1, dp);
+          }
 #pragma unroll
           for (int b = 0; b < 4; ++b) {
-            SplitB fb;
+            SplitB fb, fb2;
             split_load_b(fb, vb + t * vp + 8 * b, vp);
-            split_mma(sum[0][b], small[0][b], fa[0], fb);
-            split_mma(sum[1][b], small[1][b], fa[1], fb);
+            split_load_b(fb2, vb + (t + 8) * vp + 8 * b, vp);
+#pragma unroll
+            for (int a = 0; a < 2; ++a) split_mma(sum[a][b], small[a][b], fa[a], fa2[a], fb, fb2);
           }
         }
 #pragma unroll
@@ -611,17 +718,21 @@ __global__ void __launch_bounds__(256, 2) gated_recurrence_finish_kernel(GatedRe
       if (n0 < nv && (m0 > 0 || step <= q_steps)) {
         const float* xs = smem + (step % stages) * stage_floats + (m0 + fg) * GR_FX + fq;
         const float* ys = smem + (step % stages) * stage_floats + GR_LONG_CHUNK * GR_FX + fq * pitch + n0 + fg;
-#pragma unroll 2
-        for (int k = 0; k < GR_FK; k += 8) {
-          SplitA fa[2];
-          split_load_a(fa[0], xs + k, GR_FX, 1);
-          split_load_a(fa[1], xs + 16 * GR_FX + k, GR_FX, 1);
+#pragma unroll 1
+        for (int k = 0; k < GR_FK; k += 16) {
+          SplitA fa[2], fa2[2];
+#pragma unroll
+          for (int a = 0; a < 2; ++a) {
+            split_load_a(fa[a], xs + 16 * a * GR_FX + k, GR_FX, 1);
+            split_load_a(fa2[a], xs + 16 * a * GR_FX + k + 8, GR_FX, 1);
+          }
 #pragma unroll
           for (int b = 0; b < 4; ++b) {
-            SplitB fb;
+            SplitB fb, fb2;
             split_load_b(fb, ys + k * pitch + 8 * b, pitch);
-            split_mma(sum[0][b], small[0][b], fa[0], fb);
-            split_mma(sum[1][b], small[1][b], fa[1], fb);
+            split_load_b(fb2, ys + (k + 8) * pitch + 8 * b, pitch);
+#pragma unroll
+            for (int a = 0; a < 2; ++a) split_mma(sum[a][b], small[a][b], fa[a], fa2[a], fb, fb2);
           }
         }
       }

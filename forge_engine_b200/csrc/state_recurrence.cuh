@@ -463,8 +463,25 @@ struct OutTile {            // a warp's 32 x 16 outputs
   }
   // += X^T Y over `depth` rows (a multiple of 8) of both: x at this lane's place in [k][token], y in [k][column]
   __device__ __forceinline__ void add(const float* x, const float* y, int ldy, int depth) {
-#pragma unroll 2
-    for (int k = 0; k < depth; k += 8) {
+    int k = 0;
+#pragma unroll 1
+    for (; k + 16 <= depth; k += 16) {
+      SplitA fa[2], fa2[2];
+#pragma unroll
+      for (int a = 0; a < 2; ++a) {
+        split_load_a(fa[a], x + k * SR_TP + 16 * a, 1, SR_TP);
+        split_load_a(fa2[a], x + (k + 8) * SR_TP + 16 * a, 1, SR_TP);
+      }
+#pragma unroll
+      for (int b = 0; b < 2; ++b) {
+        SplitB fb, fb2;
+        split_load_b(fb, y + k * ldy + 8 * b, ldy);
+        split_load_b(fb2, y + (k + 8) * ldy + 8 * b, ldy);
+#pragma unroll
+        for (int a = 0; a < 2; ++a) split_mma(sum[a][b], small[a][b], fa[a], fa2[a], fb, fb2);
+      }
+    }
+    if (k < depth) {
       SplitA fa[2];
       split_load_a(fa[0], x + k * SR_TP, 1, SR_TP);
       split_load_a(fa[1], x + k * SR_TP + 16, 1, SR_TP);

@@ -263,6 +263,12 @@ def test_gated_recurrence_chunks(native, heads, dk, dv, lead, counts):
     assert torch.equal(got_state[-1].cpu(), state[-1])       # the row of no entry
 
 
+@pytest.mark.parametrize("dk", (4, 20, 36, 72, 100, 132))
+def test_gated_recurrence_channels_off_sixteen(native, dk):
+    """Products between sub-chunks over every remainder of sixteen channels; lanes with one, two and four channels."""
+    test_gated_recurrence_chunks(native, 2, dk, 8, 4, [150, 133])
+
+
 # -- delta rule: chunks ---------------------------------------------------------------------------
 @pytest.mark.parametrize("kv_heads, heads, dk, dv", ((1, 2, 64, 64), (2, 2, 72, 40), (1, 1, 128, 128), (1, 2, 160, 36), (1, 1, 176, 64), (1, 1, 152, 100), (2, 4, 6, 10), (1, 1, 13, 5), (1, 1, 65, 129)))
 @pytest.mark.parametrize("counts", ([96], [97, 160, 3], [191, 1, 192, 130]))
