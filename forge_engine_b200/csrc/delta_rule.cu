@@ -99,24 +99,10 @@ __device__ __forceinline__ void delta_prepare_gates(const DeltaPrepare& p, int t
   for (int h = threadIdx.x; h < p.heads; h += blockDim.x) delta_prepare_gate(p, t, h);
 }
 
+// An entry's edge: its first taps - 1 tokens, then the state for the next step.
 template <int V>
-__global__ void __launch_bounds__(32 * DP_WARPS) delta_prepare_kernel(DeltaPrepare p, int inner) {
-  extern __shared__ __align__(16) float smem[];      // [DP_WARPS][dk]
-  pdl_trigger();
-  pdl_wait();
-  const int back = p.taps - 1, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int r = blockIdx.y * DP_WARPS + warp, rows = 2 * p.kv_heads + p.heads;
-  float* buf = smem + warp * p.dk;
-  if ((int)blockIdx.x < inner) {
-    // a token with all its taps inside the step (inner 0: they are delta_prepare_run's)
-    const int t = blockIdx.x;
-    if (t - p.cu_tokens[p.token_entry[t]] < back) return;
-    if (r < rows) delta_prepare_row<V>(p, t, r, buf, [&](int j) { return p.proj + (size_t)(t - j) * p.ld; });
-    if (blockIdx.y == 0) delta_prepare_gates(p, t);
-    return;
-  }
-  // an entry's edge: its first taps - 1 tokens, then the state for the next step
-  const int entry = blockIdx.x - inner;
+__device__ __forceinline__ void delta_prepare_edge(const DeltaPrepare& p, int entry, int r, float* buf) {
+  const int back = p.taps - 1, lane = threadIdx.x & 31, rows = 2 * p.kv_heads + p.heads;
   const int first = p.cu_tokens[entry], count = p.cu_tokens[entry + 1] - first, edge = min(count, back);
   if (count <= 0) return;
   if (blockIdx.y == 0)
@@ -140,16 +126,43 @@ __global__ void __launch_bounds__(32 * DP_WARPS) delta_prepare_kernel(DeltaPrepa
     }
 }
 
+template <int V>
+__global__ void __launch_bounds__(32 * DP_WARPS) delta_prepare_kernel(DeltaPrepare p, int inner) {
+  extern __shared__ __align__(16) float smem[];      // [DP_WARPS][dk]
+  pdl_trigger();
+  pdl_wait();
+  const int back = p.taps - 1, warp = threadIdx.x >> 5;
+  const int r = blockIdx.y * DP_WARPS + warp, rows = 2 * p.kv_heads + p.heads;
+  float* buf = smem + warp * p.dk;
+  if ((int)blockIdx.x < inner) {
+    // a token with all its taps inside the step
+    const int t = blockIdx.x;
+    if (t - p.cu_tokens[p.token_entry[t]] < back) return;
+    if (r < rows) delta_prepare_row<V>(p, t, r, buf, [&](int j) { return p.proj + (size_t)(t - j) * p.ld; });
+    if (blockIdx.y == 0) delta_prepare_gates(p, t);
+    return;
+  }
+  delta_prepare_edge<V>(p, blockIdx.x - inner, r, buf);
+}
+
 // Tokens with all their taps inside the step, DP_RUN of them in a row by a warp for one q, k or v head of
 // at most 32 V elements: every input is read once instead of once per tap.  Bound by the bytes in and out
-// (2,048 tokens of 4,096 channels: 67 us with a warp per token and head; 24 us this way and 10 us for the entry's edge).
+// (2,048 tokens of 4,096 channels: 67 us with a warp per token and head; this way 24 us and 14 us for the entry's edge behind
+// them, 25 us with the edges' blocks, the first n_entries, beside them).
 #define DP_RUN 16
 template <int V, int TAPS>
-__global__ void __launch_bounds__(32 * DP_WARPS) delta_prepare_run_kernel(DeltaPrepare p) {
+__global__ void __launch_bounds__(32 * DP_WARPS) delta_prepare_run_kernel(DeltaPrepare p, int n_entries, int wide) {
+  extern __shared__ __align__(16) float smem[];      // [DP_WARPS][dk]
   pdl_trigger();
   pdl_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int r = blockIdx.y * DP_WARPS + warp, t0 = blockIdx.x * DP_RUN, end = min(p.n_tokens, t0 + DP_RUN);
+  const int r = blockIdx.y * DP_WARPS + warp;
+  if ((int)blockIdx.x < n_entries) {
+    if (wide) delta_prepare_edge<4>(p, blockIdx.x, r, smem + warp * p.dk);
+    else delta_prepare_edge<1>(p, blockIdx.x, r, smem + warp * p.dk);
+    return;
+  }
+  const int t0 = (blockIdx.x - n_entries) * DP_RUN, end = min(p.n_tokens, t0 + DP_RUN);
   if (blockIdx.y == 0)
     for (int i = threadIdx.x; i < (end - t0) * p.heads; i += blockDim.x) {
       const int t = t0 + i / p.heads, h = i % p.heads;
@@ -226,16 +239,15 @@ FE_EXPORT int fe_delta_prepare(const float* proj, long long ld, int b_off, int a
   if (smem > 48 * 1024 || pieces > 65535) return FE_ERR_TOO_LARGE;
   const bool wide = dk % 4 == 0 && dv % 4 == 0 && ld % 4 == 0 &&
                     (((uintptr_t)proj | (uintptr_t)conv | (uintptr_t)state | (uintptr_t)out) & 15) == 0;
-  // many tokens: runs of them, then the entries' edges alone.  Below 256 tokens there are too few runs to
+  // many tokens: runs of them, and the entries' edges beside them.  Below 256 tokens there are too few runs to
   // fill the machine, and a block per token starts all at once.
   const int most = dk > dv ? dk : dv, V = most <= 32 ? 1 : most <= 64 ? 2 : 4;
-  int inner = n_tokens;
   if (n_tokens >= 256 && taps >= 2 && taps <= 4 && most <= 128 && (V == 1 || wide || (V == 2 && dk % 2 == 0 && dv % 2 == 0 && ld % 2 == 0 &&
       (((uintptr_t)proj | (uintptr_t)conv | (uintptr_t)out) & 7) == 0))) {
-    inner = 0;
-    const dim3 runs((n_tokens + DP_RUN - 1) / DP_RUN, pieces);
+    const dim3 runs(n_entries + (n_tokens + DP_RUN - 1) / DP_RUN, pieces);
     int rc = 0;
-#define DP_RUNS(V_, TAPS) rc = fe_launch_dependent(delta_prepare_run_kernel<V_, TAPS>, runs, dim3(32 * DP_WARPS), 0, stream, p)
+#define DP_RUNS(V_, TAPS) \
+  rc = fe_launch_dependent(delta_prepare_run_kernel<V_, TAPS>, runs, dim3(32 * DP_WARPS), smem, stream, p, n_entries, (int)wide)
 #define DP_RUNS_BY_V(TAPS)        \
   do {                            \
     if (V == 1) DP_RUNS(1, TAPS); \
@@ -247,12 +259,12 @@ FE_EXPORT int fe_delta_prepare(const float* proj, long long ld, int b_off, int a
     else DP_RUNS_BY_V(4);
 #undef DP_RUNS_BY_V
 #undef DP_RUNS
-    if (rc) return rc;
+    return rc ? rc : fe_last_error();
   }
-  const dim3 grid(inner + (taps > 1 ? n_entries : 0), pieces);
+  const dim3 grid(n_tokens + (taps > 1 ? n_entries : 0), pieces);
   if (grid.x == 0) return fe_last_error();
-  const int rc = wide ? fe_launch_dependent(delta_prepare_kernel<4>, grid, dim3(32 * DP_WARPS), smem, stream, p, inner)
-                      : fe_launch_dependent(delta_prepare_kernel<1>, grid, dim3(32 * DP_WARPS), smem, stream, p, inner);
+  const int rc = wide ? fe_launch_dependent(delta_prepare_kernel<4>, grid, dim3(32 * DP_WARPS), smem, stream, p, n_tokens)
+                      : fe_launch_dependent(delta_prepare_kernel<1>, grid, dim3(32 * DP_WARPS), smem, stream, p, n_tokens);
   return rc ? rc : fe_last_error();
 }
 
@@ -265,7 +277,8 @@ struct Delta {
   int kv_heads, per;        // q/k heads; heads per q/k head
   const float* gates;       // [tokens, heads, 2]
   // chunk-parallel scratch, per (slot, head)
-  float* w;                 // [dk][SR_LONG]: W transposed
+  bf16* w;                  // [3][dk16][SR_LONG]: W transposed, split in three (mma_split.cuh); rows past dk are zero
+  bf16* k;                  // [3][SR_LONG][dk16]: the keys, split; of the first head of those that share them
   float* u;                 // [SR_LONG][dv]: U, then (chain) u
   float* before;            // [dk, dv]: the state before the chunk
   float* decays;            // [SR_LONG + 4]: e^(c_end - c_t) per token, then e^(c_end)
@@ -357,7 +370,8 @@ struct Delta {
 // thread per column solves the 16 x 16 triangle in registers and stores the result, also for the blocks
 // below.  The products (L itself, and a block's from the rows before it) run on the tensor cores, both
 // operands split; what remains is the triangles, one row after the other, and the loads before them.  Solve, chain and
-// outputs of 2,048 tokens, 32 heads of 64 channels: 307 us, 371 with tiles of multiply-adds; 3 prompts of 1,000 to 666 tokens,
+// outputs of 2,048 tokens, 32 heads of 64 channels: 263 us (307 before a warp's loads of the values went out together and W was
+// split here for the chain), 371 with tiles of multiply-adds; 3 prompts of 1,000 to 666 tokens,
 // heads of 128: 971 and 1,062; outputs' error against 64 bits 1.3e-7 and 1.9e-7, 1.3e-7 and 2.3e-7.
 #define DS_THREADS 256
 // Columns of the right sides: k in fours, then v, in eights altogether.
@@ -396,13 +410,22 @@ __global__ void __launch_bounds__(DS_THREADS) delta_solve_kernel(const Delta m, 
   __syncthreads();
   // the right sides: rows of beta e^c k and beta v, zero past the last token and between the two
   const int warp = tid >> 5, lane = tid & 31;
-  for (int t = warp; t < SR_LONG; t += DS_THREADS / 32) {
-    const bool has = t < at.count;
-    const float a = be[t], b = bt[t];
-    float* x = X + t * ldx;
-    for (int d = lane; d < v0; d += 32) x[d] = d < dk ? a * kt[d * SR_TP + t] : 0.f;
-    for (int d = lane; d < columns - v0; d += 32) x[v0 + d] = has && d < dv ? b * values.row(t)[d] : 0.f;
+  constexpr int ROWS = SR_LONG * 32 / DS_THREADS;       // of a warp: their loads are all on their way before the first is used
+  for (int d = lane; d < columns - v0; d += 32) {
+    float x[ROWS];
+#pragma unroll
+    for (int u = 0; u < ROWS; ++u) {
+      const int t = warp + u * (DS_THREADS / 32);
+      x[u] = t < at.count && d < dv ? values.row(t)[d] : 0.f;
+    }
+#pragma unroll
+    for (int u = 0; u < ROWS; ++u) {
+      const int t = warp + u * (DS_THREADS / 32);
+      X[t * ldx + v0 + d] = bt[t] * x[u];
+    }
   }
+  for (int t = warp; t < SR_LONG; t += DS_THREADS / 32)
+    for (int d = lane; d < v0; d += 32) X[t * ldx + d] = d < dk ? be[t] * kt[d * SR_TP + t] : 0.f;
   const int fg = lane >> 2, fq = lane & 3;
   {
     const int m0 = (warp >> 2) * 32, n0 = (warp & 3) * 16;
@@ -420,6 +443,21 @@ __global__ void __launch_bounds__(DS_THREADS) delta_solve_kernel(const Delta m, 
         }
   }
   const size_t cell = m.cell(p, at, head);
+  const int dk16 = (dk + 15) & ~15;
+  if (head % m.per == 0) {
+    const int pairs = dk16 >> 1, plane = SR_LONG * dk16;
+    unsigned* dst = reinterpret_cast<unsigned*>(m.k + cell * 3 * plane);
+    for (int i = tid; i < SR_LONG * pairs; i += DS_THREADS) {
+      const int t = i / pairs, d = 2 * (i - t * pairs);
+      unsigned a, b, c3;
+      split_pair(d < dk8 ? kt[d * SR_TP + t] : 0.f, d < dk8 ? kt[(d + 1) * SR_TP + t] : 0.f, a, b, c3);
+      dst[i] = a, dst[i + plane / 2] = b, dst[i + plane] = c3;
+    }
+  }
+  for (int i = tid; i < 3 * (dk16 - dk) * SR_LONG; i += DS_THREADS) {
+    const int part = i / ((dk16 - dk) * SR_LONG), at_row = i - part * (dk16 - dk) * SR_LONG;
+    m.w[(cell * 3 + part) * dk16 * SR_LONG + dk * SR_LONG + at_row] = __float2bfloat16_rn(0.f);
+  }
   for (int r0 = 0; r0 < SR_LONG; r0 += 16) {
     __syncthreads();
     if (r0 > 0) {
@@ -461,9 +499,17 @@ __global__ void __launch_bounds__(DS_THREADS) delta_solve_kernel(const Delta m, 
 #pragma unroll
       for (int t = 0; t < 16; ++t) X[(r0 + t) * ldx + i] = x[t];
       if (i < dk) {
-        float* dst = m.w + (cell * dk + i) * SR_LONG + r0;
+        bf16* dst = m.w + (cell * 3 * dk16 + i) * SR_LONG + r0;
 #pragma unroll
-        for (int t = 0; t < 16; t += 4) store4(dst + t, x + t);
+        for (int h = 0; h < 2; ++h) {
+          uint4 part[3];
+          split_pair(x[8 * h], x[8 * h + 1], part[0].x, part[1].x, part[2].x);
+          split_pair(x[8 * h + 2], x[8 * h + 3], part[0].y, part[1].y, part[2].y);
+          split_pair(x[8 * h + 4], x[8 * h + 5], part[0].z, part[1].z, part[2].z);
+          split_pair(x[8 * h + 6], x[8 * h + 7], part[0].w, part[1].w, part[2].w);
+#pragma unroll
+          for (int u = 0; u < 3; ++u) *reinterpret_cast<uint4*>(dst + (size_t)u * dk16 * SR_LONG + 8 * h) = part[u];
+        }
       } else if (i >= v0 && i - v0 < dv) {
         float* dst = m.u + (cell * SR_LONG + r0) * dv + (i - v0);
 #pragma unroll
@@ -476,16 +522,18 @@ __global__ void __launch_bounds__(DS_THREADS) delta_solve_kernel(const Delta m, 
 // The chain over an entry's chunks for one head and COLS value columns: u = U - W S, then
 // S <- e^(c_end) S + sum_j k_j (e^(c_end - c_j) u_j)^T.  What bounds it is one chunk's two products after the
 // other, so they run on the tensor cores with both operands split (mma_split.cuh): a warp takes 16 x 8
-// outputs, reads 48 numbers a lane where a 4 x 2 tile of multiply-adds read 192, and a chunk has two
-// barriers.  The state's columns stay in registers, as the warps' pieces of the second product, and in shared
-// memory for the first; the next chunk's W and keys, and what a lane needs of it besides, are on their way
-// while a chunk is worked on.
-#define DC_WP (SR_LONG + 8)          // pitches: the rows of a fragment fall into different banks
-template <int KD, int COLS>
+// outputs.  delta_solve has split W and the keys, which the blocks of a head's columns all read; the state and the
+// weighted u are split once by the lanes that hold them.  2,048 tokens, 32 heads of 64: 127 us with every warp
+// splitting what it multiplied, 96 us now.  The state's columns stay in registers, as the warps' pieces of the
+// second product, and in shared memory for the first.  Tiles (W and keys of each chunk in turn) go round SLOTS places: the next
+// SLOTS - 1 are on their way while one is worked on.
+#define DC_WP (SR_LONG + 8)          // pitches: the rows of a matrix fall into different banks
+__host__ __device__ static inline int dc_tile(int dk16) { return dk16 * DC_WP > SR_LONG * (dk16 + 8) ? dk16 * DC_WP : SR_LONG * (dk16 + 8); }
+template <int KD, int COLS, int SLOTS>
 __global__ void __launch_bounds__(16 * COLS) delta_chain_kernel(const Delta m, const StateRun p, int* status) {
   extern __shared__ __align__(16) float smem[];
   pdl_wait();
-  constexpr int KP = 64 * KD + 8, SP = COLS + 8, THREADS = 16 * COLS, WARPS = THREADS / 32;
+  constexpr int SP = COLS + 8, THREADS = 16 * COLS;
   const int head = blockIdx.x, entry = blockIdx.y, col0 = blockIdx.z * COLS, tid = threadIdx.x;
   const int first = p.cu_tokens[entry], count = p.cu_tokens[entry + 1] - first;
   if (count < p.long_from) return;
@@ -494,12 +542,12 @@ __global__ void __launch_bounds__(16 * COLS) delta_chain_kernel(const Delta m, c
     if (tid == 0 && blockIdx.z == 0) atomicOr(status, FE_STATUS_BAD_PAGE);
     return;
   }
-  const int dk = p.dk, dv = p.dv, dk8 = (dk + 7) & ~7, half = dk8 * DC_WP + SR_LONG * KP;
-  float* S = smem;                           // [64 KD][SP]
-  float* us = S + 64 * KD * SP;              // [SR_LONG][SP], weighted
-  float* buffers = us + SR_LONG * SP;        // 2 x (W transposed [dk8][DC_WP], keys [SR_LONG][KP])
+  const int dk = p.dk, dv = p.dv, dk16 = (dk + 15) & ~15, KP = dk16 + 8, tile = dc_tile(dk16);
+  bf16* S = reinterpret_cast<bf16*>(smem);   // [3][dk16][SP]
+  bf16* us = S + 3 * dk16 * SP;              // [3][SR_LONG][SP], weighted
+  bf16* tiles = us + 3 * SR_LONG * SP;       // SLOTS x 3 planes: W transposed [dk16][DC_WP] or keys [SR_LONG][KP]
   const int lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
-  const int t0 = 16 * (warp & 3) + g, n0 = 8 * (warp >> 2);        // first row and columns of this warp's pieces
+  const int m0 = 16 * (warp & 3), t0 = m0 + g, n0 = 8 * (warp >> 2);        // first row and columns of this warp's pieces
   const int col = col0 + n0 + 2 * q;                               // this lane's two columns
   const bool in0 = col < dv, in1 = col + 1 < dv, pair = in1 && (dv & 1) == 0;
   auto load2 = [&](const float* at, float& a, float& b) {
@@ -519,30 +567,27 @@ __global__ void __launch_bounds__(16 * COLS) delta_chain_kernel(const Delta m, c
       const int d = 64 * kd + t0 + 8 * h;
       s[kd][h][0] = s[kd][h][1] = 0.f;
       if (d < dk) load2(st + (size_t)d * dv, s[kd][h][0], s[kd][h][1]);
-      *reinterpret_cast<float2*>(S + d * SP + n0 + 2 * q) = make_float2(s[kd][h][0], s[kd][h][1]);
+      if (d < dk16) planes_store2(S + d * SP + n0 + 2 * q, dk16 * SP, s[kd][h][0], s[kd][h][1]);
     }
-  for (int i = tid; i < 2 * half; i += THREADS) buffers[i] = 0.f;      // channels past dk stay zero
-  __syncthreads();
   const int chunks = (count + SR_LONG - 1) / SR_LONG;
-  const size_t cell0 = (size_t)sr_slot(first, entry, 0) * p.heads + head;
-  const Rows keys{m.k_row(p, head, first), m.ld};
-  const bool wide = keys.wide(dk);
-  auto fetch = [&](int chunk, float* buf) {
-    const float* w = m.w + (cell0 + (size_t)chunk * p.heads) * dk * SR_LONG + (tid & 15) * 4;
-    float* to = buf + (tid & 15) * 4;
+  const size_t cell0 = (size_t)sr_slot(first, entry, 0) * p.heads + head, group0 = cell0 - head % m.per;
+  const int kcol = dk16 >> 3;                // 16-byte pieces of a row of keys
+  auto fetch = [&](int i) {                  // tile i: W of chunk i / 2, or its keys
+    if (i < 2 * chunks) {
+      bf16* to = tiles + (i % SLOTS) * 3 * tile;
+      const int chunk = i >> 1;
+      if ((i & 1) == 0) {
+        const bf16* from = m.w + (cell0 + (size_t)chunk * p.heads) * 3 * dk16 * SR_LONG;
+        for (int u = 0; u < 3; ++u)
 #pragma unroll 4
-    for (int d = tid >> 4; d < dk; d += THREADS / 16) sr_copy16(to + d * DC_WP, w + d * SR_LONG);
-    const int rows = min(SR_LONG, count - chunk * SR_LONG);
-    float* ks = buf + dk8 * DC_WP;
-#pragma unroll 4
-    for (int t = warp; t < SR_LONG; t += WARPS) {
-      float* dst = ks + t * KP;
-      if (t >= rows) {
-        for (int d = lane; d < dk; d += 32) dst[d] = 0.f;
-      } else if (wide) {
-        for (int d = 4 * lane; d < dk; d += 128) sr_copy16(dst + d, keys.row(chunk * SR_LONG + t) + d);
+          for (int r = tid >> 3; r < dk16; r += THREADS / 8)
+            sr_copy16(to + u * tile + r * DC_WP + (tid & 7) * 8, from + ((size_t)u * dk16 + r) * SR_LONG + (tid & 7) * 8);
       } else {
-        for (int d = lane; d < dk; d += 32) sr_copy4(dst + d, keys.row(chunk * SR_LONG + t) + d);
+        const bf16* from = m.k + (group0 + (size_t)chunk * p.heads) * 3 * dk16 * SR_LONG;
+        for (int u = 0; u < 3; ++u)
+#pragma unroll 4
+          for (int t = tid >> 3; t < SR_LONG; t += THREADS / 8)
+            for (int c = tid & 7; c < kcol; c += 8) sr_copy16(to + u * tile + t * KP + c * 8, from + ((size_t)u * SR_LONG + t) * dk16 + c * 8);
       }
     }
     sr_copy_commit();
@@ -558,15 +603,15 @@ __global__ void __launch_bounds__(16 * COLS) delta_chain_kernel(const Delta m, c
       load2(m.u + (cell * SR_LONG + t0 + 8 * h) * dv + col, x[h][0], x[h][1]);
     }
   };
-  fetch(0, buffers);
+#pragma unroll
+  for (int i = 0; i + 1 < SLOTS; ++i) fetch(i);
   ask(0);
   for (int chunk = 0; chunk < chunks; ++chunk) {
     const size_t cell = cell0 + (size_t)chunk * p.heads;
-    const float* buf = buffers + (chunk & 1) * half;
     if (chunk + 1 == chunks) pdl_trigger();    // state_out's blocks would only lie beside this one's till then
-    sr_copy_wait<0>();
-    __syncthreads();           // this chunk's tiles have landed, the state is whole; everyone is done with the other buffer
-    if (chunk + 1 < chunks) fetch(chunk + 1, buffers + ((chunk + 1) & 1) * half);
+    sr_copy_wait<SLOTS - 2>();
+    __syncthreads();           // W has landed, the state is whole; everyone is done with the keys before
+    fetch(2 * chunk + SLOTS - 1);
     // the state before the chunk, for state_out
     float* before = m.before + cell * dk * dv + col;
 #pragma unroll
@@ -577,46 +622,48 @@ __global__ void __launch_bounds__(16 * COLS) delta_chain_kernel(const Delta m, c
         if (d < dk) store2(before + (size_t)d * dv, s[kd][h][0], s[kd][h][1]);
       }
     {
-      float sum[4] = {0.f, 0.f, 0.f, 0.f}, small[4] = {0.f, 0.f, 0.f, 0.f};
-      const float* a = buf + q * DC_WP + t0;
-      const float* b = S + q * SP + n0 + g;
-#pragma unroll 8
-      for (int d = 0; d < dk8; d += 8) {
-        SplitA fa;
-        SplitB fb;
-        split_load_a(fa, a + d * DC_WP, 1, DC_WP);
-        split_load_b(fb, b + d * SP, SP);
+      float sum[4] = {}, small[5][4] = {};
+      const bf16* a = tiles + (2 * chunk % SLOTS) * 3 * tile + m0;
+      const bf16* b = S + n0;
+#pragma unroll 4
+      for (int d = 0; d < dk16; d += 16) {
+        PlanesA fa;
+        PlanesB fb;
+        planes_load_a_by_k(fa, a + d * DC_WP, DC_WP, tile);
+        planes_load_b_by_k(fb, b + d * SP, SP, dk16 * SP);
         split_mma(sum, small, fa, fb);
       }
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        x[h][0] -= split_join(sum[2 * h], small[2 * h]);
-        x[h][1] -= split_join(sum[2 * h + 1], small[2 * h + 1]);
-        *reinterpret_cast<float2*>(us + (t0 + 8 * h) * SP + n0 + 2 * q) = make_float2(x[h][0] * w[h], x[h][1] * w[h]);
+        x[h][0] -= split_join(sum[2 * h], small, 2 * h);
+        x[h][1] -= split_join(sum[2 * h + 1], small, 2 * h + 1);
+        planes_store2(us + (t0 + 8 * h) * SP + n0 + 2 * q, SR_LONG * SP, x[h][0] * w[h], x[h][1] * w[h]);
         store2(m.u + (cell * SR_LONG + t0 + 8 * h) * dv + col, x[h][0], x[h][1]);
       }
     }
     const float decay = keep;
-    __syncthreads();
+    sr_copy_wait<SLOTS - 2>();
+    __syncthreads();           // the keys have landed, u is whole; everyone is done with W
+    fetch(2 * chunk + SLOTS);
     if (chunk + 1 < chunks) ask(chunk + 1);
-    const float* b = us + q * SP + n0 + g;
+    const bf16* a = tiles + ((2 * chunk + 1) % SLOTS) * 3 * tile + m0;
 #pragma unroll
     for (int kd = 0; kd < KD; ++kd) {
-      float sum[4] = {0.f, 0.f, 0.f, 0.f}, small[4] = {0.f, 0.f, 0.f, 0.f};
-      const float* a = buf + dk8 * DC_WP + q * KP + 64 * kd + t0;
+      if (64 * kd + m0 >= dk16) break;
+      float sum[4] = {}, small[5][4] = {};
 #pragma unroll
-      for (int t = 0; t < SR_LONG; t += 8) {
-        SplitA fa;
-        SplitB fb;
-        split_load_a(fa, a + t * KP, 1, KP);
-        split_load_b(fb, b + t * SP, SP);
+      for (int t = 0; t < SR_LONG; t += 16) {
+        PlanesA fa;
+        PlanesB fb;
+        planes_load_a_by_k(fa, a + t * KP + 64 * kd, KP, tile);
+        planes_load_b_by_k(fb, us + t * SP + n0, SP, SR_LONG * SP);
         split_mma(sum, small, fa, fb);
       }
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        s[kd][h][0] = fmaf(decay, s[kd][h][0], split_join(sum[2 * h], small[2 * h]));
-        s[kd][h][1] = fmaf(decay, s[kd][h][1], split_join(sum[2 * h + 1], small[2 * h + 1]));
-        *reinterpret_cast<float2*>(S + (64 * kd + t0 + 8 * h) * SP + n0 + 2 * q) = make_float2(s[kd][h][0], s[kd][h][1]);
+        s[kd][h][0] = fmaf(decay, s[kd][h][0], split_join(sum[2 * h], small, 2 * h));
+        s[kd][h][1] = fmaf(decay, s[kd][h][1], split_join(sum[2 * h + 1], small, 2 * h + 1));
+        planes_store2(S + (64 * kd + t0 + 8 * h) * SP + n0 + 2 * q, dk16 * SP, s[kd][h][0], s[kd][h][1]);
       }
     }
   }
@@ -634,21 +681,23 @@ static size_t delta_solve_smem(int dk, int dv) {
 }
 // Value columns of a block of delta_chain: few where the heads are small, so that there are more blocks.
 static int delta_chain_cols(int dv) { return dv <= 64 ? 16 : 32; }
+// Places of its ring of tiles: what shared memory holds of the next chunk.
+static int delta_chain_slots(int dk) { return dk <= 64 ? 4 : dk <= 128 ? 3 : 2; }
 static size_t delta_chain_smem(int dk, int cols) {
-  const size_t kp = (size_t)(dk + 63) / 64 * 64, dk8 = (size_t)(dk + 7) / 8 * 8, sp = cols + 8;
-  return sizeof(float) * ((kp + SR_LONG) * sp + 2 * (dk8 * DC_WP + SR_LONG * (kp + 8)));
+  const int dk16 = (dk + 15) & ~15;
+  return sizeof(bf16) * 3 * ((size_t)(dk16 + SR_LONG) * (cols + 8) + (size_t)delta_chain_slots(dk) * dc_tile(dk16));
 }
-// Keys of up to 176 numbers with 16 columns a block and up to 152 with 32: what shared memory holds of a chunk and the
-// next one.  (The instantiations would reach 192.)
+// Keys of up to 176 numbers with 16 columns a block and up to 152 with 32; longer ones are walked.
 static bool delta_chunk_takes(int dk, int dv) {
-  return dk <= 192 && chunk_takes(dk, dv, true) && delta_solve_smem(dk, dv) <= 218 * 1024 &&
+  return dk <= (delta_chain_cols(dv) == 16 ? 176 : 152) && chunk_takes(dk, dv, true) && delta_solve_smem(dk, dv) <= 218 * 1024 &&
          delta_chain_smem(dk, delta_chain_cols(dv)) <= 226 * 1024;
 }
 
 FE_EXPORT long long fe_delta_rule_scratch(int tokens, int entries, int heads, int dk, int dv, int max_new) {
   const long long need = walk_in_stretches(dk, dv, 0) ? (long long)tokens * heads * dv : 0;
   if (max_new < SR_LONG_FROM || !delta_chunk_takes(dk, dv)) return need;
-  return (need + 3) / 4 * 4 + sr_slots(tokens, entries) * heads * ((long long)dk * SR_LONG + (long long)SR_LONG * dv + (long long)dk * dv + SR_LONG + 4);
+  return (need + 3) / 4 * 4 + sr_slots(tokens, entries) * heads *
+             (3LL * ((dk + 15) / 16 * 16) * SR_LONG + (long long)SR_LONG * dv + (long long)dk * dv + SR_LONG + 4);
 }
 
 FE_EXPORT int fe_delta_rule(const float* qkv, long long ld, const float* gates, const float* gate, long long gate_ld,
@@ -658,7 +707,7 @@ FE_EXPORT int fe_delta_rule(const float* qkv, long long ld, const float* gates, 
   if (entries <= 0 || tokens <= 0) return 0;
   if (heads < 1 || kv_heads < 1 || heads % kv_heads || dk < 1 || dv < 1 || heads > 65535 || entries > 65535) return FE_ERR_BAD_SHAPE;
   StateRun p{state, state_rows, slots, cu_tokens, heads, dk, dv, 0, qkv + 2 * kv_heads * dk, ld, norm_w, 0, gate, gate_ld, 0, eps, out, nullptr, 0};
-  Delta m{qkv, ld, kv_heads, heads / kv_heads, gates, nullptr, nullptr, nullptr, nullptr};
+  Delta m{qkv, ld, kv_heads, heads / kv_heads, gates, nullptr, nullptr, nullptr, nullptr, nullptr};
   if (walk_in_stretches(dk, dv, 0)) {
     p.raw = scratch;
     scratch = scratch ? scratch + ((size_t)tokens * heads * dv + 3) / 4 * 4 : nullptr;
@@ -670,8 +719,10 @@ FE_EXPORT int fe_delta_rule(const float* qkv, long long ld, const float* gates, 
   const int chunks = (max_new + SR_LONG - 1) / SR_LONG;
   if (chunks > 65535) return FE_ERR_TOO_LARGE;
   const size_t cells = (size_t)sr_slots(tokens, entries) * heads;
-  m.w = scratch;
-  m.u = m.w + cells * dk * SR_LONG;
+  const size_t planes = cells * 3 * ((dk + 15) / 16 * 16) * SR_LONG;
+  m.w = reinterpret_cast<bf16*>(scratch);
+  m.k = m.w + planes;
+  m.u = scratch + planes;
   m.decays = m.u + cells * SR_LONG * dv;
   m.before = m.decays + cells * (SR_LONG + 4);
   size_t smem = delta_solve_smem(dk, dv);
@@ -684,17 +735,17 @@ FE_EXPORT int fe_delta_rule(const float* qkv, long long ld, const float* gates, 
   const int cols = delta_chain_cols(dv);
   smem = delta_chain_smem(dk, cols);
   const dim3 chain(heads, entries, (dv + cols - 1) / cols);
-#define DC_LAUNCH(KD, COLS)                                                                                       \
-  do {                                                                                                            \
-    cudaFuncSetAttribute(delta_chain_kernel<KD, COLS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);   \
-    delta_chain_kernel<KD, COLS><<<chain, 16 * COLS, smem, stream>>>(m, p, status);                               \
-    rc = fe_last_error();                                                                                         \
+#define DC_LAUNCH(KD, COLS, SLOTS)                                                                                     \
+  do {                                                                                                                 \
+    cudaFuncSetAttribute(delta_chain_kernel<KD, COLS, SLOTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+    delta_chain_kernel<KD, COLS, SLOTS><<<chain, 16 * COLS, smem, stream>>>(m, p, status);                             \
+    rc = fe_last_error();                                                                                              \
   } while (0)
-#define DC_BY_DK(COLS)                 \
-  do {                                 \
-    if (dk <= 64) DC_LAUNCH(1, COLS);  \
-    else if (dk <= 128) DC_LAUNCH(2, COLS); \
-    else DC_LAUNCH(3, COLS);           \
+#define DC_BY_DK(COLS)                       \
+  do {                                       \
+    if (dk <= 64) DC_LAUNCH(1, COLS, 4);     \
+    else if (dk <= 128) DC_LAUNCH(2, COLS, 3); \
+    else DC_LAUNCH(3, COLS, 2);              \
   } while (0)
   if (cols == 16) DC_BY_DK(16);
   else DC_BY_DK(32);

@@ -85,3 +85,51 @@ __device__ __forceinline__ void split_mma(float (&sum)[4], float (&small)[4], co
   split_mma_raw(small, a.part[2], a2.part[2], b.part[0], b2.part[0]);
 }
 __device__ __forceinline__ float split_join(float sum, float small) { return sum + small; }
+
+// Tiles that are split once, by whoever writes them: three planes of bfloat16, `plane` numbers apart, rows a multiple of 16
+// bytes apart (an odd one: then the eight rows of a matrix fall into different banks).  A fragment of sixteen k, k
+// 2 q and 2 q + 1 of a lane in the low and high half of a register.
+struct PlanesA { unsigned part[3][4]; };
+struct PlanesB { unsigned part[3][2]; };
+__device__ __forceinline__ unsigned split_address(const bf16* p) { return (unsigned)__cvta_generic_to_shared(p); }
+// A[m][k], 16 x 16, at a[k * pitch + m].
+__device__ __forceinline__ void planes_load_a_by_k(PlanesA& f, const bf16* a, int pitch, int plane) {
+  const int lane = threadIdx.x & 31;
+  const unsigned at = split_address(a + ((lane >> 4) * 8 + (lane & 7)) * pitch + ((lane >> 3) & 1) * 8);
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(f.part[i][0]), "=r"(f.part[i][1]), "=r"(f.part[i][2]), "=r"(f.part[i][3]) : "r"(at + 2 * i * plane) : "memory");
+}
+// B[k][n], 16 x 8, at b[k * pitch + n].
+__device__ __forceinline__ void planes_load_b_by_k(PlanesB& f, const bf16* b, int pitch, int plane) {
+  const unsigned at = split_address(b + (threadIdx.x & 15) * pitch);
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+    asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0, %1}, [%2];"
+                 : "=r"(f.part[i][0]), "=r"(f.part[i][1]) : "r"(at + 2 * i * plane) : "memory");
+}
+// Two neighbouring numbers of a row into the planes.
+__device__ __forceinline__ void planes_store2(bf16* to, int plane, float x, float y) {
+  unsigned a, b, c;
+  split_pair(x, y, a, b, c);
+  *reinterpret_cast<unsigned*>(to) = a;
+  *reinterpret_cast<unsigned*>(to + plane) = b;
+  *reinterpret_cast<unsigned*>(to + 2 * plane) = c;
+}
+// The small products of each kind in an accumulator of their own: where little else runs, a chain of them is what is waited for.
+__device__ __forceinline__ void split_mma(float (&sum)[4], float (&small)[5][4], const PlanesA& a, const PlanesB& b) {
+  const unsigned lo[2] = {a.part[0][0], a.part[0][1]}, hi[2] = {a.part[0][2], a.part[0][3]};
+  const unsigned lo1[2] = {a.part[1][0], a.part[1][1]}, hi1[2] = {a.part[1][2], a.part[1][3]};
+  const unsigned lo2[2] = {a.part[2][0], a.part[2][1]}, hi2[2] = {a.part[2][2], a.part[2][3]};
+  split_mma_large(sum, lo, b.part[0][0]);
+  split_mma_large(sum, hi, b.part[0][1]);
+  split_mma_raw(small[0], lo, hi, b.part[1][0], b.part[1][1]);
+  split_mma_raw(small[1], lo1, hi1, b.part[0][0], b.part[0][1]);
+  split_mma_raw(small[2], lo1, hi1, b.part[1][0], b.part[1][1]);
+  split_mma_raw(small[3], lo, hi, b.part[2][0], b.part[2][1]);
+  split_mma_raw(small[4], lo2, hi2, b.part[0][0], b.part[0][1]);
+}
+__device__ __forceinline__ float split_join(float sum, const float (&small)[5][4], int i) {
+  return sum + ((small[0][i] + small[1][i]) + ((small[3][i] + small[4][i]) + small[2][i]));
+}

@@ -302,7 +302,7 @@ __device__ __forceinline__ uint64_t sr_mul2(uint64_t a, uint64_t b) {
 }
 
 // Copies of 16 or 4 bytes into shared memory that complete in the background.
-__device__ __forceinline__ void sr_copy16(float* dst, const float* src) {
+__device__ __forceinline__ void sr_copy16(void* dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
 }
 __device__ __forceinline__ void sr_copy4(float* dst, const float* src) {
