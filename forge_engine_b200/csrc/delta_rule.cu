@@ -277,8 +277,8 @@ struct Delta {
   int kv_heads, per;        // q/k heads; heads per q/k head
   const float* gates;       // [tokens, heads, 2]
   // chunk-parallel scratch, per (slot, head)
-  bf16* w;                  // [3][dk16][SR_LONG]: W transposed, split in three (mma_split.cuh); rows past dk are zero
-  bf16* k;                  // [3][SR_LONG][dk16]: the keys, split; of the first head of those that share them
+  bf16* w;                  // tiles of W transposed, split in three (mma_split.cuh); rows past dk are zero
+  bf16* k;                  // tiles of keys, split; of the first head of those that share them
   float* u;                 // [SR_LONG][dv]: U, then (chain) u
   float* before;            // [dk, dv]: the state before the chunk
   float* decays;            // [SR_LONG + 4]: e^(c_end - c_t) per token, then e^(c_end)
@@ -365,23 +365,29 @@ struct Delta {
   }
 };
 
+// A tile of the chain, as it lies in memory and in shared memory: three planes of W transposed [dk16][DC_WP] or of keys
+// [SR_LONG][dk16 + 8]; the pitches let the rows of a matrix fall into different banks.
+#define DC_WP (SR_LONG + 8)
+__host__ __device__ static constexpr int dc_tile(int dk16) { return dk16 * DC_WP > SR_LONG * (dk16 + 8) ? dk16 * DC_WP : SR_LONG * (dk16 + 8); }
+
 // W and U of one chunk of one head: the triangular system solved for the columns of beta e^c k
 // and beta v, sixteen rows at a time.  A block of rows first loses what the rows before it give, then a
 // thread per column solves the 16 x 16 triangle in registers and stores the result, also for the blocks
 // below.  The products (L itself, and a block's from the rows before it) run on the tensor cores, both
 // operands split; what remains is the triangles, one row after the other, and the loads before them.  Solve, chain and
-// outputs of 2,048 tokens, 32 heads of 64 channels: 263 us (307 before a warp's loads of the values went out together and W was
-// split here for the chain), 371 with tiles of multiply-adds; 3 prompts of 1,000 to 666 tokens,
+// outputs of 2,048 tokens, 32 heads of 64 channels: 214 us (307 before a warp's loads of the values went out together, W was
+// split here for the chain and sizes of 64 and 128 were known when compiled), 371 with tiles of multiply-adds; 3 prompts of 1,000 to 666 tokens,
 // heads of 128: 971 and 1,062; outputs' error against 64 bits 1.3e-7 and 1.9e-7, 1.3e-7 and 2.3e-7.
 #define DS_THREADS 256
 // Columns of the right sides: k in fours, then v, in eights altogether.
 __host__ __device__ static inline int ds_columns(int dk, int dv) { return (((dk + 3) & ~3) + dv + 7) & ~7; }
+template <int D>       // head sizes of both sides known when compiled; 0: any
 __global__ void __launch_bounds__(DS_THREADS) delta_solve_kernel(const Delta m, const StateRun p) {
   extern __shared__ __align__(16) float smem[];
   pdl_wait();
   ChunkAt at;
   if (!sr_locate(p, &at)) return;
-  const int head = blockIdx.x, dk = p.dk, dv = p.dv, tid = threadIdx.x;
+  const int head = blockIdx.x, dk = D ? D : p.dk, dv = D ? D : p.dv, tid = threadIdx.x;
   const int v0 = (dk + 3) & ~3, columns = ds_columns(dk, dv), ldx = columns + 8, dk8 = (dk + 7) & ~7;      // columns of k, then of v
   __shared__ double c[SR_LONG];
   __shared__ float bt[SR_LONG], be[SR_LONG];
@@ -443,20 +449,18 @@ __global__ void __launch_bounds__(DS_THREADS) delta_solve_kernel(const Delta m, 
         }
   }
   const size_t cell = m.cell(p, at, head);
-  const int dk16 = (dk + 15) & ~15;
+  const int dk16 = (dk + 15) & ~15, tile = dc_tile(dk16);
   if (head % m.per == 0) {
-    const int pairs = dk16 >> 1, plane = SR_LONG * dk16;
-    unsigned* dst = reinterpret_cast<unsigned*>(m.k + cell * 3 * plane);
+    const int pairs = dk16 >> 1;
+    bf16* dst = m.k + cell * 3 * tile;
     for (int i = tid; i < SR_LONG * pairs; i += DS_THREADS) {
       const int t = i / pairs, d = 2 * (i - t * pairs);
-      unsigned a, b, c3;
-      split_pair(d < dk8 ? kt[d * SR_TP + t] : 0.f, d < dk8 ? kt[(d + 1) * SR_TP + t] : 0.f, a, b, c3);
-      dst[i] = a, dst[i + plane / 2] = b, dst[i + plane] = c3;
+      planes_store2(dst + t * (dk16 + 8) + d, tile, d < dk8 ? kt[d * SR_TP + t] : 0.f, d < dk8 ? kt[(d + 1) * SR_TP + t] : 0.f);
     }
   }
   for (int i = tid; i < 3 * (dk16 - dk) * SR_LONG; i += DS_THREADS) {
-    const int part = i / ((dk16 - dk) * SR_LONG), at_row = i - part * (dk16 - dk) * SR_LONG;
-    m.w[(cell * 3 + part) * dk16 * SR_LONG + dk * SR_LONG + at_row] = __float2bfloat16_rn(0.f);
+    const int part = i / ((dk16 - dk) * SR_LONG), r = (i / SR_LONG) % (dk16 - dk);
+    m.w[(cell * 3 + part) * tile + (dk + r) * DC_WP + i % SR_LONG] = __float2bfloat16_rn(0.f);
   }
   for (int r0 = 0; r0 < SR_LONG; r0 += 16) {
     __syncthreads();
@@ -499,7 +503,7 @@ __global__ void __launch_bounds__(DS_THREADS) delta_solve_kernel(const Delta m, 
 #pragma unroll
       for (int t = 0; t < 16; ++t) X[(r0 + t) * ldx + i] = x[t];
       if (i < dk) {
-        bf16* dst = m.w + (cell * 3 * dk16 + i) * SR_LONG + r0;
+        bf16* dst = m.w + cell * 3 * tile + i * DC_WP + r0;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           uint4 part[3];
@@ -508,7 +512,7 @@ __global__ void __launch_bounds__(DS_THREADS) delta_solve_kernel(const Delta m, 
           split_pair(x[8 * h + 4], x[8 * h + 5], part[0].z, part[1].z, part[2].z);
           split_pair(x[8 * h + 6], x[8 * h + 7], part[0].w, part[1].w, part[2].w);
 #pragma unroll
-          for (int u = 0; u < 3; ++u) *reinterpret_cast<uint4*>(dst + (size_t)u * dk16 * SR_LONG + 8 * h) = part[u];
+          for (int u = 0; u < 3; ++u) *reinterpret_cast<uint4*>(dst + u * tile + 8 * h) = part[u];
         }
       } else if (i >= v0 && i - v0 < dv) {
         float* dst = m.u + (cell * SR_LONG + r0) * dv + (i - v0);
@@ -524,12 +528,10 @@ __global__ void __launch_bounds__(DS_THREADS) delta_solve_kernel(const Delta m, 
 // other, so they run on the tensor cores with both operands split (mma_split.cuh): a warp takes 16 x 8
 // outputs.  delta_solve has split W and the keys, which the blocks of a head's columns all read; the state and the
 // weighted u are split once by the lanes that hold them.  2,048 tokens, 32 heads of 64: 127 us with every warp
-// splitting what it multiplied, 96 us now.  The state's columns stay in registers, as the warps' pieces of the
+// splitting what it multiplied, 96 us with split tiles, 58 us with whole copies of them and sizes known when compiled.  The state's columns stay in registers, as the warps' pieces of the
 // second product, and in shared memory for the first.  Tiles (W and keys of each chunk in turn) go round SLOTS places: the next
 // SLOTS - 1 are on their way while one is worked on.
-#define DC_WP (SR_LONG + 8)          // pitches: the rows of a matrix fall into different banks
-__host__ __device__ static inline int dc_tile(int dk16) { return dk16 * DC_WP > SR_LONG * (dk16 + 8) ? dk16 * DC_WP : SR_LONG * (dk16 + 8); }
-template <int KD, int COLS, int SLOTS>
+template <int KD, int COLS, int SLOTS, bool WHOLE>
 __global__ void __launch_bounds__(16 * COLS) delta_chain_kernel(const Delta m, const StateRun p, int* status) {
   extern __shared__ __align__(16) float smem[];
   pdl_wait();
@@ -542,14 +544,14 @@ __global__ void __launch_bounds__(16 * COLS) delta_chain_kernel(const Delta m, c
     if (tid == 0 && blockIdx.z == 0) atomicOr(status, FE_STATUS_BAD_PAGE);
     return;
   }
-  const int dk = p.dk, dv = p.dv, dk16 = (dk + 15) & ~15, KP = dk16 + 8, tile = dc_tile(dk16);
+  const int dk = WHOLE ? 64 * KD : p.dk, dv = p.dv, dk16 = (dk + 15) & ~15, KP = dk16 + 8, tile = dc_tile(dk16);
   bf16* S = reinterpret_cast<bf16*>(smem);   // [3][dk16][SP]
   bf16* us = S + 3 * dk16 * SP;              // [3][SR_LONG][SP], weighted
   bf16* tiles = us + 3 * SR_LONG * SP;       // SLOTS x 3 planes: W transposed [dk16][DC_WP] or keys [SR_LONG][KP]
   const int lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3;
   const int m0 = 16 * (warp & 3), t0 = m0 + g, n0 = 8 * (warp >> 2);        // first row and columns of this warp's pieces
   const int col = col0 + n0 + 2 * q;                               // this lane's two columns
-  const bool in0 = col < dv, in1 = col + 1 < dv, pair = in1 && (dv & 1) == 0;
+  const bool in0 = WHOLE || col < dv, in1 = WHOLE || col + 1 < dv, pair = WHOLE || (in1 && (dv & 1) == 0);
   auto load2 = [&](const float* at, float& a, float& b) {
     if (pair) { const float2 x = *reinterpret_cast<const float2*>(at); a = x.x, b = x.y; }
     else { a = in0 ? at[0] : 0.f, b = in1 ? at[1] : 0.f; }
@@ -571,24 +573,13 @@ __global__ void __launch_bounds__(16 * COLS) delta_chain_kernel(const Delta m, c
     }
   const int chunks = (count + SR_LONG - 1) / SR_LONG;
   const size_t cell0 = (size_t)sr_slot(first, entry, 0) * p.heads + head, group0 = cell0 - head % m.per;
-  const int kcol = dk16 >> 3;                // 16-byte pieces of a row of keys
   auto fetch = [&](int i) {                  // tile i: W of chunk i / 2, or its keys
     if (i < 2 * chunks) {
       bf16* to = tiles + (i % SLOTS) * 3 * tile;
-      const int chunk = i >> 1;
-      if ((i & 1) == 0) {
-        const bf16* from = m.w + (cell0 + (size_t)chunk * p.heads) * 3 * dk16 * SR_LONG;
-        for (int u = 0; u < 3; ++u)
+      const size_t step = (size_t)(i >> 1) * p.heads;
+      const bf16* from = (i & 1) == 0 ? m.w + (cell0 + step) * 3 * tile : m.k + (group0 + step) * 3 * tile;
 #pragma unroll 4
-          for (int r = tid >> 3; r < dk16; r += THREADS / 8)
-            sr_copy16(to + u * tile + r * DC_WP + (tid & 7) * 8, from + ((size_t)u * dk16 + r) * SR_LONG + (tid & 7) * 8);
-      } else {
-        const bf16* from = m.k + (group0 + (size_t)chunk * p.heads) * 3 * dk16 * SR_LONG;
-        for (int u = 0; u < 3; ++u)
-#pragma unroll 4
-          for (int t = tid >> 3; t < SR_LONG; t += THREADS / 8)
-            for (int c = tid & 7; c < kcol; c += 8) sr_copy16(to + u * tile + t * KP + c * 8, from + ((size_t)u * SR_LONG + t) * dk16 + c * 8);
-      }
+      for (int at = tid * 8; at < 3 * tile; at += THREADS * 8) sr_copy16(to + at, from + at);
     }
     sr_copy_commit();
   };
@@ -697,7 +688,7 @@ FE_EXPORT long long fe_delta_rule_scratch(int tokens, int entries, int heads, in
   const long long need = walk_in_stretches(dk, dv, 0) ? (long long)tokens * heads * dv : 0;
   if (max_new < SR_LONG_FROM || !delta_chunk_takes(dk, dv)) return need;
   return (need + 3) / 4 * 4 + sr_slots(tokens, entries) * heads *
-             (3LL * ((dk + 15) / 16 * 16) * SR_LONG + (long long)SR_LONG * dv + (long long)dk * dv + SR_LONG + 4);
+             (3LL * dc_tile((dk + 15) / 16 * 16) + (long long)SR_LONG * dv + (long long)dk * dv + SR_LONG + 4);
 }
 
 FE_EXPORT int fe_delta_rule(const float* qkv, long long ld, const float* gates, const float* gate, long long gate_ld,
@@ -719,15 +710,16 @@ FE_EXPORT int fe_delta_rule(const float* qkv, long long ld, const float* gates, 
   const int chunks = (max_new + SR_LONG - 1) / SR_LONG;
   if (chunks > 65535) return FE_ERR_TOO_LARGE;
   const size_t cells = (size_t)sr_slots(tokens, entries) * heads;
-  const size_t planes = cells * 3 * ((dk + 15) / 16 * 16) * SR_LONG;
+  const size_t planes = cells * 3 * dc_tile((dk + 15) / 16 * 16);
   m.w = reinterpret_cast<bf16*>(scratch);
   m.k = m.w + planes;
   m.u = scratch + planes;
   m.decays = m.u + cells * SR_LONG * dv;
   m.before = m.decays + cells * (SR_LONG + 4);
   size_t smem = delta_solve_smem(dk, dv);
-  cudaFuncSetAttribute(delta_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  rc = fe_launch_dependent(delta_solve_kernel, dim3(heads, entries, chunks), dim3(DS_THREADS), smem, stream, m, p);
+  const auto solve = dk == 64 && dv == 64 ? delta_solve_kernel<64> : dk == 128 && dv == 128 ? delta_solve_kernel<128> : delta_solve_kernel<0>;
+  cudaFuncSetAttribute(solve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  rc = fe_launch_dependent(solve, dim3(heads, entries, chunks), dim3(DS_THREADS), smem, stream, m, p);
   if (rc) return rc;
   // delta_chain is not launched as a dependent: its blocks, fewer than the SMs or not many more, would take their
   // places while delta_solve's last blocks leave theirs, two on one SM and none on the next (measured with two tf32
@@ -735,22 +727,29 @@ FE_EXPORT int fe_delta_rule(const float* qkv, long long ld, const float* gates, 
   const int cols = delta_chain_cols(dv);
   smem = delta_chain_smem(dk, cols);
   const dim3 chain(heads, entries, (dv + cols - 1) / cols);
-#define DC_LAUNCH(KD, COLS, SLOTS)                                                                                     \
-  do {                                                                                                                 \
-    cudaFuncSetAttribute(delta_chain_kernel<KD, COLS, SLOTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-    delta_chain_kernel<KD, COLS, SLOTS><<<chain, 16 * COLS, smem, stream>>>(m, p, status);                             \
-    rc = fe_last_error();                                                                                              \
+#define DC_LAUNCH_AS(KD, COLS, SLOTS, WHOLE)                                                                                  \
+  do {                                                                                                                        \
+    cudaFuncSetAttribute(delta_chain_kernel<KD, COLS, SLOTS, WHOLE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+    delta_chain_kernel<KD, COLS, SLOTS, WHOLE><<<chain, 16 * COLS, smem, stream>>>(m, p, status);                             \
+    rc = fe_last_error();                                                                                                     \
+  } while (0)
+  // sizes that fill the warps' pieces: places and bounds known when compiled (2,048 tokens, 32 heads of 64: 96 us, 58 so)
+#define DC_LAUNCH(KD, COLS, SLOTS)                                               \
+  do {                                                                           \
+    if (dk == 64 * KD && dv % COLS == 0) DC_LAUNCH_AS(KD, COLS, SLOTS, true);    \
+    else DC_LAUNCH_AS(KD, COLS, SLOTS, false);                                   \
   } while (0)
 #define DC_BY_DK(COLS)                       \
   do {                                       \
     if (dk <= 64) DC_LAUNCH(1, COLS, 4);     \
     else if (dk <= 128) DC_LAUNCH(2, COLS, 3); \
-    else DC_LAUNCH(3, COLS, 2);              \
+    else DC_LAUNCH_AS(3, COLS, 2, false);    \
   } while (0)
   if (cols == 16) DC_BY_DK(16);
   else DC_BY_DK(32);
 #undef DC_BY_DK
 #undef DC_LAUNCH
+#undef DC_LAUNCH_AS
   if (rc) return rc;
   rc = launch_out(m, p, out_dtype, entries, chunks, stream);
   return rc ? rc : fe_last_error();

@@ -272,7 +272,8 @@ __device__ __forceinline__ void gr_inside(const float* fs, const float* qs, int 
 // two barriers per distance with q rewritten in between).  3 prompts of 1,000 to 666 tokens, 32 heads of 128: 253 us before, 195 now.
 // R: channels a lane of the sub-chunks' own blocks holds, in a slice, as few as the head needs.  32 heads of 64, 2,048
 // tokens, all kernels: 216 us with two, 225 with four; 32 heads of 16, 1,000 tokens: 77 us with one, 89 with four.
-template <int R>
+// D: key and value size known when compiled; 0: any.
+template <int R, int D>
 __global__ void __launch_bounds__(256, 2) gated_recurrence_chunk_kernel(GatedRecurrence p, int aligned) {
   extern __shared__ __align__(16) float smem[];
   pdl_trigger();
@@ -281,9 +282,9 @@ __global__ void __launch_bounds__(256, 2) gated_recurrence_chunk_kernel(GatedRec
   const int entry_first = p.cu_tokens[entry], entry_count = p.cu_tokens[entry + 1] - entry_first;
   if (entry_count < p.long_from || chunk * GR_LONG_CHUNK >= entry_count) return;
   const int first = entry_first + chunk * GR_LONG_CHUNK, count = min(GR_LONG_CHUNK, entry_count - chunk * GR_LONG_CHUNK);
-  const int dk = p.dk, dv = p.dv;
+  const int dk = D ? D : p.dk, dv = D ? D : p.dv, dkp = (dk + 3) & ~3;
   // pitches: a fragment's rows (q, k) and its columns (v) fall into different banks
-  const int dp = min(p.dkp, GR_SLICE) + 4, vp = min(dv, GR_SLICE) + 8;
+  const int dp = min(dkp, GR_SLICE) + 4, vp = min(dv, GR_SLICE) + 8;
   float* fs = smem;                              // [64][dp]: gates, then what is left of k
   float* qs = fs + GR_LONG_CHUNK * dp;           // [64][dp]; when q is done, vs [64][vp]
   float* vs = qs;
@@ -447,7 +448,7 @@ __global__ void __launch_bounds__(256, 2) gated_recurrence_chunk_kernel(GatedRec
           for (int m = sub - 1; m >= 0; --m)
 #pragma unroll
             for (int e = 0; e < 4; ++e) a[e] *= g[m][e];
-          store4(p.qb + ((size_t)(first + t) * p.heads + head) * p.dkp + d0 + d, a);
+          store4(p.qb + ((size_t)(first + t) * p.heads + head) * dkp + d0 + d, a);
         }
       }
     }
@@ -611,7 +612,7 @@ __global__ void __launch_bounds__(128) gated_recurrence_scan_kernel(GatedRecurre
 #define GR_FX (GR_FK + 4)
 __host__ __device__ static inline int gr_finish_pitch(int dv) { return ((dv < GR_SLICE ? dv : GR_SLICE) + 31) / 32 * 32 + 8; }
 __host__ __device__ static inline int gr_finish_stages(int dv) { return dv <= GR_SLICE ? 3 : 2; }
-template <typename TO>
+template <typename TO, int D>
 __global__ void __launch_bounds__(256, 2) gated_recurrence_finish_kernel(GatedRecurrence p, int v_aligned) {
   extern __shared__ __align__(16) float smem[];
   __shared__ float part[4][GR_LONG_CHUNK];
@@ -621,7 +622,7 @@ __global__ void __launch_bounds__(256, 2) gated_recurrence_finish_kernel(GatedRe
   const int entry_first = p.cu_tokens[entry], entry_count = p.cu_tokens[entry + 1] - entry_first;
   if (entry_count < p.long_from || chunk * GR_LONG_CHUNK >= entry_count) return;
   const int first = entry_first + chunk * GR_LONG_CHUNK, count = min(GR_LONG_CHUNK, entry_count - chunk * GR_LONG_CHUNK);
-  const int dk = p.dk, dv = p.dv;
+  const int dk = D ? D : p.dk, dv = D ? D : p.dv, dkp = (dk + 3) & ~3;
   const int pitch = gr_finish_pitch(dv), stages = gr_finish_stages(dv);
   const int stage_floats = GR_LONG_CHUNK * GR_FX + GR_FK * pitch;
   float* os = smem + stages * stage_floats;          // [64][dv], only where dv > 128
@@ -630,12 +631,12 @@ __global__ void __launch_bounds__(256, 2) gated_recurrence_finish_kernel(GatedRe
   const size_t at = (size_t)gr_chunk_slot(entry_first, entry, chunk) * p.heads + head;
   const float* start = p.chunk_state + at * dk * dv;
   const float* values = p.proj + (size_t)first * p.ld + p.v_off + (size_t)head * dv;
-  const int q_steps = (p.dkp + GR_FK - 1) / GR_FK, steps = q_steps + (count + GR_FK - 1) / GR_FK;
+  const int q_steps = (dkp + GR_FK - 1) / GR_FK, steps = q_steps + (count + GR_FK - 1) / GR_FK;
   // what this thread copies of a stretch: eight numbers of a row of the left operand, every eighth four of a row
   // of the right one
   const int xt = tid >> 2, xk = (tid & 3) * 8, yk = tid >> 3, yc = (tid & 7) * 4;
   const bool row = xt < count;
-  const float* x_q = p.qb + ((size_t)(first + (row ? xt : 0)) * p.heads + head) * p.dkp + xk;
+  const float* x_q = p.qb + ((size_t)(first + (row ? xt : 0)) * p.heads + head) * dkp + xk;
   const float* x_a = p.within + at * GR_LONG_CHUNK * GR_LONG_CHUNK + xt * GR_LONG_CHUNK + xk;
 
   auto stage = [&](int step, int v0, int nv) {
@@ -645,8 +646,8 @@ __global__ void __launch_bounds__(256, 2) gated_recurrence_finish_kernel(GatedRe
     const int k0 = (state ? step : step - q_steps) * GR_FK;
     const float* src = (state ? x_q : x_a) + k0;
     float* to = xs + xt * GR_FX + xk;
-    gr_copy16(to, src, row && (!state || k0 + xk < p.dkp));
-    gr_copy16(to + 4, src + 4, row && (!state || k0 + xk + 4 < p.dkp));
+    gr_copy16(to, src, row && (!state || k0 + xk < dkp));
+    gr_copy16(to + 4, src + 4, row && (!state || k0 + xk + 4 < dkp));
     const bool valid = state ? k0 + yk < dk : k0 + yk < count;
     const float* from = !valid ? start : (state ? start + (size_t)(k0 + yk) * dv : values + (size_t)(k0 + yk) * p.ld) + v0 + yc;
 #pragma unroll
@@ -884,7 +885,11 @@ FE_EXPORT int fe_gated_recurrence(const float* proj, long long ld, int q_off, in
   const int chunks = (max_new + GR_LONG_CHUNK - 1) / GR_LONG_CHUNK;
   if (chunks > 65535) return FE_ERR_TOO_LARGE;
   const size_t chunk_smem = gr_chunk_smem(dk, dv);
-  auto chunk_kernel = dk <= 32 ? gated_recurrence_chunk_kernel<1> : dk <= 64 ? gated_recurrence_chunk_kernel<2> : gated_recurrence_chunk_kernel<GR_SLICE / 32>;
+  // heads of 64 and of 128 on both sides: places and bounds known when compiled (3 prompts of 1,000 to 666
+  // tokens, 32 heads of 128: chunk kernel 195 us, 169 so; outputs 126 and 114)
+  const int whole = dk == dv && (dk == 64 || dk == 128) ? dk : 0;
+  auto chunk_kernel = whole == 64 ? gated_recurrence_chunk_kernel<2, 64> : whole == 128 ? gated_recurrence_chunk_kernel<4, 128>
+                      : dk <= 32 ? gated_recurrence_chunk_kernel<1, 0> : dk <= 64 ? gated_recurrence_chunk_kernel<2, 0> : gated_recurrence_chunk_kernel<GR_SLICE / 32, 0>;
   if (chunk_smem > 48 * 1024) cudaFuncSetAttribute(chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)chunk_smem);
   const int v_aligned = ((uintptr_t)proj & 15) == 0 && ld % 4 == 0 && v_off % 4 == 0;
   const int aligned = v_aligned && q_off % 4 == 0 && f_off % 4 == 0 && dk % 4 == 0 && (((uintptr_t)lower | (uintptr_t)f_bias) & 15) == 0;
@@ -894,16 +899,15 @@ FE_EXPORT int fe_gated_recurrence(const float* proj, long long ld, int q_off, in
                            p, status);
   if (rc) return rc;
   const size_t finish_smem = gr_finish_smem(dv);
-  if (out_dtype == FE_DTYPE_F32) {
-    if (finish_smem > 48 * 1024)
-      cudaFuncSetAttribute(gated_recurrence_finish_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)finish_smem);
-    rc = fe_launch_dependent(gated_recurrence_finish_kernel<float>, dim3(heads, entries, chunks), dim3(256), finish_smem, stream, p,
-                             v_aligned);
-  } else {
-    if (finish_smem > 48 * 1024)
-      cudaFuncSetAttribute(gated_recurrence_finish_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)finish_smem);
-    rc = fe_launch_dependent(gated_recurrence_finish_kernel<bf16>, dim3(heads, entries, chunks), dim3(256), finish_smem, stream, p,
-                             v_aligned);
-  }
+#define GR_FINISH(TO)                                                                                                          \
+  do {                                                                                                                         \
+    auto finish = whole == 64 ? gated_recurrence_finish_kernel<TO, 64> : whole == 128 ? gated_recurrence_finish_kernel<TO, 128> \
+                                                                       : gated_recurrence_finish_kernel<TO, 0>;                \
+    if (finish_smem > 48 * 1024) cudaFuncSetAttribute(finish, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)finish_smem);  \
+    rc = fe_launch_dependent(finish, dim3(heads, entries, chunks), dim3(256), finish_smem, stream, p, v_aligned);              \
+  } while (0)
+  if (out_dtype == FE_DTYPE_F32) GR_FINISH(float);
+  else GR_FINISH(bf16);
+#undef GR_FINISH
   return rc ? rc : fe_last_error();
 }

@@ -498,14 +498,14 @@ struct OutTile {            // a warp's 32 x 16 outputs
 };
 
 #define SR_OP (64 + 8)       // pitch of a tile of 64 columns
-template <class M, typename TO, int NP>
+template <class M, typename TO, int NP, int D>       // D: key and value size known when compiled; 0: any
 __global__ void __launch_bounds__(256) state_out_kernel(const M m, const StateRun p) {
   extern __shared__ __align__(16) float smem[];
   pdl_trigger();
   pdl_wait();
   ChunkAt at;
   if (!sr_locate(p, &at)) return;
-  const int head = blockIdx.x, dk = p.dk, dv = p.dv, tid = threadIdx.x, dk8 = (dk + 7) & ~7;
+  const int head = blockIdx.x, dk = D ? D : p.dk, dv = D ? D : p.dv, tid = threadIdx.x, dk8 = (dk + 7) & ~7;
   __shared__ double rt[SR_LONG], ct[SR_LONG];
   __shared__ float ea[SR_LONG], fl[SR_LONG], den[SR_LONG];
   __shared__ float part[4][SR_LONG];
@@ -653,17 +653,19 @@ template <class M>
 static int launch_out(const M& m, const StateRun& p, int out_dtype, int entries, int chunks, cudaStream_t stream) {
   const size_t smem = state_out_smem(p.dk, M::SCORES);
   int rc = FE_ERR_BAD_DTYPE;
-#define SR_OUT(TO, NP)                                                                                             \
-  do {                                                                                                             \
-    if (smem > 30 * 1024)                                                                                          \
-      cudaFuncSetAttribute(state_out_kernel<M, TO, NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);   \
-    rc = fe_launch_dependent(state_out_kernel<M, TO, NP>, dim3(p.heads, entries, chunks), dim3(256), smem, stream, m, p); \
+#define SR_OUT(TO, NP, D)                                                                                             \
+  do {                                                                                                                \
+    if (smem > 30 * 1024)                                                                                             \
+      cudaFuncSetAttribute(state_out_kernel<M, TO, NP, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);   \
+    rc = fe_launch_dependent(state_out_kernel<M, TO, NP, D>, dim3(p.heads, entries, chunks), dim3(256), smem, stream, m, p); \
   } while (0)
-#define SR_OUT_BY_DV(TO)                     \
-  do {                                       \
-    if (p.dv <= 64) SR_OUT(TO, 1);           \
-    else if (p.dv <= 128) SR_OUT(TO, 2);     \
-    else SR_OUT(TO, 4);                      \
+#define SR_OUT_BY_DV(TO)                                     \
+  do {                                                       \
+    if (p.dk == 64 && p.dv == 64) SR_OUT(TO, 1, 64);         \
+    else if (p.dk == 128 && p.dv == 128) SR_OUT(TO, 2, 128); \
+    else if (p.dv <= 64) SR_OUT(TO, 1, 0);                   \
+    else if (p.dv <= 128) SR_OUT(TO, 2, 0);                  \
+    else SR_OUT(TO, 4, 0);                                   \
   } while (0)
   if (out_dtype == FE_DTYPE_F32) SR_OUT_BY_DV(float);
   else if (out_dtype == FE_DTYPE_BF16) SR_OUT_BY_DV(bf16);

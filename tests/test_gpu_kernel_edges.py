@@ -263,7 +263,7 @@ def test_gated_recurrence_chunks(native, heads, dk, dv, lead, counts):
     assert torch.equal(got_state[-1].cpu(), state[-1])       # the row of no entry
 
 
-@pytest.mark.parametrize("dk", (4, 20, 36, 72, 100, 132))
+@pytest.mark.parametrize("dk", (4, 20, 36, 72, 100, 136))
 def test_gated_recurrence_channels_off_sixteen(native, dk):
     """Products between sub-chunks over every remainder of sixteen channels; lanes with one, two and four channels."""
     test_gated_recurrence_chunks(native, 2, dk, 8, 4, [150, 133])
