@@ -21,10 +21,11 @@ def native():
 
 
 def run_case(native, nq, nkv, d, page, window, lengths, new_counts, splits, sharp=False, merge_in_kernel=True,
-             plant=True):
+             plant=True, both=False):
     """Request r holds lengths[r] keys after the step, the last new_counts[r] of them new.
     ``plant``: the last query of every entry that takes the decode kernel is aimed at single
-    keys on the edges of its window and of its tiles (see ``plant_keys``)."""
+    keys on the edges of its window and of its tiles (see ``plant_keys``).  ``both``: the prefill and the decode
+    kernel are launched with room for longer portions, whatever the entries bring."""
     dtype = torch.bfloat16
     k_cache, v_cache, table, keys, values = paged_layout(lengths, page, nkv, d, dtype, seed=d + nq + page)
     g = torch.Generator().manual_seed(2)
@@ -48,8 +49,8 @@ def run_case(native, nq, nkv, d, page, window, lengths, new_counts, splits, shar
     native.attention_mma(
         qkv.to(DEV), stride, k_cache, v_cache, table,
         torch.tensor(cu, dtype=torch.int32, device=DEV), torch.tensor(starts, dtype=torch.int32, device=DEV),
-        len(lengths), max(new_counts), window, d ** -0.5, out, nq, status,
-        run_prefill=any(r > 16 for r in rows), run_decode=any(r <= 16 for r in rows), num_splits=splits,
+        len(lengths), max(new_counts) + (64 if both else 0), window, d ** -0.5, out, nq, status,
+        run_prefill=both or any(r > 16 for r in rows), run_decode=both or any(r <= 16 for r in rows), num_splits=splits,
         merge_in_kernel=merge_in_kernel,
     )
     assert int(status.item()) == 0
@@ -70,6 +71,15 @@ def test_prefill_and_decode_mixed(native, nq, nkv, d, page, window) -> None:
     lengths = [300, 200, 129, 1, 64, 450, 33]
     new_counts = [300, 73, 1, 1, 2, 1, 33]
     run_case(native, nq, nkv, d, page, window, lengths, new_counts, splits=3, sharp=True)
+
+
+@pytest.mark.parametrize("new_counts", ([1, 1, 1, 1, 1], [100, 40, 33, 70, 20], [1, 300, 1, 1, 2]))
+@pytest.mark.parametrize("splits", [1, 4, 8, 16])
+def test_decode_beside_prefill(native, new_counts, splits) -> None:
+    """Both kernels in one call, which run side by side: steps in which every entry is the one's, every entry is the
+    other's, and mixed ones; the splits combined in a cluster and through memory."""
+    for _ in range(3):
+        run_case(native, 32, 8, 128, 16, None, [1500, 700, 90, 257, 1024], new_counts, splits, both=True)
 
 
 @pytest.mark.parametrize("nq,nkv,d,page", [(8, 8, 64, 8), (16, 8, 128, 32), (16, 2, 128, 64), (16, 1, 64, 128),
