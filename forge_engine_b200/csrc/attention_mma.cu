@@ -90,14 +90,6 @@ struct AttnParams {
   int head_cols = 0;
   int out_dim = 0;
   int out_heads = 0;
-  // The tcgen05 prefill kernel and, right behind it, attn_decode_tma_kernel, over the same step: neither reads what the
-  // other writes, so the decode kernel runs beside the prefill's blocks.  The prefill's blocks let it start only once they have
-  // seen the kernel before them complete (its first block in any case, rows or not), which is all that the decode
-  // kernel waits for; its own first block stays until the prefill is complete, so that the next kernel, which waits for the
-  // decode kernel, finds the results of both.  1,021 new tokens
-  // after 12,288 beside 4 requests of 1,500: 258 us one after the other, 246 side by side (11 and 247 alone); 248 new ones beside 8
-  // requests of up to 2,048: 27.7 and 26.5 (what does not fit beside the prefill's blocks comes after them).
-  int beside = 0;
 };
 
 __device__ __forceinline__ unsigned smem_addr(const void* p) {
@@ -631,10 +623,8 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
   const int tok0 = p.cu_tokens[entry];
   const int n_new = p.cu_tokens[entry + 1] - tok0;
   const int rows_total = n_new * p.groups;
+  if (rows_total <= p.row_lo || rows_total > p.row_hi) return;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  // the first block leaves when the prefill beside it is complete (AttnParams::beside)
-  auto leave = [&]() { if (p.beside && tid == 0 && (blockIdx.x | blockIdx.y | blockIdx.z) == 0) pdl_wait(); };
-  if (rows_total <= p.row_lo || rows_total > p.row_hi) { leave(); return; }
   const int start = p.starts[entry];
   const int* table = p.block_table + (size_t)entry * p.max_pages;
 
@@ -673,7 +663,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
       const int rows_in_cache = p.num_pages * p.nkv * p.page_size;
       const int first_logical = tile_begin * pages_per_tile;
       const int total_pages = my_tiles * pages_per_tile;
-      bool waited = p.beside != 0, dead = false;
+      bool waited = false, dead = false;
       for (int base = 0; base < total_pages; base += 32) {
         const int logical = first_logical + base + lane;
         const int key = logical * p.page_size;
@@ -710,7 +700,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     }
   } else {
     // ---- consumers: warp w takes keys [16 w, 16 w + 16) of every tile ----
-    if (!p.beside) pdl_wait();
+    pdl_wait();
     const int pos_a = ra < rows_total ? start + ra / p.groups : -1;
     const int pos_b = rb < rows_total ? start + rb / p.groups : -1;
     if (my_tiles > 0) {
@@ -792,7 +782,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     }
   }
   if (tid == 0 && *abort_flag) atomicOr(p.status, FE_STATUS_WAIT_TIMEOUT);
-  if (p.num_splits == 1) { leave(); return; }
+  if (p.num_splits == 1) return;
 
   if (p.cluster_merge) {
     // The splits of this (entry, kv head) are the blocks of one cluster.  Every block
@@ -846,7 +836,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     }
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // partial results stay alive until read
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-    if (p.cluster_merge != 2) { leave(); return; }
+    if (p.cluster_merge != 2) return;
   }
 
   // the block that publishes its (or its cluster's) partial result last combines all of
@@ -859,7 +849,7 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     if (last_block) p.ws_count[pair] = 0u;
   }
   __syncthreads();
-  if (!last_block) { leave(); return; }
+  if (!last_block) return;
   __threadfence();
   float* weight_s = reinterpret_cast<float*>(kbuf);       // [16][MERGE_MAX_SPLITS]
   const int splits = p.cluster_merge == 2 ? p.num_splits / 8 : p.num_splits;
@@ -902,7 +892,6 @@ attn_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     const int token = row / p.groups, g = row - token * p.groups;
     p.out[((size_t)(tok0 + token) * num_q_heads + kvh * p.groups + g) * D + d] = __float2bfloat16_rn(num);
   }
-  leave();
 }
 
 // Combine the splits' (max, sum, acc) of every row: block = (entry, kv head).  The splits'
@@ -1094,8 +1083,6 @@ FE_EXPORT int SYM(fe_attention_mma_d)(const void* q, int q_stride, void* out, co
   }
   const bool use_decode = (mode & 2) != 0;
   const int decode_rows = use_decode ? DEC_ROWS : 0;
-  const bool decode_tma = use_decode && num_splits > 0 && (D % 64) == 0 && page_size <= BN && (BN % page_size) == 0 &&
-                          (num_splits == 1 || counters != nullptr);
   if (mode & 1) {
     const int max_rows = max_new * groups;
     if (max_rows > decode_rows) {
@@ -1119,7 +1106,6 @@ FE_EXPORT int SYM(fe_attention_mma_d)(const void* q, int q_stride, void* out, co
         const int query_blocks = (max_rows + TC5_BLOCK_ROWS - 1) / TC5_BLOCK_ROWS;
         if (query_blocks > 65535) return FE_ERR_TOO_LARGE;
         dim3 grid(num_kv_heads, entries, query_blocks);
-        p.beside = decode_tma ? 1 : 0;
         const int rc = fe_launch_dependent(attn_prefill_tc5_kernel<false>, grid, dim3(TC5_THREADS), TC5_SMEM, stream, mq, *mk,
                                            *mv, p);
         if (rc) return rc;
@@ -1155,8 +1141,9 @@ FE_EXPORT int SYM(fe_attention_mma_d)(const void* q, int q_stride, void* out, co
     p.row_lo = 0; p.row_hi = DEC_ROWS;
     dim3 grid(num_splits, entries, num_kv_heads);
     int rc = 0;
+    const bool tma_ok = (D % 64) == 0 && page_size <= BN && (BN % page_size) == 0 && (num_splits == 1 || counters != nullptr);
     CUtensorMap mk_copy, mv_copy;
-    const CUtensorMap* mk = decode_tma && cache_map(&mk_copy, k_cache, num_pages * num_kv_heads * page_size, page_size, true) ? &mk_copy : nullptr;
+    const CUtensorMap* mk = tma_ok && cache_map(&mk_copy, k_cache, num_pages * num_kv_heads * page_size, page_size, true) ? &mk_copy : nullptr;
     const CUtensorMap* mv = mk && cache_map(&mv_copy, v_cache, num_pages * num_kv_heads * page_size, page_size, true) ? &mv_copy : nullptr;
     if (mk && mv) {
       static bool tma_configured = false;

@@ -241,17 +241,15 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
   unsigned* tmem_slot = reinterpret_cast<unsigned*>(o_full + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  if (!p.beside) pdl_trigger();
-  // a block without rows; the first one all the same sees the kernel before this one complete (AttnParams::beside)
-  auto leave = [&]() { if (p.beside && threadIdx.x == 0 && (blockIdx.x | blockIdx.y | blockIdx.z) == 0) pdl_wait(); };
+  pdl_trigger();
   const int entry = blockIdx.y, kvh = blockIdx.x;
   const int tok0 = p.cu_tokens[entry];
   const int n_new = p.cu_tokens[entry + 1] - tok0;
   const int rows_total = n_new * p.groups;
-  if (rows_total <= p.row_lo || rows_total > p.row_hi) { leave(); return; }
+  if (rows_total <= p.row_lo || rows_total > p.row_hi) return;
   // blocks start in the order of blockIdx.x, y, z: the long query blocks of every head first
   const int row0 = (gridDim.z - 1 - blockIdx.z) * TC5_BLOCK_ROWS;
-  if (row0 >= rows_total) { leave(); return; }
+  if (row0 >= rows_total) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int start = p.starts[entry];
   const int* table = p.block_table + (size_t)entry * p.max_pages;
@@ -301,10 +299,6 @@ attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const unsigned tmem_base = *tmem_slot;
-  if (p.beside) {
-    pdl_wait();
-    pdl_trigger();
-  }
 
   if (warp == 0) {
     // ---- producer ----

@@ -76,10 +76,50 @@ def test_prefill_and_decode_mixed(native, nq, nkv, d, page, window) -> None:
 @pytest.mark.parametrize("new_counts", ([1, 1, 1, 1, 1], [100, 40, 33, 70, 20], [1, 300, 1, 1, 2]))
 @pytest.mark.parametrize("splits", [1, 4, 8, 16])
 def test_decode_beside_prefill(native, new_counts, splits) -> None:
-    """Both kernels in one call, which run side by side: steps in which every entry is the one's, every entry is the
-    other's, and mixed ones; the splits combined in a cluster and through memory."""
+    """Both kernels in one call: steps in which every entry is the one's, every entry is the other's, and mixed ones; the
+    splits combined in a cluster and through memory."""
     for _ in range(3):
         run_case(native, 32, 8, 128, 16, None, [1500, 700, 90, 257, 1024], new_counts, splits, both=True)
+
+
+@pytest.mark.parametrize("new_counts", ([1, 1, 1, 1, 1], [100, 40, 33, 70, 20], [1, 900, 1, 1, 2], [700, 1, 1, 1, 1]))
+@pytest.mark.parametrize("splits", [1, 8])
+def test_both_kernels_in_a_chain_of_dependent_ones(native, new_counts, splits) -> None:
+    """Queries, keys and values come from a kernel that lets the next one start early, and the result goes to a kernel
+    that starts early itself: the same bits as with the device idle between any two of them.  New inputs in every
+    turn, so that whoever reads too soon finds those of the turn before."""
+    nq, nkv, d, page, lengths = 32, 8, 128, 16, [1500, 950, 90, 257, 1024]
+    width, total = (nq + 2 * nkv) * d, sum(new_counts)
+    k_cache, v_cache, table, _, _ = paged_layout(lengths, page, nkv, d, torch.bfloat16, seed=9)
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)  # noqa: E731
+    starts = [n - c for n, c in zip(lengths, new_counts)]
+    cu = ints([0] + torch.tensor(new_counts).cumsum(0).tolist())
+    positions = ints([p for s, n in zip(starts, lengths) for p in range(s, n)])
+    entry = ints([e for e, c in enumerate(new_counts) for _ in range(c)])
+    starts, weight, status = ints(starts), torch.ones(nq * d, device=DEV), status_word()
+    gen = torch.Generator(device=DEV).manual_seed(1)
+
+    def step(qkv, pause):
+        out = torch.full((total, nq * d), float("nan"), dtype=torch.bfloat16, device=DEV)
+        normed, stream = torch.empty_like(out), torch.zeros((total, nq * d), device=DEV)
+        torch.cuda.synchronize()
+        native.qk_rope_cache(qkv, None, None, 1e-6, None, 0, positions, entry, k_cache, v_cache, table, nq, True, status)
+        pause()
+        native.attention_mma(qkv, width, k_cache, v_cache, table, cu, starts, len(lengths), max(new_counts) + 64, None, d ** -0.5, out,
+                             nq, status, run_prefill=True, run_decode=True, num_splits=splits)
+        pause()
+        native.add_rmsnorm(stream, out, weight, normed, 1e-6)
+        torch.cuda.synchronize()
+        return out, normed
+
+    for _ in range(6):
+        qkv = torch.randn((total, width), generator=gen, device=DEV).to(torch.bfloat16)
+        chained = step(qkv.clone(), lambda: None)
+        other = torch.randn((total, width), generator=gen, device=DEV).to(torch.bfloat16)
+        step(other, torch.cuda.synchronize)                  # other keys and values in the pages
+        alone = step(qkv.clone(), torch.cuda.synchronize)
+        assert int(status.item()) == 0
+        assert all(torch.equal(a, b) and bool(torch.isfinite(a).all()) for a, b in zip(chained, alone))
 
 
 @pytest.mark.parametrize("nq,nkv,d,page", [(8, 8, 64, 8), (16, 8, 128, 32), (16, 2, 128, 64), (16, 1, 64, 128),
