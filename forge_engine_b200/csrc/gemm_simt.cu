@@ -408,8 +408,10 @@ int split_cuts(int tile, long long tiles, int k) {
   return cuts;
 }
 
+int split_tile(int n) { return n <= 16 ? 16 : n <= 32 ? 32 : n <= 64 ? 64 : 128; }
+
 int split_product(const Product& p, int batch, bool batched, cudaStream_t stream) {
-  const int tile = p.n <= 16 ? 16 : p.n <= 32 ? 32 : p.n <= 64 ? 64 : 128;
+  const int tile = split_tile(p.n);
   const int cuts = split_cuts(tile, (long long)((p.o + 127) / 128) * ((p.n + tile - 1) / tile) * batch, p.k);
   switch (tile) {
     case 16: return launch_split<16>(p, batch, cuts, batched, stream);
@@ -483,6 +485,12 @@ int launch_coded(int x_dtype, int w_dtype, const Product& p, int batch, bool bat
 // block gives up, sets FE_STATUS_WAIT_TIMEOUT and returns.  Call with (0, -1) to go back to normal.
 FE_EXPORT void fe_gemm_simt_set_test_fault(unsigned wait_limit, int skip_stretch) {
   g_test_fault = Fault{wait_limit ? wait_limit : tc5::WAIT_LIMIT, skip_stretch};
+}
+
+// Into how many blocks a deep product of 32-bit operands cuts k, for its test.
+FE_EXPORT int fe_gemm_split_cuts(int n, int o, int k, int batch) {
+  const int tile = split_tile(n);
+  return split_cuts(tile, (long long)((o + 127) / 128) * ((n + tile - 1) / tile) * batch, k);
 }
 
 FE_EXPORT int fe_gemm_simt(const void* x, int x_dtype, const void* w, int w_dtype, const float* bias,

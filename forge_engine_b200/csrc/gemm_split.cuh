@@ -253,6 +253,9 @@ __global__ void __launch_bounds__(gst_workers(NT) + 32, NT <= 32 ? 2 : 1) gemm_s
     }
     if (!batched) pdl_wait();
     if (count > 0) b.load(x + k_of(0), p.k - k_of(0));
+    // The lanes of a warp part where a row ends, where a value is not finite and where one of them speaks for all; what the whole
+    // warp executes together (tensor memory, cluster barriers) stands behind a __syncwarp or a vote.
+    __syncwarp();
     int part = first, part_end = (int)((long long)stretches * (first + 1) / GST_PARTS);
     // the sum of the parts before `part` lies behind the accumulators (with two blocks' parts and more: the part before)
     auto close_parts = [&](int stretch) {
@@ -315,11 +318,13 @@ __global__ void __launch_bounds__(gst_workers(NT) + 32, NT <= 32 ? 2 : 1) gemm_s
       if (++s == STAGES) s = 0;
     }
     if (!ok && lane == 0 && p.status) atomicOr(p.status, FE_STATUS_WAIT_TIMEOUT);
+    __syncwarp();
     if (cuts == 1) {
       const int col = col0 + quarter * 32 + lane;
 #pragma unroll
       for (int c = 0; c < COLS; c += 8) {
         float sum[8];
+        __syncwarp();        // some lanes may have taken the chain for the columns before
         gst_tmem_load(mine + STAGES * NT + c, sum);
 #pragma unroll
         for (int e = 0; e < 8; ++e) gst_finish(p, sum[e] + acc[c + e], row0 + column + c + e, col, ok);
@@ -370,6 +375,7 @@ __global__ void __launch_bounds__(gst_workers(NT) + 32, NT <= 32 ? 2 : 1) gemm_s
         gst_finish(p, v[0], row0 + token, col0 + feature, all_ok);
       }
     }
+    __syncwarp();
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");     // the stashes stay until they are read
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   } else {

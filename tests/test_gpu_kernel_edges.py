@@ -586,6 +586,32 @@ def test_deep_product_of_values_that_are_not_finite(native, n):
     assert float((got[2, keep][sound].double() / want[2, keep][sound] - 1).abs().max()) < 1e-5
 
 
+@pytest.mark.parametrize("n, o, k", ((3, 40100, 256), (20, 20100, 320), (50, 20100, 260), (300, 4210, 448)))
+def test_values_that_are_not_finite_in_tiles_of_one_block(native, n, o, k):
+    """The same in each tile size where one block takes all of k and writes its outputs itself: single lanes take the chain
+    between two accesses of the whole warp to tensor memory, and lanes past the last column leave early."""
+    assert native.lib().fe_gemm_split_cuts(n, o, k, 1) == 1
+    gen = torch.Generator().manual_seed(n + o)
+    x, w = torch.randn((n, k), generator=gen).to(DEV), torch.randn((o, k), generator=gen).to(DEV)
+    clean = torch.empty((n, o), device=DEV)
+    native.gemm_simt(x, w, clean)
+    rows, columns = {0: float("inf"), n // 2: float("nan"), n - 1: float("-inf")}, {1: float("inf"), 70: float("nan"), o - 2: float("-inf")}
+    for row, value in rows.items():
+        x[row, (7 * row) % k] = value
+    for column, value in columns.items():
+        w[column, (5 * column + 1) % k] = value
+    got = torch.full((n, o), 7.0, device=DEV)
+    native.gemm_simt(x, w, got)
+    want = x.double() @ w.double().t()
+    keep = torch.ones((n, o), dtype=torch.bool, device=DEV)
+    keep[list(rows)] = False
+    keep[:, list(columns)] = False
+    assert torch.equal(got[keep], clean[keep])
+    assert torch.equal(got[~keep].isnan(), want[~keep].isnan())
+    infinite = ~keep & want.isinf()
+    assert bool(infinite.any()) and torch.equal(got[infinite].double(), want[infinite])
+
+
 # -- the largest logits alone ------------------------------------------------------------------------
 def drawn_among(row, temperature, top_k, top_p, min_p, u):
     """(index, distance of the target from the nearest boundary of the running sum, over the sum) in 64 bits: of equal
