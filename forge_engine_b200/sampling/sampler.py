@@ -7,6 +7,7 @@ Here all rows of a step are sampled by one kernel launch and read back by one co
 
 from __future__ import annotations
 
+import math
 import struct
 from typing import Sequence
 
@@ -17,11 +18,22 @@ from .params import SamplingParams
 
 
 _MASK64 = (1 << 64) - 1
+_PAST_32_BITS = (2.0 - 2.0**-24) * 2.0**127      # rounds to infinity in 32 bits, and so does all above
 
 
 def _to_signed64(value: int) -> int:
     value &= (1 << 64) - 1
     return value - (1 << 64) if value >= (1 << 63) else value
+
+
+def packed_rows(params: Sequence[SamplingParams], seeds: Sequence[int], counters: Sequence[int]) -> bytes:
+    """What ``native.sample_rows`` reads, the numbers as tensors of these types would hold them: a temperature past the
+    range of 32 bits is infinite (``struct`` refuses it), a top-k that is not whole is cut."""
+    fields = []
+    for p, seed, counter in zip(params, seeds, counters):
+        temperature = p.temperature if p.temperature < _PAST_32_BITS else math.inf
+        fields += (temperature, p.top_p, p.min_p, int(p.top_k or 0), seed & _MASK64, counter & _MASK64)
+    return struct.pack("=" + "3fi2Q" * len(params), *fields)
 
 
 class Sampler:
@@ -50,10 +62,7 @@ class Sampler:
             return out
         if rows <= native.SAMPLE_ROWS_BY_VALUE and all((p.top_k or 0) < 1 << 31 for p in params):
             # the parameters go with the launch: three pinned copies ahead of it took 60 us of host time
-            fields = []
-            for p, seed, counter in zip(params, seeds, counters):
-                fields += (p.temperature, p.top_p, p.min_p, p.top_k or 0, seed & _MASK64, counter & _MASK64)
-            native.sample_rows(logits, out, self.status, struct.pack("=" + "3fi2Q" * rows, *fields))
+            native.sample_rows(logits, out, self.status, packed_rows(params, seeds, counters))
             return out
         floats = torch.tensor(
             [[p.temperature for p in params], [p.top_p for p in params], [p.min_p for p in params]],

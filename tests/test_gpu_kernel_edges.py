@@ -659,3 +659,20 @@ def test_sampling_among_the_largest(native, vocab, shape):
     for r, got in enumerate(out.tolist()):
         want, gap = drawn_among(logits[r], *asked[r], twin_uniform(11 + r, 2**40 + r))
         assert got == want or gap < 1e-5, (r, got, want, gap)
+
+
+@pytest.mark.parametrize("temperature", (1e39, 3.4e38, 1e-50))
+def test_temperatures_past_32_bits(native, temperature):
+    """Finite temperatures that 32 bits hold as infinity or zero draw the same by the rows of a launch (up to 64) and by
+    arrays."""
+    from forge_engine_b200.sampling.params import SamplingParams
+    from forge_engine_b200.sampling.sampler import Sampler
+
+    logits = torch.randn((65, 5000), generator=torch.Generator().manual_seed(4)).to(DEV)
+    params = [SamplingParams(temperature=temperature, top_k=50.0 if r % 2 else None, top_p=0.9) for r in range(65)]
+    status = status_word()
+    sampler = Sampler(DEV, status)
+    seeds, counters = list(range(65)), [3] * 65
+    by_arrays = sampler.sample(logits, params, seeds, counters)
+    by_rows = [sampler.sample(logits[a:b].contiguous(), params[a:b], seeds[a:b], counters[a:b]) for a, b in ((0, 1), (1, 65))]
+    assert int(status.item()) == 0 and torch.equal(torch.cat(by_rows), by_arrays)
