@@ -612,6 +612,30 @@ def test_values_that_are_not_finite_in_tiles_of_one_block(native, n, o, k):
     assert bool(infinite.any()) and torch.equal(got[infinite].double(), want[infinite])
 
 
+@pytest.mark.parametrize("n, o, k", ((4, 32100, 256), (16, 300, 1028), (40, 700, 512), (200, 300, 448), (300, 4224, 256)))
+def test_products_without_a_finite_sum_are_chains(native, n, o, k):
+    """NaN in every row, NaN in every column, and an infinity in every row: every output is taken again, as the chain of
+    multiply-adds that kernels without tensor cores take (the same rows off 16 bytes go there), bit for bit."""
+    gen = torch.Generator().manual_seed(n + k)
+    x, w = torch.randn((n, k), generator=gen).to(DEV), torch.randn((o, k), generator=gen).to(DEV)
+    for loud in ("rows", "columns", "infinite"):
+        a, b = x.clone(), w.clone()
+        if loud == "rows":
+            a[:, 3] = float("nan")
+        elif loud == "columns":
+            b[:, k - 2] = float("nan")
+        else:
+            a[:, 9], b[:, 9] = float("inf"), b[:, 9].abs() + 0.1
+            a[0, 9] = float("-inf")
+        got, chain = torch.empty((n, o), device=DEV), torch.empty((n, o), device=DEV)
+        native.gemm_simt(a, b, got)
+        off = torch.empty(n * k + 1, device=DEV)[1:].view(n, k).copy_(a)           # rows that start off 16 bytes
+        assert off.data_ptr() % 16 != 0
+        native.gemm_simt(off, b, chain)
+        assert torch.equal(got.nan_to_num(nan=7.0), chain.nan_to_num(nan=7.0)), loud
+        assert not bool(got.isfinite().any())
+
+
 # -- the largest logits alone ------------------------------------------------------------------------
 def drawn_among(row, temperature, top_k, top_p, min_p, u):
     """(index, distance of the target from the nearest boundary of the running sum, over the sum) in 64 bits: of equal
