@@ -379,13 +379,13 @@ int launch_rows(const Product& p, int batch, cudaStream_t stream) {
 }
 
 template <int NT>
-int launch_split(const Product& p, int batch, int cuts, bool batched, cudaStream_t stream) {
+int launch_split(const Product& p, int batch, int cuts, bool ahead, cudaStream_t stream) {
   const dim3 grid((unsigned)((p.o + 127) / 128) * cuts, (p.n + NT - 1) / NT, batch);
   if (grid.y > 65535) return FE_ERR_TOO_LARGE;
   const cudaError_t err = cudaFuncSetAttribute(gemm_split_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, gst_smem(NT));
   if (err != cudaSuccess) return (int)err;
   return fe_launch_dependent_shaped(gemm_split_kernel<NT>, grid, dim3(gst_workers(NT) + 32), gst_smem(NT), stream, dim3(cuts, 1, 1), p, cuts,
-                                    batched ? 1 : 0, g_test_fault);
+                                    ahead ? 1 : 0, g_test_fault);
 }
 
 // Rows of x a block takes, and into how many blocks (a cluster) k is cut: the number for which the time below is least.
@@ -410,20 +410,20 @@ int split_cuts(int tile, long long tiles, int k) {
 
 int split_tile(int n) { return n <= 16 ? 16 : n <= 32 ? 32 : n <= 64 ? 64 : 128; }
 
-int split_product(const Product& p, int batch, bool batched, cudaStream_t stream) {
+int split_product(const Product& p, int batch, bool ahead, cudaStream_t stream) {
   const int tile = split_tile(p.n);
   const int cuts = split_cuts(tile, (long long)((p.o + 127) / 128) * ((p.n + tile - 1) / tile) * batch, p.k);
   switch (tile) {
-    case 16: return launch_split<16>(p, batch, cuts, batched, stream);
-    case 32: return launch_split<32>(p, batch, cuts, batched, stream);
-    case 64: return launch_split<64>(p, batch, cuts, batched, stream);
-    default: return launch_split<128>(p, batch, cuts, batched, stream);
+    case 16: return launch_split<16>(p, batch, cuts, ahead, stream);
+    case 32: return launch_split<32>(p, batch, cuts, ahead, stream);
+    case 64: return launch_split<64>(p, batch, cuts, ahead, stream);
+    default: return launch_split<128>(p, batch, cuts, ahead, stream);
   }
 }
 
 // Which kernel: those below give the same bits.
 template <typename TX, typename TW>
-int launch_typed(const Product& p, int batch, bool batched, cudaStream_t stream) {
+int launch_typed(const Product& p, int batch, bool ahead, cudaStream_t stream) {
   if (batch > 65535) return FE_ERR_TOO_LARGE;
   auto whole = [](const void* base, long long ld, long long step, long long k, size_t item) {
     return ((uintptr_t)base & 15) == 0 && (ld * item) % 16 == 0 && (step * item) % 16 == 0 && (k * item) % 16 == 0;
@@ -436,7 +436,7 @@ int launch_typed(const Product& p, int batch, bool batched, cudaStream_t stream)
     // of 4 layers, where a product's weights are asked for ahead, 343 / 325 altogether), 16 x 32,000 x 1,024 72 / 57, 64 x 4,096 x 1,024
     // 43 / 22, 500 x 4,096 x 1,024 119 / 45, 500 x 1,024 x 3,072 111 / 39, 1,024 x 32,000 x 1,024 1,437 / 560.  Shallower than 256
     // a tile's fixed part is more than the sum (500 x 300 x 256 13 / 16).
-    if (vec && p.k >= GST_MIN_K && p.k < (1 << 22) && p.ldx < (1 << 22)) return split_product(p, batch, batched, stream);
+    if (vec && p.k >= GST_MIN_K && p.k < (1 << 22) && p.ldx < (1 << 22)) return split_product(p, batch, ahead, stream);
   }
   const long long big = (long long)((p.o + 63) / 64) * ((p.n + 63) / 64) * batch;
   if (!vec) {
@@ -468,13 +468,13 @@ int launch_typed(const Product& p, int batch, bool batched, cudaStream_t stream)
   return launch_tile<TX, TW, 4, 4, 8, 8, true>(p, batch, stream);
 }
 
-int launch_coded(int x_dtype, int w_dtype, const Product& p, int batch, bool batched, cudaStream_t stream) {
+int launch_coded(int x_dtype, int w_dtype, const Product& p, int batch, bool ahead, cudaStream_t stream) {
   if ((p.y_dtype | x_dtype | w_dtype) & ~1) return FE_ERR_BAD_DTYPE;
   switch (x_dtype * 2 + w_dtype) {
-    case 0: return launch_typed<float, float>(p, batch, batched, stream);
-    case 1: return launch_typed<float, bf16>(p, batch, batched, stream);
-    case 2: return launch_typed<bf16, float>(p, batch, batched, stream);
-    default: return launch_typed<bf16, bf16>(p, batch, batched, stream);
+    case 0: return launch_typed<float, float>(p, batch, ahead, stream);
+    case 1: return launch_typed<float, bf16>(p, batch, ahead, stream);
+    case 2: return launch_typed<bf16, float>(p, batch, ahead, stream);
+    default: return launch_typed<bf16, bf16>(p, batch, ahead, stream);
   }
 }
 
@@ -493,12 +493,14 @@ FE_EXPORT int fe_gemm_split_cuts(int n, int o, int k, int batch) {
   return split_cuts(tile, (long long)((o + 127) / 128) * ((n + tile - 1) / tile) * batch, k);
 }
 
+// `ahead`: w is complete before the call is made and no kernel that may still run writes it (a layer's weights), so that it may be
+// read while the kernels before this one still run.  Without it w may be what the kernel before wrote.
 FE_EXPORT int fe_gemm_simt(const void* x, int x_dtype, const void* w, int w_dtype, const float* bias,
-                           void* y, int y_dtype, int n, int o, int k, int accumulate,
+                           void* y, int y_dtype, int n, int o, int k, int accumulate, int ahead,
                            int* status, cudaStream_t stream) {
   if (n <= 0 || o <= 0) return 0;
   if (k <= 0) return FE_ERR_BAD_SHAPE;
-  return launch_coded(x_dtype, w_dtype, Product{x, w, bias, y, y_dtype, n, o, k, accumulate, status, k, o, 0, 0, 0}, 1, false, stream);
+  return launch_coded(x_dtype, w_dtype, Product{x, w, bias, y, y_dtype, n, o, k, accumulate, status, k, o, 0, 0, 0}, 1, ahead != 0, stream);
 }
 
 // `batch` products at once (one per head): product b reads x + b * batch_x (rows ldx apart),
@@ -510,5 +512,5 @@ FE_EXPORT int fe_gemm_simt_batched(const void* x, int x_dtype, const void* w, in
   if (n <= 0 || o <= 0 || batch <= 0) return 0;
   if (k <= 0 || ldx < k || ldy < o) return FE_ERR_BAD_SHAPE;
   return launch_coded(x_dtype, w_dtype, Product{x, w, nullptr, y, y_dtype, n, o, k, 0, status, ldx, ldy, batch_x, batch_w, batch_y},
-                      batch, true, stream);
+                      batch, false, stream);
 }

@@ -185,7 +185,7 @@ __device__ __forceinline__ void gst_multiply(const unsigned char* stage, unsigne
 }
 
 template <int NT>
-__global__ void __launch_bounds__(gst_workers(NT) + 32, NT <= 32 ? 2 : 1) gemm_split_kernel(const __grid_constant__ Product p, int cuts, int batched, const Fault fault) {
+__global__ void __launch_bounds__(gst_workers(NT) + 32, NT <= 32 ? 2 : 1) gemm_split_kernel(const __grid_constant__ Product p, int cuts, int ahead, const Fault fault) {
   constexpr int WORKERS = gst_workers(NT);
   constexpr int COLS = NT * 128 / WORKERS, STEP = 8;          // columns of a thread, and of a piece of them
   constexpr int STAGES = gst_stages(NT);
@@ -216,9 +216,9 @@ __global__ void __launch_bounds__(gst_workers(NT) + 32, NT <= 32 ? 2 : 1) gemm_s
                  "r"(gst_tmem_cols(NT)) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  // Weights: nobody writes them meanwhile, so they do not wait for the kernel before: the first stages of them are split, and
-  // L2 is asked for the first stretches (a row each thread.  2 stretches: 4 x 32,000 x 1,024 55 us, 8 58, all 61, none 57).
-  if (!batched && blockIdx.y == 0 && threadIdx.x < 128 && col0 + (int)threadIdx.x < p.o && count > 0) {
+  // With `ahead` w is not the result of an earlier kernel that may still run, and does not wait for it: the first stages of w are
+  // split, and L2 is asked for the first stretches (a row each thread.  2 stretches: 4 x 32,000 x 1,024 55 us, 8 58, all 61, none 57).
+  if (ahead && blockIdx.y == 0 && threadIdx.x < 128 && col0 + (int)threadIdx.x < p.o && count > 0) {
     const int k_begin = s_begin * GST_K, bytes = (min(p.k, min(s_end, s_begin + GST_L2) * GST_K) - k_begin) * 4;
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(w + (size_t)threadIdx.x * p.k + k_begin), "r"(bytes) : "memory");
   }
@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(gst_workers(NT) + 32, NT <= 32 ? 2 : 1) gemm_s
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const unsigned tmem = *tmem_slot;
   pdl_trigger();         // after the allocation: a block of the next kernel that held the columns would wait for this one's end
-  if (batched) pdl_wait();
+  if (!ahead) pdl_wait();
 
   bool ok = true;
   unsigned again = 0u;       // sums of this thread that are taken again, at the end
@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(gst_workers(NT) + 32, NT <= 32 ? 2 : 1) gemm_s
       for (unsigned t = 0; t < tc5::WAIT_LIMIT && !ended; ++t) ended = tc5::mbar_try_wait(&done[(issued - 1) % STAGES], ((issued - 1) / STAGES) & 1);
     }
     __syncwarp();
-    if (!batched) pdl_wait();
+    if (ahead) pdl_wait();
   } else {
     const int quarter = warp & 3, column = (warp >> 2) * COLS;
     const unsigned mine = tmem + ((unsigned)(quarter * 32) << 16) + column;
@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(gst_workers(NT) + 32, NT <= 32 ? 2 : 1) gemm_s
     float acc[COLS];
 #pragma unroll
     for (int c = 0; c < COLS; ++c) acc[c] = 0.f;
-    const int split_ahead = batched ? 0 : min(count, STAGES);
+    const int split_ahead = ahead ? min(count, STAGES) : 0;
     // stretch i of this block's, and past the last one that again
     auto k_of = [&](int i) { return (s_begin + min(i, count - 1)) * GST_K; };
     if (count > 0) a.load(w + k_of(0), p.k - k_of(0));
@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(gst_workers(NT) + 32, NT <= 32 ? 2 : 1) gemm_s
       a.put(smem + i * gst_stage_bytes(NT), p.k - k_of(i));
       a.load(w + k_of(i + 1), p.k - k_of(i + 1));
     }
-    if (!batched) pdl_wait();
+    if (ahead) pdl_wait();
     if (count > 0) b.load(x + k_of(0), p.k - k_of(0));
     // The lanes of a warp part where a row ends, where a value is not finite and where one of them speaks for all; what the whole
     // warp executes together (tensor memory, cluster barriers) stands behind a __syncwarp or a vote.

@@ -92,7 +92,7 @@ def _declare(handle: ctypes.CDLL) -> None:
         "fe_attention_simt_scratch": [i, i, i, i, i, i],
         "fe_attention_simt_units": [i, i, i, i, i, i],
         "fe_attention_simt_tile_scratch": [i, i, i, i, i, i, i],
-        "fe_gemm_simt": [p, i, p, i, p, p, i, i, i, i, i, p, p],
+        "fe_gemm_simt": [p, i, p, i, p, p, i, i, i, i, i, i, p, p],
         "fe_sample": [p, i, i, p, p, p, p, p, p, p, p, p],
         "fe_sample_rows": [p, i, i, ctypes.c_char_p, p, p, p],
         "fe_gemm_tc5": [p, p, p, p, i, i, i, i, i, p, p, p, f, f, p],
@@ -1059,7 +1059,7 @@ def linear_recurrence(
 
 
 def gemm_simt_batched(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, status: torch.Tensor | None = None) -> None:
-    """out[n, b, :] = x[n, b, :] @ w[b].T with plain 32-bit FMAs, for x [n, batch, k] and out
+    """out[n, b, :] = x[n, b, :] @ w[b].T in 32 bits (as ``gemm_simt``), for x [n, batch, k] and out
     [n, batch, o] that may be strided in their first two extents, and w [batch, o, k]
     contiguous.  ``status`` as in ``gemm_simt``."""
     _dense(w, "w")
@@ -1586,9 +1586,12 @@ def gemm_simt(
     bias: torch.Tensor | None = None,
     accumulate: bool = False,
     status: torch.Tensor | None = None,
+    ahead: bool = False,
 ) -> None:
-    """out = x @ w.T (+ bias) (+ out) with plain 32-bit FMAs; w is [out, in].  A wait that runs out inside the kernel
-    for few rows sets its bit in the device word ``status`` and leaves NaN."""
+    """out = x @ w.T (+ bias) (+ out) in 32 bits; w is [out, in].  Deep products of 32-bit operands run on the tensor cores, both
+    split into three bfloat16 numbers, others as chains of multiply-adds.  A wait that runs out inside a kernel sets its bit in the
+    device word ``status`` and leaves NaN.  ``ahead``: w is a layer's weights, which no kernel of the step writes; they may be
+    read while the kernels before this one still run."""
     _dense(x, "x"), _dense(w, "w"), _dense(out, "out")
     n, k = x.shape
     o = w.shape[0]
@@ -1596,7 +1599,7 @@ def gemm_simt(
     assert bias is None or (bias.dtype == torch.float32 and bias.numel() == o)
     check(
         lib().fe_gemm_simt(ptr(x), code(x), ptr(w), code(w), ptr(bias), ptr(out), code(out), n, o, k,
-                           1 if accumulate else 0, ptr(status), stream()),
+                           1 if accumulate else 0, 1 if ahead else 0, ptr(status), stream()),
         "gemm_simt",
     )
 

@@ -90,7 +90,7 @@ class Linear:
             if bias is not None and out_dtype == torch.float32 and _addmm_out_dtype_works(x.device):
                 return torch.addmm(bias, x, self.weight.t(), out_dtype=torch.float32)
         out = torch.empty((n, self.out_features), dtype=out_dtype, device=x.device)
-        native.gemm_simt(x, self.weight, out, bias, status=self.status)
+        native.gemm_simt(x, self.weight, out, bias, status=self.status, ahead=True)
         return out
 
 

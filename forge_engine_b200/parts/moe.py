@@ -175,7 +175,7 @@ class RoutedMLP(FeedForward):
             if self.width <= 48 * 1024:
                 native.moe_logits(x, self.router, logits, self.router_bias)
             else:
-                native.gemm_simt(x, self.router, logits, self.router_bias, status=self.ctx.status)
+                native.gemm_simt(x, self.router, logits, self.router_bias, status=self.ctx.status, ahead=True)
         tile_rows = self.tile_rows(slots) if self.fused else 0
         max_tiles = native.moe_max_tiles(slots, self.experts, tile_rows)
         with section("ffn.route"):

@@ -636,6 +636,30 @@ def test_products_without_a_finite_sum_are_chains(native, n, o, k):
         assert not bool(got.isfinite().any())
 
 
+@pytest.mark.parametrize("n, o, k", ((4, 2048, 1024), (40, 3000, 512), (300, 4224, 1024)))
+def test_operands_that_the_kernel_before_writes(native, n, o, k):
+    """Both operands are products of the kernels right before, which let the next one start early: the same bits as with the
+    device idle in between.  New operands in every turn, so that whoever reads too soon finds those of the turn before."""
+    gen = torch.Generator(device=DEV).manual_seed(n)
+    rand = lambda *shape: torch.randn(shape, generator=gen, device=DEV)  # noqa: E731
+    x, w, got, want = torch.empty((n, k), device=DEV), torch.empty((o, k), device=DEV), torch.empty((n, o), device=DEV), torch.empty((n, o), device=DEV)
+
+    def chain(left, right, mix, out, pause):
+        torch.cuda.synchronize()
+        for a, b in ((left, x), (right, w)):
+            native.gemm_simt(a, mix, b)
+            pause()
+        native.gemm_simt(x, w, out)
+        torch.cuda.synchronize()
+
+    for _ in range(6):
+        left, right, mix = rand(n, 256), rand(o, 256), rand(k, 256) / 16
+        chain(left, right, mix, got, lambda: None)
+        chain(rand(n, 256), rand(o, 256), mix, want, torch.cuda.synchronize)
+        chain(left, right, mix, want, torch.cuda.synchronize)
+        assert torch.equal(got, want)
+
+
 # -- the largest logits alone ------------------------------------------------------------------------
 def drawn_among(row, temperature, top_k, top_p, min_p, u):
     """(index, distance of the target from the nearest boundary of the running sum, over the sum) in 64 bits: of equal
