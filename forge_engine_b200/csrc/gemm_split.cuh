@@ -1,7 +1,8 @@
 // 32-bit products of deep rows on the 5th-generation tensor cores (part of gemm_simt.cu).
 //
 // Every operand is split into three bfloat16 numbers on its way to shared memory: x = a + b + c, each rounded to
-// nearest of what the ones before left, so that nothing of the 24 bits is lost.  x y is taken as
+// nearest of what the ones before left, so that nothing of the 24 bits of a number from 2^-110 on is lost (of smaller ones
+// what lies below 2^-133, where bfloat16 ends).  x y is taken as
 // (ab + ba + bb + ac + ca) + aa; the three products left out are 2^-25 of x y and below.  The products of 64 k are
 // summed in tensor memory, the small ones first; what a stretch of 64 gives is added to the 32-bit sum outside, rounded
 // to nearest, because the tensor core cuts off what falls below the 24 bits of its sum.  Of the eight parts of k
@@ -21,10 +22,12 @@
 // operands, depth 256 / 1,024 / 3,072: 0.9e-7, 1.0e-7 and 1.1e-7 (of it along the result -0.6e-7); one chain of 32-bit
 // multiply-adds 2.9e-7, 5.7e-7 and 9.9e-7.
 //
-// A sum that is not finite is taken again as one chain of multiply-adds, so that infinities and numbers that round to
-// infinity give what they give there; a warp takes the chains of eight rows of x together.  1,024 x 32,000 x 1,024: 0.54 ms
-// finite, 0.65 with a NaN in one row, 0.80 in one column, 8.2 in every row (every lane its own chains, one after the other: 0.66,
-// 1.5 and 124; multiply-adds alone 1.44).
+// A sum that is not finite, or not zero and below 2^-70, is taken again as one chain of multiply-adds: so infinities, numbers
+// that round to infinity and rows of numbers that bfloat16 does not hold give what they give there.  (Numbers about 2^-118 are
+// off by 9e-6 of themselves in three parts, about 2^-126 by 2e-3.  What they lose moves a sum from 2^-70 on by less than 2^-24 of
+// it while the other operand's numbers add up to less than 2^40; where all numbers are below 2^-134 the sum is zero.)
+// A warp takes the chains of eight rows of x together.  1,024 x 32,000 x 1,024: 0.54 ms finite, 0.65 with a NaN in one row, 0.80 in
+// one column, 8.2 in every row (every lane its own chains, one after the other: 0.66, 1.5 and 124; multiply-adds alone 1.44).
 #pragma once
 #include "tcgen05.cuh"
 
@@ -32,6 +35,7 @@
 #define GST_PARTS 8
 #define GST_L2 2             // stretches of w asked for ahead
 #define GST_MIN_K 256        // depth from which on 32-bit operands go this way
+#define GST_SMALL 8.4703295e-22f     // 2^-70
 
 namespace {
 
@@ -108,7 +112,7 @@ __device__ __forceinline__ void gst_tmem_store8(unsigned taddr, const float* v) 
                "r"(__float_as_uint(v[4])), "r"(__float_as_uint(v[5])), "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7])) : "memory");
 }
 
-// The chains of multiply-adds that take the place of sums that are not finite (bits of `which`): N rows of x, `step` apart from
+// The chains of multiply-adds that take the place of sums (bits of `which`): N rows of x, `step` apart from
 // `row` on (the last one again where the product has no more), with this lane's row of w.  A warp takes them together: a row of w
 // is then read once for N chains, and they fill one another's waits.
 template <int N>
@@ -134,7 +138,7 @@ __device__ __noinline__ void gst_chains(const Product& p, int row, int step, int
 // Stores a sum, or says that it has to be taken again.
 __device__ __forceinline__ unsigned gst_finish(const Product& p, float v, int row, int col, bool ok) {
   if (row >= p.n || col >= p.o) return 0u;
-  if (ok && !isfinite(v)) return 1u;
+  if (ok && !(v == 0.f || (fabsf(v) >= GST_SMALL && isfinite(v)))) return 1u;
   gs_store(p, ok ? v : __int_as_float(0x7fffffff), row, col);
   return 0u;
 }

@@ -660,6 +660,30 @@ def test_operands_that_the_kernel_before_writes(native, n, o, k):
         assert torch.equal(got, want)
 
 
+@pytest.mark.parametrize("exponent", (-100, -111, -118, -126, -130))
+@pytest.mark.parametrize("n, o, k", ((3, 300, 1024), (40, 150, 256), (300, 4224, 448)))
+def test_deep_product_of_small_numbers(native, n, o, k, exponent):
+    """Rows of either operand whose numbers lie where bfloat16 ends (2^-133): no further from 64 bits than a chain of
+    multiply-adds may be, (k + 1) 2^-24 of the sum of magnitudes and half a step of 2^-149 an addition.  Zeros stay zeros,
+    and the other rows and columns keep their bits."""
+    gen = torch.Generator().manual_seed(n - exponent)
+    x, w = torch.randn((n, k), generator=gen).to(DEV), torch.randn((o, k), generator=gen).to(DEV)
+    clean, got = torch.empty((n, o), device=DEV), torch.empty((n, o), device=DEV)
+    native.gemm_simt(x, w, clean)
+    rows, columns = [0, n // 2], [5, o - 1]
+    x[rows], w[columns] = (x[rows].double() * 2.0**exponent).float(), (w[columns].double() * 2.0**exponent).float()
+    x[n - 1], w[o // 2] = 0.0, 0.0
+    native.gemm_simt(x, w, got)
+    want, size = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+    assert bool(((got.double() - want).abs() <= size * (k + 1) * 2.0**-24 + k * 2.0**-149).all())
+    off = (got.double() - want)[rows][:, 6 : o // 2].norm() / want[rows][:, 6 : o // 2].norm()
+    assert float(off) < (2e-6 if exponent > -120 else 1e-5)
+    assert float(got[n - 1].abs().max()) == float(got[:, o // 2].abs().max()) == 0.0
+    keep = torch.ones((n, o), dtype=torch.bool, device=DEV)
+    keep[rows + [n - 1]], keep[:, columns + [o // 2]] = False, False
+    assert torch.equal(got[keep], clean[keep])
+
+
 # -- the largest logits alone ------------------------------------------------------------------------
 def drawn_among(row, temperature, top_k, top_p, min_p, u):
     """(index, distance of the target from the nearest boundary of the running sum, over the sum) in 64 bits: of equal
