@@ -144,7 +144,7 @@ __device__ __forceinline__ unsigned gst_finish(const Product& p, float v, int ro
 }
 
 __host__ __device__ constexpr int gst_stage_bytes(int nt) { return 3 * (128 + nt) * 128; }
-// Threads that read, split and add up: with few rows of x half as many, so that two blocks share an SM.
+// Threads that read, split and add up: with few rows of x half as many, so that (up to 16 rows: 110 KB a block) two blocks share an SM.
 __host__ __device__ constexpr int gst_workers(int nt) { return nt <= 32 ? 256 : 512; }
 __host__ __device__ constexpr int gst_stages(int nt) { return nt == 64 ? 3 : 2; }
 __host__ __device__ constexpr int gst_smem(int nt) { return gst_stages(nt) * gst_stage_bytes(nt) + 1024 + 128; }
@@ -189,7 +189,7 @@ __device__ __forceinline__ void gst_multiply(const unsigned char* stage, unsigne
 }
 
 template <int NT>
-__global__ void __launch_bounds__(gst_workers(NT) + 32, NT <= 32 ? 2 : 1) gemm_split_kernel(const __grid_constant__ Product p, int cuts, int ahead, const Fault fault) {
+__global__ void __launch_bounds__(gst_workers(NT) + 32, NT <= 16 ? 2 : 1) gemm_split_kernel(const __grid_constant__ Product p, int cuts, int ahead, const Fault fault) {
   constexpr int WORKERS = gst_workers(NT);
   constexpr int COLS = NT * 128 / WORKERS, STEP = 8;          // columns of a thread, and of a piece of them
   constexpr int STAGES = gst_stages(NT);
