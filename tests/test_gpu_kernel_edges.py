@@ -99,6 +99,30 @@ def test_a_wait_that_runs_out_is_reported(native, n, o, k):
     assert torch.equal(again, good)
 
 
+@pytest.mark.parametrize("xd, wd", [(torch.float32, torch.bfloat16), (torch.bfloat16, torch.float32), (torch.bfloat16, torch.bfloat16), (torch.float32, torch.float32)])
+@pytest.mark.parametrize("n, o, k", ((1, 100, 1152), (4, 5000, 2048), (16, 9000, 1152), (4, 40100, 1024)))
+def test_a_wait_that_runs_out_in_either_kernel_for_few_rows(native, xd, wd, n, o, k):
+    """The kernel of multiply-adds, whose ring these depths go round (operands of mixed types and of 16 bits go there whatever their
+    depth), and the one on the tensor cores where one block takes all of k."""
+    assert xd != wd or wd != torch.float32 or o < 40000 or native.lib().fe_gemm_split_cuts(n, o, k, 1) == 1
+    gen = torch.Generator().manual_seed(o)
+    x, w = torch.randn((n, k), generator=gen).to(xd).to(DEV), torch.randn((o, k), generator=gen).to(wd).to(DEV)
+    good, bad, again = (torch.empty((n, o), device=DEV) for _ in range(3))
+    status = status_word()
+    native.gemm_simt(x, w, good, status=status)
+    bound = (x.double().abs() @ w.double().abs().t()) * (k + 1) * 2.0**-24
+    assert int(status.item()) == 0 and bool(((good.double() - x.double() @ w.double().t()).abs() <= bound).all())
+    try:
+        native.gemm_simt_set_test_fault(2000, 2)
+        native.gemm_simt(x, w, bad, status=status)
+        torch.cuda.synchronize()
+    finally:
+        native.gemm_simt_set_test_fault()
+    assert int(status.item()) == 8 and not bool(torch.isfinite(bad).any())
+    native.gemm_simt(x, w, again, status=status_word())
+    assert torch.equal(again, good)
+
+
 def test_layers_give_products_their_status_word(native, monkeypatch):
     from forge_engine_b200.parts.linear import Linear
 
@@ -106,6 +130,22 @@ def test_layers_give_products_their_status_word(native, monkeypatch):
     monkeypatch.setattr(native, "gemm_simt", lambda *args, status=None, **kw: seen.append(status))
     Linear(torch.randn(8, 16, device=DEV), status=status)(torch.randn(2, 16, device=DEV))
     assert len(seen) == 1 and seen[0] is status
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("n, rows, k", ((1185, 8, 36), (1186, 3, 37), (1187, 9, 48), (1184, 8, 1), (600, 12, 130), (593, 16, 6400), (593, 16, 6408)))
+def test_router_logits_of_many_tokens(native, dtype, n, rows, k):
+    """Four tokens a block, with a rest of one to three and widths off eight and off four: the bits of a token a block (few
+    tokens go there), and within a chain's bound of 64 bits.  The last width is the first whose four tokens do not fit."""
+    gen = torch.Generator().manual_seed(n + k)
+    x, w, bias = torch.randn((n, k), generator=gen).to(dtype).to(DEV), torch.randn((rows, k), generator=gen).to(DEV), torch.randn(rows, generator=gen).to(DEV)
+    got, alone = torch.empty((n, rows), device=DEV), torch.empty((n, rows), device=DEV)
+    native.moe_logits(x, w, got, bias)
+    for at in range(0, n, 100):
+        native.moe_logits(x[at : at + 100].contiguous(), w, alone[at : at + 100], bias)
+    assert torch.equal(got, alone)
+    bound = (x.double().abs() @ w.double().abs().t() + bias.double().abs()) * (k + 2) * 2.0**-24
+    assert bool(((got.double() - x.double() @ w.double().t() - bias.double()).abs() <= bound).all())
 
 
 # -- 32-bit attention --------------------------------------------------------------------------------
@@ -142,6 +182,39 @@ def test_attention_of_entries(native, dtype, nq, nkv, d, page, window):
         assert torch.equal(attend(rows, table[e : e + 1].contiguous(), [0, count]), together[rows])
         want = dense_attention(q[rows], keys[e], values[e], torch.tensor([positions[r] for r in rows]), d ** -0.5, window)
         mine = together[rows].view(count, nq, d).double().cpu()
+        torch.testing.assert_close(mine, want, **(dict(atol=2e-5, rtol=1e-5) if dtype == torch.float32 else dict(atol=2e-2, rtol=2e-2)))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("nq, nkv, d, window", [(32, 32, 64, None), (30, 30, 40, 150), (16, 16, 128, 300), (32, 16, 256, None)])
+def test_attention_of_portions_that_fill_the_chip(native, dtype, nq, nkv, d, window):
+    """A portion of enough row tiles that a block folds all spans of its rows itself, after cached keys and beside a shorter
+    one: the bits of the same tokens in pieces small enough that every span has blocks of its own, and the dense result."""
+    page, lengths, counts = 16, [900, 300], [840, 33]
+    k_cache, v_cache, table, keys, values = paged_layout(lengths, page, nkv, d, dtype, seed=d)
+    positions = [p for n, c in zip(lengths, counts) for p in range(n - c, n)]
+    entry = [e for e, c in enumerate(counts) for _ in range(c)]
+    q = torch.randn((len(positions), nq, d), generator=torch.Generator().manual_seed(5)).to(dtype)
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)  # noqa: E731
+    floats, status = native.lib().fe_attention_simt_tile_scratch, status_word()
+
+    def attend(rows, table, cu):
+        out = torch.empty((len(rows), nq * d), dtype=dtype, device=DEV)
+        native.attention_simt(q[rows].reshape(len(rows), nq * d).to(DEV), nq * d, k_cache, v_cache, table, ints([positions[r] for r in rows]),
+                              ints([0 if table.shape[0] == 1 else entry[r] for r in rows]), window, d ** -0.5, out, nq, status,
+                              entries=(ints(cu), len(cu) - 1, max(b - a for a, b in zip(cu, cu[1:]))))
+        return out
+
+    assert floats(len(positions), 2, nq, nkv, d, table.shape[1], page) == 0
+    together = attend(list(range(len(positions))), table, [0, 840, 873])
+    for first, last in ((0, 31), (31, 64), (64, 164), (164, 290), (290, 417), (417, 500), (740, 840), (840, 873)):
+        one = table[entry[first] : entry[first] + 1].contiguous()
+        assert floats(last - first, 1, nq, nkv, d, one.shape[1], page) > 0
+        assert torch.equal(attend(list(range(first, last)), one, [0, last - first]), together[first:last]), first
+    assert int(status.item()) == 0
+    for e, at in ((0, 0), (1, 840)):
+        want = dense_attention(q[at : at + counts[e]], keys[e], values[e], torch.tensor(positions[at : at + counts[e]]), d ** -0.5, window)
+        mine = together[at : at + counts[e]].view(counts[e], nq, d).double().cpu()
         torch.testing.assert_close(mine, want, **(dict(atol=2e-5, rtol=1e-5) if dtype == torch.float32 else dict(atol=2e-2, rtol=2e-2)))
 
 
