@@ -6,6 +6,8 @@
 // cores (gemm_split.cuh); for the others each output element is summed over k in ascending order by one
 // thread, in both kernels below.  Which of the two does not depend on the number of rows, so a row's result
 // does not depend on how many other rows are in the call, nor on the tile.
+// (A row's bits do depend on which of the two it is: from 256 numbers on, where both operands are 32 bits and lie on 16 bytes,
+// rows and strides too and below 2^22 numbers, the tensor cores; a layer's products are all of one kind.)
 //
 // Tiles of both operands lie in shared memory as they lie in memory, rows of k with 16 bytes
 // of padding, so that a 16-byte read of 4 k by eight neighbouring rows touches every bank once.
@@ -432,9 +434,10 @@ int launch_typed(const Product& p, int batch, bool ahead, cudaStream_t stream) {
                    whole(p.w, p.k, batch > 1 ? p.batch_w : 0, p.k, sizeof(TW));
   if constexpr (sizeof(TX) == 4 && sizeof(TW) == 4) {
     // Deep rows of 32-bit numbers go to the tensor cores, however many there are, so that a row's bits do not depend on that.  us,
-    // the kernels below against those: 4 x 4,096 x 1,024 14 / 18, 4 x 1,024 x 3,072 18 / 20, 4 x 32,000 x 1,024 45 / 55 (in a decode step
-    // of 4 layers, where a product's weights are asked for ahead, 343 / 325 altogether), 16 x 32,000 x 1,024 72 / 57, 64 x 4,096 x 1,024
-    // 43 / 22, 500 x 4,096 x 1,024 119 / 45, 500 x 1,024 x 3,072 111 / 39, 1,024 x 32,000 x 1,024 1,437 / 560.  Shallower than 256
+    // the kernels below against those: alone, up to four rows lose, 4 x 4,096 x 1,024 14.6 / 17.3, 4 x 6,144 x 1,024 19.4 / 20.5,
+    // 4 x 32,000 x 1,024 46 / 51, 4 x 1,024 x 3,072 19.4 / 19.4 (in a decode step of 4 layers, where a product's weights are asked for
+    // ahead, 343 / 326 altogether); 16 x 4,096 x 1,024 20.5 / 17.3, 16 x 32,000 x 1,024 72 / 52, 32 x 32,000 x 1,024 116 / 60, 64 x 4,096 x
+    // 1,024 43 / 20, 500 x 4,096 x 1,024 118 / 43, 500 x 1,024 x 3,072 111 / 36, 1,024 x 32,000 x 1,024 1,439 / 540.  Shallower than 256
     // a tile's fixed part is more than the sum (500 x 300 x 256 13 / 16).
     if (vec && p.k >= GST_MIN_K && p.k < (1 << 22) && p.ldx < (1 << 22)) return split_product(p, batch, ahead, stream);
   }
@@ -447,10 +450,12 @@ int launch_typed(const Product& p, int batch, bool ahead, cudaStream_t stream) {
     if (p.n > 32 && (big >= 296 || (p.n <= 64 && big >= 64))) return launch_tile<TX, TW, 8, 4, 8, 16, false>(p, batch, stream);
     return launch_tile<TX, TW, 4, 4, 8, 8, false>(p, batch, stream);
   }
-  // Few rows: as many columns a block as still give every SM one.  Measured with 32-bit operands, us
-  // (8 / 16 / 32 columns): 4 x 1,024 x 3,072 14.7 / 16.0 / 16.8, 4 x 4,096 x 1,024 9.1 / 7.9 / 9.6,
-  // 4 x 32,000 x 1,024 43 / 44 / 36; 16 x 1,024 x 3,072 23.0 / 25.7 / 26.7, 16 x 4,096 x 1,024 18.4 / 13.4 / 16.6,
-  // 16 x 32,000 x 1,024 115 / 78 / 66 (the 64 x 64 tiles that all sizes took before: 57 to 180).
+  // From here on operands of which one or both are bfloat16, and 32-bit ones shallower than 256.  Few rows: as many columns a
+  // block as still give every SM one.  Measured, us (8 / 16 / 32 columns), bfloat16 weights, then bfloat16 rows, then both:
+  // 4 x 1,024 x 3,072 19.4 / 22.5 / 20.5, 20.5 / 25.5 / 21.3, 22.5 / 26.7 / 22.6; 4 x 4,096 x 1,024 14.3 / 13.3 / 12.4,
+  // 15.2 / 15.3 / 13.3, 15.1 / 14.4 / 12.4; 4 x 32,000 x 1,024 42 / 36 / 37, 51 / 49 / 43, 43 / 39 / 40; 16 x 1,024 x 3,072
+  // 20.5 / 22.6 / 30.8, 20.5 / 25.6 / 36.9, 22.6 / 28.7 / 39.9; 16 x 4,096 x 1,024 22.6 / 17.4 / 15.4, 27.6 / 18.5 / 18.5,
+  // 22.6 / 18.5 / 18.6; 16 x 32,000 x 1,024 107 / 75 / 67, 99 / 81 / 70, 98 / 82 / 74.
   if (p.n <= 4) {
     if (p.o <= 2048) return launch_rows<TX, TW, 8, 8, 1>(p, batch, stream);
     if (p.o <= 8192) return launch_rows<TX, TW, 16, 16, 2>(p, batch, stream);
@@ -461,10 +466,14 @@ int launch_typed(const Product& p, int batch, bool ahead, cudaStream_t stream) {
     if (p.o <= 8192) return launch_rows<TX, TW, 16, 8, 2>(p, batch, stream);
     return launch_rows<TX, TW, 32, 16, 4>(p, batch, stream);
   }
-  // Many rows: tiles of 64 x 64 by 128 threads (8 x 4 each) where they fill the SMs twice, else of
-  // 32 x 32 by 64 threads: 500 x 1,024 x 3,072 165 us against 211, 2,000 x 4,096 x 1,024 415 against 371 (45 TFLOP/s),
-  // 64 x 4,096 x 1,024 43 against 37; 256 threads with 4 x 4 each, as before, 227 and 412.
-  if (big >= 296 || (p.n <= 64 && big >= 64)) return launch_tile<TX, TW, 8, 4, 8, 16, true>(p, batch, stream);
+  // Many rows: tiles of 64 x 64 by 128 threads (8 x 4 each) where there are about as many as the chip holds twice, else of
+  // 32 x 32 by 64 threads.  Measured, us (32 x 32 / 64 x 64), bfloat16 weights, then bfloat16 rows, then shallow 32-bit products
+  // (k 192): 20 x 32,000 x 1,024 74 / 119, 72 / 117, 23 / 29; 64 x 4,096 x 1,024 31 / 45, 33 / 43, 12.3 / 16.4; 48 x 8,192 x 1,024
+  // 45.2 / 43.7, 45.1 / 43.0, 14.4 / 16.4; 64 x 32,000 x 1,024 137 / 122, 127 / 119, 35 / 31; 100 x 8,192 x 3,072 199 / 193,
+  // 199 / 188, 20.5 / 20.5; 200 x 2,048 x 1,024 45.1 / 45.1, 43.0 / 43.7, 14.3 / 16.4; 200 x 16,384 x 3,072 656 / 580, 655 / 576, 49 / 47.
+  // (The line of 64 tiles up to 64 rows that 32-bit products once had cost 20 to 64 rows of these up to 1.7 times the time.)
+  constexpr int LINE = sizeof(TX) + sizeof(TW) == 8 ? 296 : 256;       // shallow 32-bit ones: 200 x 4,096 x 192 18.5 / 20.5
+  if (p.n > 32 && (big >= LINE || (p.n <= 64 && big >= 128))) return launch_tile<TX, TW, 8, 4, 8, 16, true>(p, batch, stream);
   return launch_tile<TX, TW, 4, 4, 8, 8, true>(p, batch, stream);
 }
 
@@ -480,8 +489,8 @@ int launch_coded(int x_dtype, int w_dtype, const Product& p, int batch, bool ahe
 
 }  // namespace
 
-// For tests of the bounded waits only: later launches of the kernel for few rows poll at most `wait_limit` times per
-// wait (0: the usual bound) and their loaders do not report stretch `skip_stretch` of k (-1: none), so that the
+// For tests of the bounded waits only: later launches of the kernel for few rows and of the one on the tensor cores poll at most
+// `wait_limit` times per wait (0: the usual bound) and do not report stretch `skip_stretch` of 128 k (-1: none), so that the
 // block gives up, sets FE_STATUS_WAIT_TIMEOUT and returns.  Call with (0, -1) to go back to normal.
 FE_EXPORT void fe_gemm_simt_set_test_fault(unsigned wait_limit, int skip_stretch) {
   g_test_fault = Fault{wait_limit ? wait_limit : tc5::WAIT_LIMIT, skip_stretch};

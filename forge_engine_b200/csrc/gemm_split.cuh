@@ -18,7 +18,7 @@
 //
 // What bounds it: with 128 rows of x the instructions that split (a stretch takes 3,100 cycles, of which its products need
 // 1,536); with 16 a stretch's chain of load, split, 24 products of 35 cycles each to issue, and sum (2,200 cycles).
-// 500 x 4,096 x 1,024 takes 45 us, 500 x 1,024 x 3,072 39 (multiply-adds: 119 and 111).  Relative error against 64 bits, random normal
+// 500 x 4,096 x 1,024 takes 43 us, 500 x 1,024 x 3,072 36 (multiply-adds: 118 and 111).  Relative error against 64 bits, random normal
 // operands, depth 256 / 1,024 / 3,072: 0.9e-7, 1.0e-7 and 1.1e-7 (of it along the result -0.6e-7); one chain of 32-bit
 // multiply-adds 2.9e-7, 5.7e-7 and 9.9e-7.
 //

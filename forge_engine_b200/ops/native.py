@@ -1605,8 +1605,8 @@ def gemm_simt(
 
 
 def gemm_simt_set_test_fault(wait_limit: int = 0, skip_stretch: int = -1) -> None:
-    """For tests of the bounded waits: later ``gemm_simt`` launches for few rows poll at most ``wait_limit`` times per
-    wait (0: the usual bound) and do not report stretch ``skip_stretch`` of 128 k (-1: none)."""
+    """For tests of the bounded waits: later ``gemm_simt`` launches for few rows or on the tensor cores poll at most
+    ``wait_limit`` times per wait (0: the usual bound) and do not report stretch ``skip_stretch`` of 128 k (-1: none)."""
     fn = lib().fe_gemm_simt_set_test_fault
     fn.argtypes, fn.restype = [ctypes.c_uint, c_int], None
     fn(int(wait_limit), int(skip_stretch))
