@@ -738,12 +738,16 @@ static int resident_clusters(int parts) {
 }
 
 // How many blocks share a row: the number for which the rounds of clusters that run at once, times what a
-// block's slice takes, is least.  A slice takes 30 us and 1.4 us per 1,000 logits where it is kept in shared
-// memory, 45 and 1.85 where every pass reads it again, from L2 (3.3 where the rows at hand do not fit there); top-k 50
-// and top-p 0.95.  Measured, 1 / 2 / 4 / 8 blocks a row, us: 8 rows of
+// block's slice takes, is least.  The times are those of the passes over the row (no top-k, or one past 512): a slice takes 30 us and
+// 1.4 us per 1,000 logits where it is kept in shared memory, 45 and 1.85 where every pass reads it again, from L2 (3.3 where the
+// rows at hand do not fit there); top-k 50 and top-p 0.95 by passes.  Measured so, 1 / 2 / 4 / 8 blocks a row, us: 8 rows of
 // 151,936 330 / 187 / 88 / 64, 16 rows 326 / 187 / 86 / 122, 40 rows 327 / 186 / 168 / 185, 64 rows 328 / 188 /
 // 172 / 302, 128 rows 333 / 368 / 336 / 544; 40 rows of 32,000 70 / 51 / 76 / 118, 256 rows 135 / 191 / 300 / 663; 64 rows
-// of 300,000 611 / 337 / 372 / 436, 128 rows 1047 / 715 / 757 / 815.
+// of 300,000 611 / 337 / 372 / 436, 128 rows 1047 / 715 / 757 / 815.  A top-k of up to 512, decided among the largest logits, has its
+// least time at the same number or within 2 us of it: 1 row of 151,936 351 / 200 / 36 / 34, 8 rows 368 / 221 / 56 / 52, 16 rows 366 / 206 /
+// 36 / 52, 40 rows 366 / 206 / 58 / 73, 64 rows 368 / 212 / 69 / 110, 128 rows 394 / 409 / 124 / 190; of 32,000 1 row 32 / 28 / 26 / 28,
+// 16 rows 32 / 28 / 28 / 42, 40 rows 32 / 28 / 40 / 58, 64 rows 32 / 28 / 48 / 83, 256 rows 58 / 97 / 149 / 276 (one and two blocks keep no
+// slice of 151,936 in shared memory and take the passes).
 static int sample_parts(int rows, int vocab) {
   int best = 1;
   double least = 0.0;

@@ -304,7 +304,7 @@ class LatentAttention(Mixer):
 
     def _per_head(self, x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
         """out[n, h] = x[n, h] @ w[h].T for x [N, heads, k], w [heads, o, k], out [N, heads, o]
-        (x and out may be strided).  The 32-bit engine uses the plain FFMA kernel; bfloat16
+        (x and out may be strided).  The 32-bit engine uses the 32-bit kernels; bfloat16
         the library's batched product, as the large projections do."""
         if x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and x.shape[0] > native.TC5_MAX_ROWS:
             out.copy_(torch.bmm(x.transpose(0, 1), w.transpose(1, 2)).transpose(0, 1))

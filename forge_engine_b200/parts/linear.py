@@ -4,8 +4,9 @@ Which kernel runs is decided by the dtypes alone:
 
 * weight and input both bfloat16 - the tensor-core product (library GEMM, as upstream
   uses ``nn.Linear`` for every projection, src/forge_engine/qwen3.py:113-122);
-* anything else (the 32-bit path, or a tensor the checkpoint stores in 32-bit) - the
-  plain FFMA kernel, which never uses a reduced-precision matrix mode.
+* anything else (the 32-bit path, or a tensor the checkpoint stores in 32-bit) - the 32-bit
+  kernels: multiply-adds, or the tensor cores with both operands split into three bfloat16
+  numbers, which keep all of their 24 bits.
 """
 
 from __future__ import annotations

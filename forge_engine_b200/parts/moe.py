@@ -154,10 +154,13 @@ class RoutedMLP(FeedForward):
     def tile_rows(self, slots: int) -> int:
         """Rows of a row tile of the tcgen05 products: few rows per expert (decoding) take the narrow tiles,
         whose rings are deepest; more take the tile that most experts fill once, because every further row tile
-        reads the expert's weights again.  Whole layer, 16 experts of 4,864 (of 2,432) at width 2,560, us with
-        tiles of 32 / 64 / 128 rows: 32 rows an expert 261 / 258 / 302 (147 / 154 / 183), 40 rows 282 / 279 / 305
-        (155 / 154 / 184), 75 rows 405 / 309 / 315 (211 / 177 / 188), 87 rows 429 / 359 / 325 (229 / 197 / 190),
-        125 rows 549 / 413 / 371 (285 / 233 / 203)."""
+        reads the expert's weights again.  A tile brings the rows it has, in sixteens, so that a wide one costs few
+        rows little.  Whole layer, 16 experts of 4,864 (of 2,432) at width 2,560, us with tiles of 32 / 64 / 128 rows:
+        8 rows an expert 221 / 228 / 236 (141 / 143 / 143), 32 rows 275 / 268 / 282 (167 / 170 / 179), 36 rows
+        288 / 273 / 287 (176 / 174 / 182), 48 rows 329 / 284 / 289 (196 / 177 / 186), 64 rows 354 / 306 / 292
+        (209 / 188 / 183), 80 rows 418 / 308 / 314 (237 / 191 / 189), 87 rows 428 / 354 / 323 (242 / 213 / 194), 125 rows
+        558 / 453 / 390 (289 / 241 / 215); tiles of 16 rows 239, 326, 344 and 418 at 8 to 48.  Either side of both lines the
+        two tiles lie within 5 %."""
         wish = int(os.environ.get("FORGE_ENGINE_MOE_TILE", "0"))
         if wish in (16, 32, 64, 128):
             return wish
