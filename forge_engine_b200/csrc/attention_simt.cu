@@ -25,6 +25,8 @@
 // a block, all spans of a row by one block and the value product without pairs of columns).
 #include "attention_common.cuh"
 
+#include <algorithm>
+
 namespace {
 
 constexpr int SPAN = 128;          // key positions of a block of the span kernel
@@ -49,6 +51,7 @@ struct Simt {
   int unit0;                // of this launch: the units go through the workspace in slices
   float* partial;           // [unit of the slice][kv head][row tile][span][row][D + 2]
   int n_tokens;
+  int share;                // blocks of a row tile and kv head (1: all spans by one block)
   int* status;
 };
 
@@ -339,8 +342,8 @@ __device__ __forceinline__ bool find_tile(const Simt& p, int index, int& entry, 
   return false;
 }
 
-// SPLIT: the block takes one span of the keys (blockIdx.y = span * kv heads + kv head) and leaves its maxima and sums to
-// attention_simt_fold_kernel.
+// SPLIT: `share` blocks take a row tile of a kv head, each every share-th span of the keys that its rows see, and leave the spans'
+// maxima and sums to attention_simt_fold_kernel.
 template <typename T, int DMAX, bool SPLIT>
 __global__ void __launch_bounds__(TILE_THREADS) attention_simt_tile_kernel(const Simt p) {
   constexpr int CH = 16 / (int)sizeof(T), CG = DMAX / 64;      // groups of four output columns of a thread
@@ -348,7 +351,7 @@ __global__ void __launch_bounds__(TILE_THREADS) attention_simt_tile_kernel(const
   __shared__ int ok[TILE_KEYS];
   pdl_trigger();
   pdl_wait();
-  const int D = p.cache.head_dim, kvh = blockIdx.y % p.cache.num_kv_heads, span = blockIdx.y / p.cache.num_kv_heads;
+  const int D = p.cache.head_dim, nkv = p.cache.num_kv_heads, kvh = blockIdx.y % nkv;
   int entry = 0, tile = 0, tiles = 0;
   if (!find_tile(p, blockIdx.x, entry, tile, tiles)) return;
   const int token0 = p.cu_tokens[entry], count = p.cu_tokens[entry + 1] - token0;
@@ -360,6 +363,14 @@ __global__ void __launch_bounds__(TILE_THREADS) attention_simt_tile_kernel(const
   T* ks = (T*)(ps + TILE_ROWS * P_PITCH);                       // [key][D + CH]
   T* vs = ks + TILE_KEYS * (D + CH);                            // [key][D]
   const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+  const int* table = p.cache.block_table + (size_t)entry * p.cache.max_pages;
+  const int low = p.positions[token0 + row0 / p.groups], last = p.positions[token0 + (min(row0 + TILE_ROWS, total) - 1) / p.groups];
+  const int lo = p.window > 0 ? max(0, low - p.window + 1) : 0;
+  const int which = blockIdx.y / nkv;
+  if (SPLIT && which == 0 && last >= p.spans * SPAN && threadIdx.x == 0) atomicOr(p.status, FE_STATUS_BAD_PAGE);   // past the block table
+  const int stop = SPLIT ? min(last / SPAN, p.spans - 1) : 0;
+  int span = SPLIT ? lo / SPAN + which : 0;
+  if (span > stop) return;
   for (int i = threadIdx.x; i < TILE_ROWS * D; i += TILE_THREADS) {
     const int r = i / D, d = i - r * D, row = row0 + r;
     const int token = token0 + row / p.groups, head = kvh * p.groups + row % p.groups;
@@ -372,157 +383,154 @@ __global__ void __launch_bounds__(TILE_THREADS) attention_simt_tile_kernel(const
     upto[i] = row < total ? p.positions[token0 + row / p.groups] : -1;
     from[i] = p.window > 0 ? max(0, upto[i] - p.window + 1) : 0;
   }
-  const int* table = p.cache.block_table + (size_t)entry * p.cache.max_pages;
-  const int low = p.positions[token0 + row0 / p.groups], last = p.positions[token0 + (min(row0 + TILE_ROWS, total) - 1) / p.groups];
-  const int lo = p.window > 0 ? max(0, low - p.window + 1) : 0;
-  const int high = SPLIT ? min(last, span * SPAN + SPAN - 1) : last;
-  if (SPLIT && span == 0 && last >= p.spans * SPAN && threadIdx.x == 0) atomicOr(p.status, FE_STATUS_BAD_PAGE);   // past the block table
-  if (SPLIT && (high < span * SPAN || lo > high)) return;
-  // of the span at hand, and of the spans before it
-  float m[RT], l[RT], top[SPLIT ? 1 : RT], den[SPLIT ? 1 : RT], num[SPLIT ? 1 : RT][CG][4];
-  uint64_t acc[RT][CG][2];           // two neighbouring columns each
+  for (; span <= stop; span += p.share) {
+    const int high = SPLIT ? min(last, span * SPAN + SPAN - 1) : last;
+    // of the span at hand, and of the spans before it
+    float m[RT], l[RT], top[SPLIT ? 1 : RT], den[SPLIT ? 1 : RT], num[SPLIT ? 1 : RT][CG][4];
+    uint64_t acc[RT][CG][2];           // two neighbouring columns each
 #pragma unroll
-  for (int i = 0; i < RT; ++i) {
-    m[i] = -INFINITY;
-    l[i] = 0.f;
-    if (!SPLIT) top[i] = -INFINITY, den[i] = 0.f;
+    for (int i = 0; i < RT; ++i) {
+      m[i] = -INFINITY;
+      l[i] = 0.f;
+      if (!SPLIT) top[i] = -INFINITY, den[i] = 0.f;
 #pragma unroll
-    for (int g = 0; g < CG; ++g)
+      for (int g = 0; g < CG; ++g)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        acc[i][g][e / 2] = 0;
-        if (!SPLIT) num[i][g][e] = 0.f;
-      }
-  }
-  for (int first = max(lo, SPLIT ? span * SPAN : 0) / TILE_KEYS * TILE_KEYS; first <= high; first += TILE_KEYS) {
-    __syncthreads();
-    stage_keys<T, TILE_KEYS, TILE_THREADS>(p, table, kvh, first, lo, high, ks, vs, ok);
-    commit();
-    wait<0>();
-    __syncthreads();
-    uint64_t dot[RT][4];
-#pragma unroll
-    for (int i = 0; i < RT; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) dot[i][j] = 0;
-#pragma unroll 4
-    for (int d = 0; d < D; d += 4) {
-      uint64_t a[RT][2], b[4][2];
-#pragma unroll
-      for (int i = 0; i < RT; ++i) pairs4(qs + (ty * RT + i) * qpitch + d, a[i]);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) pairs4(ks + (tx + 16 * j) * (D + CH) + d, b[j]);
-#pragma unroll
-      for (int e = 0; e < 2; ++e)
-#pragma unroll
-        for (int i = 0; i < RT; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) fma2(dot[i][j], a[i][e], b[j][e]);
-    }
-    // by row and thirty-two of keys: maxima, corrections of what came before, sums
-    float score[RT][4], most[2 * RT], corr[2][RT];
-#pragma unroll
-    for (int i = 0; i < RT; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int key = first + tx + 16 * j;
-        score[i][j] = ok[tx + 16 * j] && key >= from[i] && key <= upto[i] ? __fmul_rn(sum2(dot[i][j]), p.scale) : -INFINITY;
-        if (j & 1) most[2 * i + j / 2] = fmaxf(score[i][j - 1], score[i][j]);
-      }
-    reduce4<true>(most, threadIdx.x & 31);
-#pragma unroll
-    for (int i = 0; i < RT; ++i)
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const float now = fmaxf(m[i], most[2 * i + h]);
-        corr[h][i] = m[i] == -INFINITY ? 0.f : expf(m[i] - now);
-        m[i] = now;
-        float e[2];
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          e[j] = score[i][2 * h + j] == -INFINITY ? 0.f : expf(score[i][2 * h + j] - now);
-          ps[(ty * RT + i) * P_PITCH + 32 * h + 16 * j + tx] = e[j];
+        for (int e = 0; e < 4; ++e) {
+          acc[i][g][e / 2] = 0;
+          if (!SPLIT) num[i][g][e] = 0.f;
         }
-        most[2 * i + h] = e[0] + e[1];
+    }
+    for (int first = max(lo, SPLIT ? span * SPAN : 0) / TILE_KEYS * TILE_KEYS; first <= high; first += TILE_KEYS) {
+      __syncthreads();
+      stage_keys<T, TILE_KEYS, TILE_THREADS>(p, table, kvh, first, lo, high, ks, vs, ok);
+      commit();
+      wait<0>();
+      __syncthreads();
+      uint64_t dot[RT][4];
+#pragma unroll
+      for (int i = 0; i < RT; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) dot[i][j] = 0;
+#pragma unroll 4
+      for (int d = 0; d < D; d += 4) {
+        uint64_t a[RT][2], b[4][2];
+#pragma unroll
+        for (int i = 0; i < RT; ++i) pairs4(qs + (ty * RT + i) * qpitch + d, a[i]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) pairs4(ks + (tx + 16 * j) * (D + CH) + d, b[j]);
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+          for (int i = 0; i < RT; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) fma2(dot[i][j], a[i][e], b[j][e]);
       }
-    reduce4<false>(most, threadIdx.x & 31);
+      // by row and thirty-two of keys: maxima, corrections of what came before, sums
+      float score[RT][4], most[2 * RT], corr[2][RT];
 #pragma unroll
-    for (int i = 0; i < RT; ++i) l[i] = fmaf(fmaf(l[i], corr[0][i], most[2 * i]), corr[1][i], most[2 * i + 1]);
-    __syncwarp();                    // a row's probabilities are written and read by the same warp
-    // Where some row of the tile does not see some key, that key's value is left out for it: a
-    // zero probability would not keep an infinity out.
-    const bool edge = first < max(0, p.window > 0 ? last - p.window + 1 : 0) || first + TILE_KEYS - 1 > low;
-    for (int key = 0; key < TILE_KEYS; key += 4) {
-      if (key % 32 == 0) {
+      for (int i = 0; i < RT; ++i)
 #pragma unroll
-        for (int i = 0; i < RT; ++i)
+        for (int j = 0; j < 4; ++j) {
+          const int key = first + tx + 16 * j;
+          score[i][j] = ok[tx + 16 * j] && key >= from[i] && key <= upto[i] ? __fmul_rn(sum2(dot[i][j]), p.scale) : -INFINITY;
+          if (j & 1) most[2 * i + j / 2] = fmaxf(score[i][j - 1], score[i][j]);
+        }
+      reduce4<true>(most, threadIdx.x & 31);
 #pragma unroll
-          for (int g = 0; g < CG; ++g)
+      for (int i = 0; i < RT; ++i)
 #pragma unroll
-            for (int e = 0; e < 2; ++e) acc[i][g][e] = scale2(acc[i][g][e], key == 0 ? corr[0][i] : corr[1][i]);
-      }
-      float e[RT][4];
+        for (int h = 0; h < 2; ++h) {
+          const float now = fmaxf(m[i], most[2 * i + h]);
+          corr[h][i] = m[i] == -INFINITY ? 0.f : expf(m[i] - now);
+          m[i] = now;
+          float e[2];
 #pragma unroll
-      for (int i = 0; i < RT; ++i) load4(ps + (ty * RT + i) * P_PITCH + key, e[i]);
+          for (int j = 0; j < 2; ++j) {
+            e[j] = score[i][2 * h + j] == -INFINITY ? 0.f : expf(score[i][2 * h + j] - now);
+            ps[(ty * RT + i) * P_PITCH + 32 * h + 16 * j + tx] = e[j];
+          }
+          most[2 * i + h] = e[0] + e[1];
+        }
+      reduce4<false>(most, threadIdx.x & 31);
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        uint64_t v[CG][2];
+      for (int i = 0; i < RT; ++i) l[i] = fmaf(fmaf(l[i], corr[0][i], most[2 * i]), corr[1][i], most[2 * i + 1]);
+      __syncwarp();                    // a row's probabilities are written and read by the same warp
+      // Where some row of the tile does not see some key, that key's value is left out for it: a
+      // zero probability would not keep an infinity out.
+      const bool edge = first < max(0, p.window > 0 ? last - p.window + 1 : 0) || first + TILE_KEYS - 1 > low;
+      for (int key = 0; key < TILE_KEYS; key += 4) {
+        if (key % 32 == 0) {
 #pragma unroll
-        for (int g = 0; g < CG; ++g)
-          if (tx * 4 + 64 * g < D) pairs4(vs + (key + u) * D + tx * 4 + 64 * g, v[g]);
-          else v[g][0] = v[g][1] = 0;
-#pragma unroll
-        for (int i = 0; i < RT; ++i) {
-          if (!edge || (first + key + u >= from[i] && first + key + u <= upto[i])) {
-            const uint64_t both = twice(e[i][u]);
+          for (int i = 0; i < RT; ++i)
 #pragma unroll
             for (int g = 0; g < CG; ++g)
 #pragma unroll
-              for (int c = 0; c < 2; ++c) fma2(acc[i][g][c], both, v[g][c]);
+              for (int e = 0; e < 2; ++e) acc[i][g][e] = scale2(acc[i][g][e], key == 0 ? corr[0][i] : corr[1][i]);
+        }
+        float e[RT][4];
+#pragma unroll
+        for (int i = 0; i < RT; ++i) load4(ps + (ty * RT + i) * P_PITCH + key, e[i]);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          uint64_t v[CG][2];
+#pragma unroll
+          for (int g = 0; g < CG; ++g)
+            if (tx * 4 + 64 * g < D) pairs4(vs + (key + u) * D + tx * 4 + 64 * g, v[g]);
+            else v[g][0] = v[g][1] = 0;
+#pragma unroll
+          for (int i = 0; i < RT; ++i) {
+            if (!edge || (first + key + u >= from[i] && first + key + u <= upto[i])) {
+              const uint64_t both = twice(e[i][u]);
+#pragma unroll
+              for (int g = 0; g < CG; ++g)
+#pragma unroll
+                for (int c = 0; c < 2; ++c) fma2(acc[i][g][c], both, v[g][c]);
+            }
           }
         }
       }
-    }
-    if constexpr (!SPLIT) if ((first + TILE_KEYS) % SPAN == 0 || first + TILE_KEYS > high) {
+      if constexpr (!SPLIT) if ((first + TILE_KEYS) % SPAN == 0 || first + TILE_KEYS > high) {
 #pragma unroll
-      for (int i = 0; i < RT; ++i) {
-        float old, mine;
-        fold_factors(top[i], m[i], old, mine);
-        den[i] = fmaf(l[i], mine, __fmul_rn(den[i], old));
-        m[i] = -INFINITY;
-        l[i] = 0.f;
+        for (int i = 0; i < RT; ++i) {
+          float old, mine;
+          fold_factors(top[i], m[i], old, mine);
+          den[i] = fmaf(l[i], mine, __fmul_rn(den[i], old));
+          m[i] = -INFINITY;
+          l[i] = 0.f;
 #pragma unroll
-        for (int g = 0; g < CG; ++g)
+          for (int g = 0; g < CG; ++g)
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            num[i][g][e] = fmaf(half2_of(acc[i][g][e / 2], e & 1), mine, __fmul_rn(num[i][g][e], old));
-            if (e & 1) acc[i][g][e / 2] = 0;
-          }
+            for (int e = 0; e < 4; ++e) {
+              num[i][g][e] = fmaf(half2_of(acc[i][g][e / 2], e & 1), mine, __fmul_rn(num[i][g][e], old));
+              if (e & 1) acc[i][g][e / 2] = 0;
+            }
+        }
       }
     }
-  }
 #pragma unroll
-  for (int i = 0; i < RT; ++i) {
-    const int row = row0 + ty * RT + i;
-    if (row >= total) continue;
-    if constexpr (SPLIT) {
-      const size_t rows = (size_t)p.n_tokens * p.groups, at = (size_t)blockIdx.y * rows + (size_t)token0 * p.groups + row;
-      float* sums = p.partial + at * D;
+    for (int i = 0; i < RT; ++i) {
+      const int row = row0 + ty * RT + i;
+      if (row >= total) continue;
+      if constexpr (SPLIT) {
+        const size_t rows = (size_t)p.n_tokens * p.groups, at = ((size_t)span * nkv + kvh) * rows + (size_t)token0 * p.groups + row;
+        float* sums = p.partial + at * D;
 #pragma unroll
-      for (int g = 0; g < CG; ++g)
-        if (tx * 4 + 64 * g < D) *reinterpret_cast<ulonglong2*>(sums + tx * 4 + 64 * g) = make_ulonglong2(acc[i][g][0], acc[i][g][1]);
-      if (tx == 0) *reinterpret_cast<float2*>(p.partial + (size_t)gridDim.y * rows * D + 2 * at) = make_float2(m[i], l[i]);
-      continue;
-    }
-    T* out = (T*)p.out + ((size_t)(token0 + row / p.groups) * p.num_q_heads + kvh * p.groups + row % p.groups) * D;
+        for (int g = 0; g < CG; ++g)
+          if (tx * 4 + 64 * g < D) *reinterpret_cast<ulonglong2*>(sums + tx * 4 + 64 * g) = make_ulonglong2(acc[i][g][0], acc[i][g][1]);
+        if (tx == 0) *reinterpret_cast<float2*>(p.partial + (size_t)p.spans * nkv * rows * D + 2 * at) = make_float2(m[i], l[i]);
+        continue;
+      }
+      T* out = (T*)p.out + ((size_t)(token0 + row / p.groups) * p.num_q_heads + kvh * p.groups + row % p.groups) * D;
 #pragma unroll
-    for (int g = 0; g < CG; ++g) {
-      const int d = tx * 4 + 64 * g;
-      if (d < D) {
-        float o[4];
+      for (int g = 0; g < CG; ++g) {
+        const int d = tx * 4 + 64 * g;
+        if (d < D) {
+          float o[4];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) o[c] = den[SPLIT ? 0 : i] > 0.f ? num[SPLIT ? 0 : i][g][c] / den[SPLIT ? 0 : i] : 0.f;
-        store4(out + d, o);
+          for (int c = 0; c < 4; ++c) o[c] = den[SPLIT ? 0 : i] > 0.f ? num[SPLIT ? 0 : i][g][c] / den[SPLIT ? 0 : i] : 0.f;
+          store4(out + d, o);
+        }
       }
     }
   }
@@ -620,11 +628,23 @@ long long tile_floats(int n_tokens, int num_q_heads, int num_kv_heads, int head_
 }
 
 template <typename T, bool SPLIT>
-int run_tiles(const Simt& p, cudaStream_t stream) {
+int run_tiles(Simt p, cudaStream_t stream) {
   const int D = p.cache.head_dim;
   const size_t smem = (size_t)4 * TILE_ROWS * (D + 4 + P_PITCH) + (size_t)TILE_KEYS * (2 * D * sizeof(T) + 16);
   // tiles of all entries one after the other; an entry's last one may be short
-  const dim3 grid((unsigned)(((long long)p.n_tokens * p.groups + TILE_ROWS - 1) / TILE_ROWS + p.units), p.cache.num_kv_heads * (SPLIT ? p.spans : 1));
+  const long long heads = p.cache.num_kv_heads, tiles = ((long long)p.n_tokens * p.groups + TILE_ROWS - 1) / TILE_ROWS + p.units;
+  // Blocks that share a tile: about eight times what the chip holds altogether, and no more than there are spans in a window.  How
+  // many spans a tile has is known on the device; a block for each that the block table has room for took 190 us for a prompt of
+  // 60 tokens beside a request of 32,768 (16 heads of 128; 28 now), and 81 for 100 tokens with a window of 256 (49).  With 600
+  // blocks 200 tokens after 3,000 of 16 heads of 128 take 330 us, 1,200 304, 2,400 322, 4,700 331; 40 tokens beside 50 decoding
+  // requests, 16 heads of 96, 153, 135, 111 and 111.
+  p.share = 1;
+  if (SPLIT) {
+    long long share = std::min<long long>(p.spans, (8 * 296 + tiles * heads - 1) / (tiles * heads));
+    if (p.window > 0) share = std::min<long long>(share, ((long long)p.window + TILE_ROWS / p.groups + SPAN) / SPAN + 1);
+    p.share = (int)share;
+  }
+  const dim3 grid((unsigned)tiles, (unsigned)(heads * p.share));
   int code;
   if (D <= 64) code = launch(attention_simt_tile_kernel<T, 64, SPLIT>, grid, TILE_THREADS, smem, stream, p);
   else if (D <= 128) code = launch(attention_simt_tile_kernel<T, 128, SPLIT>, grid, TILE_THREADS, smem, stream, p);
@@ -686,7 +706,7 @@ FE_EXPORT int fe_attention_simt(const void* q, int q_stride, int dtype, const vo
   const int row_tiles = (groups + R - 1) / R;
   if (spans > 0x7fffffff || (long long)num_kv_heads * row_tiles > 65535) return FE_ERR_TOO_LARGE;
   Simt p{q, q_stride, cache, positions, token_entry, cu_tokens, units, window, scale, out, num_q_heads, groups,
-         (int)spans, row_tiles, 0, workspace, n_tokens, status};
+         (int)spans, row_tiles, 0, workspace, n_tokens, 1, status};
   if (dtype == FE_DTYPE_F32) return run<float>(p, n_tokens, max_new, stream);
   if (dtype == FE_DTYPE_BF16) return run<bf16>(p, n_tokens, max_new, stream);
   return FE_ERR_BAD_DTYPE;

@@ -218,6 +218,37 @@ def test_attention_of_portions_that_fill_the_chip(native, dtype, nq, nkv, d, win
         torch.testing.assert_close(mine, want, **(dict(atol=2e-5, rtol=1e-5) if dtype == torch.float32 else dict(atol=2e-2, rtol=2e-2)))
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("nq, nkv, d, window, wide", [(16, 16, 64, None, 0), (32, 8, 40, None, 300), (16, 16, 128, 700, 0), (16, 2, 256, None, 0), (8, 8, 64, 100, 400)])
+def test_attention_spans_that_blocks_share(native, dtype, nq, nkv, d, window, wide):
+    """More spans than blocks share a row tile of a long portion, windows that leave most spans unseen, and block tables far
+    wider than a request's pages: the bits of the same tokens in pieces with blocks for every span, and the dense result."""
+    page, lengths, counts = 16, [3000, 60], [190, 60]
+    k_cache, v_cache, table, keys, values = paged_layout(lengths, page, nkv, d, dtype, seed=d)
+    table = torch.nn.functional.pad(table, (0, wide), value=-1)
+    positions = [p for n, c in zip(lengths, counts) for p in range(n - c, n)]
+    q = torch.randn((len(positions), nq, d), generator=torch.Generator().manual_seed(5)).to(dtype)
+    ints = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)  # noqa: E731
+    status = status_word()
+
+    def attend(first, last, entry):
+        out = torch.empty((last - first, nq * d), dtype=dtype, device=DEV)
+        one = table[entry : entry + 1].contiguous()
+        assert native.lib().fe_attention_simt_tile_scratch(last - first, 1, nq, nkv, d, one.shape[1], page) > 0
+        native.attention_simt(q[first:last].reshape(last - first, nq * d).to(DEV), nq * d, k_cache, v_cache, one, ints(positions[first:last]),
+                              ints([0] * (last - first)), window, d ** -0.5, out, nq, status, entries=(ints([0, last - first]), 1, last - first))
+        return out
+
+    for entry, first, last, step in ((0, 0, 190, 19), (1, 190, 250, 2)):
+        together = attend(first, last, entry)
+        for at in range(first, last, step):
+            assert torch.equal(attend(at, at + step, entry), together[at - first : at - first + step]), at
+        want = dense_attention(q[first:last], keys[entry], values[entry], torch.tensor(positions[first:last]), d ** -0.5, window)
+        mine = together.view(last - first, nq, d).double().cpu()
+        torch.testing.assert_close(mine, want, **(dict(atol=2e-5, rtol=1e-5) if dtype == torch.float32 else dict(atol=2e-2, rtol=2e-2)))
+    assert int(status.item()) == 0
+
+
 def test_attention_marks_missing_pages_and_keeps_later_infinities_out(native):
     """A position without a page sets the status bit; an infinite value of a later token of the same tile
     changes no earlier row."""
