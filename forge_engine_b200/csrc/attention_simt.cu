@@ -15,14 +15,15 @@
 //   requests.
 // attention_simt_tile: entries of several tokens.  A block takes 32 rows (token, query head) of one
 //   kv head over all their keys in tiles of 64, as two small FFMA products from shared memory; where that leaves
-//   the chip idle, over one span of them, and attention_simt_fold folds a row's spans.  Bound by instructions (two
-//   blocks of 8 warps an SM issue in 53 % of the cycles; with 4 warps of twice the rows 30 %).
+//   the chip idle, over a share of their spans, and attention_simt_fold folds a row's spans.  Bound by instructions (heads of 128:
+//   two blocks of 8 warps an SM issue in 53 % of the cycles; with 4 warps of twice the rows 30 %).
 //
 // A row's bits depend on nothing but its token and the keys it sees: not on what else is in the batch, nor on
 // how its portion was cut.  Both kernels take a span's keys, counted from position 0, in thirty-twos with one
 // running maximum, sum over positions (or elements of a head: even and odd ones apart) in ascending order,
-// and fold the spans one after the other (fold_factors).  500 tokens of 16 heads of 128 take 108 us in a layer (150 by 4 warps
-// a block, all spans of a row by one block and the value product without pairs of columns).
+// and fold the spans one after the other (fold_factors).  us, 16 heads of 128, before (4 warps a block, all spans of a row by one block, one
+// head's tiles after the other's, the value product without pairs of columns) and now: 500 tokens 158 / 104, 2,048 1,243 / 806, 200 after
+// 3,000 696 / 302; 32 heads of 64 111 / 92, 985 / 862, 461 / 307; 40 of 64 in bfloat16 104 / 98, 1,102 / 1,061, 455 / 368.
 #include "attention_common.cuh"
 
 #include <algorithm>
@@ -33,8 +34,7 @@ constexpr int SPAN = 128;          // key positions of a block of the span kerne
 constexpr int SPAN_KEYS = 32;      // of one stage of its ring
 constexpr int SPAN_STAGES = 3;
 constexpr int SPAN_THREADS = 128;
-constexpr int TILE_ROWS = 32, TILE_KEYS = 64, TILE_THREADS = 256;
-constexpr int RT = TILE_ROWS / (TILE_THREADS / 16);      // rows of a thread
+constexpr int TILE_ROWS = 32, TILE_KEYS = 64;
 constexpr int P_PITCH = TILE_KEYS + 4;
 
 struct Simt {
@@ -91,12 +91,13 @@ __device__ __forceinline__ void pairs4(const bf16* p, uint64_t (&out)[2]) {
   out[1] = (uint64_t)(raw.y << 16) | ((uint64_t)(raw.y & 0xffff0000u) << 32);
 }
 
-// Sums (or maxima) of four numbers over 16 neighbouring lanes, for all of them, in the order of warp_sum's last
+// Sums (or maxima) of N (four or eight) numbers over 16 neighbouring lanes, for all of them, in the order of warp_sum's last
 // four steps: half of the numbers go to the partner at a time, and come back whole.
-template <bool MAX>
-__device__ __forceinline__ void reduce4(float (&x)[4], int lane) {
+template <bool MAX, int N>
+__device__ __forceinline__ void reduce_all(float (&x)[N], int lane) {
+  int bit = 8;
 #pragma unroll
-  for (int half = 2, bit = 8; half > 0; half >>= 1, bit >>= 1) {
+  for (int half = N / 2; half > 0; half >>= 1, bit >>= 1) {
     const bool upper = (lane & bit) != 0;
 #pragma unroll
     for (int i = 0; i < half; ++i) {
@@ -107,12 +108,12 @@ __device__ __forceinline__ void reduce4(float (&x)[4], int lane) {
   }
   float mine = x[0];
 #pragma unroll
-  for (int bit = 2; bit > 0; bit >>= 1) {
-    const float got = __shfl_xor_sync(0xffffffffu, mine, bit);
+  for (int b = 8 / N; b > 0; b >>= 1) {
+    const float got = __shfl_xor_sync(0xffffffffu, mine, b);
     mine = MAX ? fmaxf(mine, got) : mine + got;
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i) x[i] = __shfl_sync(0xffffffffu, mine, (lane & 16) | (i << 2));
+  for (int i = 0; i < N; ++i) x[i] = __shfl_sync(0xffffffffu, mine, (lane & 16) | (i * (16 / N)));
 }
 
 // A span (maximum m) joins those before it (maximum top): their sums take `old`, its own `mine`.
@@ -344,16 +345,21 @@ __device__ __forceinline__ bool find_tile(const Simt& p, int index, int& entry, 
 
 // SPLIT: `share` blocks take a row tile of a kv head, each every share-th span of the keys that its rows see, and leave the spans'
 // maxima and sums to attention_simt_fold_kernel.
-template <typename T, int DMAX, bool SPLIT>
-__global__ void __launch_bounds__(TILE_THREADS) attention_simt_tile_kernel(const Simt p) {
+// Whole tiles: the kv heads of a row tile one after the other, so that the tiles with the most keys start first in all of them (one
+// head's tiles after the other: 1,000 tokens of 16 heads of 128 324 us, 223 so; 32 heads of 64 314 and 256).  Shares of a tile lie tile by tile.
+template <typename T, int DMAX, bool SPLIT, int THREADS>
+__global__ void __launch_bounds__(THREADS, DMAX == 256 && sizeof(T) == 4 ? 1 : THREADS == 256 ? 2 : 3) attention_simt_tile_kernel(const Simt p) {
+  constexpr int RT = TILE_ROWS / (THREADS / 16);               // rows of a thread
   constexpr int CH = 16 / (int)sizeof(T), CG = DMAX / 64;      // groups of four output columns of a thread
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ int ok[TILE_KEYS];
   pdl_trigger();
   pdl_wait();
-  const int D = p.cache.head_dim, nkv = p.cache.num_kv_heads, kvh = blockIdx.y % nkv;
+  const int D = p.cache.head_dim, nkv = p.cache.num_kv_heads;
+  const unsigned per = nkv * (SPLIT ? p.share : 1), tiles_all = gridDim.x / per;
+  const int part = (int)(SPLIT ? blockIdx.x / tiles_all : blockIdx.x % per), kvh = part % nkv, which = part / nkv;
   int entry = 0, tile = 0, tiles = 0;
-  if (!find_tile(p, blockIdx.x, entry, tile, tiles)) return;
+  if (!find_tile(p, (int)(SPLIT ? blockIdx.x % tiles_all : blockIdx.x / per), entry, tile, tiles)) return;
   const int token0 = p.cu_tokens[entry], count = p.cu_tokens[entry + 1] - token0;
   const int total = count * p.groups;
   const int row0 = (tiles - 1 - tile) * TILE_ROWS;    // the tiles with the most keys first
@@ -366,12 +372,11 @@ __global__ void __launch_bounds__(TILE_THREADS) attention_simt_tile_kernel(const
   const int* table = p.cache.block_table + (size_t)entry * p.cache.max_pages;
   const int low = p.positions[token0 + row0 / p.groups], last = p.positions[token0 + (min(row0 + TILE_ROWS, total) - 1) / p.groups];
   const int lo = p.window > 0 ? max(0, low - p.window + 1) : 0;
-  const int which = blockIdx.y / nkv;
   if (SPLIT && which == 0 && last >= p.spans * SPAN && threadIdx.x == 0) atomicOr(p.status, FE_STATUS_BAD_PAGE);   // past the block table
   const int stop = SPLIT ? min(last / SPAN, p.spans - 1) : 0;
   int span = SPLIT ? lo / SPAN + which : 0;
   if (span > stop) return;
-  for (int i = threadIdx.x; i < TILE_ROWS * D; i += TILE_THREADS) {
+  for (int i = threadIdx.x; i < TILE_ROWS * D; i += THREADS) {
     const int r = i / D, d = i - r * D, row = row0 + r;
     const int token = token0 + row / p.groups, head = kvh * p.groups + row % p.groups;
     qs[r * qpitch + d] = row < total ? to_float(((const T*)p.q)[(size_t)token * p.q_stride + (size_t)head * D + d]) : 0.f;
@@ -383,6 +388,9 @@ __global__ void __launch_bounds__(TILE_THREADS) attention_simt_tile_kernel(const
     upto[i] = row < total ? p.positions[token0 + row / p.groups] : -1;
     from[i] = p.window > 0 ? max(0, upto[i] - p.window + 1) : 0;
   }
+  int column[CG];                      // columns past the head's last are its last ones again, and are not stored
+#pragma unroll
+  for (int g = 0; g < CG; ++g) column[g] = min(tx * 4 + 64 * g, D - 4);
   for (; span <= stop; span += p.share) {
     const int high = SPLIT ? min(last, span * SPAN + SPAN - 1) : last;
     // of the span at hand, and of the spans before it
@@ -403,7 +411,7 @@ __global__ void __launch_bounds__(TILE_THREADS) attention_simt_tile_kernel(const
     }
     for (int first = max(lo, SPLIT ? span * SPAN : 0) / TILE_KEYS * TILE_KEYS; first <= high; first += TILE_KEYS) {
       __syncthreads();
-      stage_keys<T, TILE_KEYS, TILE_THREADS>(p, table, kvh, first, lo, high, ks, vs, ok);
+      stage_keys<T, TILE_KEYS, THREADS>(p, table, kvh, first, lo, high, ks, vs, ok);
       commit();
       wait<0>();
       __syncthreads();
@@ -436,7 +444,7 @@ __global__ void __launch_bounds__(TILE_THREADS) attention_simt_tile_kernel(const
           score[i][j] = ok[tx + 16 * j] && key >= from[i] && key <= upto[i] ? __fmul_rn(sum2(dot[i][j]), p.scale) : -INFINITY;
           if (j & 1) most[2 * i + j / 2] = fmaxf(score[i][j - 1], score[i][j]);
         }
-      reduce4<true>(most, threadIdx.x & 31);
+      reduce_all<true>(most, threadIdx.x & 31);
 #pragma unroll
       for (int i = 0; i < RT; ++i)
 #pragma unroll
@@ -452,7 +460,7 @@ __global__ void __launch_bounds__(TILE_THREADS) attention_simt_tile_kernel(const
           }
           most[2 * i + h] = e[0] + e[1];
         }
-      reduce4<false>(most, threadIdx.x & 31);
+      reduce_all<false>(most, threadIdx.x & 31);
 #pragma unroll
       for (int i = 0; i < RT; ++i) l[i] = fmaf(fmaf(l[i], corr[0][i], most[2 * i]), corr[1][i], most[2 * i + 1]);
       __syncwarp();                    // a row's probabilities are written and read by the same warp
@@ -475,18 +483,21 @@ __global__ void __launch_bounds__(TILE_THREADS) attention_simt_tile_kernel(const
         for (int u = 0; u < 4; ++u) {
           uint64_t v[CG][2];
 #pragma unroll
-          for (int g = 0; g < CG; ++g)
-            if (tx * 4 + 64 * g < D) pairs4(vs + (key + u) * D + tx * 4 + 64 * g, v[g]);
-            else v[g][0] = v[g][1] = 0;
+          for (int g = 0; g < CG; ++g) pairs4(vs + (key + u) * D + column[g], v[g]);
+          auto add = [&](int i) {
+            const uint64_t both = twice(e[i][u]);
 #pragma unroll
-          for (int i = 0; i < RT; ++i) {
-            if (!edge || (first + key + u >= from[i] && first + key + u <= upto[i])) {
-              const uint64_t both = twice(e[i][u]);
+            for (int g = 0; g < CG; ++g)
 #pragma unroll
-              for (int g = 0; g < CG; ++g)
+              for (int c = 0; c < 2; ++c) fma2(acc[i][g][c], both, v[g][c]);
+          };
+          if (!edge) {
 #pragma unroll
-                for (int c = 0; c < 2; ++c) fma2(acc[i][g][c], both, v[g][c]);
-            }
+            for (int i = 0; i < RT; ++i) add(i);
+          } else {
+#pragma unroll
+            for (int i = 0; i < RT; ++i)
+              if (first + key + u >= from[i] && first + key + u <= upto[i]) add(i);
           }
         }
       }
@@ -617,14 +628,15 @@ int run_spans(Simt p, cudaStream_t stream) {
   return code;
 }
 
-// Whether entries of several tokens are cut into spans of their keys: while their row tiles are fewer than 400 blocks (the
-// chip holds 296, two an SM) and what the spans leave fits the workspace.  16 heads of 128, us, whole / in spans: 500 tokens (264
-// blocks) 132 / 118, 40 after 900 cached ones (32) 148 / 52, 100 after 5,000 (64) 720 / 298, 700 after 400 (360) 353 / 318,
-// 700 (360) 181 / 183, 1,000 (512) 323 / 337.
+// Whether entries of several tokens are cut into spans of their keys: while their row tiles are fewer than 340 blocks (the
+// chip holds 296, two an SM; 444 with heads of 64) and what the spans leave fits the workspace.  us, whole / in spans, 16 heads of 128: 250 tokens
+// (136 blocks) 54 / 50, 500 (264) 105 / 104, 600 (312) 136 / 124, 700 (360) 150 / 157, 850 (432) 182 / 220; 100 after 5,000 cached ones
+// (64) 740 / 275, 300 after 900 (160) 249 / 181, 700 after 400 (360) 242 / 278.  32 heads of 64: 250 tokens (264) 51 / 46, 500 (512)
+// 93 / 112; 24 heads of 64 and one kv head: 500 (376) 92 / 85, 600 (451) 111 / 113; 40 in bfloat16: 250 (316) 54 / 54, 300 after 900 (378) 202 / 224.
 long long tile_floats(int n_tokens, int num_q_heads, int num_kv_heads, int head_dim, long long spans, int units) {
   const long long tiles = ((long long)n_tokens * (num_q_heads / num_kv_heads) + TILE_ROWS - 1) / TILE_ROWS + units;
   const long long floats = (long long)n_tokens * num_q_heads * spans * (head_dim + 2);
-  return spans < 2 || tiles * num_kv_heads >= 400 || floats > SIMT_WORKSPACE || spans * num_kv_heads > 65535 ? 0 : floats;
+  return spans < 2 || tiles * num_kv_heads >= 340 || floats > SIMT_WORKSPACE || spans * num_kv_heads > 65535 ? 0 : floats;
 }
 
 template <typename T, bool SPLIT>
@@ -636,7 +648,7 @@ int run_tiles(Simt p, cudaStream_t stream) {
   // Blocks that share a tile: about eight times what the chip holds altogether, and no more than there are spans in a window.  How
   // many spans a tile has is known on the device; a block for each that the block table has room for took 190 us for a prompt of
   // 60 tokens beside a request of 32,768 (16 heads of 128; 28 now), and 81 for 100 tokens with a window of 256 (49).  With 600
-  // blocks 200 tokens after 3,000 of 16 heads of 128 take 330 us, 1,200 304, 2,400 322, 4,700 331; 40 tokens beside 50 decoding
+  // blocks 200 tokens after 3,000 of 16 heads of 128 took 330 us, 1,200 304, 2,400 322, 4,700 331; 40 tokens beside 50 decoding
   // requests, 16 heads of 96, 153, 135, 111 and 111.
   p.share = 1;
   if (SPLIT) {
@@ -644,11 +656,17 @@ int run_tiles(Simt p, cudaStream_t stream) {
     if (p.window > 0) share = std::min<long long>(share, ((long long)p.window + TILE_ROWS / p.groups + SPAN) / SPAN + 1);
     p.share = (int)share;
   }
-  const dim3 grid((unsigned)tiles, (unsigned)(heads * p.share));
+  if (tiles * heads * p.share > 0x7fffffffLL) return FE_ERR_TOO_LARGE;
+  const dim3 grid((unsigned)(tiles * heads * p.share));
+  // Threads: what a block holds in shared memory leaves three blocks an SM with up to 32 KB of keys and values (heads of 64, of 128 in
+  // bfloat16); four warps of four rows a thread then read less for a multiply-add than eight of two.  Otherwise two blocks fit, and eight
+  // warps hide more.  us, 128 / 256 threads: 2,048 tokens of 32 heads of 64 991 / 1,094, 40 heads of 64 in bfloat16 1,167 / 1,528, of 128
+  // 1,692 / 1,997; 16 heads of 128 1,261 (other changes besides) / 955.
+  constexpr int SMALL = 128, LARGE = 256, MID = sizeof(T) == 2 ? SMALL : LARGE;
   int code;
-  if (D <= 64) code = launch(attention_simt_tile_kernel<T, 64, SPLIT>, grid, TILE_THREADS, smem, stream, p);
-  else if (D <= 128) code = launch(attention_simt_tile_kernel<T, 128, SPLIT>, grid, TILE_THREADS, smem, stream, p);
-  else code = launch(attention_simt_tile_kernel<T, 256, SPLIT>, grid, TILE_THREADS, smem, stream, p);
+  if (D <= 64) code = launch(attention_simt_tile_kernel<T, 64, SPLIT, SMALL>, grid, SMALL, smem, stream, p);
+  else if (D <= 128) code = launch(attention_simt_tile_kernel<T, 128, SPLIT, MID>, grid, MID, smem, stream, p);
+  else code = launch(attention_simt_tile_kernel<T, 256, SPLIT, LARGE>, grid, LARGE, smem, stream, p);
   if (code || !SPLIT) return code;
   const long long rows = (long long)p.n_tokens * p.num_q_heads;
   return launch(attention_simt_fold_kernel<T>, dim3((unsigned)((rows + 7) / 8)), 256, 0, stream, p);
