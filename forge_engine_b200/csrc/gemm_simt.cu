@@ -394,7 +394,9 @@ int launch_split(const Product& p, int batch, int cuts, bool ahead, cudaStream_t
 // Measured, us, w out of memory: by one block a tile 16 rows x 4,096 x 1,024 29, 1,024 x 2,048 47, 1,024 x 3,072 66 and by eight 18, 16
 // and 20; 128 rows of 500 x 4,096 x 1,024 45, 1,024 x 2,048 70, by four 78 and 31, by eight 113 and 51.  So a stretch takes
 // 1.15 to 1.6 us, a tile 10 to 19 besides; blocks beyond what the SMs hold start when others have ended (with up to 16 rows two
-// share an SM, and the time of a stretch).
+// share an SM, and the time of a stretch).  Clusters lie in one group of SMs: with a block an SM 15 of eight and 33 of four run at
+// once, us, 15 and 16 tiles by eight blocks, 16 by four: 128 rows, depth 1,024 18.5 / 28.7 / 24.5, 3,072 26.6 / 45 / 39, 64 rows, 1,024 16.4 / 24.6 /
+// 18.5; 33 and 34 tiles of 32 rows by four, depth 512 14.4 and 24.6, 34 by one 20.5.
 int split_cuts(int tile, long long tiles, int k) {
   const int stretches = (k + GST_K - 1) / GST_K;
   const double stretch = tile == 16 ? 1.15 : tile == 32 ? 1.2 : tile == 64 ? 1.3 : 1.6, again = tile == 16 ? 2.5 : tile == 128 ? 11.0 : 8.0;
@@ -402,7 +404,7 @@ int split_cuts(int tile, long long tiles, int k) {
   int cuts = 1;
   double least = 0.0;
   for (int c = 1; c <= 8; c = c == 1 ? 4 : 2 * c) {
-    const int at_once = c == 8 ? 128 : c == 4 ? 136 : 148;        // clusters lie in one group of SMs
+    const int at_once = tile == 16 ? (c == 8 ? 128 : c == 4 ? 136 : 148) : c == 8 ? 120 : c == 4 ? 132 : 148;
     const double layers = (double)((tiles * c + at_once - 1) / at_once);
     const double time = (c == 1 ? fixed : tile == 16 ? 12.5 : 16.0) + (stretches + c - 1) / c * stretch * layers + again * (layers - 1.0);
     if (c == 1 || time < least) cuts = c, least = time;
@@ -438,7 +440,8 @@ int launch_typed(const Product& p, int batch, bool ahead, cudaStream_t stream) {
     // 4 x 32,000 x 1,024 46 / 51, 4 x 1,024 x 3,072 19.4 / 19.4 (in a decode step of 4 layers, where a product's weights are asked for
     // ahead, 343 / 326 altogether); 16 x 4,096 x 1,024 20.5 / 17.3, 16 x 32,000 x 1,024 72 / 52, 32 x 32,000 x 1,024 116 / 60, 64 x 4,096 x
     // 1,024 43 / 20, 500 x 4,096 x 1,024 118 / 43, 500 x 1,024 x 3,072 111 / 36, 1,024 x 32,000 x 1,024 1,439 / 540.  Shallower than 256
-    // a tile's fixed part is more than the sum (500 x 300 x 256 13 / 16).
+    // a tile's fixed part is more than the sum; up to about 512 it still is with few outputs, 4 x 512 x 256 8 / 12, 200 x 512 x 256 12 / 17,
+    // 64 x 512 x 512 16.4 / 13.3, and is not with many, 2,000 x 2,048 x 256 60 / 39 (the line is where the sums are as exact all the same).
     if (vec && p.k >= GST_MIN_K && p.k < (1 << 22) && p.ldx < (1 << 22)) return split_product(p, batch, ahead, stream);
   }
   const long long big = (long long)((p.o + 63) / 64) * ((p.n + 63) / 64) * batch;

@@ -690,6 +690,18 @@ def test_deep_product_of_values_that_are_not_finite(native, n):
     assert float((got[2, keep][sound].double() / want[2, keep][sound] - 1).abs().max()) < 1e-5
 
 
+@pytest.mark.parametrize("n, tiles, k, cuts", ((128, 15, 1024, 8), (128, 16, 1024, 4), (64, 16, 3072, 4), (32, 33, 512, 4), (32, 34, 512, 1), (4, 16, 1024, 8)))
+def test_products_are_cut_into_clusters_that_run_at_once(native, n, tiles, k, cuts):
+    """15 clusters of eight blocks and 33 of four fit the chip where a block has an SM; the bits of any cut are the same."""
+    assert native.lib().fe_gemm_split_cuts(n, tiles * 128, k, 1) == cuts
+    gen = torch.Generator().manual_seed(n + k)
+    x, w = torch.randn((n, k), generator=gen).to(DEV), torch.randn((tiles * 128, k), generator=gen).to(DEV)
+    got, alone = torch.empty((n, tiles * 128), device=DEV), torch.empty((n, 128), device=DEV)
+    native.gemm_simt(x, w, got)
+    native.gemm_simt(x, w[-128:].contiguous(), alone)
+    assert torch.equal(got[:, -128:], alone)
+
+
 @pytest.mark.parametrize("n, o, k", ((3, 40100, 256), (20, 20100, 320), (50, 20100, 260), (300, 4210, 448)))
 def test_values_that_are_not_finite_in_tiles_of_one_block(native, n, o, k):
     """The same in each tile size where one block takes all of k and writes its outputs itself: single lanes take the chain
